@@ -97,14 +97,16 @@ struct PinBuf {
 
 // ---- passes ----------------------------------------------------------------------------
 
-// PK_AFFINE16 and PK_CHAIN16 only classify buckets: an affine pass the packed 16-bit kernel
-// runs, and a chain of sorted-text passes it runs in order.
+// PK_AFFINE16, PK_CHAIN16 and PK_WAVE16 only classify buckets: an affine pass the packed 16-bit
+// row kernel runs, a chain of sorted-text passes it runs in order, and an affine pass the
+// anti-diagonal kernel runs (its class: an index into kWave).
 enum PassKind : uint8_t {
   PK_MYERS = 0,
   PK_AFFINE = 1,
   PK_LOCAL = 2,
   PK_AFFINE16 = 3,
-  PK_CHAIN16 = 4
+  PK_CHAIN16 = 4,
+  PK_WAVE16 = 5
 };
 
 // One DP pass as the reference's `affine_dp` / `distance` / `local_band_core` receive it.
@@ -151,6 +153,7 @@ struct Bucket {
   int c = 0;       // affine: cells per lane; Myers: blocks per lane
   bool wide = false, tb = false;
   int lanes = 32;  // Myers: lanes per pair
+  int per_warp = 1;  // anti-diagonal kernel: passes per warp
   uint32_t first = 0, count = 0;  // range in the order array
   int grid = 0, block = 128;
   uint64_t scratch_off = 0;       // wide rows: this bucket's slice of the scratch (int32s)
@@ -206,6 +209,9 @@ struct sf_plan {
   uint64_t launches = 0;
   // The transcript store SF_TEXT_STORE texts were resolved in (the context's at build time).
   const sf_store* store = nullptr;
+  // Whether anti-diagonal passes take the fastest class a pass (few passes) or the cheapest a
+  // cell: -1 by the plan's passes, else as set (the autotuner's trial plans).
+  int lean = -1;
   // Class overrides for this plan only (the autotuner's trial plans); else the context's.
   const sfe::TuneTable* tune_override = nullptr;
   // Host-side build arrays kept between builds (sf_plan.cu).
@@ -298,8 +304,16 @@ bool ok_sc(const sf_affine_t* sc);
 // Kernel classes (sf_plan.cu).
 bool allow16();
 int default_lanes16();
-void classify_affine(const Pass& p, uint32_t flags, int64_t wmax, bool use16, PassKind& kind,
-                     int& c, bool& wide, int& lanes, int lanes16 = 32);
+void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax, bool use16,
+                     bool lean, PassKind& kind, int& c, bool& wide, int& lanes,
+                     int lanes16 = 32);
+// The band cells the anti-diagonal kernel lays out for a pass.
+int64_t wave_width(const DJob& j);
+// Whether a plan of np passes takes the anti-diagonal kernel's fastest classes a pass.
+bool lean_plan(size_t np, int sms);
+// A class as its reports show it: cells a lane and lanes a pass.
+int shown_c(int kind, int c);
+int shown_lanes(int kind, int c, int lanes);
 int choose_myers_class(uint32_t m, int& b, int& lanes);
 DJob make_djob(const Pass& p, uint32_t& flags);
 // Whether large sf_batch_run batches may run in segments (SF_BATCH_SEGMENTS).

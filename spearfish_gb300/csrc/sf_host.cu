@@ -16,6 +16,7 @@
 
 #include "sf_engine.h"
 #include "sf_hostpool.h"
+#include "sf_wave16.h"
 
 using namespace sfe;
 
@@ -1149,7 +1150,7 @@ int sf_batch_run(sf_context* ctx, const uint8_t* pool, uint64_t pool_bytes, cons
 namespace {
 
 // A pass's class before any override, and the Myers blocks it needs.
-int default_class(const Pass& p, bool use16, ClassKey& key, int64_t& blocks) {
+int default_class(const Pass& p, bool use16, bool lean, ClassKey& key, int64_t& blocks) {
   if (p.kind == PK_MYERS) {
     int b = 1, lanes = 1;
     int rc = choose_myers_class(p.m, b, lanes);
@@ -1164,10 +1165,10 @@ int default_class(const Pass& p, bool use16, ClassKey& key, int64_t& blocks) {
   int c = 4, lanes = 32;
   bool wide = false;
   PassKind kind = PK_AFFINE;
-  classify_affine(p, flags, wmax, use16, kind, c, wide, lanes, default_lanes16());
+  classify_affine(p, j, flags, wmax, use16, lean, kind, c, wide, lanes, default_lanes16());
   const bool tb = p.want_cigar && p.kind != PK_LOCAL;
   key = ClassKey{kind, c, wide ? 1 : 0, tb ? 1 : 0, lanes};
-  blocks = wmax;  // affine: the group's widest row
+  blocks = kind == PK_WAVE16 ? wave_width(j) : wmax;  // affine: the group's widest row
   return SF_OK;
 }
 
@@ -1187,6 +1188,12 @@ std::vector<ClassChoice> tune_candidates(const ClassKey& key, int64_t blocks) {
       for (const auto& c : out) dup = dup || (c.c == b && c.lanes == lanes);
       if (!dup) out.push_back(ClassChoice{b, lanes});
     }
+  } else if (key.kind == PK_WAVE16) {
+    // The next two classes that hold the group's widest band, and the fastest one a pass.
+    for (int c = 0; c < sfk::kWaveN; ++c)
+      if (c != key.c && sfk::wave_cap(sfk::kWave[c]) >= blocks && (int)out.size() < 4 &&
+          (c > key.c || key.c >= sfk::kWaveN0))
+        out.push_back(ClassChoice{c, key.lanes});
   } else if (!key.wide) {
     // The 16-bit classes for 16, 32 and 64 lanes a pass.
     auto classes16 = [](int lanes, const int*& cs, int& nc) {
@@ -1235,13 +1242,14 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   if (reps == 0) reps = 1;
   const auto t0 = std::chrono::steady_clock::now();
   const bool use16 = allow16();
+  const bool lean = P->lean >= 0 ? P->lean != 0 : lean_plan(P->passes.size(), ctx->sms);
   // Group the passes by their default class.
   std::map<ClassKey, std::vector<size_t>> groups;
   std::map<ClassKey, int64_t> gblocks;
   for (size_t q = 0; q < P->passes.size(); ++q) {
     ClassKey k;
     int64_t blocks = 0;
-    int rc = default_class(P->passes[q], use16, k, blocks);
+    int rc = default_class(P->passes[q], use16, lean, k, blocks);
     if (rc) return rc;
     groups[k].push_back(q);
     gblocks[k] = std::max(gblocks[k], blocks);
@@ -1249,6 +1257,7 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   sf_plan S;  // trial plan, its buffers reused across trials
   S.ctx = ctx;
   S.pool_bytes = P->pool_bytes;
+  S.lean = lean;
   void* uploaded = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CK(cudaEventCreate(&e0));
@@ -1283,7 +1292,8 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
       ms /= (float)reps;
       char buf[96];
       std::snprintf(buf, sizeof buf, "%s{\"c\": %d, \"lanes\": %d, \"ms\": %.4f}", ci ? ", " : "",
-                    cands[ci].c, cands[ci].lanes, ms);
+                    shown_c(key.kind, cands[ci].c), shown_lanes(key.kind, cands[ci].c, cands[ci].lanes),
+                    ms);
       tried += buf;
       if (best_ms < 0 || ms < best_ms) {
         best_ms = ms;
@@ -1303,9 +1313,12 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
                   gi++ ? ", " : "",
                   key.kind == PK_MYERS ? "myers"
                                        : (key.kind == PK_LOCAL ? "local"
-                                                               : (key.kind == PK_AFFINE16 ? "affine16" : "affine")),
-                  key.c, key.wide ? "true" : "false", key.tb ? "true" : "false", key.lanes,
-                  g.second.size(), best.c, best.lanes);
+                                                               : (key.kind == PK_AFFINE16 ? "affine16"
+                                                                  : key.kind == PK_WAVE16 ? "wave16"
+                                                                                          : "affine")),
+                  shown_c(key.kind, key.c), key.wide ? "true" : "false", key.tb ? "true" : "false",
+                  shown_lanes(key.kind, key.c, key.lanes), g.second.size(), shown_c(key.kind, best.c),
+                  shown_lanes(key.kind, best.c, best.lanes));
     rep += buf + tried + "]}";
   }
   cudaEventDestroy(e0);

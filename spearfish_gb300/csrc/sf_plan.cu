@@ -15,6 +15,7 @@
 
 #include "sf_engine.h"
 #include "sf_hostpool.h"
+#include "sf_wave16.h"
 
 namespace sfe {
 
@@ -86,16 +87,53 @@ bool fits16(const Pass& p, uint32_t flags, int64_t wmax) {
   return spread + 2 * 64 * step + 2 * (go + s.mis + s.ext) + s.mat + 256 <= 16384;
 }
 
-// SF_AFFINE16=0 in the environment turns the 16-bit kernel off (every pass then runs on the
+// The band cells the anti-diagonal kernel lays out for a pass (its bl is odd).
+int64_t wave_width(const DJob& j) { return (j.below | 1) + j.above + 1; }
+
+// Whether a pass runs on the anti-diagonal kernel (sf_wave16_impl.cuh): a Global pass of a
+// finite band without clip or cut.  Its band edges rest on mis = 2 ext (a mismatch costs what
+// the two gap bases around it would extend for) and open >= 1.  Its fields hold four times the
+// value: the largest rises by (mat + 2 ext) a row step between rebases, and a band cell lies at
+// most (mat + 2 ext) * width / 2 + open below it (a gap from the best path, extension free in
+// the kernel's potential).  A band much wider than the text (or the pattern) is left to the
+// row kernels, whose rows stop at the text's end.
+bool fits_wave(const Pass& p, const DJob& j, uint32_t flags) {
+  if (p.kind != PK_AFFINE || (flags & (F_FULL | F_ROWMAX)) || p.mode != SF_GLOBAL) return false;
+  const sf_affine_t& s = p.sc;
+  if (s.mat < 0 || s.mat > 1000 || s.ext < 0 || s.ext > 1000 || s.mis != 2 * s.ext) return false;
+  if (s.open < 1 || s.open > 900) return false;
+  const int64_t w = wave_width(j);
+  if (p.m < 1 || p.n < 1 || w > 2 * ((int64_t)std::min(p.m, p.n) + 1)) return false;
+  if (w > sfk::wave_cap(sfk::kWave[sfk::kWaveN0 - 1])) return false;
+  const int64_t g = (int64_t)s.mat + 2 * s.ext;
+  if (4 * g * (sfk::kWaveRebaseRows + 1) >
+      std::min<int64_t>(0xffff - (int64_t)sfk::kWaveTop, sfk::kWaveNeg))
+    return false;
+  return 4 * (g * (w / 2 + 2) + 2 * (int64_t)s.open + 16) <=
+         (int64_t)sfk::kWaveTop - (int64_t)sfk::kWaveNeg;
+}
+
+// Few passes: each takes the fastest class.  Measured on 2 kb passes with band 128 and CIGARs:
+// 600 passes 0.47 ms on 4 words x 32 lanes, 0.84 on 10 x 8; 1,200 passes 0.64 against 1.37 on
+// 12 x 6; 8,200 passes 3.49 against 2.54 (four a warp): the lines cross near 20 an SM.
+bool lean_plan(size_t np, int sms) { return np <= (size_t)sms * 20; }
+
+int shown_c(int kind, int c) { return kind == PK_WAVE16 ? 4 * sfk::kWave[c].q : c; }
+int shown_lanes(int kind, int c, int lanes) {
+  return kind == PK_WAVE16 ? sfk::kWave[c].lanes : lanes;
+}
+
+// SF_AFFINE16=0 in the environment turns the 16-bit kernels off (every pass then runs on the
 // 32-bit kernel); read once per plan.
 bool allow16() {
   const char* env = std::getenv("SF_AFFINE16");
   return !(env && env[0] == '0');
 }
 
-// Lanes per 16-bit pass by default: 32 (with 64 for rows wider than 32 x 40 cells), or with
+// Lanes per 16-bit row pass by default: 32 (with 64 for rows wider than 32 x 40 cells), or with
 // SF_AFFINE16_LANES in the environment 16 (two passes per warp) or 64 (two warps per pass,
-// every pass a 64-lane class holds); the autotuner chooses per length bucket either way.
+// every pass a 64-lane class holds), which also keeps every 16-bit pass on the row kernels;
+// the autotuner chooses per length bucket either way.
 int default_lanes16() {
   const char* env = std::getenv("SF_AFFINE16_LANES");
   if (env && env[0] == '1' && env[1] == '6') return 16;
@@ -133,12 +171,19 @@ bool allow_w64() {
   return !(env && env[0] == '0');
 }
 
-// Kernel class of an affine or local pass: the packed 16-bit kernel when the pass fits it,
-// else the 32-bit register kernel, else (rows wider than 32 * 48 cells) the wide-row kernel.
-void classify_affine(const Pass& p, uint32_t flags, int64_t wmax, bool use16, PassKind& kind,
-                     int& c, bool& wide, int& lanes, int lanes16) {
+// Kernel class of an affine or local pass: the anti-diagonal 16-bit kernel when the pass fits
+// it, else the packed 16-bit row kernel, else the 32-bit register kernel, else (rows wider than 32 * 48 cells) the wide-row kernel.
+void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax, bool use16,
+                     bool lean, PassKind& kind, int& c, bool& wide, int& lanes, int lanes16) {
   wide = false;
   lanes = 32;
+  if (use16 && lanes16 == 32 && fits_wave(p, j, flags)) {
+    const int64_t w = wave_width(j);
+    kind = PK_WAVE16;
+    for (c = lean ? sfk::kWaveN0 : 0; sfk::wave_cap(sfk::kWave[c]) < w; ++c) {
+    }
+    return;
+  }
   if (use16 && fits16(p, flags, wmax)) {
     if (lanes16 == 16)
       for (int q = 0; q < sfk::kAffine16HNC; ++q)
@@ -530,6 +575,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   const sf_context* ctx = P->ctx;
   const size_t np = P->passes.size();
   const int lanes16 = default_lanes16();
+  const bool lean = P->lean >= 0 ? P->lean != 0 : lean_plan(np, ctx->sms);
   const TuneTable* tune = P->tune_override ? P->tune_override : &ctx->tune;
   const auto& word_of = S.word_of;
   auto& dj = S.dj;
@@ -644,14 +690,16 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       bool wide = false;
       PassKind kind = PK_AFFINE;
       int ln = 32;
-      classify_affine(p, flags, wmax, use16, kind, c, wide, ln, lanes16);
+      classify_affine(p, j, flags, wmax, use16, lean, kind, c, wide, ln, lanes16);
       const bool tb = p.want_cigar && p.kind != PK_LOCAL;
       if (!wide) tuned(kind, c, false, tb, ln);
       TJob t{};
       if (tb) {
         flags |= F_TB;
         const int64_t chunks = wide ? wide_chunks(c, wmax) : 1;
-        tb_need[sl] = (uint64_t)p.m * (tb_row_words(c, chunks) * (uint64_t)ln / 32);
+        tb_need[sl] = kind == PK_WAVE16
+                          ? sfk::wave_tb_words(sfk::kWave[c], ((uint64_t)p.m + p.n + 1) / 2)
+                          : (uint64_t)p.m * (tb_row_words(c, chunks) * (uint64_t)ln / 32);
         const uint64_t cap = (uint64_t)p.m + p.n + 2;
         ops_need[sl] = cap;
         t.ops_cap = (uint32_t)std::min<uint64_t>(cap, 0xffffffffull);
@@ -674,7 +722,10 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       pr.ext = p.sc.ext;
       const uint64_t work = (uint64_t)std::max<uint32_t>(p.m, 1) * (uint64_t)std::max<int64_t>(wmax, 1);
       pass_work[q] = work;
-      const uint64_t row_cost = (uint64_t)c * (wide ? (uint64_t)wide_chunks(c, wmax) : 1u) + 8u;
+      // Anti-diagonal row steps: about (60 + 32 Q) / 45 of this unit (a row's 45 cycles).
+      const uint64_t row_cost = kind == PK_WAVE16
+                                    ? 2u + (uint64_t)(2 * sfk::kWave[c].q / 3)
+                                    : (uint64_t)c * (wide ? (uint64_t)wide_chunks(c, wmax) : 1u) + 8u;
       pass_lat[q] = (uint64_t)std::max<uint32_t>(p.m, 1) * row_cost;
       has_item[q] = !P->chained[q];
       if (has_item[q]) per[q] = {Key2{kind, c, wide, tb, ln}, Item{sl, work, pass_lat[q]}};
@@ -1002,6 +1053,15 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
       const uint64_t warps = (b.count + per_warp - 1) / per_warp;
       const uint64_t wpb = (uint64_t)b.block / 32;
       b.grid = (int)std::min<uint64_t>((warps + wpb - 1) / wpb, (uint64_t)ctx->sms * (2048 / b.block));
+    } else if (b.kind == PK_WAVE16) {
+      // As many passes a warp as its lanes hold; in the fast classes fewer, while that leaves
+      // schedulers empty.
+      b.block = 128;
+      const int64_t most = 32 / sfk::kWave[b.c].lanes;
+      b.per_warp = (int)(b.c < sfk::kWaveN0 ? most
+                                            : std::max<int64_t>(1, std::min<int64_t>(most, b.count / (4 * (int64_t)ctx->sms))));
+      const uint64_t blocks = (b.count + 4 * b.per_warp - 1) / (4 * b.per_warp);
+      b.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)ctx->sms * 16));
     } else {
       // Two-warp passes: one pass per 64-thread block; otherwise a 4-warp block holds 4
       // passes (chains), or 8 with 16 lanes a pass.
@@ -1154,9 +1214,11 @@ void describe_plan(sf_plan* P, const BuildScratch& S) {
                   : b.kind == PK_LOCAL   ? "local"
                   : b.kind == PK_AFFINE16 ? "affine16"
                   : b.kind == PK_CHAIN16 ? "chain16"
+                  : b.kind == PK_WAVE16  ? "wave16"
                                          : "affine",
-                  b.c,
-                  b.wide ? "true" : "false", b.tb ? "true" : "false", b.lanes, b.count, b.grid,
+                  shown_c(b.kind, b.c),
+                  b.wide ? "true" : "false", b.tb ? "true" : "false",
+                  shown_lanes(b.kind, b.c, b.lanes), b.count, b.grid,
                   b.block, (unsigned long long)b.work);
     d += buf;
   }
@@ -1302,7 +1364,9 @@ int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* ev
       al.links = P->d_links.as<DLink>();
       al.want = P->d_want.as<uint32_t>();
       al.snap = P->d_snap.as<uint32_t>();
-      if (b.kind == PK_CHAIN16)
+      if (b.kind == PK_WAVE16)
+        CK(sfk::launch_wave16(b.c, b.tb, al, b.per_warp, b.grid, bs));
+      else if (b.kind == PK_CHAIN16)
         CK(sfk::launch_affine16_chain(b.c, al, b.grid, b.block, bs));
       else if (b.kind == PK_AFFINE16 && b.lanes == 64)
         CK(sfk::launch_affine16w(b.c, b.tb, al, b.grid, b.block, bs));
@@ -1629,9 +1693,18 @@ uint64_t plan_bytes_estimate(const std::vector<Pass>& passes, uint64_t pool_byte
     bool wide = false;
     PassKind kind = PK_AFFINE;
     int ln = 32;
-    classify_affine(p, flags, wmax, use16, kind, c, wide, ln, lanes16);
+    uint64_t tb_wave = 0;
+    // The classes either way of `lean`: the larger traceback.
+    for (int lean = 0; lean < 2 && p.want_cigar && p.kind != PK_LOCAL; ++lean) {
+      classify_affine(p, j, flags, wmax, use16, lean != 0, kind, c, wide, ln, lanes16);
+      if (kind != PK_WAVE16) break;
+      tb_wave = std::max(tb_wave, sfk::wave_tb_words(sfk::kWave[c], ((uint64_t)p.m + p.n + 1) / 2) * 4);
+    }
+    classify_affine(p, j, flags, wmax, use16, false, kind, c, wide, ln, lanes16);
     if (p.want_cigar && p.kind != PK_LOCAL) {
-      b += (uint64_t)p.m * tb_row_words(c, wide ? wide_chunks(c, wmax) : 1) * 4 * ln / 32;
+      b += kind == PK_WAVE16
+               ? tb_wave
+               : (uint64_t)p.m * tb_row_words(c, wide ? wide_chunks(c, wmax) : 1) * 4 * ln / 32;
       b += 2 * ((uint64_t)p.m + p.n + 2) * 4;
     }
     if (wide) scratch = std::max<uint64_t>(scratch, (uint64_t)wide_chunks(c, wmax) * 32 * c);

@@ -1,0 +1,484 @@
+// Global banded affine (Gotoh) passes swept by anti-diagonals, two cells per 32-bit register and
+// several passes per warp (align.rs:2446-2666 `run_core` in Mode::Global without clip or cut).
+// Results and traceback decisions equal the row kernels' (sf_affine16_impl.cuh).
+//
+// Cells.  Band offset K = j - i + bl of cell (i, j) sits at a fixed place: lane K / 4Q of the
+// pass's L lanes, and along anti-diagonal i + j = t the cells of one parity of K are computed
+// together, each from its neighbours K - 1 (left), K + 1 (above) and its own last value (the
+// diagonal).  No cell of a step depends on another, so a step has no scan and no serial chain:
+// two neighbour shuffles, then 2Q independent cells a lane.  A row step a is one even and one
+// odd step; cell K = 2k (+1) is then row i = a - k, column j = a + k - bl (+1).
+//
+// Fields.  A 16-bit field holds 4 * (value + ext * (i + j)) + offset: the potential makes gap
+// extension free, so E = max(Hleft - open, Eleft) and F = max(Hup - open, Fup) are one
+// two-operand maximum each (the subtraction is an IMAD, off the pipe the maxima use), and with
+// mis = 2 * ext a mismatch adds 0.  The factor 4 leaves two low bits for the traceback: the
+// diagonal carries 2, F 1, E 0, so that one three-way maximum also says which won, ties in the
+// walk's order (diagonal, F, E); an opened gap carries 2 against an extended one's 0 (E) or 1
+// (F), so that a tie opens.  Per cell and row four bits are kept: (winner << 2) | (E opened
+// << 1) | F extended.
+//
+// Band edges.  Left of the band lane 0 takes NEG from outside.  Right of it (and at K = 0 when
+// `below` is even, which keeps bl odd) pad cells are computed with every match masked.  A path
+// through them leaves the band and returns by gaps and mismatches only, so it costs at least
+// 2 * open + 2 * ext * d for the d diagonals it gains, where the band's edge offers d mismatches
+// at 2 * ext each: with open >= 1 it never reaches a band cell's maximum, and where an extended
+// gap ties an opened one the opened one wins, as in the row kernels.  Cells before row 1 or
+// column 1 are masked too, so row 0 and column 0 come out of the recurrence itself, from the
+// one seed at (0, 0).  Cells past the text or pattern hold values nothing in the matrix reads.
+//
+// Bound: the ALU pipe (one instruction every other cycle a scheduler): 8.5 of a word's 14.5
+// instructions with traceback, 4.5 of 6.5 without.  With 12 words a lane and 6 lanes a pass a
+// row step issues 443 instructions for five 2 kb passes of band 128 (258 on the ALU pipe), the
+// row kernel 254 for one; score only 221 against 150.  20,000 such pairs on GB300: 10.25 ->
+// 5.2 ms with CIGARs, 5.7 -> 2.4 ms without.
+#pragma once
+#include "sf_affine_impl.cuh"
+#include "sf_wave16.h"
+
+namespace {
+
+constexpr uint32_t kWTop = sfk::kWaveTop, kWNeg = sfk::kWaveNeg;
+constexpr uint32_t kW2 = 0x00010001u;
+constexpr int kWRebase = sfk::kWaveRebaseRows;
+
+// The 16 two-bit fields of x in reverse order.
+__device__ __forceinline__ uint32_t rev2(uint32_t x) {
+  const uint32_t y = __brev(x);
+  return ((y >> 1) & 0x55555555u) | ((y & 0x55555555u) << 1);
+}
+
+// Bit 2e set for e < c (register r of the mask: e = 16r ..).
+__device__ __forceinline__ uint32_t low_fields(int32_t c, int r) {
+  const int32_t k = min(max(c - 16 * r, 0), 16);
+  return (uint32_t)((uint64_t(1) << (2 * k)) - 1u) & 0x55555555u;
+}
+
+// (x & m) | o in one instruction, with the constants in registers.
+__device__ __forceinline__ uint32_t and_or(uint32_t x, uint32_t m, uint32_t o) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(x), "r"(m), "r"(o));
+  return d;
+}
+// x's bits where m is set, y's elsewhere.
+__device__ __forceinline__ uint32_t pick(uint32_t x, uint32_t y, uint32_t m) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(d) : "r"(x), "r"(y), "r"(m));
+  return d;
+}
+
+// Walks the pass's path from (m, n), the whole warp on one pass.  Each lane caches eight band
+// offsets (two quads of four) of one group of four row steps, so the warp holds 128 row steps
+// around the path; a run of diagonal steps, which keeps its band offset, is found by one ballot
+// over the cached nibbles.
+template <int Q>
+__device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, int L, int lane) {
+  const DJob J = a.jobs[jid];
+  const TJob T = a.tjobs[jid];
+  const int32_t m = (int32_t)J.m, n = (int32_t)J.n;
+  const int32_t bl = clamp30(J.below) | 1, W = bl + clamp30(J.above) + 1;
+  const int32_t a1 = (bl >> 1) + 1;  // the row step that row-step index 0 stands for
+  const int32_t gstride = (Q / 2) * L;  // uint4s per group of four row steps
+  const uint4* tb = reinterpret_cast<const uint4*>(a.tb + J.tb_word);
+  uint32_t* out = a.ops + T.ops_off;
+  const uint32_t cap = T.ops_cap;
+  uint32_t n_ops = 0, cur_op = 15, cur_len = 0;
+  int status = 0;
+  auto push = [&](uint32_t op, uint32_t len) {
+    if (len == 0) return;
+    if (op == cur_op) {
+      cur_len += len;
+      return;
+    }
+    if (cur_len) {
+      if (n_ops == cap) {
+        status = -1;
+        return;
+      }
+      if (lane == 0) out[n_ops] = (cur_len << 4) | cur_op;
+      ++n_ops;
+    }
+    cur_op = op;
+    cur_len = len;
+  };
+  int32_t i = m, j = n, K = n - m + bl;
+  int state = 0;                      // 0 H, 1 E, 2 F
+  int32_t G0 = -1, q0 = -1;           // lane d caches group G0 - d of offsets 4 q0 .. 4 q0 + 7
+  uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0;  // offsets 4 q0 + (0, 1), (2, 3), (4, 5), (6, 7)
+  // One quad of four offsets: the low or the high fields of its four words.
+  auto quad = [&](int32_t g, int32_t kq, uint32_t& x, uint32_t& y) {
+    x = y = 0;
+    if (g < 0 || kq < 0 || kq >= Q * L) return;
+    const int32_t ln = kq / Q, rem = kq - ln * Q, hi = rem >= Q / 2;
+    const uint4 w = tb[(int64_t)g * gstride + (rem - (hi ? Q / 2 : 0)) * L + ln];
+    const uint32_t s = hi ? 0x7632u : 0x5410u;
+    x = __byte_perm(w.x, w.y, s);
+    y = __byte_perm(w.z, w.w, s);
+  };
+  const int64_t guard = 3 * ((int64_t)m + n) + 64;
+  for (int64_t it = 0;; ++it) {
+    if (it > guard || status) {
+      if (!status) status = 1;
+      break;
+    }
+    if (state == 0 && i == 0) {
+      push(2, (uint32_t)j);
+      break;
+    }
+    if (state == 0 && j == 0) {
+      push(1, (uint32_t)i);
+      break;
+    }
+    if (i <= 0 || j <= 0 || K < 0 || K >= W) {
+      status = 1;
+      break;
+    }
+    const int32_t rho = i + (K >> 1) - a1, g = rho >> 2;
+    if (K < 4 * q0 || K >= 4 * q0 + 8 || q0 < 0 || g > G0 || g <= G0 - 32) {
+      q0 = max(K - 2, 0) >> 2;
+      G0 = g;
+      quad(g - lane, q0, c0, c1);
+      quad(g - lane, q0 + 1, c2, c3);
+    }
+    const int32_t x = K - 4 * q0;  // 0 .. 7
+    const uint32_t w01 = x & 2 ? c1 : c0, w23 = x & 2 ? c3 : c2;
+    const uint32_t w = x & 4 ? w23 : w01;
+    const uint32_t v = (x & 1) ? w >> 16 : w & 0xffffu;  // this lane's four nibbles at K
+    const int32_t d = G0 - g, r0 = rho & 3;
+    const uint32_t nib = (__shfl_sync(FULL, v, d) >> (4 * (3 - r0))) & 15u;
+    if (state == 0) {
+      const uint32_t win = nib >> 2;
+      if (win == 2u) {
+        // Row step 3 of a group is nibble 0.  Rows after the path's own count as diagonal.
+        uint32_t dg = (v >> 3) & ~(v >> 2) & 0x1111u;
+        if (lane == d) dg |= 0x1111u & ((1u << (4 * (3 - r0))) - 1u);
+        const uint32_t part = ((uint32_t)__ffs((int)(~dg & 0x11111u)) - 1u) >> 2;  // 0 .. 4
+        const uint32_t nf = __ballot_sync(FULL, dg != 0x1111u) >> d;
+        const int32_t z = nf ? __ffs((int)nf) - 1 : 32 - d;  // whole groups from lane d on
+        const int32_t tail = (int32_t)__shfl_sync(FULL, part, (d + z) & 31);
+        int32_t run = 4 * z - (3 - r0) + (nf ? tail : 0);
+        run = min(run, min(i, j));
+        push(0, (uint32_t)run);
+        i -= run;
+        j -= run;
+      } else {
+        state = win == 1u ? 2 : 1;
+      }
+    }
+    if (state == 1) {
+      push(2, 1);
+      state = (nib & 2u) ? 0 : 1;
+      --j;
+      --K;
+    } else if (state == 2) {
+      push(1, 1);
+      state = (nib & 1u) ? 2 : 0;
+      --i;
+      ++K;
+    }
+  }
+  if (!status && cur_len) {
+    if (n_ops == cap)
+      status = -1;
+    else if (lane == 0)
+      out[n_ops] = (cur_len << 4) | cur_op;
+    ++n_ops;
+  }
+  if (lane == 0) {
+    TRes tr;
+    tr.score = a.out[jid].score;
+    tr.status = status;
+    tr.end_i = (uint32_t)m;
+    tr.end_j = (uint32_t)n;
+    tr.text_start = 0;
+    tr.n_ops = status == 0 ? n_ops : 0;
+    a.tres[jid] = tr;
+  }
+}
+
+// One warp's passes, one per segment of L lanes: `jid` is the lane's own pass (any valid one
+// where `has` is false: computed, not stored).
+template <int Q, bool TB>
+__device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t jid, bool has, int L,
+                                            int np, int lane, int seg) {
+  constexpr int NT = (2 * Q + 15) / 16;  // 16-base registers of a lane's text (pattern) window
+  constexpr int NC = (Q + 7) / 8;        // registers of a step's match bits
+  static_assert(Q % 2 == 0 && Q >= 4 && Q <= 16, "words per lane and parity");
+  const int l = lane - seg * L;
+  const DJob J = a.jobs[jid];
+  const DParams S = a.params[jid];
+  const int32_t m = (int32_t)J.m, n = (int32_t)J.n;
+  const int32_t below = clamp30(J.below), above = clamp30(J.above);
+  const int32_t bl = below | 1, W = bl + above + 1;
+  const int32_t k0 = 2 * Q * l;  // the lane's first pair of offsets
+  const int32_t a1 = (bl >> 1) + 1;
+  const int32_t N = (m + n + 1) >> 1;  // row steps until cell (m, n) is done
+
+  const uint32_t one = (uint32_t)opaque_one(), mone = 0u - one;
+  const uint32_t sixteen = one << 4, four = one << 2, mfour = 0u - four;
+  // The tag masks, opaque so that each use is one three-input instruction.
+  const uint32_t mlow = 0xfffcfffcu * one, kone = kW2 * one, ktwo = 2u * kone, msel = ~kone;
+  const uint32_t g2 = 4u * (uint32_t)S.open * kW2;
+  const uint32_t v1 = (uint32_t)(S.mat + S.mis), v4 = 4u * v1;
+  constexpr uint32_t kH = TB ? 2u : 0u, kF = TB ? 1u : 0u;  // a clean field's low bits
+  constexpr uint32_t kNegH = (kWNeg + kH) * kW2, kNegE = kWNeg * kW2, kNegF = (kWNeg + kF) * kW2;
+
+  uint32_t HA[Q], HB[Q], E[Q], F[Q], acc[TB ? 2 * Q : 1];
+#pragma unroll
+  for (int k = 0; k < Q; ++k) {
+    // The seed at (0, 0): offset bl, odd.
+    const int32_t e = (bl >> 1) - k0;
+    const uint32_t top = kWTop + kH, neg = kWNeg + kH;
+    HA[k] = kNegH;
+    HB[k] = (e == k ? top : neg) | ((e == Q + k ? top : neg) << 16);
+    E[k] = kNegE;
+    F[k] = kNegF;
+    if constexpr (TB) acc[2 * k] = acc[2 * k + 1] = 0;
+  }
+  int32_t off = -(int32_t)kWTop;
+
+  // Windows: T[r] holds the text bases of columns from a + k0 - bl + 16 r on (T[NT]: the bases
+  // that shift in next), P[r] the pattern bases of rows from a - k0 - 16 r downwards, Pn the
+  // ones that come next, first at the top.  Both move by one base a row step.
+  const int32_t tlim = (n >> 4) + 64, plim = (m >> 4) + 64;  // the pool's slack covers 100 words
+  auto word = [&](uint64_t w, int32_t x, int32_t lim) {
+    return __ldg(a.pool + w + (uint32_t)min(max(x, 0), lim));
+  };
+  auto chunk = [&](uint64_t w, int32_t x, int32_t lim) {
+    return __funnelshift_r(word(w, x >> 4, lim), word(w, (x >> 4) + 1, lim), 2 * (x & 15));
+  };
+  uint32_t T[NT + 1], P[NT], Pn;
+  const int32_t tx = a1 + k0 - bl, px = a1 - k0;  // at row-step index 0
+#pragma unroll
+  for (int r = 0; r <= NT; ++r) T[r] = chunk(J.t_word, tx + 16 * r, tlim);
+#pragma unroll
+  for (int r = 0; r < NT; ++r) P[r] = rev2(chunk(J.p_word, px - 16 * r - 15, plim));
+  Pn = rev2(chunk(J.p_word, px + 1, plim));
+  uint32_t t0 = 0, t1 = 0, p0 = 0, p1 = 0;  // the next chunk's words, loaded 16 row steps ahead
+  const int32_t tsh = 2 * (tx & 15), psh = 2 * ((px + 1) & 15);
+
+  uint32_t Me[NT], Mo[NT];  // match masks of the even and odd step
+  // Cells of row step index r that lie in the matrix and the band.
+  auto masks = [&](int32_t r) {
+    const int32_t x = a1 + r;
+    const int32_t rows = x - k0;  // e < rows: row 1 or later
+    const int32_t lo_e = max(bl + 1 - x - k0, l == 0 ? bl - below : 0);
+    const int32_t lo_o = bl - x - k0;
+    const int32_t hi_e = min(rows, ((W + 1) >> 1) - k0), hi_o = min(rows, (W >> 1) - k0);
+#pragma unroll
+    for (int r2 = 0; r2 < NT; ++r2) {
+      Me[r2] = low_fields(min(hi_e, 2 * Q), r2) & ~low_fields(lo_e, r2);
+      Mo[r2] = low_fields(min(hi_o, 2 * Q), r2) & ~low_fields(lo_o, r2);
+    }
+  };
+  // Row steps after which every cell of the band is in the matrix (masks constant).
+  int32_t rF = max(min(2 * Q * L, (W >> 1) + 1), bl + 1) - a1;
+  int32_t Rtot = has ? N : 0;
+  rF = __reduce_max_sync(FULL, rF);
+  Rtot = (__reduce_max_sync(FULL, Rtot) + 3) & ~3;
+  int32_t next_end = __reduce_min_sync(FULL, has ? N : INT32_MAX);
+
+  // A step's match bits: cell k's low field at bit 2 (k % 8) of register k / 8, its high field
+  // (cell k + Q) 16 bits up.
+  auto matches = [&](const uint32_t (&M)[NT], uint32_t (&cb)[NC]) {
+    uint32_t eq[NT];
+#pragma unroll
+    for (int r = 0; r < NT; ++r) {
+      const uint32_t x = T[r] ^ P[r];
+      eq[r] = ~(x | (x >> 1)) & M[r];
+    }
+    if constexpr (Q == 8) {
+      cb[0] = eq[0];
+    } else if constexpr (Q < 8) {
+      cb[0] = __byte_perm(eq[0], eq[0] << (16 - 2 * Q), 0x7610);
+    } else {
+      const uint32_t hi = Q == 16 ? eq[1] : __funnelshift_r(eq[0], eq[1], 2 * Q);
+      cb[0] = __byte_perm(eq[0], hi, 0x5410);
+      cb[NC - 1] = __byte_perm(eq[0], hi, 0x7632);
+    }
+  };
+  // Word k's cells: e and f are the gap values entering them; h their diagonal, then their H.
+  auto cell = [&](int k, const uint32_t (&cb)[NC], uint32_t& h, uint32_t et, uint32_t ft,
+                  uint32_t& eo, uint32_t& fo, uint32_t& ac) {
+    const uint32_t c = cb[k >> 3] >> (4 * ((k & 7) >> 1));
+    const uint32_t dg = (k & 1) ? (c & (4u * kW2)) * v1 + h : (c & kW2) * v4 + h;
+    if constexpr (TB) {
+      const uint32_t ec = et & 0xfffcfffcu, fc = and_or(ft, mlow, kone);
+      const uint32_t ht = __vimax3_u16x2(dg, fc, ec);
+      const uint32_t hs = and_or(ht, mlow, ktwo);
+      const uint32_t y = pick(et, ft, msel);  // E opened << 1 | F extended
+      ac = ac * sixteen + y;
+      ac = ec * mone + ac;
+      ac = ht * four + ac;
+      ac = hs * mfour + ac;  // (winner - 2) << 2: the flush adds the 8 a nibble
+      h = hs;
+      eo = ec;
+      fo = fc;
+    } else {
+      (void)ac;
+      h = __vimax3_u16x2(dg, ft, et);
+      eo = et;
+      fo = ft;
+    }
+  };
+  uint4* tbp = nullptr;
+  if constexpr (TB) tbp = reinterpret_cast<uint4*>(a.tb + J.tb_word) + l;
+
+  for (int32_t r = 0; r < Rtot;) {
+    if ((r & 15) == 0) {
+      if (r > 0) {
+        T[NT] = __funnelshift_r(t0, t1, tsh);
+        Pn = rev2(__funnelshift_r(p0, p1, psh));
+      }
+      // The chunk after this one.
+      const int32_t xt = (tx + r + 16 * (NT + 1)) >> 4, xp = (px + 1 + r + 16) >> 4;
+      t0 = word(J.t_word, xt, tlim);
+      t1 = word(J.t_word, xt + 1, tlim);
+      p0 = word(J.p_word, xp, plim);
+      p1 = word(J.p_word, xp + 1, plim);
+    }
+    if (r <= rF) masks(r);
+    uint32_t G[Q], cb[NC];
+    // Even step: offsets 2k from their odd neighbours.
+    matches(Me, cb);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) G[k] = HB[k] * one - g2;
+    {
+      uint32_t sG = __shfl_up_sync(FULL, G[Q - 1], 1), sE = __shfl_up_sync(FULL, E[Q - 1], 1);
+      if (l == 0) sG = sE = kNegE;
+      const uint32_t gl = __byte_perm(sG, G[Q - 1], 0x5432), el = __byte_perm(sE, E[Q - 1], 0x5432);
+#pragma unroll
+      for (int k = Q - 1; k >= 0; --k) {
+        const uint32_t et = __vmaxu2(k ? G[k ? k - 1 : 0] : gl, k ? E[k ? k - 1 : 0] : el);
+        const uint32_t ft = __vmaxu2(G[k], F[k]);
+        cell(k, cb, HA[k], et, ft, E[k], F[k], acc[TB ? 2 * k : 0]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NT; ++q) T[q] = __funnelshift_r(T[q], T[q + 1], 2);
+    T[NT] >>= 2;
+    // Odd step: offsets 2k + 1 from their even neighbours.
+    matches(Mo, cb);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) G[k] = HA[k] * one - g2;
+    {
+      uint32_t sG = __shfl_down_sync(FULL, G[0], 1), sF = __shfl_down_sync(FULL, F[0], 1);
+      if (l == L - 1) {
+        sG = kNegE;
+        sF = kNegF;
+      }
+      const uint32_t gu = __byte_perm(G[0], sG, 0x5432), fu = __byte_perm(F[0], sF, 0x5432);
+#pragma unroll
+      for (int k = 0; k < Q; ++k) {
+        const uint32_t et = __vmaxu2(G[k], E[k]);
+        const uint32_t ft = __vmaxu2(k + 1 < Q ? G[k + 1 < Q ? k + 1 : 0] : gu,
+                                     k + 1 < Q ? F[k + 1 < Q ? k + 1 : 0] : fu);
+        cell(k, cb, HB[k], et, ft, E[k], F[k], acc[TB ? 2 * k + 1 : 0]);
+      }
+    }
+#pragma unroll
+    for (int q = NT - 1; q > 0; --q) P[q] = __funnelshift_l(P[q - 1], P[q], 2);
+    P[0] = __funnelshift_l(Pn, P[0], 2);
+    Pn = Pn * four;
+    ++r;
+    if constexpr (TB) {
+      if ((r & 3) == 0) {
+        // Four row steps: one 16-byte store per quad of words, lane-fastest.
+        const bool st = has && r < N + 4;
+#pragma unroll
+        for (int q = 0; q < Q / 2; ++q) {
+          const uint4 w = make_uint4(acc[4 * q] + 0x88888888u, acc[4 * q + 1] + 0x88888888u,
+                                     acc[4 * q + 2] + 0x88888888u, acc[4 * q + 3] + 0x88888888u);
+          if (st) tbp[q * L] = w;
+        }
+        if (st) tbp += (Q / 2) * L;
+#pragma unroll
+        for (int k = 0; k < 2 * Q; ++k) acc[k] = 0;
+      }
+    }
+    if (r == next_end) {
+      // Passes whose cell (m, n) this row step computed.
+      const int32_t Kend = n - m + bl, ke = (Kend >> 1) - k0;
+      if (has && r == N && ke >= 0 && ke < 2 * Q) {
+        uint32_t u = 0;
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+          const uint32_t h = (Kend & 1) ? HB[k] : HA[k];
+          if (ke == k) u = h & 0xffffu;
+          if (ke == Q + k) u = h >> 16;
+        }
+        DRes o{};
+        o.score = (((int32_t)(u & ~3u) + off) >> 2) - S.ext * (m + n);
+        o.cut_score = NEG;
+        o.score_col = (uint32_t)n;
+        o.text_read = (uint32_t)min(m + above, n);
+        o.last_row = o.rows = (uint32_t)m;
+        o.cells = band_cells(m, below, above, n);
+        a.out[jid] = o;
+      }
+      next_end = __reduce_min_sync(FULL, has && N > r ? N : INT32_MAX);
+    }
+    if ((r & (kWRebase - 1)) == 0) {
+      // Each pass's largest field back to the top.
+      uint32_t v = 0;
+#pragma unroll
+      for (int k = 0; k < Q; ++k) v = __vimax3_u16x2(v, HA[k], HB[k]);
+      v = max(v & 0xffffu, v >> 16);
+      for (int s = 1; s < L; s <<= 1) {
+        const uint32_t u = __shfl_down_sync(FULL, v, s);
+        if (l + s < L) v = max(v, u);
+      }
+      v = __shfl_sync(FULL, v, min(seg * L, 31));
+      const int32_t delta = (int32_t)(v - kH) - (int32_t)kWTop;
+      const uint32_t dd = ((uint32_t)(-delta) & 0xffffu) * kW2;
+#pragma unroll
+      for (int k = 0; k < Q; ++k) {
+        HA[k] = __viaddmax_u16x2(HA[k], dd, kNegH);
+        HB[k] = __viaddmax_u16x2(HB[k], dd, kNegH);
+        E[k] = __viaddmax_u16x2(E[k], dd, kNegE);
+        F[k] = __viaddmax_u16x2(F[k], dd, kNegF);
+      }
+      off += delta;
+    }
+  }
+  if constexpr (TB) {
+    __syncwarp();
+    for (int s = 0; s < np; ++s) {
+      const uint32_t js = __shfl_sync(FULL, jid, s * L);
+      if (__shfl_sync(FULL, (int)has, s * L)) walk_wave<Q>(a, js, L, lane);
+      __syncwarp();
+    }
+  }
+  __syncwarp();
+}
+
+template <int Q, bool TB>
+__global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB)) wave16_kernel(sfk::AffLaunch a, int L,
+                                                                           int np) {
+  const int lane = threadIdx.x & 31, seg = lane / L;
+  for (;;) {
+    uint32_t q = 0;
+    if (lane == 0) q = atomicAdd(a.counter, (uint32_t)np);
+    q = __shfl_sync(FULL, q, 0);
+    if (q >= a.njobs) break;
+    const uint32_t mine = q + (uint32_t)seg;
+    const bool has = seg < np && mine < a.njobs;
+    wave_passes<Q, TB>(a, a.order[has ? mine : q], has, L, np, lane, seg);
+  }
+}
+
+}  // namespace
+
+namespace sfk {
+
+template <int Q>
+cudaError_t launch_wave16_q(bool tb, const AffLaunch& a, int lanes, int per_warp, int grid,
+                            cudaStream_t s) {
+  if (tb)
+    wave16_kernel<Q, true><<<grid, 128, 0, s>>>(a, lanes, per_warp);
+  else
+    wave16_kernel<Q, false><<<grid, 128, 0, s>>>(a, lanes, per_warp);
+  return cudaGetLastError();
+}
+
+}  // namespace sfk

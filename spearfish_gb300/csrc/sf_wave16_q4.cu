@@ -1,0 +1,9 @@
+// Anti-diagonal 16-bit kernels with 4 words a lane and parity.
+#include "sf_wave16_impl.cuh"
+
+namespace sfk {
+cudaError_t launch_wave16_4(bool tb, const AffLaunch& a, int lanes, int per_warp, int grid,
+                             cudaStream_t s) {
+  return launch_wave16_q<4>(tb, a, lanes, per_warp, grid, s);
+}
+}  // namespace sfk

@@ -1,0 +1,170 @@
+"""The anti-diagonal 16-bit kernel (sf_wave16_impl.cuh) against the oracle: scores, end cells,
+DP cells and CIGARs of Global banded passes, bit-exact, where its layout can go wrong -- every
+class filled to its last band cell, several passes of uneven length to a warp, bands that start
+at column 0 for many rows, one-base sequences, row steps around the stores (4), the window
+chunks (16) and the rebase (32), paths along the band's edges, long passes, and score sets on
+both sides of its admission rule."""
+import json
+
+import numpy as np
+import pytest
+
+import oracle as O
+import refcases as R
+
+pytestmark = pytest.mark.gpu
+
+# Few passes run one to a warp; more than this many on any GPU this library is built for run
+# several to a warp.
+PACKED = 3400
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from spearfish_gb300 import build
+    build.build()
+    from spearfish_gb300 import batch as B
+    c = B.Context(0)
+    yield c
+    c.close()
+
+
+def _run(ctx, rows, scores):
+    """rows: (pattern, text, band, cigar, score index).  Returns the output and the plan's
+    (kind, cells a lane, lanes) buckets."""
+    from spearfish_gb300 import batch as B
+    pb = B.PoolBuilder()
+    jobs = B.new_jobs(len(rows))
+    for j, (p, t, band, cig, sci) in zip(jobs, rows):
+        j["p_off"], j["m"] = pb.add(p), len(p)
+        j["t_off"], j["n"] = pb.add(t), len(t)
+        j["kind"], j["mode"], j["band"], j["want_cigar"] = B.JOB_AFFINE, 2, band, cig
+        j["sc_index"] = sci
+    plan = B.Plan(ctx, jobs, pb.size, scores)
+    try:
+        plan.upload(pb.build())
+        plan.execute()
+        out = plan.download()
+        plan.execute()  # replayed from the plan's graph
+        again = plan.download()
+        kinds = {(b["kind"], b["c"], b["lanes"]) for b in json.loads(plan.describe())["buckets"]}
+    finally:
+        plan.close()
+    assert np.array_equal(out.results, again.results) and np.array_equal(out.ops, again.ops)
+    return out, kinds
+
+
+def _check(rows, out, scores):
+    for q, (p, t, band, cig, sci) in enumerate(rows):
+        r = out.results[q]
+        o = O.traceback(p, t, O.TB_AFFINE, O.GLOBAL, scores[sci], band)
+        where = (q, len(p), len(t), band, sci)
+        assert (int(r["status"]), int(r["score"]), int(r["text_end"]), int(r["pattern_end"])) == \
+            (0, o["score"], len(t), len(p)), where
+        if cig:
+            assert out.cigar(q) == o["cigar"], where
+
+
+def _noisy(rng, m, rate):
+    q = rng.integers(0, 4, m)
+    return q.tolist(), R.mutate(q.tolist(), R.rand_edits(rng, int(m * rate), m))
+
+
+def _shifted(rng, m, d):
+    """A pair whose path leaves the main diagonal by d columns and comes back."""
+    q = rng.integers(0, 4, m).tolist()
+    cut = m // 2
+    if d > 0:
+        t = q[:cut] + rng.integers(0, 4, d).tolist() + q[cut:m - d]
+    else:
+        t = q[:cut] + q[cut - d:] + rng.integers(0, 4, -d).tolist()
+    return q, t
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_every_class_to_its_last_cell(ctx, packed):
+    """Bands whose cells fill each class exactly, miss it by one, or pass it by one; paths that
+    touch both band edges."""
+    rng = np.random.default_rng(2601 + packed)
+    rows = []
+    caps = (48, 64, 72, 80, 96, 120, 128, 144, 160, 192, 200, 240, 256, 288, 320, 384, 400, 480,
+            512, 640, 768, 1024, 1280, 1536)
+    for cap in caps:
+        for w in (cap - 1, cap, cap + 1):
+            band, extra = (w - 2) // 2, (w - 2) % 2
+            m = band + 30 + int(rng.integers(0, 90))
+            d = int(rng.integers(-band, band + 1))
+            p, t = _shifted(rng, m, d)
+            t = (t + rng.integers(0, 4, extra).tolist())
+            rows.append((p, t, band, 1 + 0 * cap, int(rng.integers(0, 2))))
+    while packed and len(rows) < PACKED:
+        band = int(rng.integers(1, 70))
+        p, t = _noisy(rng, int(rng.integers(band + 2, 4 * band + 40)), 0.1)
+        rows.append((p, t, band, int(rng.integers(0, 2)), int(rng.integers(0, 2))))
+    scores = (R.ONT, R.HIFI)
+    out, kinds = _run(ctx, rows, scores)
+    wave = {(c, n) for k, c, n in kinds if k == "wave16"}
+    want = {(16, 3), (24, 4), (40, 8), (48, 10), (32, 16), (48, 32)} if packed else \
+        {(16, 8), (16, 16), (16, 32), (24, 32), (32, 32), (40, 32), (48, 32)}
+    assert wave >= want, sorted(kinds)
+    _check(rows, out, scores)
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_small_and_uneven(ctx, packed):
+    """One to a few dozen bases, every remainder of the row steps, passes of very different
+    length side by side, bands wider than half the sequences."""
+    rng = np.random.default_rng(2611 + packed)
+    rows = []
+    for m in list(range(1, 70)) + [127, 128, 129]:
+        p, t = _noisy(rng, m, 0.15)
+        t = t or [int(rng.integers(0, 4))]
+        rows.append((p, t, int(rng.integers(0, max(1, m // 2) + 1)), m % 3 != 0, m % 2))
+    rows.append(([0], [3], 0, 1, 0))
+    rows.append(([0, 1, 2, 3] * 10, [2] * 75, 3, 1, 0))
+    for _ in range(PACKED - len(rows) if packed else 40):
+        m = int(np.exp(rng.uniform(np.log(4), np.log(600))))
+        rate = float(rng.choice([0.0, 0.05, 0.3]))
+        p, t = _noisy(rng, m, rate)
+        if rng.random() < 0.15:
+            t = rng.integers(0, 2, int(rng.integers(1, 2 * m + 2))).tolist()  # unrelated
+        rows.append((p, t or [1], int(rng.integers(0, min(60, m) + 1)), int(rng.integers(0, 2)),
+                     int(rng.integers(0, 2))))
+    scores = (R.ONT, R.HIFI)
+    out, _ = _run(ctx, rows, scores)
+    _check(rows, out, scores)
+
+
+def test_long_passes(ctx):
+    """Thousands of row steps: identical sequences (the largest field climbs most), unrelated
+    ones (it hardly moves), 10% errors; widths of the widest classes."""
+    rng = np.random.default_rng(2621)
+    rows = []
+    for m, band, kind in ((20000, 40, "same"), (9000, 64, "unrelated"), (12000, 512, "noisy"),
+                          (4000, 700, "noisy"), (3000, 700, "same"), (2500, 620, "unrelated")):
+        q = rng.integers(0, 4, m).tolist()
+        t = list(q) if kind == "same" else rng.integers(0, 4, m).tolist() \
+            if kind == "unrelated" else R.mutate(q, R.rand_edits(rng, m // 10, m))
+        rows += [(q, t, band, cig, sci) for cig in (0, 1) for sci in (0, 1)]
+    scores = (R.ONT, R.HIFI)
+    out, kinds = _run(ctx, rows, scores)
+    assert any(k == "wave16" for k, _, _ in kinds), kinds
+    _check(rows, out, scores)
+
+
+def test_admission(ctx):
+    """Score sets the kernel takes (mis = 2 ext, open >= 1) at its bounds, and ones it leaves to
+    the row kernels: the same results either way."""
+    rng = np.random.default_rng(2631)
+    scores = ((3, 2, 1, 1), (7, 0, 5, 0), (0, 4, 1, 2), (59, 2, 900, 1), (61, 2, 5, 1),
+              (20, 20, 10, 10), (2, 4, 0, 2), (2, 5, 4, 2), (2, 3, 4, 2), (0, 0, 1, 0))
+    rows = []
+    for sci in range(len(scores)):
+        for band in (0, 5, 60, 150, 230, 330):
+            p, t = _noisy(rng, int(rng.integers(max(20, band), 900)), 0.15)
+            rows.append((p, t, band, 1, sci))
+            p, t = _shifted(rng, 2 * band + 50, int(rng.integers(-band, band + 1)))
+            rows.append((p, t, band, 1, sci))
+    out, kinds = _run(ctx, rows, scores)
+    assert {"wave16", "affine16"} <= {k for k, _, _ in kinds}, kinds
+    _check(rows, out, scores)
