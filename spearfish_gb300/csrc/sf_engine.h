@@ -153,13 +153,22 @@ struct Bucket {
   int c = 0;       // affine: cells per lane; Myers: blocks per lane
   bool wide = false, tb = false;
   int lanes = 32;  // Myers: lanes per pair
-  int per_warp = 1;  // anti-diagonal kernel: passes per warp
+  int per_warp = 1;  // Myers and anti-diagonal kernels: pairs (passes) per warp
+  uint32_t task_first = 0, task_count = 0;  // its tasks (what a warp takes at a time)
   uint32_t first = 0, count = 0;  // range in the order array
   int grid = 0, block = 128;
   uint64_t scratch_off = 0;       // wide rows: this bucket's slice of the scratch (int32s)
   uint64_t work = 0;              // estimated work (cells of its passes' widest rows)
   uint64_t lat = 0;               // its longest pass's time, roughly (launch order)
   int stream = 0;                 // auxiliary stream it runs on
+};
+
+// One launch: a bucket, or the Myers (anti-diagonal) buckets that one kernel runs -- the same
+// blocks (words) a lane, whatever their lanes a pair -- as one task list.
+struct Group {
+  uint32_t bucket = 0;                      // its first bucket (kind, c, tb)
+  uint32_t task_first = 0, task_count = 0;  // none: the bucket's own order range
+  int grid = 0, block = 128, stream = 0;
 };
 
 }  // namespace sfe
@@ -172,6 +181,7 @@ struct BuildScratch;
 struct sf_plan {
   using Pass = sfe::Pass;
   using Bucket = sfe::Bucket;
+  using Group = sfe::Group;
   using DevBuf = sfe::DevBuf;
   using PinBuf = sfe::PinBuf;
   sf_context* ctx = nullptr;
@@ -186,12 +196,13 @@ struct sf_plan {
   uint32_t n_aff = 0, n_my = 0, n_walk = 0;
   bool myers_kcut = false;  // a Myers pass is Global or Prefix with k < m + n
   std::vector<Bucket> buckets;
+  std::vector<Group> groups;
   uint64_t tb_words = 0, ops_words = 0, scratch_cells = 0;
   int wide_warps = 0;
   std::string desc;
   // Device buffers.
   DevBuf d_bytes, d_pool, d_seq, d_djobs, d_params, d_res, d_mjobs, d_mout, d_tjobs, d_tres,
-      d_tb, d_ops, d_opsc, d_offs, d_order, d_counters, d_wlist, d_cls, d_scratch, d_total,
+      d_tb, d_ops, d_opsc, d_offs, d_order, d_tasks, d_counters, d_wlist, d_cls, d_scratch, d_total,
       d_chains, d_links, d_want, d_snap;
   // Chains of sorted-call passes the plan runs on the chain kernel, their passes, and per
   // pass whether it is one of them.
@@ -209,9 +220,10 @@ struct sf_plan {
   uint64_t launches = 0;
   // The transcript store SF_TEXT_STORE texts were resolved in (the context's at build time).
   const sf_store* store = nullptr;
-  // Whether anti-diagonal passes take the fastest class a pass (few passes) or the cheapest a
+  // Whether passes take the class that finishes one fastest (few passes) or the cheapest a
   // cell: -1 by the plan's passes, else as set (the autotuner's trial plans).
   int lean = -1;
+  int most = 0;  // Myers pairs a warp at most, likewise (0: by the plan's passes)
   // Class overrides for this plan only (the autotuner's trial plans); else the context's.
   const sfe::TuneTable* tune_override = nullptr;
   // Host-side build arrays kept between builds (sf_plan.cu).
@@ -243,9 +255,10 @@ struct sf_context {
   int dev = 0;
   int sms = 0;
   cudaStream_t s = nullptr;
-  // Auxiliary streams: kMain that buckets share round robin, then kSide for buckets of a
-  // few long passes, so that no other bucket waits behind them.
-  static constexpr int kMain = 8, kSide = 4, kAux = kMain + kSide;
+  // Auxiliary streams that launches share round robin: as many as the device has hardware
+  // queues by default.  More would share queues, and a launch would wait for another stream's
+  // (with twelve, config 3's four streams past the eighth held back a third of its buckets).
+  static constexpr int kAux = 8;
   cudaStream_t aux[kAux] = {};
   cudaEvent_t fork = nullptr, join[kAux] = {};
   std::unique_ptr<sf_plan> cache;  // reused by sf_batch_run
@@ -309,12 +322,15 @@ void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax,
                      int lanes16 = 32);
 // The band cells the anti-diagonal kernel lays out for a pass.
 int64_t wave_width(const DJob& j);
-// Whether a plan of np passes takes the anti-diagonal kernel's fastest classes a pass.
+// Whether a plan of np passes takes the Myers and anti-diagonal classes that finish a pass
+// fastest, rather than the cheapest ones a cell.
 bool lean_plan(size_t np, int sms);
+bool plan_is_lean(const sf_plan* P);
 // A class as its reports show it: cells a lane and lanes a pass.
 int shown_c(int kind, int c);
 int shown_lanes(int kind, int c, int lanes);
-int choose_myers_class(uint32_t m, int& b, int& lanes);
+int choose_myers_class(uint32_t m, bool lean, int most, int& b, int& lanes);
+int most_pairs(const sf_plan* P);
 DJob make_djob(const Pass& p, uint32_t& flags);
 // Whether large sf_batch_run batches may run in segments (SF_BATCH_SEGMENTS).
 bool batch_segments_on();
@@ -322,8 +338,8 @@ bool batch_segments_on();
 // far; stage_wait waits for that before it is written again.
 int stage_wait(sf_plan* P);
 int stage_done(sf_plan* P);
-// One execute in parts: the pack and the buckets (each on its auxiliary stream, the main
-// ones rotated by soff; also a single bucket with fan_one; `used` collects the streams),
+// One execute in parts: the pack and the launches (each on its auxiliary stream, rotated by
+// soff; also a single bucket with fan_one; `used` collects the streams),
 // the auxiliary streams joined back into `s`, then the CIGAR compaction.  plan_launch runs
 // all three; with `evs`, everything runs in order on `s` with an event after each stage.
 int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* evs, int soff,

@@ -227,7 +227,7 @@ const char* sf_last_error(void) { return last_error().c_str(); }
 
 const char* sf_version(void) {
   return "spearfish_gb300 sf_align 0.1 (sm_103a; affine C={4,6,8,9,10,11,12,14,16,20,24,28,32,40,48}+wide; "
-         "myers B={1,2,3,4,6,8,12,16})";
+         "myers B={1,2,3,4})";
 }
 
 int sf_set_device(int device) {
@@ -1080,7 +1080,7 @@ int batch_run_segments(sf_context* ctx, int nseg, const uint8_t* pool, uint64_t 
       (void)cudaStreamSynchronize(ctx->tail);
       return fail(rc, msg);
     }
-    soff = (soff + (int)std::max<size_t>(P->buckets.size(), 1)) % sf_context::kMain;
+    soff = (soff + (int)std::max<size_t>(P->groups.size(), 1)) % sf_context::kAux;
   }
   // Results, segment by segment as their tails end: the records converted while later
   // segments run, the CIGARs copied to the caller after the earlier segments' ones.
@@ -1150,10 +1150,10 @@ int sf_batch_run(sf_context* ctx, const uint8_t* pool, uint64_t pool_bytes, cons
 namespace {
 
 // A pass's class before any override, and the Myers blocks it needs.
-int default_class(const Pass& p, bool use16, bool lean, ClassKey& key, int64_t& blocks) {
+int default_class(const Pass& p, bool use16, bool lean, int most, ClassKey& key, int64_t& blocks) {
   if (p.kind == PK_MYERS) {
     int b = 1, lanes = 1;
-    int rc = choose_myers_class(p.m, b, lanes);
+    int rc = choose_myers_class(p.m, lean, most, b, lanes);
     if (rc) return rc;
     key = ClassKey{PK_MYERS, b, 0, 0, lanes};
     blocks = ((int64_t)p.m + 63) / 64;
@@ -1168,7 +1168,7 @@ int default_class(const Pass& p, bool use16, bool lean, ClassKey& key, int64_t& 
   classify_affine(p, j, flags, wmax, use16, lean, kind, c, wide, lanes, default_lanes16());
   const bool tb = p.want_cigar && p.kind != PK_LOCAL;
   key = ClassKey{kind, c, wide ? 1 : 0, tb ? 1 : 0, lanes};
-  blocks = kind == PK_WAVE16 ? wave_width(j) : wmax;  // affine: the group's widest row
+  blocks = wmax;  // affine: the group's widest row
   return SF_OK;
 }
 
@@ -1179,19 +1179,21 @@ std::vector<ClassChoice> tune_candidates(const ClassKey& key, int64_t blocks) {
   std::vector<ClassChoice> out;
   out.push_back(ClassChoice{key.c, key.lanes});
   if (key.kind == PK_MYERS) {
-    for (int q = 0; q < sfk::kMyersNB; ++q) {
-      const int b = sfk::kMyersB[q];
-      int lanes = 1;
-      while ((int64_t)lanes * b < blocks) lanes <<= 1;
-      if (lanes > 32) continue;
-      bool dup = false;
-      for (const auto& c : out) dup = dup || (c.c == b && c.lanes == lanes);
-      if (!dup) out.push_back(ClassChoice{b, lanes});
-    }
+    // Every class that holds all the default class does (later plans' pairs of it too).
+    const int hold = key.c * key.lanes;
+    for (int b = 1; b <= sfk::kMyersMaxB; ++b)
+      for (int lanes : {(hold + b - 1) / b, 64, 128}) {
+        if ((lanes > 32 && lanes != 64 && lanes != 128) || lanes * b < hold) continue;
+        if (lanes > 32 && hold <= 32) continue;
+        bool dup = false;
+        for (const auto& c : out) dup = dup || (c.c == b && c.lanes == lanes);
+        if (!dup) out.push_back(ClassChoice{b, lanes});
+      }
   } else if (key.kind == PK_WAVE16) {
-    // The next two classes that hold the group's widest band, and the fastest one a pass.
+    // The next classes that hold all the default class does (later plans' passes of it too).
     for (int c = 0; c < sfk::kWaveN; ++c)
-      if (c != key.c && sfk::wave_cap(sfk::kWave[c]) >= blocks && (int)out.size() < 4 &&
+      if (c != key.c && sfk::wave_cap(sfk::kWave[c]) >= sfk::wave_cap(sfk::kWave[key.c]) &&
+          (int)out.size() < 4 &&
           (c > key.c || key.c >= sfk::kWaveN0))
         out.push_back(ClassChoice{c, key.lanes});
   } else if (!key.wide) {
@@ -1242,14 +1244,15 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   if (reps == 0) reps = 1;
   const auto t0 = std::chrono::steady_clock::now();
   const bool use16 = allow16();
-  const bool lean = P->lean >= 0 ? P->lean != 0 : lean_plan(P->passes.size(), ctx->sms);
+  const bool lean = plan_is_lean(P);
+  const int most = most_pairs(P);
   // Group the passes by their default class.
   std::map<ClassKey, std::vector<size_t>> groups;
   std::map<ClassKey, int64_t> gblocks;
   for (size_t q = 0; q < P->passes.size(); ++q) {
     ClassKey k;
     int64_t blocks = 0;
-    int rc = default_class(P->passes[q], use16, lean, k, blocks);
+    int rc = default_class(P->passes[q], use16, lean, most, k, blocks);
     if (rc) return rc;
     groups[k].push_back(q);
     gblocks[k] = std::max(gblocks[k], blocks);
@@ -1258,6 +1261,7 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   S.ctx = ctx;
   S.pool_bytes = P->pool_bytes;
   S.lean = lean;
+  S.most = most;
   void* uploaded = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CK(cudaEventCreate(&e0));

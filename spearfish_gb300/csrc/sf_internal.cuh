@@ -185,6 +185,9 @@ struct AffLaunch {
   const sf::DParams* params;  // per job
   const uint32_t* order;      // job indices of this bucket, longest first
   uint32_t njobs;
+  // Anti-diagonal kernel: what a warp takes at a time, passes order[x ..], y = lanes a pass |
+  // passes << 8 (njobs: how many tasks).
+  const uint2* tasks;
   uint32_t* counter;          // work-queue head
   const uint32_t* pool;
   const uint8_t* bytes;       // byte pool (local band reads)
@@ -232,17 +235,20 @@ cudaError_t launch_affine16_chain(int c, const AffLaunch& a, int grid, int block
 struct MyersLaunch {
   const sf::MJob* jobs;
   const uint32_t* order;
-  uint32_t njobs;
+  // What a warp (a team: a block) takes at a time: pairs order[x ..], y = lanes a pair |
+  // pairs << 8.
+  const uint2* tasks;
+  uint32_t ntasks;
   uint32_t* counter;
   const uint32_t* pool;
   uint32_t* out;
-  int lanes;  // lanes per pair (power of two <= 32)
+  int team;   // one pair per block of 2 or 4 warps
   int kcut;   // some pair is Global or Prefix with k < m + n: stop pairs early (see kernel)
 };
+// Pairs of up to 64 * blocks_per_lane * lanes pattern bases; blocks_per_lane 1 .. kMyersMaxB.
 cudaError_t launch_myers(int blocks_per_lane, const MyersLaunch& a, int grid, int block,
                          cudaStream_t s);
-extern const int kMyersB[];
-extern const int kMyersNB;
+constexpr int kMyersMaxB = 4;
 
 // Sequences of a batch into its packed pool: from the byte pool, or (byte_off with bit 63
 // set) sliced from the transcript store's packed words at that base position; bit 62 reads

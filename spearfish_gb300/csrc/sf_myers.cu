@@ -1,10 +1,30 @@
-// Myers' bit-parallel edit distance (align.rs:47-168), one pair per P-lane segment of a warp.
+// Myers' bit-parallel edit distance (align.rs:47-168): one pair per P lanes of a warp, or, for
+// patterns of many blocks, per team of two or four warps (P = 64, 128).
 //
-// The pattern's 64-row blocks are spread over the segment's lanes, B consecutive blocks per
-// lane.  Within one text column the blocks form a chain (block b needs the horizontal delta
-// leaving block b - 1), across columns each block depends only on itself, so the segment runs
-// a diagonal pipeline: at step t lane l processes column t - l, taking the delta (and the
-// column's text base) that lane l - 1 produced at step t - 1 through one __shfl_up per step.
+// The pattern's 64-row blocks are spread over the pair's lanes, B consecutive blocks a lane.
+// Within one text column the blocks form a chain (block b needs the horizontal delta leaving
+// block b - 1), across columns each block depends only on itself, so the lanes run a diagonal
+// pipeline: lane l is at column t - l at step t, and takes the delta that lane l - 1 left at
+// step t - 1 with two shuffles.
+//
+//  - The pattern is aligned to the lanes' end: the free rows lie above it, as rows that change
+//    nothing (Infix: rows that match every base, so the zeros of row 0 reach the pattern's first
+//    row; Global and Prefix: rows that match none, through which row 0's +1 passes).  So every
+//    block's last row is bit 63, a delta travels as the sign bits of the block's two delta
+//    words, ready to shift into the next block, and the distance is read at one lane.
+//  - Match masks sit in shared memory by code, a lane to its own banks: one 8-byte load a block
+//    instead of the four logic instructions that derive them from bit planes.  A fifth code
+//    matches only the free rows: with no delta entering, a column of it leaves a lane's state
+//    as it is, so lanes wait for column 0 on it.
+//  - A lane reads its own columns' bases (a 16-base word every 16 steps), so no base travels.
+//  - A lane's deltas of 32 steps collect in two words; the distance and its least value over
+//    the columns come from their bit counts once every 32 steps, a column a lane.
+//
+// A team's warps run 63 steps apart, so the 32 deltas that leave a warp in one chunk of 32 steps
+// are exactly those its neighbour takes in the next: two words through shared memory and one
+// block barrier a chunk.
+//
+// Bound: the ALU pipe: 22 instructions a block and step and about 12 a step besides.
 //
 // Every block of every column is computed (no Ukkonen band): the reference's cutoff is
 // exact whenever the distance is <= k and reports None otherwise (align.rs:87-168, pinned by
@@ -12,15 +32,14 @@
 // with k gives the same Option<u32>.  The band's skipped blocks would save no time here: the
 // lanes holding them still step every column their upper neighbours step.
 //
-// What does save time is the end of a capped Global or Prefix pair (KC): once every cell of
-// a column exceeds k -- row 0 holds the column index there, and each block's bottom row is
-// at least k + 64, so its 64 rows exceed k -- every later cell does too (every path to a
-// later column crosses this one), and the pair's answer is fixed: None (Global) or the best
-// so far (Prefix).  Each lane tracks its blocks' bottom-row scores; the verdict for a column
-// travels down the segment with the column's pipeline payload, and the warp stops when every
-// segment has its verdict or has run out of text.  Infix pairs never stop (row 0 is 0).
+// What does save time is the end of a capped Global or Prefix pair: once every cell of the
+// lanes' current columns exceeds k + 1 (and row 0 does), every later cell exceeds k, since a
+// path to it crosses those columns, or the one beside them where it steps down between two
+// lanes; then the pair's answer is fixed: None (Global) or the best so far (Prefix).  Checked
+// once every 32 steps from each lane's bottom score (the bit counts) less its +1 vertical
+// deltas.  Between two warps of a team 32 columns lie open, so the bound is 32 higher there.
+// Infix pairs never stop (row 0 is 0).
 #include <type_traits>
-#include <utility>
 
 #include "sf_internal.cuh"
 
@@ -28,268 +47,278 @@ namespace {
 
 using sf::FULL;
 
-__device__ __forceinline__ uint32_t match16(uint32_t w, uint32_t c) {
-  // Bit k of the result: base k of the 16-base word w equals c.
-  uint32_t x = w ^ (c * 0x55555555u);
-  uint32_t y = ~(x | (x >> 1)) & 0x55555555u;
-  y = (y | (y >> 1)) & 0x33333333u;
-  y = (y | (y >> 2)) & 0x0F0F0F0Fu;
-  y = (y | (y >> 4)) & 0x00FF00FFu;
-  y = (y | (y >> 8)) & 0x0000FFFFu;
-  return y;
+constexpr int kCodes = 5;                    // A, C, G, T and "no column yet"
+constexpr int kCodeBytes = 32 * 8;           // a code's masks: 8 bytes a lane
+constexpr int kBlockBytes = kCodes * kCodeBytes;
+
+// The low (hi) bits of the 16 codes of w, gathered into 16 bits.
+__device__ __forceinline__ uint32_t gather16(uint32_t x) {
+  x &= 0x55555555u;
+  x = (x | (x >> 1)) & 0x33333333u;
+  x = (x | (x >> 2)) & 0x0F0F0F0Fu;
+  x = (x | (x >> 4)) & 0x00FF00FFu;
+  return (x | (x >> 8)) & 0x0000FFFFu;
 }
 
-// Calls f(std::integral_constant<int, k>{}) for k = 0 .. 15.
-template <class F, int... K>
-__device__ __forceinline__ void sf_unroll16_impl(F&& f, std::integer_sequence<int, K...>) {
-  (f(std::integral_constant<int, K>{}), ...);
-}
-template <class F>
-__device__ __forceinline__ void sf_unroll16(F&& f) {
-  sf_unroll16_impl(f, std::make_integer_sequence<int, 16>{});
+__device__ __forceinline__ int popc64(uint2 v) { return __popc(v.x) + __popc(v.y); }
+
+// align.rs:50-66 `block` on 32-bit halves.  in_p / in_m: the words whose sign bits are the +1 /
+// -1 delta entering the block; on return those of the delta leaving it.
+__device__ __forceinline__ void myers_block(uint2& pv, uint2& mv, uint2 eq, uint32_t& in_p,
+                                            uint32_t& in_m) {
+  const uint32_t xvl = eq.x | mv.x, xvh = eq.y | mv.y;
+  const uint32_t el = eq.x | (in_m >> 31);
+  uint32_t sl, sh;
+  asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, %5;"
+      : "=&r"(sl), "=r"(sh)
+      : "r"(el & pv.x), "r"(pv.x), "r"(eq.y & pv.y), "r"(pv.y));
+  const uint32_t xl = (sl ^ pv.x) | el, xh = (sh ^ pv.y) | eq.y;
+  const uint32_t pl = mv.x | ~(xl | pv.x), ph = mv.y | ~(xh | pv.y);
+  const uint32_t ml = pv.x & xl, mh = pv.y & xh;
+  const uint32_t spl = __funnelshift_l(in_p, pl, 1), sph = __funnelshift_l(pl, ph, 1);
+  const uint32_t sml = __funnelshift_l(in_m, ml, 1), smh = __funnelshift_l(ml, mh, 1);
+  pv.x = sml | ~(xvl | spl);
+  pv.y = smh | ~(xvh | sph);
+  mv.x = spl & xvl;
+  mv.y = sph & xvh;
+  in_p = ph;
+  in_m = mh;
 }
 
-// align.rs:50-66 `block`.  The horizontal delta entering and leaving the block travels as
-// two bits (pos: +1, neg: -1); the delta leaving is read at the block's last row `ob`
-// (63, or the pattern's last row in its last block), as bit 0 of
-// funnelshift_rc(lo, hi, ob) >> sub with sub = max(ob - 32, 0).
-__device__ __forceinline__ void myers_step(uint64_t& pv, uint64_t& mv, uint64_t eq,
-                                           uint32_t& pos, uint32_t& neg, uint32_t ob,
-                                           uint32_t sub) {
-  const uint64_t p = pv, m = mv;
-  const uint64_t xv = eq | m;
-  eq |= neg;
-  const uint64_t xh = (((eq & p) + p) ^ p) | eq;
-  uint64_t ph = m | ~(xh | p);
-  uint64_t mh = p & xh;
-  const uint32_t po =
-      (__funnelshift_rc((uint32_t)ph, (uint32_t)(ph >> 32), ob) >> sub) & 1u;
-  const uint32_t no =
-      (__funnelshift_rc((uint32_t)mh, (uint32_t)(mh >> 32), ob) >> sub) & 1u;
-  ph = (ph << 1) | pos;
-  mh = (mh << 1) | neg;
-  pv = mh | ~(xv | ph);
-  mv = ph & xv;
-  pos = po;
-  neg = no;
-}
+// Shared memory: the warps' match masks, then (teams) the chunk's words and votes by parity.
+template <int B>
+struct Team {
+  uint32_t acc[2][4][2];
+  uint32_t past[2][4];
+  uint32_t task;
+};
 
-template <int B, bool KC>
-__global__ void __launch_bounds__(B <= 4 ? 128 : (B <= 8 ? 64 : 32))
-    myers_kernel(sfk::MyersLaunch a) {
-  constexpr bool SMEM = B > 4;
+template <int B, bool TEAM>
+__global__ void __launch_bounds__(128, B <= 2 ? 8 : (B == 3 ? 6 : 5)) myers_kernel(sfk::MyersLaunch a) {
   extern __shared__ uint64_t smem[];
-  const int lane = threadIdx.x & 31;
-  const int P = a.lanes;
-  const int seg = lane / P, l = lane % P, nseg = 32 / P;
-  uint64_t* speq = smem + (size_t)(threadIdx.x >> 5) * 32 * B * 4;
+  __shared__ Team<B> X;
+  const int lane = threadIdx.x & 31, w = TEAM ? threadIdx.x >> 5 : 0;
+  const int W = TEAM ? blockDim.x >> 5 : 1;
+  // A lane's masks: code c of block bb at byte bb * kBlockBytes + c * kCodeBytes + 8 * lane.
+  const char* eqb = reinterpret_cast<const char*>(smem) +
+                    (threadIdx.x >> 5) * (B * kBlockBytes) + lane * 8;
+  char* eqw = const_cast<char*>(eqb);
 
   for (;;) {
-    uint32_t q0 = 0;
-    if (lane == 0) q0 = atomicAdd(a.counter, (uint32_t)nseg);
-    q0 = __shfl_sync(FULL, q0, 0);
-    if (q0 >= a.njobs) break;
-    const uint32_t qi = q0 + seg;
-    const bool has = qi < a.njobs;
-    sf::MJob J{};
-    uint32_t jid = 0;
-    if (has) {
-      jid = a.order[qi];
-      J = a.jobs[jid];
+    uint32_t q = 0;
+    if constexpr (TEAM) {
+      if (threadIdx.x == 0) X.task = atomicAdd(a.counter, 1u);
+      __syncthreads();
+      q = X.task;
+      __syncthreads();
+    } else {
+      if (lane == 0) q = atomicAdd(a.counter, 1u);
+      q = __shfl_sync(FULL, q, 0);
     }
-    const uint32_t m = J.m, n = J.n;
-    const uint32_t blocks = (m + 63) / 64;
-    const uint32_t last_block = blocks ? blocks - 1 : 0;
-    const uint32_t last_bit = m ? (m - 1) % 64 : 0;
+    if (q >= a.ntasks) break;
+    const uint2 task = a.tasks[q];
+    const int P = TEAM ? 32 * W : (int)(task.y & 0xffu), np = TEAM ? 1 : (int)(task.y >> 8);
+    const int seg = TEAM ? 0 : lane / P;
+    const int l = TEAM ? 32 * w + lane : lane - seg * P;
+    const bool has = seg < np;
+    const uint32_t jid = a.order[task.x + (has ? (uint32_t)seg : 0u)];
+    const sf::MJob J = a.jobs[jid];
+    const int m = (int)J.m, n = (int)J.n;
+    const bool infix = J.mode == 0, glob = J.mode == 2;
+    const int free_rows = P * B * 64 - m;  // above the pattern
 
-    // Match masks of this lane's blocks (align.rs:75-84): in shared memory per code for wide
-    // lanes; in registers as the pattern's two bit planes otherwise, eq(c) = bits whose code
-    // equals c.  Bits past the pattern's last row (and blocks past it) hold codes too: the
-    // row recurrences only move information to higher rows, so they never reach the rows the
-    // distance is read at.
-    uint64_t pl0[SMEM ? 1 : B], pl1[SMEM ? 1 : B];
-    uint64_t pv[B], mv[B];
-    uint32_t ob[B], osub[B];
-    // KC: each block's bottom-row score in this lane's current column (D[i][0] = i), and
-    // the threshold a block must reach for all its 64 rows to exceed k.
-    int32_t sb[KC ? B : 1];
-    const int64_t kk = (int64_t)min((uint64_t)J.k, (uint64_t)m + (uint64_t)n);
-    const int64_t thr = kk + 64;
+    uint2 pv[B], mv[B];
+    const int plim = (m >> 4) + 1;
 #pragma unroll
     for (int bb = 0; bb < B; ++bb) {
-      const uint32_t b = (uint32_t)l * B + bb;
-      uint64_t q[4] = {0, 0, 0, 0}, b0 = 0, b1 = 0;
-      if (has && b < blocks) {
+      const int row0 = (l * B + bb) * 64 - free_rows;  // the pattern row of bit 0
+      uint32_t lo[2] = {0, 0}, hi[2] = {0, 0};
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          const uint64_t wi = J.p_word + (uint64_t)b * 4 + h;
-          const uint32_t w = __funnelshift_r(__ldg(a.pool + wi), __ldg(a.pool + wi + 1), 2);
-          if constexpr (SMEM) {
+      for (int h = 0; h < 4; ++h) {
+        const int x = row0 + 16 * h + 1;  // packed position (one leading pad base)
+        const int i0 = min(max(x >> 4, 0), plim), i1 = min(max((x >> 4) + 1, 0), plim);
+        const uint32_t u = __funnelshift_r(__ldg(a.pool + J.p_word + i0), __ldg(a.pool + J.p_word + i1),
+                                           2 * (x & 15));
+        lo[h >> 1] |= gather16(u) << (16 * (h & 1));
+        hi[h >> 1] |= gather16(u >> 1) << (16 * (h & 1));
+      }
+      // Bits of free rows.
+      const int f = min(max(-row0, 0), 64);
+      const uint32_t fr[2] = {f >= 32 ? ~0u : (1u << f) - 1u,
+                              f >= 64 ? ~0u : (f <= 32 ? 0u : (1u << (f - 32)) - 1u)};
 #pragma unroll
-            for (int c = 0; c < 4; ++c) q[c] |= (uint64_t)match16(w, (uint32_t)c) << (16 * h);
-          } else {
-            // Gather the 16 codes' low and high bits.
-            uint32_t lo = w & 0x55555555u, hi = (w >> 1) & 0x55555555u;
-            lo = (lo | (lo >> 1)) & 0x33333333u;
-            lo = (lo | (lo >> 2)) & 0x0F0F0F0Fu;
-            lo = (lo | (lo >> 4)) & 0x00FF00FFu;
-            lo = (lo | (lo >> 8)) & 0x0000FFFFu;
-            hi = (hi | (hi >> 1)) & 0x33333333u;
-            hi = (hi | (hi >> 2)) & 0x0F0F0F0Fu;
-            hi = (hi | (hi >> 4)) & 0x00FF00FFu;
-            hi = (hi | (hi >> 8)) & 0x0000FFFFu;
-            b0 |= (uint64_t)lo << (16 * h);
-            b1 |= (uint64_t)hi << (16 * h);
-          }
+      for (int c = 0; c < kCodes; ++c) {
+        uint2 e;
+        uint32_t* eh[2] = {&e.x, &e.y};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t k = (c & 1 ? lo[h] : ~lo[h]) & (c & 2 ? hi[h] : ~hi[h]);
+          *eh[h] = c == 4 ? fr[h] : (k & ~fr[h]) | (infix ? fr[h] : 0u);
         }
+        *reinterpret_cast<uint2*>(eqw + bb * kBlockBytes + c * kCodeBytes) = e;
       }
-      if constexpr (SMEM) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) speq[((size_t)bb * 4 + c) * 32 + lane] = q[c];
-      } else {
-        pl0[bb] = b0;
-        pl1[bb] = b1;
-      }
-      pv[bb] = ~0ull;
-      mv[bb] = 0;
-      if constexpr (KC) sb[bb] = has && b < blocks ? (int32_t)min((b + 1) * 64u, m) : INT32_MAX / 2;
-      ob[bb] = b == last_block ? last_bit : 63u;
-      osub[bb] = ob[bb] >= 32 ? ob[bb] - 32 : 0u;
+      pv[bb] = make_uint2(~fr[0], ~fr[1]);
+      mv[bb] = make_uint2(0, 0);
     }
-    if constexpr (SMEM) __syncwarp();
+    __syncwarp();
 
-    const int top = J.mode == 0 ? 0 : 1;  // Infix: free text start
-    const bool owner = has && m > 0 && (uint32_t)l == last_block / B;
-    const int own_bb = (int)(last_block % B);
-    int score = (int)m, best = (int)m;
-    const int seg_steps = has && m > 0 ? (int)n + P - 1 : 0;
-    const int steps = __reduce_max_sync(FULL, seg_steps);
-    uint32_t payload = 0;  // (column past k << 4) | (text code << 2) | (pos << 1) | neg
-    bool dead = false;     // KC, the segment's last lane: a column wholly past k went by
-    uint32_t tw = 0;       // the text word holding base t + 1 (used by lane 0)
-    const bool glob = J.mode == 2;
-    // One step of the pipeline.  Lanes keep their state only while they are past the fill
-    // (FILL: some lanes have not reached column 0 yet); past its text's end a lane computes
-    // on state nothing reads any more, so the steady loop needs no masking and no branches.
-    // K < 0: the step reads its text base itself; K = 0..15: the step is the K-th of a run of
-    // 16 whose bases all sit in `tw`, loaded before the run.  Every lane keeps a running
-    // score (only the owner's is used): the column's distance while the lane's column lies in
-    // the text, and the least of them (Infix, Prefix; Global takes the last).
-    const int jend = (int)n + l;  // steps t < jend have this lane's column j = t - l < n
-    auto step = [&](int t, auto fill, auto kk) {
-      constexpr bool FILL = decltype(fill)::value;
-      constexpr int K = decltype(kk)::value;
-      const int j = t - l;
-      const bool live = FILL ? (j >= 0 && t < jend) : t < jend;
-      const uint32_t in = __shfl_up_sync(FULL, payload, 1, P);
-      uint32_t c0;
-      if constexpr (K < 0) {
-        // A new text word every 16 steps, read only while it lies inside this text (base
-        // t + 1 of a text of n bases sits in word (t + 1) / 16 after the leading pad base).
-        if ((((t + 1) & 15) == 0 || t == 0) && (uint32_t)(t + 1) <= n)
-          tw = __ldg(a.pool + J.t_word + ((uint32_t)(t + 1) >> 4));
-        c0 = (tw >> (2 * ((t + 1) & 15))) & 3u;
-      } else {
-        c0 = (tw >> (2 * K)) & 3u;
-      }
-      const uint32_t c = l == 0 ? c0 : ((in >> 2) & 3u);
-      uint32_t pos = l == 0 ? (uint32_t)top : (in >> 1) & 1u;
-      uint32_t neg = l == 0 ? 0u : in & 1u;
-      // eq(c) from the bit planes: both code bits equal c's.
-      [[maybe_unused]] const uint64_t m0 = (c & 1u) ? ~0ull : 0ull, m1 = (c & 2u) ? ~0ull : 0ull;
-      int hlast = 0;
-#pragma unroll
-      for (int bb = 0; bb < B; ++bb) {
-        uint64_t eq;
-        if constexpr (SMEM)
-          eq = speq[((size_t)bb * 4 + c) * 32 + lane];
-        else
-          eq = ~(pl0[bb] ^ m0) & ~(pl1[bb] ^ m1);
-        if constexpr (FILL) {
-          uint64_t p2 = pv[bb], m2 = mv[bb];
-          myers_step(p2, m2, eq, pos, neg, ob[bb], osub[bb]);
-          if (j >= 0) {
-            pv[bb] = p2;
-            mv[bb] = m2;
-            if constexpr (KC) sb[bb] += (int32_t)pos - (int32_t)neg;
+    // Lane l is at column s - delay at step s.
+    const int delay = TEAM ? 63 * w + lane : l;
+    const int tlim = (n >> 4) + 1;
+    auto bases = [&](int s) {  // the 16 columns from step s on
+      const int x = s - delay + 1;
+      const int i0 = min(max(x >> 4, 0), tlim), i1 = min(max((x >> 4) + 1, 0), tlim);
+      return __funnelshift_r(__ldg(a.pool + J.t_word + i0), __ldg(a.pool + J.t_word + i1), 2 * (x & 15));
+    };
+    const int last = TEAM ? 63 * (W - 1) + 31 : P - 1;  // the delay of the pattern's last row
+    const int mine = has && m > 0 && n > 0 ? (n - 1 + last) / 32 + 1 : 0;
+    const int chunks = TEAM ? mine : (int)__reduce_max_sync(FULL, mine);
+
+    int score = m, best = glob ? INT32_MAX : m;
+    // This lane's bottom score in its current column (D[i][0] = i), for the cap.
+    int bottom = max((l + 1) * B * 64 - free_rows, 0);
+    const bool capped = a.kcut && has && !infix && (uint64_t)J.k < (uint64_t)m + (uint64_t)n;
+    const int far = (int)min((uint64_t)J.k, (uint64_t)0x3fffffff) + (TEAM ? 34 : 2);
+    const bool any_cap = __any_sync(FULL, capped);
+    bool dead = false;
+    uint32_t out_p = 0, out_m = 0;  // the deltas leaving this lane
+    // What enters the pair's first lane: row 0's delta, or (teams) the last warp's words, a
+    // column at their sign bit, moved on by a multiplication (the FMA pipe).
+    const bool first = l == 0 || (TEAM && lane == 0);
+    const bool relay = TEAM && w > 0;
+    const uint32_t step_mul = relay ? 2u : 1u;
+    uint32_t src_p = infix || relay ? 0u : 0x80000000u, src_m = 0;
+    const uint32_t top = src_p;
+
+    uint32_t tw = 0;  // the next 16 columns' bases
+    auto chunk = [&](int s, auto filltag) {
+      constexpr bool FILL = decltype(filltag)::value;
+      uint32_t acc_p = 0, acc_m = 0;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        const uint32_t tn = bases(s + 16 * half + 16);
+#pragma unroll(B <= 2 ? 4 : 2)
+        for (int k = 0; k < 16; ++k) {
+          uint32_t ip = __shfl_up_sync(FULL, out_p, 1), im = __shfl_up_sync(FULL, out_m, 1);
+          uint32_t c = tw & 3u;
+          if constexpr (FILL) {
+            const bool wait = s + 16 * half + k < delay;
+            if (wait) c = 4;
+            if (first) {
+              ip = wait && !relay ? 0u : src_p;
+              im = src_m;
+            }
+          } else if (first) {
+            ip = src_p;
+            im = src_m;
           }
-        } else {
-          myers_step(pv[bb], mv[bb], eq, pos, neg, ob[bb], osub[bb]);
-          if constexpr (KC) sb[bb] += (int32_t)pos - (int32_t)neg;
-        }
-        hlast = bb == own_bb ? (int)pos - (int)neg : hlast;
-      }
-      score += live ? hlast : 0;
-      best = min(best, score);
-      uint32_t past = 0;
-      if constexpr (KC) {
-        // Column j wholly past k down to this lane's blocks: row 0 (lane 0: D[0][j + 1] =
-        // j + 1) and every block above, as the lane before found; then this lane's blocks.
-        bool ex = l == 0 ? (int64_t)t + 1 > kk : ((in >> 4) & 1u) != 0;
+          if constexpr (TEAM) {
+            src_p *= step_mul;
+            src_m *= step_mul;
+          }
+          tw >>= 2;
+          const char* at = eqb + c * kCodeBytes;
 #pragma unroll
-        for (int bb = 0; bb < B; ++bb) ex = ex && sb[bb] >= thr;
-        ex = ex && live;
-        if (ex && l == P - 1) dead = true;
-        past = ex ? 16u : 0u;
+          for (int bb = 0; bb < B; ++bb)
+            myers_block(pv[bb], mv[bb], *reinterpret_cast<const uint2*>(at + bb * kBlockBytes), ip, im);
+          out_p = ip;
+          out_m = im;
+          acc_p = __funnelshift_l(ip, acc_p, 1);
+          acc_m = __funnelshift_l(im, acc_m, 1);
+        }
+        tw = tn;
       }
-      payload = past | (c << 2) | (pos << 1) | neg;
+      return make_uint2(acc_p, acc_m);
     };
-    // KC: every segment has its column past k, or has stepped through its text.
-    auto all_done = [&](int t) -> bool {
-      const uint32_t bal = __ballot_sync(FULL, dead);
-      const bool sd = ((bal >> (seg * P + P - 1)) & 1u) != 0;
-      return __all_sync(FULL, sd || t >= seg_steps);
-    };
-    bool stop = false;
-    using kAny = std::integral_constant<int, -1>;
-    const int fill = steps < P - 1 ? steps : P - 1;
-    int t = 0;
-    for (; t < fill; ++t) step(t, std::true_type{}, kAny{});
-    // Steady steps: with register blocks, single ones up to a text-word boundary, then runs of
-    // 16 with one load each (wider lanes keep the loop short: their step is long already).
-    if constexpr (!SMEM) {
-      for (; t < steps && ((t + 1) & 15) != 0; ++t) step(t, std::false_type{}, kAny{});
-      for (; t + 16 <= steps; t += 16) {
-        if constexpr (KC) {
-          if (all_done(t)) {
-            stop = true;
+
+    for (int ch = 0; ch < chunks; ++ch) {
+      const int s = 32 * ch;
+      uint2 acc = make_uint2(0, 0);
+      if constexpr (TEAM) {
+        // A warp whose first column is still to come leaves no deltas.
+        if (s + 31 >= 63 * w) {
+          if (s <= 63 * w) tw = bases(s);  // the warp's first chunk
+          if (relay) {
+            src_p = ch > 0 ? X.acc[(ch + 1) & 1][w - 1][0] : 0u;
+            src_m = ch > 0 ? X.acc[(ch + 1) & 1][w - 1][1] : 0u;
+          } else {
+            src_p = top;
+          }
+          acc = s < 63 * w + 31 ? chunk(s, std::true_type{}) : chunk(s, std::false_type{});
+        }
+      } else {
+        if (ch == 0) tw = bases(0);
+        acc = ch == 0 ? chunk(s, std::true_type{}) : chunk(s, std::false_type{});
+      }
+      bottom += __popc(acc.x) - __popc(acc.y);
+      // The pair's last lane holds the last row's deltas: columns s - last .. + 31.
+      const int own = TEAM ? 31 : min(seg * P + P - 1, 31);
+      const uint32_t op = __shfl_sync(FULL, acc.x, own), om = __shfl_sync(FULL, acc.y, own);
+      if (!TEAM || w == W - 1) {
+        const int c0 = s - last;
+        for (int t = TEAM ? lane : l; t < 32; t += TEAM ? 32 : P) {
+          const int c = c0 + t;
+          if (c >= 0 && c < n && (!glob || c == n - 1))
+            best = min(best, score + __popc(op >> (31 - t)) - __popc(om >> (31 - t)));
+        }
+        score += __popc(op) - __popc(om);
+      }
+      bool past = false;
+      if (any_cap) {
+        int ups = 0;
+#pragma unroll
+        for (int bb = 0; bb < B; ++bb) ups += popc64(pv[bb]);
+        past = bottom - ups >= far && (!first || relay || s + 32 >= far);
+      }
+      if constexpr (TEAM) {
+        if (lane == 31) {
+          X.acc[ch & 1][w][0] = acc.x;
+          X.acc[ch & 1][w][1] = acc.y;
+        }
+        const bool all = __all_sync(FULL, past);
+        if (lane == 0) X.past[ch & 1][w] = all;
+        __syncthreads();
+        if (capped && ch + 1 < mine) {
+          bool every = true;
+          for (int u = 0; u < W; ++u) every = every && X.past[ch & 1][u];
+          if (every) {
+            dead = true;
             break;
           }
         }
-        if ((uint32_t)(t + 1) <= n) tw = __ldg(a.pool + J.t_word + ((uint32_t)(t + 1) >> 4));
-        sf_unroll16([&](auto kt) { step(t + decltype(kt)::value, std::false_type{}, kt); });
+      } else if (any_cap) {
+        const uint32_t lanes = (P == 32 ? FULL : (1u << P) - 1u) << min(seg * P, 31);
+        const uint32_t bal = __ballot_sync(FULL, past);
+        if (capped && ch + 1 < mine && (bal & lanes) == lanes) dead = true;
+        if (__all_sync(FULL, dead || ch + 1 >= mine)) break;
       }
     }
-    for (; t < steps && !stop; ++t) {
-      if constexpr (KC) {
-        if ((t & 15) == 0 && all_done(t)) break;
-      }
-      step(t, std::false_type{}, kAny{});
-    }
-    if (glob) best = score;
-    if constexpr (KC) {
-      // A segment whose column went past k: Global ends past k; Prefix keeps its best.
-      const uint32_t bal = __ballot_sync(FULL, dead);
-      if (((bal >> (seg * P + P - 1)) & 1u) && glob) best = INT32_MAX;
-    }
-    if (has) {
-      if (m == 0) {
-        if (l == 0) {
-          const uint32_t d = J.mode == 2 ? n : 0;
-          a.out[jid] = d <= J.k ? d : 0xffffffffu;
-        }
-      } else if (owner) {
+    if (dead && glob) best = INT32_MAX;
+    if constexpr (TEAM) {
+      best = __reduce_min_sync(FULL, best);
+      if (w == W - 1 && lane == 0) {
+        if (m == 0 || n == 0) best = m == 0 ? (glob ? n : 0) : m;
         a.out[jid] = (uint32_t)best <= J.k ? (uint32_t)best : 0xffffffffu;
       }
+      __syncthreads();
+    } else {
+      for (int t = 1; t < P; t <<= 1) {
+        const int o = __shfl_down_sync(FULL, best, t);
+        if (l + t < P) best = min(best, o);
+      }
+      if (has && l == 0) {
+        if (m == 0 || n == 0) best = m == 0 ? (glob ? n : 0) : m;
+        a.out[jid] = (uint32_t)best <= J.k ? (uint32_t)best : 0xffffffffu;
+      }
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 
 template <int B>
 cudaError_t launch_b(const sfk::MyersLaunch& a, int grid, int block, cudaStream_t s) {
-  const size_t sm = B > 4 ? (size_t)(block / 32) * 32 * B * 4 * sizeof(uint64_t) : 0;
-  if (a.kcut)
+  const size_t sm = (size_t)(block / 32) * B * kBlockBytes;
+  if (a.team)
     myers_kernel<B, true><<<grid, block, sm, s>>>(a);
   else
     myers_kernel<B, false><<<grid, block, sm, s>>>(a);
@@ -300,19 +329,12 @@ cudaError_t launch_b(const sfk::MyersLaunch& a, int grid, int block, cudaStream_
 
 namespace sfk {
 
-const int kMyersB[] = {1, 2, 3, 4, 6, 8, 12, 16};
-const int kMyersNB = 8;
-
 cudaError_t launch_myers(int b, const MyersLaunch& a, int grid, int block, cudaStream_t s) {
   switch (b) {
     case 1: return launch_b<1>(a, grid, block, s);
     case 2: return launch_b<2>(a, grid, block, s);
     case 3: return launch_b<3>(a, grid, block, s);
     case 4: return launch_b<4>(a, grid, block, s);
-    case 6: return launch_b<6>(a, grid, block, s);
-    case 8: return launch_b<8>(a, grid, block, s);
-    case 12: return launch_b<12>(a, grid, block, s);
-    case 16: return launch_b<16>(a, grid, block, s);
     default: return cudaErrorInvalidValue;
   }
 }

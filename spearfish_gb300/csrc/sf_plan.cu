@@ -117,6 +117,14 @@ bool fits_wave(const Pass& p, const DJob& j, uint32_t flags) {
 // 600 passes 0.47 ms on 4 words x 32 lanes, 0.84 on 10 x 8; 1,200 passes 0.64 against 1.37 on
 // 12 x 6; 8,200 passes 3.49 against 2.54 (four a warp): the lines cross near 20 an SM.
 bool lean_plan(size_t np, int sms) { return np <= (size_t)sms * 20; }
+bool plan_is_lean(const sf_plan* P) {
+  return P->lean >= 0 ? P->lean != 0 : lean_plan(P->passes.size(), P->ctx->sms);
+}
+// Myers pairs a warp at most: four warps a scheduler before more pairs share one.
+int most_pairs(const sf_plan* P) {
+  if (P->most) return P->most;
+  return (int)std::max<size_t>(1, std::min<size_t>(32, P->passes.size() / ((size_t)P->ctx->sms * 16)));
+}
 
 int shown_c(int kind, int c) { return kind == PK_WAVE16 ? 4 * sfk::kWave[c].q : c; }
 int shown_lanes(int kind, int c, int lanes) {
@@ -222,31 +230,37 @@ void apply_tune(const TuneTable* tune, int kind, int& c, bool wide, bool tb, int
 }
 
 // Whether choose_myers_class takes a pattern of m bases (a check that sets no error).
-bool myers_class_ok(uint32_t m) {
-  if (m > SF_MYERS_MAX_PATTERN) return false;
-  const uint32_t blocks = (m + 63) / 64;
-  if (blocks <= 32) return true;
-  for (int q = 0; q < sfk::kMyersNB; ++q)
-    if (32u * (uint32_t)sfk::kMyersB[q] >= blocks) return true;
-  return false;
-}
+bool myers_class_ok(uint32_t m) { return m <= SF_MYERS_MAX_PATTERN; }
 
-int choose_myers_class(uint32_t m, int& b, int& lanes) {
-  const uint32_t blocks = (m + 63) / 64;
+// Blocks a lane and lanes a pair for a pattern of m bases.  A warp's step with B blocks a lane
+// was measured at 74, 140, 190 and 250 cycles of a scheduler, whatever its lanes hold: many
+// pairs take the B whose share of a step is least, of at most `most` pairs a warp (10,000 1 kb
+// pairs: 0.33 ms at 2 x 8 and 1 x 16 lanes, 0.36 at 4 x 4, which leaves two warps a scheduler);
+// few pairs one block a lane, over several warps from 33 blocks on (100 of 5 kb: 0.29 ms at
+// 1 x 128, 0.58 at 4 x 32).  Past 128 blocks a pair takes four warps either way (a 20 kb pattern
+// on one warp ran 8.1 ms alone, and among other kernels it set an uneven batch's time; on four
+// 2.3 ms).
+int choose_myers_class(uint32_t m, bool lean, int most, int& b, int& lanes) {
   if (m > SF_MYERS_MAX_PATTERN) return fail(SF_ERR_TOO_LONG, "Myers pattern longer than SF_MYERS_MAX_PATTERN");
-  if (blocks <= 32) {
-    b = 1;
-    lanes = 1;
-    while ((uint32_t)lanes < blocks) lanes <<= 1;
+  const int blocks = std::max(1, (int)((m + 63) / 64));
+  if (blocks > 128 || (lean && blocks > 32)) {
+    lanes = lean && blocks <= 64 ? 64 : 128;
+    b = (blocks + lanes - 1) / lanes;
     return SF_OK;
   }
-  lanes = 32;
-  for (int q = 0; q < sfk::kMyersNB; ++q)
-    if (32u * (uint32_t)sfk::kMyersB[q] >= blocks) {
-      b = sfk::kMyersB[q];
-      return SF_OK;
+  int best = INT32_MAX;
+  for (int c = 1; c <= (lean ? 1 : sfk::kMyersMaxB); ++c) {
+    const int p = (blocks + c - 1) / c;
+    if (p > 32) continue;
+    constexpr int kStep[sfk::kMyersMaxB] = {74, 140, 190, 250};
+    const int cost = 64 * kStep[c - 1] / std::min(32 / p, most);
+    if (cost < best) {
+      best = cost;
+      b = c;
+      lanes = p;
     }
-  return fail(SF_ERR_TOO_LONG, "pattern too long for the Myers kernels");
+  }
+  return SF_OK;
 }
 
 DJob make_djob(const Pass& p, uint32_t& flags) {
@@ -313,6 +327,7 @@ struct BuildScratch {
   std::vector<uint16_t> cls;
   std::vector<MJob> mj;
   std::vector<uint32_t> wlist, kid, order;
+  std::vector<uint2> tasks;
   std::vector<std::pair<BucketKey, BucketItem>> items, per;
   std::vector<uint8_t> has_item;
   std::vector<std::pair<uint64_t, uint32_t>> byb, byb_tmp;
@@ -575,7 +590,8 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   const sf_context* ctx = P->ctx;
   const size_t np = P->passes.size();
   const int lanes16 = default_lanes16();
-  const bool lean = P->lean >= 0 ? P->lean != 0 : lean_plan(np, ctx->sms);
+  const bool lean = plan_is_lean(P);
+  const int most = most_pairs(P);
   const TuneTable* tune = P->tune_override ? P->tune_override : &ctx->tune;
   const auto& word_of = S.word_of;
   auto& dj = S.dj;
@@ -605,7 +621,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   for (int k = 0; k < kT; ++k) {
     if (bad[k] != UINT64_MAX) {
       int b = 1, l = 1;
-      return choose_myers_class(P->passes[bad[k]].m, b, l);  // sets the error
+      return choose_myers_class(P->passes[bad[k]].m, lean, 1, b, l);  // sets the error
     }
     nmy[k + 1] += nmy[k];
   }
@@ -663,7 +679,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       const uint32_t sl = P->slot[q];
       if (p.kind == PK_MYERS) {
         int b = 1, lanes = 1;
-        (void)choose_myers_class(p.m, b, lanes);
+        (void)choose_myers_class(p.m, lean, most, b, lanes);
         tuned(PK_MYERS, b, false, false, lanes);
         MJob& m = mj[sl];
         m = MJob{};
@@ -675,7 +691,8 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
         m.k = p.k;
         if (p.mode != SF_INFIX && (uint64_t)p.k < (uint64_t)p.m + p.n) kcut[worker] = true;
         per[q] = {Key2{PK_MYERS, b, 0, 0, lanes},
-                  Item{sl, (uint64_t)p.n, ((uint64_t)p.n + (uint64_t)lanes) * (4u * (uint64_t)b + 4u)}};
+                  // A step takes about (70 + 25 B) / 45 of a row's unit.
+                  Item{sl, (uint64_t)p.n, ((uint64_t)p.n + (uint64_t)lanes) * ((uint64_t)b + 3u) / 2u}};
         has_item[q] = 1;
         pass_work[q] = pass_lat[q] = 0;
         continue;
@@ -854,20 +871,24 @@ void build_chains(sf_plan* P, BuildScratch& S) {
 void build_buckets(sf_plan* P, BuildScratch& S) {
   using Key2 = BucketKey;
   const sf_context* ctx = P->ctx;
+  const bool lean = plan_is_lean(P);
   const auto& items = S.items;
   const size_t ni = items.size();
   constexpr int kT = 16;
   // Buckets in key order; within a bucket, longest work first (ties in job order).
   // Each item's bucket first: keys pack into 15-bit codes ordered as the keys are (kind < 8,
-  // C < 128, lanes a power of two up to 64, coded by its log2), so a bit set of the codes
-  // present lists the buckets in order and a code's bucket is the number of codes below it.
-  // Keys outside those bounds (never built) take a search instead.
+  // C < 128, lanes a power of two up to 64, coded by its log2; Myers: up to 4 blocks a lane and
+  // 128 lanes), so a bit set of the codes present lists the buckets in order and a code's bucket
+  // is the number of codes below it.  Keys outside those bounds (never built) take a search
+  // instead.
   auto& kid = S.kid;
   kid.resize(ni);
   std::vector<Key2> keys;  // the buckets' keys, in order
   {
     constexpr uint32_t kWords = (1u << 15) / 64;
     auto fits = [](const Key2& k) {
+      if (k.kind == PK_MYERS)
+        return k.c >= 1 && k.c <= 8 && !k.wide && !k.tb && k.lanes >= 1 && k.lanes <= 512;
       return k.kind >= 0 && k.kind < 8 && k.c >= 0 && k.c < 128 && (k.wide & ~1) == 0 &&
              (k.tb & ~1) == 0 && k.lanes >= 1 && k.lanes <= 64 && (k.lanes & (k.lanes - 1)) == 0;
     };
@@ -884,9 +905,11 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
           packed[k] = false;
           return;
         }
-        const uint32_t c = (uint32_t)key.kind << 12 | (uint32_t)key.c << 5 |
-                           (uint32_t)key.wide << 4 | (uint32_t)key.tb << 3 |
-                           (uint32_t)__builtin_ctz((uint32_t)key.lanes);
+        const uint32_t c = key.kind == PK_MYERS
+                               ? (uint32_t)(key.c - 1) << 9 | (uint32_t)(key.lanes - 1)
+                               : (uint32_t)key.kind << 12 | (uint32_t)key.c << 5 |
+                                     (uint32_t)key.wide << 4 | (uint32_t)key.tb << 3 |
+                                     (uint32_t)__builtin_ctz((uint32_t)key.lanes);
         kid[q] = c;
         w[c >> 6] |= uint64_t(1) << (c & 63);
       }
@@ -900,7 +923,10 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
         below[w + 1] = below[w] + (uint32_t)__builtin_popcountll(x);
         for (; x; x &= x - 1) {
           const int c = (int)(w * 64 + (uint32_t)__builtin_ctzll(x));
-          keys.push_back(Key2{(int)(c >> 12), (int)((c >> 5) & 127), (int)((c >> 4) & 1),
+          if (c >> 12 == PK_MYERS)
+            keys.push_back(Key2{PK_MYERS, (c >> 9) + 1, 0, 0, (c & 511) + 1});
+          else
+            keys.push_back(Key2{(int)(c >> 12), (int)((c >> 5) & 127), (int)((c >> 4) & 1),
                               (int)((c >> 3) & 1), 1 << (c & 7)});
         }
       }
@@ -1046,22 +1072,24 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
   // may run concurrently (fan-out streams), so each gets its own scratch slice.
   int wide_warps = 0;
   uint64_t scratch_total = 0;
+  auto warps_grid = [&](uint64_t warps, int block) {
+    const uint64_t wpb = (uint64_t)block / 32;
+    return (int)std::max<uint64_t>(
+        1, std::min<uint64_t>((warps + wpb - 1) / wpb, (uint64_t)ctx->sms * (2048 / block)));
+  };
   for (auto& b : P->buckets) {
-    if (b.kind == PK_MYERS) {
-      b.block = b.c <= 4 ? 128 : (b.c <= 8 ? 64 : 32);
-      const uint64_t per_warp = (uint64_t)(32 / b.lanes);
-      const uint64_t warps = (b.count + per_warp - 1) / per_warp;
-      const uint64_t wpb = (uint64_t)b.block / 32;
-      b.grid = (int)std::min<uint64_t>((warps + wpb - 1) / wpb, (uint64_t)ctx->sms * (2048 / b.block));
-    } else if (b.kind == PK_WAVE16) {
-      // As many passes a warp as its lanes hold; in the fast classes fewer, while that leaves
+    if (b.kind == PK_MYERS || b.kind == PK_WAVE16) {
+      // As many pairs a warp as its lanes hold; in the fast classes fewer, while that leaves
       // schedulers empty.
-      b.block = 128;
-      const int64_t most = 32 / sfk::kWave[b.c].lanes;
-      b.per_warp = (int)(b.c < sfk::kWaveN0 ? most
-                                            : std::max<int64_t>(1, std::min<int64_t>(most, b.count / (4 * (int64_t)ctx->sms))));
-      const uint64_t blocks = (b.count + 4 * b.per_warp - 1) / (4 * b.per_warp);
-      b.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)ctx->sms * 16));
+      const bool my = b.kind == PK_MYERS;
+      const int64_t most =
+          my ? std::min(most_pairs(P), std::max(1, 32 / b.lanes)) : 32 / sfk::kWave[b.c].lanes;
+      const bool fast = my ? lean : b.c >= sfk::kWaveN0;
+      b.per_warp = (int)(!fast ? most
+                               : std::max<int64_t>(1, std::min<int64_t>(most, b.count / (4 * (int64_t)ctx->sms))));
+      b.task_count = (b.count + b.per_warp - 1) / b.per_warp;
+      b.block = my && b.lanes > 32 ? b.lanes : 128;
+      b.grid = warps_grid((uint64_t)b.task_count * (my && b.lanes > 32 ? b.lanes / 32 : 1), b.block);
     } else {
       // Two-warp passes: one pass per 64-thread block; otherwise a 4-warp block holds 4
       // passes (chains), or 8 with 16 lanes a pass.
@@ -1079,18 +1107,44 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
   }
   P->wide_warps = wide_warps;
   S.scratch_total = scratch_total;
-  // Streams.  The first buckets (in launch order) of fewer warps than the device has SMs -- a
-  // few long passes: the widest rows, the longest patterns -- take a side stream each, so
-  // that no bucket queues behind their long run; the others go round robin over the main
-  // streams in launch order, so that their tails overlap.  Measured on 100,000 uneven pairs:
-  // 87.5 -> 86.8 ms an execute; every bucket on a stream of its own (16 or 32 streams) took
-  // 106-112 ms, the long passes then starting late among the other kernels' blocks.
-  int nmain = 0, nside = 0;
-  for (auto& b : P->buckets) {
-    if ((int64_t)b.grid * (b.block / 32) < ctx->sms && nside < sf_context::kSide)
-      b.stream = sf_context::kMain + nside++;
-    else
-      b.stream = nmain++ % sf_context::kMain;
+  // Launches, in the order of their first buckets: the Myers and the anti-diagonal buckets that
+  // differ only in the lanes a pair takes are one launch over all their tasks, longest bucket
+  // first, so that a batch of many lengths is a few kernels and not one for each length.
+  P->groups.clear();
+  S.tasks.clear();
+  auto merges = [](const Bucket& x, const Bucket& y) {
+    if (x.kind != y.kind) return false;
+    if (x.kind == PK_WAVE16) return sfk::kWave[x.c].q == sfk::kWave[y.c].q && x.tb == y.tb;
+    return x.c == y.c && (x.lanes > 32 ? x.lanes == y.lanes : y.lanes <= 32);
+  };
+  std::vector<uint8_t> done(nb, 0);
+  for (size_t u = 0; u < nb; ++u) {
+    if (done[u]) continue;
+    Bucket& b = P->buckets[u];
+    Group g;
+    g.bucket = (uint32_t)u;
+    g.grid = b.grid;
+    g.block = b.block;
+    if (b.kind == PK_MYERS || b.kind == PK_WAVE16) {
+      g.task_first = (uint32_t)S.tasks.size();
+      for (size_t v = u; v < nb; ++v) {
+        Bucket& x = P->buckets[v];
+        if (done[v] || !merges(b, x)) continue;
+        done[v] = 1;
+        x.task_first = (uint32_t)S.tasks.size();
+        const uint32_t lanes = (uint32_t)(x.kind == PK_MYERS ? x.lanes : sfk::kWave[x.c].lanes);
+        for (uint32_t t = 0; t < x.task_count; ++t) {
+          const uint32_t at = t * (uint32_t)x.per_warp;
+          S.tasks.push_back(make_uint2(
+              x.first + at, lanes | std::min<uint32_t>((uint32_t)x.per_warp, x.count - at) << 8));
+        }
+      }
+      g.task_count = (uint32_t)S.tasks.size() - g.task_first;
+      g.grid = warps_grid((uint64_t)g.task_count * (b.kind == PK_MYERS && b.lanes > 32 ? b.lanes / 32 : 1),
+                          g.block);
+    }
+    g.stream = (int)(P->groups.size() % sf_context::kAux);
+    P->groups.push_back(g);
   }
 }
 
@@ -1104,6 +1158,7 @@ int upload_plan(sf_plan* P, BuildScratch& S) {
   const auto& mj = S.mj;
   const auto& wlist = S.wlist;
   const auto& order = S.order;
+  const auto& tasks = S.tasks;
   const auto& chains = S.chains;
   const auto& links = S.links;
   const auto& want = S.want;
@@ -1128,6 +1183,7 @@ int upload_plan(sf_plan* P, BuildScratch& S) {
   if ((rc = P->d_offs.ensure(wlist.size() * 8 + 64))) return rc;
   if ((rc = P->d_total.ensure(64))) return rc;
   if ((rc = P->d_order.ensure(order.size() * 4 + 64))) return rc;
+  if ((rc = P->d_tasks.ensure(tasks.size() * sizeof(uint2) + 64))) return rc;
   if ((rc = P->d_counters.ensure(P->buckets.size() * 4 + 64))) return rc;
   if ((rc = P->d_wlist.ensure(wlist.size() * 4 + 64))) return rc;
   if ((rc = P->d_scratch.ensure(scratch_total * 4 + 64))) return rc;
@@ -1167,6 +1223,7 @@ int upload_plan(sf_plan* P, BuildScratch& S) {
   put(P->d_cls, {{cls.data(), cls.size() * 2}});
   put(P->d_mjobs, {{mj.data(), mj.size() * sizeof(MJob)}});
   put(P->d_order, {{order.data(), order.size() * 4}});
+  put(P->d_tasks, {{tasks.data(), tasks.size() * sizeof(uint2)}});
   put(P->d_wlist, {{wlist.data(), wlist.size() * 4}});
   put(P->d_chains, {{chains.data(), chains.size() * sizeof(DChain)}});
   put(P->d_links, {{links.data(), links.size() * sizeof(DLink)}});
@@ -1292,9 +1349,9 @@ int mark_stage(std::vector<cudaEvent_t>* evs, cudaStream_t s) {
   return SF_OK;
 }
 
-// The first part of an execute: the pack on `s`, then the buckets, fanned out over the
-// auxiliary streams so that their tails overlap (each bucket on its stream, the main ones
-// rotated by `soff`; also a single bucket with `fan_one`).  `used` collects the auxiliary
+// The first part of an execute: the pack on `s`, then the launches, fanned out over the
+// auxiliary streams so that their tails overlap (each on its stream, rotated by `soff`; also
+// a single one with `fan_one`).  `used` collects the auxiliary
 // streams launched on.
 // With `evs`, everything runs in order on `s` with an event after each stage.
 int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* evs, int soff,
@@ -1318,38 +1375,45 @@ int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* ev
     launches += nseq ? 1 : 0;
   }
   if ((mrc = mark_stage(evs, s))) return mrc;
-  const int nb = (int)P->buckets.size();
+  // Timed stages run bucket by bucket, in order; otherwise one launch a group.
+  const int nb = (int)(evs ? P->buckets.size() : P->groups.size());
   const bool fan = !evs && (nb > 1 || (fan_one && nb == 1));
   bool mine[sf_context::kAux] = {};
   if (fan) CK(cudaEventRecord(ctx->fork, s));
   for (int q = 0; q < nb; ++q) {
-    const Bucket& b = P->buckets[q];
+    const Bucket& b = P->buckets[evs ? (uint32_t)q : P->groups[q].bucket];
+    const uint32_t task_first = evs ? b.task_first : P->groups[q].task_first;
+    const uint32_t task_count = evs ? b.task_count : P->groups[q].task_count;
+    const int grid = evs ? b.grid : P->groups[q].grid;
     cudaStream_t bs = s;
     if (fan) {
-      const int si = b.stream < sf_context::kMain ? (b.stream + soff) % sf_context::kMain : b.stream;
+      const int si = (P->groups[q].stream + soff) % sf_context::kAux;
       bs = ctx->aux[si];
       if (!mine[si]) CK(cudaStreamWaitEvent(bs, ctx->fork, 0));
       mine[si] = used[si] = true;
     }
     uint32_t* counter = P->d_counters.as<uint32_t>() + q;
     const uint32_t* order = P->d_order.as<uint32_t>() + b.first;
+    const uint2* tasks = P->d_tasks.as<uint2>() + task_first;
     if (b.kind == PK_MYERS) {
       sfk::MyersLaunch ml;
       ml.jobs = P->d_mjobs.as<MJob>();
-      ml.order = order;
-      ml.njobs = b.count;
+      ml.order = P->d_order.as<uint32_t>();
+      ml.tasks = tasks;
+      ml.ntasks = task_count;
       ml.counter = counter;
       ml.pool = P->d_pool.as<uint32_t>();
       ml.out = P->d_mout.as<uint32_t>();
-      ml.lanes = b.lanes;
+      ml.team = b.lanes > 32 ? 1 : 0;
       ml.kcut = P->myers_kcut ? 1 : 0;
-      CK(sfk::launch_myers(b.c, ml, b.grid, b.block, bs));
+      CK(sfk::launch_myers(b.c, ml, grid, b.block, bs));
     } else {
       sfk::AffLaunch al;
       al.jobs = P->d_djobs.as<DJob>();
       al.params = P->d_params.as<DParams>();
       al.order = order;
       al.njobs = b.count;
+      al.tasks = nullptr;
       al.counter = counter;
       al.pool = P->d_pool.as<uint32_t>();
       al.bytes = plan_dev_bytes(P);
@@ -1364,18 +1428,22 @@ int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* ev
       al.links = P->d_links.as<DLink>();
       al.want = P->d_want.as<uint32_t>();
       al.snap = P->d_snap.as<uint32_t>();
-      if (b.kind == PK_WAVE16)
-        CK(sfk::launch_wave16(b.c, b.tb, al, b.per_warp, b.grid, bs));
-      else if (b.kind == PK_CHAIN16)
+      if (b.kind == PK_WAVE16) {
+        al.order = P->d_order.as<uint32_t>();
+        al.tasks = tasks;
+        al.njobs = task_count;
+        CK(sfk::launch_wave16(sfk::kWave[b.c].q, b.tb, al, grid, bs));
+      } else if (b.kind == PK_CHAIN16) {
         CK(sfk::launch_affine16_chain(b.c, al, b.grid, b.block, bs));
-      else if (b.kind == PK_AFFINE16 && b.lanes == 64)
+      } else if (b.kind == PK_AFFINE16 && b.lanes == 64) {
         CK(sfk::launch_affine16w(b.c, b.tb, al, b.grid, b.block, bs));
-      else if (b.kind == PK_AFFINE16 && b.lanes == 16)
+      } else if (b.kind == PK_AFFINE16 && b.lanes == 16) {
         CK(sfk::launch_affine16h(b.c, b.tb, al, b.grid, b.block, bs));
-      else if (b.kind == PK_AFFINE16)
+      } else if (b.kind == PK_AFFINE16) {
         CK(sfk::launch_affine16(b.c, b.tb, al, b.grid, b.block, bs));
-      else
+      } else {
         CK(sfk::launch_affine(b.c, b.wide, b.tb, b.kind == PK_LOCAL, al, b.grid, b.block, bs));
+      }
     }
     launches++;
     if ((mrc = mark_stage(evs, s))) return mrc;

@@ -32,8 +32,6 @@ __host__ __device__ constexpr int wave_blocks(int q, bool tb) {
   return tb ? (q <= 4 ? 6 : q <= 6 ? 5 : q <= 8 ? 4 : 3) : (q <= 6 ? 8 : q <= 8 ? 6 : q <= 10 ? 5 : 4);
 }
 
-// per_warp: passes a warp takes, at most 32 / L.
-cudaError_t launch_wave16(int cls, bool tb, const AffLaunch& a, int per_warp, int grid,
-                          cudaStream_t s);
+cudaError_t launch_wave16(int q, bool tb, const AffLaunch& a, int grid, cudaStream_t s);
 
 }  // namespace sfk

@@ -4,11 +4,11 @@
 
 namespace sfk {
 
-cudaError_t launch_wave16_4(bool, const AffLaunch&, int, int, int, cudaStream_t);
-cudaError_t launch_wave16_6(bool, const AffLaunch&, int, int, int, cudaStream_t);
-cudaError_t launch_wave16_8(bool, const AffLaunch&, int, int, int, cudaStream_t);
-cudaError_t launch_wave16_10(bool, const AffLaunch&, int, int, int, cudaStream_t);
-cudaError_t launch_wave16_12(bool, const AffLaunch&, int, int, int, cudaStream_t);
+cudaError_t launch_wave16_4(bool, const AffLaunch&, int, cudaStream_t);
+cudaError_t launch_wave16_6(bool, const AffLaunch&, int, cudaStream_t);
+cudaError_t launch_wave16_8(bool, const AffLaunch&, int, cudaStream_t);
+cudaError_t launch_wave16_10(bool, const AffLaunch&, int, cudaStream_t);
+cudaError_t launch_wave16_12(bool, const AffLaunch&, int, cudaStream_t);
 
 // Classes by the cells they hold.  The first kWaveN0 are the cheapest a band cell: a row step
 // costs a warp about 32 Q + 60 issue slots whatever it holds, so many lanes' worth of cells a
@@ -20,15 +20,13 @@ const WaveClass kWave[] = {
     {4, 8}, {4, 16}, {4, 32}, {6, 32}, {8, 32}, {10, 32}, {12, 32}};
 const int kWaveN = 31, kWaveN0 = 24;
 
-cudaError_t launch_wave16(int cls, bool tb, const AffLaunch& a, int per_warp, int grid,
-                          cudaStream_t s) {
-  const int lanes = kWave[cls].lanes;
-  switch (kWave[cls].q) {
-    case 4: return launch_wave16_4(tb, a, lanes, per_warp, grid, s);
-    case 6: return launch_wave16_6(tb, a, lanes, per_warp, grid, s);
-    case 8: return launch_wave16_8(tb, a, lanes, per_warp, grid, s);
-    case 10: return launch_wave16_10(tb, a, lanes, per_warp, grid, s);
-    case 12: return launch_wave16_12(tb, a, lanes, per_warp, grid, s);
+cudaError_t launch_wave16(int q, bool tb, const AffLaunch& a, int grid, cudaStream_t s) {
+  switch (q) {
+    case 4: return launch_wave16_4(tb, a, grid, s);
+    case 6: return launch_wave16_6(tb, a, grid, s);
+    case 8: return launch_wave16_8(tb, a, grid, s);
+    case 10: return launch_wave16_10(tb, a, grid, s);
+    case 12: return launch_wave16_12(tb, a, grid, s);
     default: return cudaErrorInvalidValue;
   }
 }

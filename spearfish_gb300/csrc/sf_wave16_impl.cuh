@@ -453,17 +453,17 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
 }
 
 template <int Q, bool TB>
-__global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB)) wave16_kernel(sfk::AffLaunch a, int L,
-                                                                           int np) {
-  const int lane = threadIdx.x & 31, seg = lane / L;
+__global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB)) wave16_kernel(sfk::AffLaunch a) {
+  const int lane = threadIdx.x & 31;
   for (;;) {
     uint32_t q = 0;
-    if (lane == 0) q = atomicAdd(a.counter, (uint32_t)np);
+    if (lane == 0) q = atomicAdd(a.counter, 1u);
     q = __shfl_sync(FULL, q, 0);
     if (q >= a.njobs) break;
-    const uint32_t mine = q + (uint32_t)seg;
-    const bool has = seg < np && mine < a.njobs;
-    wave_passes<Q, TB>(a, a.order[has ? mine : q], has, L, np, lane, seg);
+    const uint2 task = a.tasks[q];
+    const int L = (int)(task.y & 0xffu), np = (int)(task.y >> 8), seg = lane / L;
+    const bool has = seg < np;
+    wave_passes<Q, TB>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, np, lane, seg);
   }
 }
 
@@ -472,12 +472,11 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB)) wave16_kernel(sf
 namespace sfk {
 
 template <int Q>
-cudaError_t launch_wave16_q(bool tb, const AffLaunch& a, int lanes, int per_warp, int grid,
-                            cudaStream_t s) {
+cudaError_t launch_wave16_q(bool tb, const AffLaunch& a, int grid, cudaStream_t s) {
   if (tb)
-    wave16_kernel<Q, true><<<grid, 128, 0, s>>>(a, lanes, per_warp);
+    wave16_kernel<Q, true><<<grid, 128, 0, s>>>(a);
   else
-    wave16_kernel<Q, false><<<grid, 128, 0, s>>>(a, lanes, per_warp);
+    wave16_kernel<Q, false><<<grid, 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 

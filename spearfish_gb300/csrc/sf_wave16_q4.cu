@@ -2,8 +2,7 @@
 #include "sf_wave16_impl.cuh"
 
 namespace sfk {
-cudaError_t launch_wave16_4(bool tb, const AffLaunch& a, int lanes, int per_warp, int grid,
-                             cudaStream_t s) {
-  return launch_wave16_q<4>(tb, a, lanes, per_warp, grid, s);
+cudaError_t launch_wave16_4(bool tb, const AffLaunch& a, int grid, cudaStream_t s) {
+  return launch_wave16_q<4>(tb, a, grid, s);
 }
 }  // namespace sfk
