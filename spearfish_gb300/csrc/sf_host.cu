@@ -192,9 +192,10 @@ void link_sorted(std::vector<Pass>& ps, size_t q0, size_t count, F text) {
 // from its passes' whole-pass results res(u) (every result equals the separate pass's).  A
 // pass takes the previous text's result when that pass read nothing the two texts differ in
 // (with clip) or stopped within the rows they share, and counts nothing; else it counts the
-// rows after its resume row.
+// rows after its resume row.  Adds to `cells` and `rows`.
 template <class R>
-void count_sorted(const std::vector<Pass>& ps, size_t q0, size_t count, R res) {
+void count_sorted(const std::vector<Pass>& ps, size_t q0, size_t count, R res, uint64_t& cells,
+                  uint64_t& rows) {
   const bool full = count && (ps[q0].mode == SF_INFIX || ps[q0].band == SF_NOLIMIT);
   size_t src = q0;  // the pass whose result the previous text took
   for (size_t k = 0; k < count; ++k) {
@@ -210,8 +211,8 @@ void count_sorted(const std::vector<Pass>& ps, size_t q0, size_t count, R res) {
     const DRes& d = res(src);
     uint32_t flags = 0;
     const DJob j = make_djob(p, flags);
-    g_dp_rows += d.rows - p.resume;
-    g_dp_cells += d.cells - band_cells(p.resume, j.below, j.above, p.n);
+    rows += d.rows - p.resume;
+    cells += d.cells - band_cells(p.resume, j.below, j.above, p.n);
   }
 }
 
@@ -390,7 +391,7 @@ int sf_affine_sorted(const uint8_t* pattern, uint64_t m, const uint8_t* const* t
   std::vector<DRes> r;
   int rc = run_passes(ps, g, &r, nullptr, nullptr, nullptr, nullptr);
   if (rc) return rc;
-  count_sorted(ps, 0, count, [&](size_t u) -> const DRes& { return r[u]; });
+  count_sorted(ps, 0, count, [&](size_t u) -> const DRes& { return r[u]; }, g_dp_cells, g_dp_rows);
   for (uint64_t q = 0; q < count; ++q) out[q] = r[q].score;
   return SF_OK;
 }
@@ -423,7 +424,7 @@ int sf_affine_extend_sorted_cut_bonus(const uint8_t* pattern, uint64_t m,
   std::vector<DRes> r;
   int rc = run_passes(ps, g, &r, nullptr, nullptr, nullptr, nullptr);
   if (rc) return rc;
-  count_sorted(ps, 0, count, [&](size_t u) -> const DRes& { return r[u]; });
+  count_sorted(ps, 0, count, [&](size_t u) -> const DRes& { return r[u]; }, g_dp_cells, g_dp_rows);
   for (uint64_t q = 0; q < count; ++q) {
     // align.rs:929-948
     const DRes& d = r[q];
@@ -790,54 +791,76 @@ int sf_extend_ends_batch(sf_context* ctx, const uint8_t* pool, uint64_t pool_byt
   const sf_store* store = ctx->store;
   // lib.rs:2021: the transcript flank searched: the read flank plus pad + flank / pad_div.
   auto window = [&](uint32_t x) { return (uint64_t)x + e->pad + x / e->pad_div; };
-  std::vector<Pass> ps;
-  std::vector<std::pair<uint64_t, int>> slot;  // (hit, 0 left / 1 right) per pass
-  for (uint64_t q = 0; q < n; ++q) {
-    const sf_hit_t& h = hits[q];
-    if (h.read_off > pool_bytes || h.read_len > pool_bytes - h.read_off)
-      return fail(SF_ERR_INVALID, "read outside the pool");
+  // Each hit's passes in hit order, the left one first: counted per chunk of hits, then written.
+  auto bad_hit = [&](const sf_hit_t& h) -> const char* {
+    if (h.read_off > pool_bytes || h.read_len > pool_bytes - h.read_off) return "read outside the pool";
     if (h.tx_start > store->bases || h.tx_len > store->bases - h.tx_start)
-      return fail(SF_ERR_INVALID, "transcript outside the store");
+      return "transcript outside the store";
     if (h.qstart > h.qend || h.qend > h.read_len || h.tstart > h.tend || h.tend > h.tx_len)
-      return fail(SF_ERR_INVALID, "bad hit span");
-    Pass p;
-    p.kind = PK_AFFINE;
-    p.mode = SF_PREFIX;
-    p.band = e->band;
-    p.clip = true;
-    p.cell = true;
-    p.xdrop = e->xdrop;
-    p.end_bonus = e->end_bonus;
-    p.tb_kind = 1;
-    p.sc = e->sc;
-    if (h.qstart > 0 && h.tstart > 0) {
-      // lib.rs:2022-2031: the read prefix and the transcript flank before tstart, backwards.
-      const uint64_t w = window(h.qstart);
-      const uint64_t lo = h.tstart > w ? h.tstart - w : 0;
-      Pass L = p;
-      L.p_off = kRevFlag | h.read_off;
-      L.m = h.qstart;
-      L.t_off = kStoreFlag | kRevFlag | (h.tx_start + lo + kStorePad);
-      L.n = (uint32_t)(h.tstart - lo);
-      L.geom = std::max<uint64_t>(w, L.n);
-      ps.push_back(L);
-      slot.push_back({q, 0});
+      return "bad hit span";
+    return nullptr;
+  };
+  auto goes_left = [](const sf_hit_t& h) { return h.qstart > 0 && h.tstart > 0; };
+  auto goes_right = [](const sf_hit_t& h) { return h.read_len > h.qend && h.tend < h.tx_len; };
+  constexpr int kT = 16;
+  uint64_t first_bad[kT], cnt[kT + 1] = {};
+  std::fill(first_bad, first_bad + kT, UINT64_MAX);
+  parallel_chunks(n, 2048, kT, [&](size_t q0, size_t q1, int k) {
+    for (size_t q = q0; q < q1; ++q) {
+      if (bad_hit(hits[q])) {
+        first_bad[k] = q;
+        return;
+      }
+      cnt[k + 1] += goes_left(hits[q]) + goes_right(hits[q]);
     }
-    const uint32_t rest = h.read_len - h.qend;
-    if (rest > 0 && h.tend < h.tx_len) {
-      // lib.rs:2046-2073: the read suffix and the flank after tend, cut at the transcript's end.
-      const uint64_t w = window(rest);
-      const uint64_t hi = std::min<uint64_t>(h.tend + w, h.tx_len);
-      Pass R = p;
-      R.p_off = h.read_off + h.qend;
-      R.m = rest;
-      R.t_off = kStoreFlag | (h.tx_start + h.tend + kStorePad);
-      R.n = (uint32_t)(hi - h.tend);
-      R.geom = std::max<uint64_t>(w, R.n);
-      ps.push_back(R);
-      slot.push_back({q, 1});
+  });
+  const uint64_t bad = *std::min_element(first_bad, first_bad + kT);
+  if (bad != UINT64_MAX) return fail(SF_ERR_INVALID, bad_hit(hits[bad]));
+  for (int k = 0; k < kT; ++k) cnt[k + 1] += cnt[k];
+  std::vector<Pass> ps(cnt[kT]);
+  std::vector<std::pair<uint64_t, int>> slot(cnt[kT]);  // (hit, 0 left / 1 right) per pass
+  parallel_chunks(n, 2048, kT, [&](size_t q0, size_t q1, int k) {
+    uint64_t at = cnt[k];
+    for (size_t q = q0; q < q1; ++q) {
+      const sf_hit_t& h = hits[q];
+      Pass p;
+      p.kind = PK_AFFINE;
+      p.mode = SF_PREFIX;
+      p.band = e->band;
+      p.clip = true;
+      p.cell = true;
+      p.xdrop = e->xdrop;
+      p.end_bonus = e->end_bonus;
+      p.tb_kind = 1;
+      p.sc = e->sc;
+      if (goes_left(h)) {
+        // lib.rs:2022-2031: the read prefix and the transcript flank before tstart, backwards.
+        const uint64_t w = window(h.qstart);
+        const uint64_t lo = h.tstart > w ? h.tstart - w : 0;
+        Pass& L = ps[at] = p;
+        L.p_off = kRevFlag | h.read_off;
+        L.m = h.qstart;
+        L.t_off = kStoreFlag | kRevFlag | (h.tx_start + lo + kStorePad);
+        L.n = (uint32_t)(h.tstart - lo);
+        L.geom = std::max<uint64_t>(w, L.n);
+        slot[at++] = {q, 0};
+      }
+      if (goes_right(h)) {
+        // lib.rs:2046-2073: the read suffix and the flank after tend, cut at the transcript's
+        // end.
+        const uint32_t rest = h.read_len - h.qend;
+        const uint64_t w = window(rest);
+        const uint64_t hi = std::min<uint64_t>(h.tend + w, h.tx_len);
+        Pass& R = ps[at] = p;
+        R.p_off = h.read_off + h.qend;
+        R.m = rest;
+        R.t_off = kStoreFlag | (h.tx_start + h.tend + kStorePad);
+        R.n = (uint32_t)(hi - h.tend);
+        R.geom = std::max<uint64_t>(w, R.n);
+        slot[at++] = {q, 1};
+      }
     }
-  }
+  });
   if (ps.empty()) return SF_OK;
   if (!ctx->cache) {
     ctx->cache.reset(new sf_plan);
@@ -875,43 +898,72 @@ int sf_sorted_batch(sf_context* ctx, const uint8_t* pool, uint64_t pool_bytes,
   if (!ctx || (n_calls && !calls) || (n_texts && (!texts || !out)) || (pool_bytes && !pool) ||
       (n_scores && !scores))
     return fail(SF_ERR_INVALID, "bad argument");
-  std::vector<Pass> ps;
-  std::vector<uint64_t> text_of;
-  for (uint64_t c = 0; c < n_calls; ++c) {
-    const sf_sorted_call_t& k = calls[c];
+  // Every call checked, in call order: the error, and how many passes come before each call.
+  auto bad_call = [&](const sf_sorted_call_t& k, std::string& msg) -> int {
+    auto err = [&](int code, const char* m) {
+      msg = m;
+      return code;
+    };
     if (k.sc_index >= n_scores || !ok_sc(&scores[k.sc_index]))
-      return fail(SF_ERR_INVALID, "bad scoring index");
-    if (k.kind > SF_SORTED_EXTEND_CUT) return fail(SF_ERR_INVALID, "bad sorted call kind");
-    if (k.kind == SF_SORTED_AFFINE && !ok_mode((int)k.mode)) return fail(SF_ERR_INVALID, "bad mode");
+      return err(SF_ERR_INVALID, "bad scoring index");
+    if (k.kind > SF_SORTED_EXTEND_CUT) return err(SF_ERR_INVALID, "bad sorted call kind");
+    if (k.kind == SF_SORTED_AFFINE && !ok_mode((int)k.mode)) return err(SF_ERR_INVALID, "bad mode");
     if (k.first > n_texts || k.count > n_texts - k.first)
-      return fail(SF_ERR_INVALID, "call's texts outside the text list");
+      return err(SF_ERR_INVALID, "call's texts outside the text list");
     if (k.p_off > pool_bytes || k.m > pool_bytes - k.p_off)
-      return fail(SF_ERR_INVALID, "pattern outside the pool");
-    if (k.m >= 0x7fffffffu) return fail(SF_ERR_TOO_LONG, "sequence too long");
-    const sf_affine_t* sc = &scores[k.sc_index];
-    const size_t q0 = ps.size();
+      return err(SF_ERR_INVALID, "pattern outside the pool");
+    if (k.m >= 0x7fffffffu) return err(SF_ERR_TOO_LONG, "sequence too long");
     for (uint64_t q = 0; q < k.count; ++q) {
       const sf_span_t& t = texts[k.first + q];
       if (t.off > pool_bytes || t.len > pool_bytes - t.off)
-        return fail(SF_ERR_INVALID, "text outside the pool");
-      if (t.len >= 0x7fffffffu) return fail(SF_ERR_TOO_LONG, "sequence too long");
-      if (k.kind == SF_SORTED_AFFINE) {
-        // align.rs:854-861 `affine_sorted`: one Global/Prefix/Infix pass per text.
-        ps.push_back(affine_pass(k.p_off, k.m, t.off, t.len, (int)k.mode, sc, k.band));
-      } else {
-        // align.rs:903-949 `affine_extend_sorted_cut_bonus` (the passes of 917-928).
-        Pass p = affine_pass(k.p_off, k.m, t.off, t.len, SF_PREFIX, sc, k.band);
-        p.geom = k.diagonal ? std::min<uint64_t>(k.m, t.len) : std::max<uint64_t>(t.len, k.window);
-        p.clip = true;
-        p.xdrop = k.xdrop;
-        p.cell = k.track_cut && k.cut != SF_NOLIMIT;
-        p.cut = k.cut;
-        ps.push_back(p);
-      }
-      text_of.push_back(k.first + q);
+        return err(SF_ERR_INVALID, "text outside the pool");
+      if (t.len >= 0x7fffffffu) return err(SF_ERR_TOO_LONG, "sequence too long");
     }
-    link_sorted(ps, q0, k.count, [&](size_t u) { return pool + texts[text_of[u]].off; });
+    return SF_OK;
+  };
+  constexpr int kT = 16;
+  uint64_t first_bad[kT];
+  std::fill(first_bad, first_bad + kT, UINT64_MAX);
+  parallel_chunks(n_calls, 512, kT, [&](size_t c0, size_t c1, int k) {
+    std::string msg;
+    for (size_t c = c0; c < c1; ++c)
+      if (bad_call(calls[c], msg) != SF_OK) {
+        first_bad[k] = c;
+        return;
+      }
+  });
+  const uint64_t bad = *std::min_element(first_bad, first_bad + kT);
+  if (bad != UINT64_MAX) {
+    std::string msg;
+    const int code = bad_call(calls[bad], msg);
+    return fail(code, msg);
   }
+  std::vector<uint64_t> at(n_calls + 1, 0);
+  for (uint64_t c = 0; c < n_calls; ++c) at[c + 1] = at[c] + calls[c].count;
+  std::vector<Pass> ps(at[n_calls]);
+  parallel_chunks(n_calls, 512, kT, [&](size_t c0, size_t c1, int) {
+    for (size_t c = c0; c < c1; ++c) {
+      const sf_sorted_call_t& k = calls[c];
+      const sf_affine_t* sc = &scores[k.sc_index];
+      for (uint64_t q = 0; q < k.count; ++q) {
+        const sf_span_t& t = texts[k.first + q];
+        Pass& p = ps[at[c] + q];
+        if (k.kind == SF_SORTED_AFFINE) {
+          // align.rs:854-861 `affine_sorted`: one Global/Prefix/Infix pass per text.
+          p = affine_pass(k.p_off, k.m, t.off, t.len, (int)k.mode, sc, k.band);
+        } else {
+          // align.rs:903-949 `affine_extend_sorted_cut_bonus` (the passes of 917-928).
+          p = affine_pass(k.p_off, k.m, t.off, t.len, SF_PREFIX, sc, k.band);
+          p.geom = k.diagonal ? std::min<uint64_t>(k.m, t.len) : std::max<uint64_t>(t.len, k.window);
+          p.clip = true;
+          p.xdrop = k.xdrop;
+          p.cell = k.track_cut && k.cut != SF_NOLIMIT;
+          p.cut = k.cut;
+        }
+      }
+      link_sorted(ps, at[c], k.count, [&](size_t u) { return pool + texts[k.first + (u - at[c])].off; });
+    }
+  });
   if (ps.empty()) return SF_OK;
   if (!ctx->cache) {
     ctx->cache.reset(new sf_plan);
@@ -926,27 +978,38 @@ int sf_sorted_batch(sf_context* ctx, const uint8_t* pool, uint64_t pool_bytes,
   if ((rc = plan_execute(P, false))) return rc;
   if ((rc = plan_fetch(P))) return rc;
   const DRes* rs = P->h_res.as<DRes>();
-  size_t u = 0;
-  for (uint64_t c = 0; c < n_calls; ++c) {
-    const sf_sorted_call_t& k = calls[c];
-    count_sorted(P->passes, u, k.count, [&](size_t v) -> const DRes& { return rs[P->slot[v]]; });
-    for (uint64_t q = 0; q < k.count; ++q, ++u) {
-      const DRes& d = rs[P->slot[u]];
-      sf_cut_t& o = out[text_of[u]];
-      if (k.kind == SF_SORTED_AFFINE) {
-        // lib.rs:1442-1445: an affine_sorted score stands for whole and cut, no columns.
-        o.whole = o.cut = d.score;
-        o.cols = 0;
-        continue;
+  uint64_t cells[kT] = {}, rows[kT] = {};
+  // Calls whose texts overlap write one after another, as they stand.
+  bool apart = true;
+  for (uint64_t c = 1; c < n_calls; ++c)
+    apart = apart && calls[c].first >= calls[c - 1].first + calls[c - 1].count;
+  parallel_chunks(n_calls, 512, apart ? kT : 1, [&](size_t c0, size_t c1, int w) {
+    for (size_t c = c0; c < c1; ++c) {
+      const sf_sorted_call_t& k = calls[c];
+      count_sorted(P->passes, at[c], k.count, [&](size_t v) -> const DRes& { return rs[P->slot[v]]; },
+                   cells[w], rows[w]);
+      for (uint64_t q = 0; q < k.count; ++q) {
+        const DRes& d = rs[P->slot[at[c] + q]];
+        sf_cut_t& o = out[k.first + q];
+        if (k.kind == SF_SORTED_AFFINE) {
+          // lib.rs:1442-1445: an affine_sorted score stands for whole and cut, no columns.
+          o.whole = o.cut = d.score;
+          o.cols = 0;
+          continue;
+        }
+        // align.rs:929-948
+        const int32_t end = (k.bonus_within_cut && k.cut != SF_NOLIMIT)
+                                ? std::max(d.score, sat_add32(d.cut_score, k.end_bonus))
+                                : sat_add32(d.score, k.end_bonus);
+        o.whole = std::max(d.clip_best, end);
+        o.cols = d.clip_best >= end ? d.clip_j : d.score_col;
+        o.cut = k.cut == SF_NOLIMIT ? o.whole : std::max(d.cut_best, sat_add32(d.cut_score, k.end_bonus));
       }
-      // align.rs:929-948
-      const int32_t end = (k.bonus_within_cut && k.cut != SF_NOLIMIT)
-                              ? std::max(d.score, sat_add32(d.cut_score, k.end_bonus))
-                              : sat_add32(d.score, k.end_bonus);
-      o.whole = std::max(d.clip_best, end);
-      o.cols = d.clip_best >= end ? d.clip_j : d.score_col;
-      o.cut = k.cut == SF_NOLIMIT ? o.whole : std::max(d.cut_best, sat_add32(d.cut_score, k.end_bonus));
     }
+  });
+  for (int w = 0; w < kT; ++w) {
+    g_dp_cells += cells[w];
+    g_dp_rows += rows[w];
   }
   return SF_OK;
 }
