@@ -68,6 +68,15 @@ struct DevBuf {
   }
 };
 
+// An array in a device buffer.
+struct DevView {
+  void* p = nullptr;
+  template <class T>
+  T* as() const {
+    return static_cast<T*>(p);
+  }
+};
+
 struct PinBuf {
   void* p = nullptr;
   size_t cap = 0;
@@ -194,6 +203,7 @@ struct sf_plan {
   // Per pass: index in its kind's device arrays.
   std::vector<uint32_t> slot;
   uint32_t n_aff = 0, n_my = 0, n_walk = 0;
+  uint32_t n_tasks = 0;  // tasks of all launches (d_tasks: the tasks, then the job order)
   bool myers_kcut = false;  // a Myers pass is Global or Prefix with k < m + n
   std::vector<Bucket> buckets;
   std::vector<Group> groups;
@@ -201,9 +211,11 @@ struct sf_plan {
   int wide_warps = 0;
   std::string desc;
   // Device buffers.
-  DevBuf d_bytes, d_pool, d_seq, d_djobs, d_params, d_res, d_mjobs, d_mout, d_tjobs, d_tres,
-      d_tb, d_ops, d_opsc, d_offs, d_order, d_tasks, d_counters, d_wlist, d_cls, d_scratch, d_total,
-      d_chains, d_links, d_want, d_snap;
+  DevBuf d_bytes, d_pool, d_res, d_mout, d_tres, d_tb, d_ops, d_opsc, d_offs, d_counters, d_scratch,
+      d_total, d_snap;
+  // The descriptors: one buffer, one copy, and each array's place in it.
+  DevBuf d_desc;
+  sfe::DevView d_seq, d_djobs, d_params, d_mjobs, d_tjobs, d_tasks, d_wlist, d_chains, d_links, d_want;
   // Chains of sorted-call passes the plan runs on the chain kernel, their passes, and per
   // pass whether it is one of them.
   uint32_t n_chains = 0, n_chained = 0;

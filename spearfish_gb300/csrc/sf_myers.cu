@@ -104,18 +104,10 @@ __global__ void __launch_bounds__(128, B <= 2 ? 8 : (B == 3 ? 6 : 5)) myers_kern
                     (threadIdx.x >> 5) * (B * kBlockBytes) + lane * 8;
   char* eqw = const_cast<char*>(eqb);
 
-  for (;;) {
-    uint32_t q = 0;
-    if constexpr (TEAM) {
-      if (threadIdx.x == 0) X.task = atomicAdd(a.counter, 1u);
-      __syncthreads();
-      q = X.task;
-      __syncthreads();
-    } else {
-      if (lane == 0) q = atomicAdd(a.counter, 1u);
-      q = __shfl_sync(FULL, q, 0);
-    }
-    if (q >= a.ntasks) break;
+  // The first task by place; the queue hands out those after the grid's first ones.
+  const uint32_t grid_tasks = TEAM ? gridDim.x : (gridDim.x * blockDim.x) >> 5;
+  uint32_t q = TEAM ? blockIdx.x : __shfl_sync(FULL, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, 0);
+  for (bool more = q < a.ntasks; more;) {
     const uint2 task = a.tasks[q];
     const int P = TEAM ? 32 * W : (int)(task.y & 0xffu), np = TEAM ? 1 : (int)(task.y >> 8);
     const int seg = TEAM ? 0 : lane / P;
@@ -251,12 +243,13 @@ __global__ void __launch_bounds__(128, B <= 2 ? 8 : (B == 3 ? 6 : 5)) myers_kern
         acc = ch == 0 ? chunk(s, std::true_type{}) : chunk(s, std::false_type{});
       }
       bottom += __popc(acc.x) - __popc(acc.y);
-      // The pair's last lane holds the last row's deltas: columns s - last .. + 31.
-      const int own = TEAM ? 31 : min(seg * P + P - 1, 31);
+      // The pair's last lane holds the last row's deltas: columns s - last .. + 31, shared out
+      // over the pair's lanes (all of the warp's, if it is the only pair).
+      const int own = TEAM ? 31 : (np == 1 ? P - 1 : min(seg * P + P - 1, 31));
       const uint32_t op = __shfl_sync(FULL, acc.x, own), om = __shfl_sync(FULL, acc.y, own);
       if (!TEAM || w == W - 1) {
         const int c0 = s - last;
-        for (int t = TEAM ? lane : l; t < 32; t += TEAM ? 32 : P) {
+        for (int t = TEAM || np == 1 ? lane : l; t < 32; t += TEAM || np == 1 ? 32 : P) {
           const int c = c0 + t;
           if (c >= 0 && c < n && (!glob || c == n - 1))
             best = min(best, score + __popc(op >> (31 - t)) - __popc(om >> (31 - t)));
@@ -300,11 +293,14 @@ __global__ void __launch_bounds__(128, B <= 2 ? 8 : (B == 3 ? 6 : 5)) myers_kern
         if (m == 0 || n == 0) best = m == 0 ? (glob ? n : 0) : m;
         a.out[jid] = (uint32_t)best <= J.k ? (uint32_t)best : 0xffffffffu;
       }
-      __syncthreads();
     } else {
-      for (int t = 1; t < P; t <<= 1) {
-        const int o = __shfl_down_sync(FULL, best, t);
-        if (l + t < P) best = min(best, o);
+      if (np == 1) {
+        best = __reduce_min_sync(FULL, best);
+      } else {
+        for (int t = 1; t < P; t <<= 1) {
+          const int o = __shfl_down_sync(FULL, best, t);
+          if (l + t < P) best = min(best, o);
+        }
       }
       if (has && l == 0) {
         if (m == 0 || n == 0) best = m == 0 ? (glob ? n : 0) : m;
@@ -312,6 +308,17 @@ __global__ void __launch_bounds__(128, B <= 2 ? 8 : (B == 3 ? 6 : 5)) myers_kern
       }
       __syncwarp();
     }
+    if (a.ntasks <= grid_tasks) break;
+    if constexpr (TEAM) {
+      if (threadIdx.x == 0) X.task = grid_tasks + atomicAdd(a.counter, 1u);
+      __syncthreads();
+      q = X.task;
+      __syncthreads();
+    } else {
+      if (lane == 0) q = grid_tasks + atomicAdd(a.counter, 1u);
+      q = __shfl_sync(FULL, q, 0);
+    }
+    more = q < a.ntasks;
   }
 }
 

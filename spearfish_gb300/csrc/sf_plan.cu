@@ -324,7 +324,6 @@ struct BuildScratch {
   std::vector<DJob> dj;
   std::vector<DParams> dp;
   std::vector<TJob> tj;
-  std::vector<uint16_t> cls;
   std::vector<MJob> mj;
   std::vector<uint32_t> wlist, kid, order;
   std::vector<uint2> tasks;
@@ -490,7 +489,9 @@ int build_sequences(sf_plan* P, BuildScratch& S) {
       }
     });
   }
-  P->pool_words = words + 512;  // slack: kernels read whole windows past a sequence's end
+  // Slack: kernels read whole windows past a sequence's end.  No result depends on what stands
+  // there, after the last sequence as after the others.
+  P->pool_words = words + 512;
   return SF_OK;
 }
 
@@ -563,7 +564,6 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   auto& dj = S.dj;
   auto& dp = S.dp;
   auto& tj = S.tj;
-  auto& cls = S.cls;
   auto& mj = S.mj;
   // Slots in each kind's arrays, in pass order: each chunk's Myers passes counted, then the
   // slots written.  Myers classes are checked here, so that the parallel part below cannot
@@ -603,7 +603,6 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   dj.resize(n_affine);
   dp.resize(n_affine);
   tj.resize(n_affine);
-  cls.resize(n_affine);
   auto& pass_work = S.pass_work;
   auto& pass_lat = S.pass_lat;
   auto& tb_need = S.tb_need;
@@ -715,7 +714,6 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       dj[sl] = j;
       dp[sl] = pr;
       tj[sl] = t;
-      cls[sl] = (uint16_t)(c | (wide ? 0x100 : 0) | (kind == PK_AFFINE16 ? 0x200 : 0));
     }
   };
   parallel_chunks(np, 2048, kMaxThreads, describe);
@@ -1120,7 +1118,6 @@ int upload_plan(sf_plan* P, BuildScratch& S) {
   const auto& dj = S.dj;
   const auto& dp = S.dp;
   const auto& tj = S.tj;
-  const auto& cls = S.cls;
   const auto& mj = S.mj;
   const auto& wlist = S.wlist;
   const auto& order = S.order;
@@ -1134,51 +1131,36 @@ int upload_plan(sf_plan* P, BuildScratch& S) {
   if (!P->bytes_from && (rc = P->d_bytes.ensure(std::max<uint64_t>(P->pool_bytes, 16)))) return rc;
   if ((rc = P->d_pool.ensure(P->pool_words * 4))) return rc;
   const size_t nseq = P->seq_boff.size();
-  if ((rc = P->d_seq.ensure(nseq * 20 + 64))) return rc;
-  if ((rc = P->d_djobs.ensure(dj.size() * sizeof(DJob) + 64))) return rc;
-  if ((rc = P->d_params.ensure(dp.size() * sizeof(DParams) + 64))) return rc;
   if ((rc = P->d_res.ensure(dj.size() * sizeof(DRes) + 64))) return rc;
-  if ((rc = P->d_tjobs.ensure(tj.size() * sizeof(TJob) + 64))) return rc;
   if ((rc = P->d_tres.ensure(tj.size() * sizeof(TRes) + 64))) return rc;
-  if ((rc = P->d_cls.ensure(cls.size() * 2 + 64))) return rc;
-  if ((rc = P->d_mjobs.ensure(mj.size() * sizeof(MJob) + 64))) return rc;
   if ((rc = P->d_mout.ensure(mj.size() * 4 + 64))) return rc;
   if ((rc = P->d_tb.ensure(tb_words * 4 + 64))) return rc;
   if ((rc = P->d_ops.ensure(ops_words * 4 + 64))) return rc;
   if ((rc = P->d_opsc.ensure(ops_words * 4 + 64))) return rc;
   if ((rc = P->d_offs.ensure(wlist.size() * 8 + 64))) return rc;
   if ((rc = P->d_total.ensure(64))) return rc;
-  if ((rc = P->d_order.ensure(order.size() * 4 + 64))) return rc;
-  if ((rc = P->d_tasks.ensure(tasks.size() * sizeof(uint2) + 64))) return rc;
+  P->n_tasks = (uint32_t)tasks.size();
   if ((rc = P->d_counters.ensure(P->buckets.size() * 4 + 64))) return rc;
-  if ((rc = P->d_wlist.ensure(wlist.size() * 4 + 64))) return rc;
   if ((rc = P->d_scratch.ensure(scratch_total * 4 + 64))) return rc;
-  if ((rc = P->d_chains.ensure(chains.size() * sizeof(DChain) + 64))) return rc;
-  if ((rc = P->d_links.ensure(links.size() * sizeof(DLink) + 64))) return rc;
-  if ((rc = P->d_want.ensure(want.size() * 4 + 64))) return rc;
   if ((rc = P->d_snap.ensure(snap_words * 4 + 64))) return rc;
   // Descriptors -> device (one pinned staging area, one stream).  Every array goes into the
-  // staging (on host threads, in pieces), then one copy per device buffer.  The sequence
-  // table is byte offsets, word offsets (both 8-byte aligned), then lengths.
+  // staging (on host threads, in pieces) and all of it to the device in one copy: a small call
+  // spent 20 of its 90 us on a copy an array.  The sequence table is byte offsets, word offsets
+  // (both 8-byte aligned), then lengths.
   struct Part {
     const void* src;
     size_t bytes, at;
   };
-  struct Copy {
-    DevBuf* d;
-    size_t at, bytes;
-  };
   std::vector<Part> parts;
-  std::vector<Copy> copies;
+  std::vector<std::pair<DevView*, size_t>> views;
   size_t at = 0;
-  auto put = [&](DevBuf& d, std::initializer_list<std::pair<const void*, size_t>> srcs) {
+  auto put = [&](DevView& d, std::initializer_list<std::pair<const void*, size_t>> srcs) {
     size_t bytes = 0;
     for (const auto& sp : srcs) {
       if (sp.second) parts.push_back(Part{sp.first, sp.second, at + bytes});
       bytes += sp.second;
     }
-    if (!bytes) return;
-    copies.push_back(Copy{&d, at, bytes});
+    views.push_back({&d, at});
     at += (bytes + 15) & ~size_t(15);
   };
   put(P->d_seq, {{P->seq_boff.data(), nseq * 8}, {P->seq_woff.data(), nseq * 8},
@@ -1186,16 +1168,16 @@ int upload_plan(sf_plan* P, BuildScratch& S) {
   put(P->d_djobs, {{dj.data(), dj.size() * sizeof(DJob)}});
   put(P->d_params, {{dp.data(), dp.size() * sizeof(DParams)}});
   put(P->d_tjobs, {{tj.data(), tj.size() * sizeof(TJob)}});
-  put(P->d_cls, {{cls.data(), cls.size() * 2}});
   put(P->d_mjobs, {{mj.data(), mj.size() * sizeof(MJob)}});
-  put(P->d_order, {{order.data(), order.size() * 4}});
-  put(P->d_tasks, {{tasks.data(), tasks.size() * sizeof(uint2)}});
+  put(P->d_tasks, {{tasks.data(), tasks.size() * sizeof(uint2)}, {order.data(), order.size() * 4}});
   put(P->d_wlist, {{wlist.data(), wlist.size() * 4}});
   put(P->d_chains, {{chains.data(), chains.size() * sizeof(DChain)}});
   put(P->d_links, {{links.data(), links.size() * sizeof(DLink)}});
   put(P->d_want, {{want.data(), want.size() * 4}});
   if ((rc = stage_wait(P))) return rc;
   if ((rc = P->h_stage.ensure(at + 16))) return rc;
+  if ((rc = P->d_desc.ensure(at + 64))) return rc;
+  for (const auto& v : views) v.first->p = P->d_desc.as<uint8_t>() + v.second;
   uint8_t* h = P->h_stage.as<uint8_t>();
   {
     constexpr size_t kPiece = size_t(256) << 10;
@@ -1210,10 +1192,7 @@ int upload_plan(sf_plan* P, BuildScratch& S) {
       }
     });
   }
-  for (const Copy& c : copies)
-    CK(cudaMemcpyAsync(c.d->p, h + c.at, c.bytes, cudaMemcpyHostToDevice, ctx->s));
-  // The pool's slack words stay zero.
-  CK(cudaMemsetAsync(P->d_pool.p, 0, P->pool_words * 4, ctx->s));
+  if (at) CK(cudaMemcpyAsync(P->d_desc.p, h, at, cudaMemcpyHostToDevice, ctx->s));
   if ((rc = stage_done(P))) return rc;
   if (P->graph) {
     cudaGraphExecDestroy(P->graph);
@@ -1359,12 +1338,13 @@ int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* ev
       mine[si] = used[si] = true;
     }
     uint32_t* counter = P->d_counters.as<uint32_t>() + q;
-    const uint32_t* order = P->d_order.as<uint32_t>() + b.first;
+    const uint32_t* orders = reinterpret_cast<const uint32_t*>(P->d_tasks.as<uint2>() + P->n_tasks);
+    const uint32_t* order = orders + b.first;
     const uint2* tasks = P->d_tasks.as<uint2>() + task_first;
     if (b.kind == PK_MYERS) {
       sfk::MyersLaunch ml;
       ml.jobs = P->d_mjobs.as<MJob>();
-      ml.order = P->d_order.as<uint32_t>();
+      ml.order = orders;
       ml.tasks = tasks;
       ml.ntasks = task_count;
       ml.counter = counter;
@@ -1395,7 +1375,7 @@ int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* ev
       al.want = P->d_want.as<uint32_t>();
       al.snap = P->d_snap.as<uint32_t>();
       if (b.kind == PK_WAVE16) {
-        al.order = P->d_order.as<uint32_t>();
+        al.order = orders;
         al.tasks = tasks;
         al.njobs = task_count;
         CK(sfk::launch_wave16(sfk::kWave[b.c].q, b.tb, al, grid, bs));
@@ -1700,10 +1680,9 @@ int plan_results(sf_plan* P, sf_result_t* results, uint32_t* ops, uint64_t ops_c
 }
 
 uint64_t plan_bytes_held(const sf_plan* P) {
-  const DevBuf* bufs[] = {&P->d_bytes, &P->d_pool, &P->d_seq, &P->d_djobs, &P->d_params,
-                          &P->d_res, &P->d_mjobs, &P->d_mout, &P->d_tjobs, &P->d_tres,
-                          &P->d_tb, &P->d_ops, &P->d_opsc, &P->d_offs, &P->d_order,
-                          &P->d_counters, &P->d_wlist, &P->d_cls, &P->d_scratch, &P->d_total};
+  const DevBuf* bufs[] = {&P->d_bytes, &P->d_pool, &P->d_desc, &P->d_res, &P->d_mout, &P->d_tres,
+                          &P->d_tb, &P->d_ops, &P->d_opsc, &P->d_offs, &P->d_counters,
+                          &P->d_scratch, &P->d_total, &P->d_snap};
   uint64_t b = 0;
   for (const DevBuf* d : bufs) b += d->cap;
   return b;

@@ -455,15 +455,19 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
 template <int Q, bool TB>
 __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB)) wave16_kernel(sfk::AffLaunch a) {
   const int lane = threadIdx.x & 31;
-  for (;;) {
-    uint32_t q = 0;
-    if (lane == 0) q = atomicAdd(a.counter, 1u);
-    q = __shfl_sync(FULL, q, 0);
-    if (q >= a.njobs) break;
+  // The first task by place; the queue hands out those after the grid's first ones.
+  const uint32_t grid_tasks = (gridDim.x * blockDim.x) >> 5;
+  // (Every q is a shuffle's: the compiler then keeps what follows from it in uniform registers.)
+  uint32_t q = __shfl_sync(FULL, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, 0);
+  while (q < a.njobs) {
     const uint2 task = a.tasks[q];
     const int L = (int)(task.y & 0xffu), np = (int)(task.y >> 8), seg = lane / L;
     const bool has = seg < np;
     wave_passes<Q, TB>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, np, lane, seg);
+    if (a.njobs <= grid_tasks) break;
+    uint32_t next = 0;
+    if (lane == 0) next = atomicAdd(a.counter, 1u);
+    q = __shfl_sync(FULL, grid_tasks + next, 0);
   }
 }
 
