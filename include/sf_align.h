@@ -29,8 +29,10 @@
  * Environment (read when a plan is built; results never depend on them)
  *  - SF_AFFINE16=0: every affine pass on the 32-bit rows (no packed 16-bit
  *    rows).
- *  - SF_AFFINE16_LANES=16: 16-bit passes on half warps by default (the
- *    autotuner chooses per length bucket either way).
+ *  - SF_AFFINE16_LANES=32 (16, 64): every 16-bit pass on the row kernels,
+ *    one to a warp (two to a warp, one to two warps); the autotuner chooses
+ *    per length bucket either way.  Unset: Global and Prefix passes that fit
+ *    it run on the anti-diagonal kernel.
  *  - SF_SORTED_CHAINS=1: the sorted entry points run the passes that can
  *    share rows as chains (below, at sf_affine_sorted).
  *  - SF_BATCH_SEGMENTS=0: sf_batch_run builds every batch as one plan (no

@@ -107,15 +107,16 @@ struct PinBuf {
 // ---- passes ----------------------------------------------------------------------------
 
 // PK_AFFINE16, PK_CHAIN16 and PK_WAVE16 only classify buckets: an affine pass the packed 16-bit
-// row kernel runs, a chain of sorted-text passes it runs in order, and an affine pass the
-// anti-diagonal kernel runs (its class: an index into kWave).
+// row kernel runs, a chain of sorted-text passes it runs in order, and a Global or a Prefix pass
+// the anti-diagonal kernel runs (its class: an index into kWave).
 enum PassKind : uint8_t {
   PK_MYERS = 0,
   PK_AFFINE = 1,
   PK_LOCAL = 2,
   PK_AFFINE16 = 3,
   PK_CHAIN16 = 4,
-  PK_WAVE16 = 5
+  PK_WAVE16 = 5,
+  PK_WAVE16X = 6
 };
 
 // One DP pass as the reference's `affine_dp` / `distance` / `local_band_core` receive it.
@@ -338,6 +339,9 @@ int64_t wave_width(const DJob& j);
 // fastest, rather than the cheapest ones a cell.
 bool lean_plan(size_t np, int sms);
 bool plan_is_lean(const sf_plan* P);
+inline bool is_wave(int kind) { return kind == PK_WAVE16 || kind == PK_WAVE16X; }
+// Row steps of a pass on the anti-diagonal kernel.
+uint64_t wave_steps(const DJob& j, int kind);
 // A class as its reports show it: cells a lane and lanes a pass.
 int shown_c(int kind, int c);
 int shown_lanes(int kind, int c, int lanes);

@@ -1252,11 +1252,11 @@ std::vector<ClassChoice> tune_candidates(const ClassKey& key, int64_t blocks) {
         for (const auto& c : out) dup = dup || (c.c == b && c.lanes == lanes);
         if (!dup) out.push_back(ClassChoice{b, lanes});
       }
-  } else if (key.kind == PK_WAVE16) {
+  } else if (is_wave(key.kind)) {
     // The next classes that hold all the default class does (later plans' passes of it too).
     for (int c = 0; c < sfk::kWaveN; ++c)
       if (c != key.c && sfk::wave_cap(sfk::kWave[c]) >= sfk::wave_cap(sfk::kWave[key.c]) &&
-          (int)out.size() < 4 &&
+          (int)out.size() < 4 && (key.kind == PK_WAVE16 || sfk::kWave[c].q <= sfk::kWaveMaxX) &&
           (c > key.c || key.c >= sfk::kWaveN0))
         out.push_back(ClassChoice{c, key.lanes});
   } else if (!key.wide) {
@@ -1381,8 +1381,9 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
                   key.kind == PK_MYERS ? "myers"
                                        : (key.kind == PK_LOCAL ? "local"
                                                                : (key.kind == PK_AFFINE16 ? "affine16"
-                                                                  : key.kind == PK_WAVE16 ? "wave16"
-                                                                                          : "affine")),
+                                                                  : key.kind == PK_WAVE16  ? "wave16"
+                                                                  : key.kind == PK_WAVE16X ? "wave16x"
+                                                                                           : "affine")),
                   shown_c(key.kind, key.c), key.wide ? "true" : "false", key.tb ? "true" : "false",
                   shown_lanes(key.kind, key.c, key.lanes), g.second.size(), shown_c(key.kind, best.c),
                   shown_lanes(key.kind, best.c, best.lanes));

@@ -90,26 +90,37 @@ bool fits16(const Pass& p, uint32_t flags, int64_t wmax) {
 // The band cells the anti-diagonal kernel lays out for a pass (its bl is odd).
 int64_t wave_width(const DJob& j) { return (j.below | 1) + j.above + 1; }
 
-// Whether a pass runs on the anti-diagonal kernel (sf_wave16_impl.cuh): a Global pass of a
-// finite band without clip or cut.  Its band edges rest on mis = 2 ext (a mismatch costs what
-// the two gap bases around it would extend for) and open >= 1.  Its fields hold four times the
-// value: the largest rises by (mat + 2 ext) a row step between rebases, and a band cell lies at
-// most (mat + 2 ext) * width / 2 + open below it (a gap from the best path, extension free in
-// the kernel's potential).  A band much wider than the text (or the pattern) is left to the
-// row kernels, whose rows stop at the text's end.
-bool fits_wave(const Pass& p, const DJob& j, uint32_t flags) {
-  if (p.kind != PK_AFFINE || (flags & (F_FULL | F_ROWMAX)) || p.mode != SF_GLOBAL) return false;
+// Row steps until a Global pass's cell (m, n), or a Prefix pass's last cell of row m, is done.
+uint64_t wave_steps(const DJob& j, int kind) {
+  if (kind == PK_WAVE16) return ((uint64_t)j.m + j.n + 1) / 2;
+  return (uint64_t)((int64_t)j.m + (wave_width(j) - 1) / 2 - (j.below | 1) / 2);
+}
+
+// Whether a pass runs on the anti-diagonal kernel (sf_wave16_impl.cuh), and as which kind: a
+// Global pass of a finite band without clip or cut, or a Prefix pass of one without cut.  Its
+// band edges rest on mis = 2 ext (a mismatch costs what the two gap bases around it would extend
+// for) and open >= 1.  Its fields hold four times the value: the largest rises by (mat + 2 ext) a
+// row step between rebases, and a band cell lies at most (mat + 2 ext) * width / 2 + open below it
+// (a gap from the best path, extension free in the kernel's potential); a Prefix pass's row
+// maxima rise by ext a cell across the band on either side of that.  A band much wider than the
+// text (or the pattern) is left to the row kernels, whose rows stop at the text's end.
+bool fits_wave(const Pass& p, const DJob& j, uint32_t flags, PassKind& kind) {
+  if (p.kind != PK_AFFINE || (flags & (F_FULL | F_CUT))) return false;
+  const bool prefix = p.mode == SF_PREFIX;
+  if (!prefix && (p.mode != SF_GLOBAL || (flags & F_ROWMAX))) return false;
   const sf_affine_t& s = p.sc;
   if (s.mat < 0 || s.mat > 1000 || s.ext < 0 || s.ext > 1000 || s.mis != 2 * s.ext) return false;
   if (s.open < 1 || s.open > 900) return false;
-  const int64_t w = wave_width(j);
-  if (p.m < 1 || p.n < 1 || w > 2 * ((int64_t)std::min(p.m, p.n) + 1)) return false;
-  if (w > sfk::wave_cap(sfk::kWave[sfk::kWaveN0 - 1])) return false;
+  const int64_t w = wave_width(j), shorter = std::min(p.m, p.n);
+  if (p.m < 1 || p.n < 1 || w > (prefix ? 4 * (shorter + 1) + 64 : 2 * (shorter + 1))) return false;
+  if (prefix && (int64_t)p.m > (int64_t)p.n + j.below) return false;  // ends past the text
+  if (w > sfk::wave_cap(sfk::kWave[prefix ? sfk::kWaveN - 1 : sfk::kWaveN0 - 1])) return false;
   const int64_t g = (int64_t)s.mat + 2 * s.ext;
   if (4 * g * (sfk::kWaveRebaseRows + 1) >
       std::min<int64_t>(0xffff - (int64_t)sfk::kWaveTop, sfk::kWaveNeg))
     return false;
-  return 4 * (g * (w / 2 + 2) + 2 * (int64_t)s.open + 16) <=
+  kind = prefix ? PK_WAVE16X : PK_WAVE16;
+  return 4 * (g * (w / 2 + 2) + 2 * (int64_t)s.open + 16) + (prefix ? 8 * (int64_t)s.ext * (w + 1) : 0) <=
          (int64_t)sfk::kWaveTop - (int64_t)sfk::kWaveNeg;
 }
 
@@ -126,9 +137,9 @@ int most_pairs(const sf_plan* P) {
   return (int)std::max<size_t>(1, std::min<size_t>(32, P->passes.size() / ((size_t)P->ctx->sms * 16)));
 }
 
-int shown_c(int kind, int c) { return kind == PK_WAVE16 ? 4 * sfk::kWave[c].q : c; }
+int shown_c(int kind, int c) { return is_wave(kind) ? 4 * sfk::kWave[c].q : c; }
 int shown_lanes(int kind, int c, int lanes) {
-  return kind == PK_WAVE16 ? sfk::kWave[c].lanes : lanes;
+  return is_wave(kind) ? sfk::kWave[c].lanes : lanes;
 }
 
 // SF_AFFINE16=0 in the environment turns the 16-bit kernels off (every pass then runs on the
@@ -138,14 +149,15 @@ bool allow16() {
   return !(env && env[0] == '0');
 }
 
-// Lanes per 16-bit row pass by default: 32 (with 64 for rows wider than 32 x 40 cells), or with
-// SF_AFFINE16_LANES in the environment 16 (two passes per warp) or 64 (two warps per pass,
-// every pass a 64-lane class holds), which also keeps every 16-bit pass on the row kernels;
-// the autotuner chooses per length bucket either way.
+// SF_AFFINE16_LANES in the environment keeps every 16-bit pass on the row kernels, with 32
+// lanes a pass (and 64 for rows wider than 32 x 40 cells), 16 (two passes per warp) or 64 (two
+// warps per pass, every pass a 64-lane class holds).  Unset (0): the anti-diagonal kernel where
+// a pass fits it, else 32; the autotuner chooses per length bucket either way.
 int default_lanes16() {
   const char* env = std::getenv("SF_AFFINE16_LANES");
-  if (env && env[0] == '1' && env[1] == '6') return 16;
-  if (env && env[0] == '6' && env[1] == '4') return 64;
+  if (!env || !env[0]) return 0;
+  if (env[0] == '1' && env[1] == '6') return 16;
+  if (env[0] == '6' && env[1] == '4') return 64;
   return 32;
 }
 
@@ -185,10 +197,9 @@ void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax,
                      bool lean, PassKind& kind, int& c, bool& wide, int& lanes, int lanes16) {
   wide = false;
   lanes = 32;
-  if (use16 && lanes16 == 32 && fits_wave(p, j, flags)) {
+  if (use16 && lanes16 == 0 && fits_wave(p, j, flags, kind)) {
     const int64_t w = wave_width(j);
-    kind = PK_WAVE16;
-    for (c = lean ? sfk::kWaveN0 : 0; sfk::wave_cap(sfk::kWave[c]) < w; ++c) {
+    for (c = lean ? sfk::kWaveN0 : (kind == PK_WAVE16X ? sfk::kWaveX0 : 0); sfk::wave_cap(sfk::kWave[c]) < w; ++c) {
     }
     return;
   }
@@ -679,8 +690,8 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       if (tb) {
         flags |= F_TB;
         const int64_t chunks = wide ? wide_chunks(c, wmax) : 1;
-        tb_need[sl] = kind == PK_WAVE16
-                          ? sfk::wave_tb_words(sfk::kWave[c], ((uint64_t)p.m + p.n + 1) / 2)
+        tb_need[sl] = is_wave(kind)
+                          ? sfk::wave_tb_words(sfk::kWave[c], wave_steps(j, kind))
                           : (uint64_t)p.m * (tb_row_words(c, chunks) * (uint64_t)ln / 32);
         const uint64_t cap = (uint64_t)p.m + p.n + 2;
         ops_need[sl] = cap;
@@ -705,7 +716,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       const uint64_t work = (uint64_t)std::max<uint32_t>(p.m, 1) * (uint64_t)std::max<int64_t>(wmax, 1);
       pass_work[q] = work;
       // Anti-diagonal row steps: about (60 + 32 Q) / 45 of this unit (a row's 45 cycles).
-      const uint64_t row_cost = kind == PK_WAVE16
+      const uint64_t row_cost = is_wave(kind)
                                     ? 2u + (uint64_t)(2 * sfk::kWave[c].q / 3)
                                     : (uint64_t)c * (wide ? (uint64_t)wide_chunks(c, wmax) : 1u) + 8u;
       pass_lat[q] = (uint64_t)std::max<uint32_t>(p.m, 1) * row_cost;
@@ -1042,13 +1053,13 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
         1, std::min<uint64_t>((warps + wpb - 1) / wpb, (uint64_t)ctx->sms * (2048 / block)));
   };
   for (auto& b : P->buckets) {
-    if (b.kind == PK_MYERS || b.kind == PK_WAVE16) {
+    if (b.kind == PK_MYERS || is_wave(b.kind)) {
       // As many pairs a warp as its lanes hold; in the fast classes fewer, while that leaves
       // schedulers empty.
       const bool my = b.kind == PK_MYERS;
       const int64_t most =
           my ? std::min(most_pairs(P), std::max(1, 32 / b.lanes)) : 32 / sfk::kWave[b.c].lanes;
-      const bool fast = my ? lean : b.c >= sfk::kWaveN0;
+      const bool fast = my ? lean : b.c >= sfk::kWaveN0 && b.c < sfk::kWaveX0;
       b.per_warp = (int)(!fast ? most
                                : std::max<int64_t>(1, std::min<int64_t>(most, b.count / (4 * (int64_t)ctx->sms))));
       b.task_count = (b.count + b.per_warp - 1) / b.per_warp;
@@ -1078,7 +1089,7 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
   S.tasks.clear();
   auto merges = [](const Bucket& x, const Bucket& y) {
     if (x.kind != y.kind) return false;
-    if (x.kind == PK_WAVE16) return sfk::kWave[x.c].q == sfk::kWave[y.c].q && x.tb == y.tb;
+    if (is_wave(x.kind)) return sfk::kWave[x.c].q == sfk::kWave[y.c].q && x.tb == y.tb;
     return x.c == y.c && (x.lanes > 32 ? x.lanes == y.lanes : y.lanes <= 32);
   };
   std::vector<uint8_t> done(nb, 0);
@@ -1089,7 +1100,7 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
     g.bucket = (uint32_t)u;
     g.grid = b.grid;
     g.block = b.block;
-    if (b.kind == PK_MYERS || b.kind == PK_WAVE16) {
+    if (b.kind == PK_MYERS || is_wave(b.kind)) {
       g.task_first = (uint32_t)S.tasks.size();
       for (size_t v = u; v < nb; ++v) {
         Bucket& x = P->buckets[v];
@@ -1217,6 +1228,7 @@ void describe_plan(sf_plan* P, const BuildScratch& S) {
                   : b.kind == PK_AFFINE16 ? "affine16"
                   : b.kind == PK_CHAIN16 ? "chain16"
                   : b.kind == PK_WAVE16  ? "wave16"
+                  : b.kind == PK_WAVE16X ? "wave16x"
                                          : "affine",
                   shown_c(b.kind, b.c),
                   b.wide ? "true" : "false", b.tb ? "true" : "false",
@@ -1374,11 +1386,11 @@ int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* ev
       al.links = P->d_links.as<DLink>();
       al.want = P->d_want.as<uint32_t>();
       al.snap = P->d_snap.as<uint32_t>();
-      if (b.kind == PK_WAVE16) {
+      if (is_wave(b.kind)) {
         al.order = orders;
         al.tasks = tasks;
         al.njobs = task_count;
-        CK(sfk::launch_wave16(sfk::kWave[b.c].q, b.tb, al, grid, bs));
+        CK(sfk::launch_wave16(sfk::kWave[b.c].q, b.kind == PK_WAVE16X, b.tb, al, grid, bs));
       } else if (b.kind == PK_CHAIN16) {
         CK(sfk::launch_affine16_chain(b.c, al, b.grid, b.block, bs));
       } else if (b.kind == PK_AFFINE16 && b.lanes == 64) {
@@ -1710,12 +1722,12 @@ uint64_t plan_bytes_estimate(const std::vector<Pass>& passes, uint64_t pool_byte
     // The classes either way of `lean`: the larger traceback.
     for (int lean = 0; lean < 2 && p.want_cigar && p.kind != PK_LOCAL; ++lean) {
       classify_affine(p, j, flags, wmax, use16, lean != 0, kind, c, wide, ln, lanes16);
-      if (kind != PK_WAVE16) break;
-      tb_wave = std::max(tb_wave, sfk::wave_tb_words(sfk::kWave[c], ((uint64_t)p.m + p.n + 1) / 2) * 4);
+      if (!is_wave(kind)) break;
+      tb_wave = std::max(tb_wave, sfk::wave_tb_words(sfk::kWave[c], wave_steps(j, kind)) * 4);
     }
     classify_affine(p, j, flags, wmax, use16, false, kind, c, wide, ln, lanes16);
     if (p.want_cigar && p.kind != PK_LOCAL) {
-      b += kind == PK_WAVE16
+      b += is_wave(kind)
                ? tb_wave
                : (uint64_t)p.m * tb_row_words(c, wide ? wide_chunks(c, wmax) : 1) * 4 * ln / 32;
       b += 2 * ((uint64_t)p.m + p.n + 2) * 4;

@@ -20,7 +20,10 @@ struct WaveClass {
   int q, lanes;
 };
 extern const WaveClass kWave[];
-extern const int kWaveN, kWaveN0;
+// [0, kWaveN0): the cheapest a cell, Global; [kWaveN0, kWaveX0): the fastest a pass (Prefix
+// passes: those of up to kWaveMaxX words); [kWaveX0, kWaveN): the cheapest a cell, Prefix.
+constexpr int kWaveN0 = 24, kWaveX0 = 31, kWaveN = 43;
+constexpr int kWaveMaxX = 8;
 inline int wave_cap(const WaveClass& c) { return 4 * c.q * c.lanes; }
 // Traceback words of a pass of `steps` row steps: 2Q words a lane and group of four.
 inline uint64_t wave_tb_words(const WaveClass& c, uint64_t steps) {
@@ -28,10 +31,13 @@ inline uint64_t wave_tb_words(const WaveClass& c, uint64_t steps) {
 }
 
 // 4-warp blocks per SM the registers are held to.
-__host__ __device__ constexpr int wave_blocks(int q, bool tb) {
-  return tb ? (q <= 4 ? 6 : q <= 6 ? 5 : q <= 8 ? 4 : 3) : (q <= 6 ? 8 : q <= 8 ? 6 : q <= 10 ? 5 : 4);
+__host__ __device__ constexpr int wave_blocks(int q, bool tb, bool ext) {
+  return ext ? (tb ? (q <= 4 ? 5 : q <= 6 ? 4 : 3) : (q <= 4 ? 6 : q <= 6 ? 5 : 4))
+             : tb ? (q <= 4 ? 6 : q <= 6 ? 5 : q <= 8 ? 4 : 3) : (q <= 6 ? 8 : q <= 8 ? 6 : q <= 10 ? 5 : 4);
 }
 
-cudaError_t launch_wave16(int q, bool tb, const AffLaunch& a, int grid, cudaStream_t s);
+// prefix: Prefix passes, else Global ones.
+cudaError_t launch_wave16(int q, bool prefix, bool tb, const AffLaunch& a, int grid,
+                          cudaStream_t s);
 
 }  // namespace sfk

@@ -10,23 +10,29 @@ cudaError_t launch_wave16_8(bool, const AffLaunch&, int, cudaStream_t);
 cudaError_t launch_wave16_10(bool, const AffLaunch&, int, cudaStream_t);
 cudaError_t launch_wave16_12(bool, const AffLaunch&, int, cudaStream_t);
 
-// Classes by the cells they hold.  The first kWaveN0 are the cheapest a band cell: a row step
-// costs a warp about 32 Q + 60 issue slots whatever it holds, so many lanes' worth of cells a
-// lane and many passes a warp.  The others are the fastest a pass: few words a lane.
-const WaveClass kWave[] = {
+cudaError_t launch_wave16x_4(bool, const AffLaunch&, int, cudaStream_t);
+cudaError_t launch_wave16x_6(bool, const AffLaunch&, int, cudaStream_t);
+cudaError_t launch_wave16x_8(bool, const AffLaunch&, int, cudaStream_t);
+
+// Classes by the cells they hold, within each range.  The cheapest a band cell: a row step costs
+// a warp about 32 Q + 60 issue slots whatever it holds, so many cells a lane and many passes a
+// warp; Prefix passes keep two more registers a word and stop at 8 words.  The fastest a pass:
+// few words a lane.
+const WaveClass kWave[kWaveN] = {
     {4, 3},  {4, 4},  {6, 3},  {4, 5},  {6, 4},   {10, 3},  {8, 4},   {12, 3},
     {10, 4}, {12, 4}, {10, 5}, {12, 5}, {8, 8},   {12, 6},  {10, 8},  {12, 8},
     {10, 10}, {12, 10}, {8, 16}, {10, 16}, {12, 16}, {8, 32}, {10, 32}, {12, 32},
-    {4, 8}, {4, 16}, {4, 32}, {6, 32}, {8, 32}, {10, 32}, {12, 32}};
-const int kWaveN = 31, kWaveN0 = 24;
+    {4, 8}, {4, 16}, {4, 32}, {6, 32}, {8, 32}, {10, 32}, {12, 32},
+    {4, 3}, {4, 4}, {6, 3}, {4, 5}, {6, 4}, {8, 4}, {8, 5}, {8, 6}, {8, 8}, {8, 10}, {8, 16}, {8, 32}};
 
-cudaError_t launch_wave16(int q, bool tb, const AffLaunch& a, int grid, cudaStream_t s) {
+cudaError_t launch_wave16(int q, bool prefix, bool tb, const AffLaunch& a, int grid,
+                          cudaStream_t s) {
   switch (q) {
-    case 4: return launch_wave16_4(tb, a, grid, s);
-    case 6: return launch_wave16_6(tb, a, grid, s);
-    case 8: return launch_wave16_8(tb, a, grid, s);
-    case 10: return launch_wave16_10(tb, a, grid, s);
-    case 12: return launch_wave16_12(tb, a, grid, s);
+    case 4: return prefix ? launch_wave16x_4(tb, a, grid, s) : launch_wave16_4(tb, a, grid, s);
+    case 6: return prefix ? launch_wave16x_6(tb, a, grid, s) : launch_wave16_6(tb, a, grid, s);
+    case 8: return prefix ? launch_wave16x_8(tb, a, grid, s) : launch_wave16_8(tb, a, grid, s);
+    case 10: return prefix ? cudaErrorInvalidValue : launch_wave16_10(tb, a, grid, s);
+    case 12: return prefix ? cudaErrorInvalidValue : launch_wave16_12(tb, a, grid, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -1,6 +1,7 @@
-// Global banded affine (Gotoh) passes swept by anti-diagonals, two cells per 32-bit register and
-// several passes per warp (align.rs:2446-2666 `run_core` in Mode::Global without clip or cut).
-// Results and traceback decisions equal the row kernels' (sf_affine16_impl.cuh).
+// Global and Prefix banded affine (Gotoh) passes swept by anti-diagonals, two cells per 32-bit
+// register and several passes per warp (align.rs:2446-2666 `run_core` in Mode::Global without
+// clip or cut, and in Mode::Prefix with or without clip, without cut).  Results and traceback
+// decisions equal the row kernels' (sf_affine16_impl.cuh).
 //
 // Cells.  Band offset K = j - i + bl of cell (i, j) sits at a fixed place: lane K / 4Q of the
 // pass's L lanes, and along anti-diagonal i + j = t the cells of one parity of K are computed
@@ -27,12 +28,21 @@
 // column 1 are masked too, so row 0 and column 0 come out of the recurrence itself, from the
 // one seed at (0, 0).  Cells past the text or pattern hold values nothing in the matrix reads.
 //
+// Prefix passes (EXT) need each row's largest value and its leftmost column, in row order: for
+// the clip score, its cell and the X-drop stop, and for the last row's score.  Both travel along
+// the row from left to right, a cell a step, as E does: M(K) = max(M(K - 1), H(K)) with the
+// leftmost offset it was reached at, and leave the band at its last cell, where one lane keeps
+// the pass's books, one row a row step, in row order.  The rows that run ahead of a stop are
+// computed and left out.  Columns past the text count for nothing (the last rows of a pass).
+//
 // Bound: the ALU pipe (one instruction every other cycle a scheduler): 8.5 of a word's 14.5
 // instructions with traceback, 4.5 of 6.5 without.  With 12 words a lane and 6 lanes a pass a
 // row step issues 443 instructions for five 2 kb passes of band 128 (258 on the ALU pipe), the
 // row kernel 254 for one; score only 221 against 150.  20,000 such pairs on GB300: 10.25 ->
 // 5.2 ms with CIGARs, 5.7 -> 2.4 ms without.
 #pragma once
+#include <type_traits>
+
 #include "sf_affine_impl.cuh"
 #include "sf_wave16.h"
 
@@ -67,7 +77,7 @@ __device__ __forceinline__ uint32_t pick(uint32_t x, uint32_t y, uint32_t m) {
   return d;
 }
 
-// Walks the pass's path from (m, n), the whole warp on one pass.  Each lane caches eight band
+// Walks the pass's path from its end cell, the whole warp on one pass.  Each lane caches eight band
 // offsets (two quads of four) of one group of four row steps, so the warp holds 128 row steps
 // around the path; a run of diagonal steps, which keeps its band offset, is found by one ballot
 // over the cached nibbles.
@@ -75,6 +85,7 @@ template <int Q>
 __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, int L, int lane) {
   const DJob J = a.jobs[jid];
   const TJob T = a.tjobs[jid];
+  const DRes R = a.out[jid];
   const int32_t m = (int32_t)J.m, n = (int32_t)J.n;
   const int32_t bl = clamp30(J.below) | 1, W = bl + clamp30(J.above) + 1;
   const int32_t a1 = (bl >> 1) + 1;  // the row step that row-step index 0 stands for
@@ -101,7 +112,19 @@ __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, int L, int lane
     cur_op = op;
     cur_len = len;
   };
-  int32_t i = m, j = n, K = n - m + bl;
+  // End cell (align.rs:2643-2650 score_col; 975-981 the window's choice).
+  int32_t score = R.score, i = m, j = (int32_t)R.score_col;
+  if (T.kind != 0) {
+    score = sat_add(R.score, T.end_bonus);
+    if (R.clip_best >= score) {
+      score = R.clip_best;
+      i = (int32_t)R.clip_i;
+      j = (int32_t)R.clip_j;
+      push(4, (uint32_t)(m - i));
+    }
+  }
+  const int32_t ei = i, ej = j;
+  int32_t K = j - i + bl;
   int state = 0;                      // 0 H, 1 E, 2 F
   int32_t G0 = -1, q0 = -1;           // lane d caches group G0 - d of offsets 4 q0 .. 4 q0 + 7
   uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0;  // offsets 4 q0 + (0, 1), (2, 3), (4, 5), (6, 7)
@@ -186,10 +209,10 @@ __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, int L, int lane
   }
   if (lane == 0) {
     TRes tr;
-    tr.score = a.out[jid].score;
+    tr.score = score;
     tr.status = status;
-    tr.end_i = (uint32_t)m;
-    tr.end_j = (uint32_t)n;
+    tr.end_i = (uint32_t)ei;
+    tr.end_j = (uint32_t)ej;
     tr.text_start = 0;
     tr.n_ops = status == 0 ? n_ops : 0;
     a.tres[jid] = tr;
@@ -198,7 +221,7 @@ __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, int L, int lane
 
 // One warp's passes, one per segment of L lanes: `jid` is the lane's own pass (any valid one
 // where `has` is false: computed, not stored).
-template <int Q, bool TB>
+template <int Q, bool TB, bool EXT>
 __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t jid, bool has, int L,
                                             int np, int lane, int seg) {
   constexpr int NT = (2 * Q + 15) / 16;  // 16-base registers of a lane's text (pattern) window
@@ -212,7 +235,9 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
   const int32_t bl = below | 1, W = bl + above + 1;
   const int32_t k0 = 2 * Q * l;  // the lane's first pair of offsets
   const int32_t a1 = (bl >> 1) + 1;
-  const int32_t N = (m + n + 1) >> 1;  // row steps until cell (m, n) is done
+  // Row steps until cell (m, n) is done; EXT: until row m's last band cell is.
+  const int32_t kw = (W - 1) >> 1;  // the pair of offsets the band's last cell is in
+  const int32_t N = EXT ? m + kw - a1 + 1 : (m + n + 1) >> 1;
 
   const uint32_t one = (uint32_t)opaque_one(), mone = 0u - one;
   const uint32_t sixteen = one << 4, four = one << 2, mfour = 0u - four;
@@ -223,19 +248,26 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
   constexpr uint32_t kH = TB ? 2u : 0u, kF = TB ? 1u : 0u;  // a clean field's low bits
   constexpr uint32_t kNegH = (kWNeg + kH) * kW2, kNegE = kWNeg * kW2, kNegF = (kWNeg + kF) * kW2;
 
+  // EXT: M's potential rises by 4 ext a step, so the top leaves room for a row's width of them.
+  const int32_t wtop = EXT ? (int32_t)kWTop - 4 * S.ext * (W + 1) : (int32_t)kWTop;
   uint32_t HA[Q], HB[Q], E[Q], F[Q], acc[TB ? 2 * Q : 1];
+  uint32_t M[EXT ? Q : 1], MK[EXT ? Q : 1];  // a row's largest value so far and its offset K
 #pragma unroll
   for (int k = 0; k < Q; ++k) {
     // The seed at (0, 0): offset bl, odd.
     const int32_t e = (bl >> 1) - k0;
-    const uint32_t top = kWTop + kH, neg = kWNeg + kH;
+    const uint32_t top = (uint32_t)wtop + kH, neg = kWNeg + kH;
     HA[k] = kNegH;
     HB[k] = (e == k ? top : neg) | ((e == Q + k ? top : neg) << 16);
     E[k] = kNegE;
     F[k] = kNegF;
     if constexpr (TB) acc[2 * k] = acc[2 * k + 1] = 0;
+    if constexpr (EXT) {
+      M[k] = kNegH | kW2;
+      MK[k] = 0;
+    }
   }
-  int32_t off = -(int32_t)kWTop;
+  int32_t off = -wtop;
 
   // Windows: T[r] holds the text bases of columns from a + k0 - bl + 16 r on (T[NT]: the bases
   // that shift in next), P[r] the pattern bases of rows from a - k0 - 16 r downwards, Pn the
@@ -297,6 +329,44 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       cb[NC - 1] = __byte_perm(eq[0], hi, 0x7632);
     }
   };
+  // EXT: the row maximum and its offset after word k's cells, from those left of them.  h: the
+  // cells' values, or 0 where they count for nothing; kc: their offsets.  The maximum is kept one
+  // step ahead (4 ext more) and with bit 0 set, which no H has: a tie keeps the left one, and bit
+  // 0 says which won.
+  const uint32_t m4 = 4u * (uint32_t)S.ext * kW2 + kW2, kc0 = 4u * (uint32_t)Q * (uint32_t)l * kW2;
+  const uint32_t ones = 0xffffu * one;
+  auto row_max = [&](uint32_t h, uint32_t kc, uint32_t ml, uint32_t pl, uint32_t& mo, uint32_t& po) {
+    const uint32_t x = __vmaxu2(ml, h);
+    const uint32_t kept = x & kW2;
+    po = pick(pl, kc, kept * ones);
+    mo = kept * mone + (x * one + m4);
+  };
+  // The band's last cell: one lane's word and half, in the even or the odd step.
+  const bool last_odd = (W - 1) & 1;
+  const int32_t last_e = kw - k0;  // 0 .. 2Q - 1 in the lane that holds it
+  const bool books = EXT && has && last_e >= 0 && last_e < 2 * Q;
+  const bool any_even = EXT && __any_sync(FULL, books && !last_odd);
+  const bool any_odd = EXT && __any_sync(FULL, books && last_odd);
+  const uint32_t pad0 = l == 0 && bl != below ? 0xffff0000u : ~0u;  // offset 0 is a pad
+  int32_t rmax_f = 0, rmax_k = 0;  // the finished row's largest field and its offset
+  auto take_last = [&](bool mine) {
+    uint32_t u = 0, p = 0;
+#pragma unroll
+    for (int k = 0; k < (EXT ? Q : 1); ++k) {
+      if (last_e == k || last_e == Q + k) {
+        u = M[k];
+        p = MK[k];
+      }
+    }
+    if (mine) {
+      rmax_f = (int32_t)(last_e >= Q ? u >> 16 : u & 0xffffu);
+      rmax_k = (int32_t)(last_e >= Q ? p >> 16 : p & 0xffffu);
+    }
+  };
+  Book b;
+  bool fin = false;
+  // Row steps from which some cell lies past the text.
+  const int32_t r_tail = __reduce_min_sync(FULL, has ? n + bl - kw - a1 : INT32_MAX);
   // Word k's cells: e and f are the gap values entering them; h their diagonal, then their H.
   auto cell = [&](int k, const uint32_t (&cb)[NC], uint32_t& h, uint32_t et, uint32_t ft,
                   uint32_t& eo, uint32_t& fo, uint32_t& ac) {
@@ -324,7 +394,8 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
   uint4* tbp = nullptr;
   if constexpr (TB) tbp = reinterpret_cast<uint4*>(a.tb + J.tb_word) + l;
 
-  for (int32_t r = 0; r < Rtot;) {
+  auto row_step = [&](int32_t r, auto tailtag) {
+    constexpr bool TAIL = decltype(tailtag)::value;
     if ((r & 15) == 0) {
       if (r > 0) {
         T[NT] = __funnelshift_r(t0, t1, tsh);
@@ -338,6 +409,11 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       p1 = word(J.p_word, xp + 1, plim);
     }
     if (r <= rF) masks(r);
+    // EXT, some columns past the text: cells e <= te lie in it (the odd step's: e < te).
+    [[maybe_unused]] const int32_t te = n + bl - (a1 + r) - k0;
+    auto in_text = [&](int k, int32_t t) -> uint32_t {
+      return (k <= t ? 0xffffu : 0u) | (Q + k <= t ? 0xffff0000u : 0u);
+    };
     uint32_t G[Q], cb[NC];
     // Even step: offsets 2k from their odd neighbours.
     matches(Me, cb);
@@ -353,6 +429,20 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
         const uint32_t ft = __vmaxu2(G[k], F[k]);
         cell(k, cb, HA[k], et, ft, E[k], F[k], acc[TB ? 2 * k : 0]);
       }
+    }
+    if constexpr (EXT) {
+      uint32_t sM = __shfl_up_sync(FULL, M[Q - 1], 1);
+      const uint32_t sK = __shfl_up_sync(FULL, MK[Q - 1], 1);
+      if (l == 0) sM = kNegH | kW2;
+      const uint32_t ml = __byte_perm(sM, M[Q - 1], 0x5432), pl = __byte_perm(sK, MK[Q - 1], 0x5432);
+#pragma unroll
+      for (int k = Q - 1; k >= 0; --k) {
+        uint32_t h = k == 0 ? HA[0] & pad0 : HA[k];
+        if constexpr (TAIL) h &= in_text(k, te);
+        row_max(h, kc0 + (uint32_t)(2 * k) + ((uint32_t)(2 * (Q + k)) << 16), k ? M[k ? k - 1 : 0] : ml,
+                k ? MK[k ? k - 1 : 0] : pl, M[k], MK[k]);
+      }
+      if (any_even) take_last(!last_odd);
     }
 #pragma unroll
     for (int q = 0; q < NT; ++q) T[q] = __funnelshift_r(T[q], T[q + 1], 2);
@@ -376,11 +466,50 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
         cell(k, cb, HB[k], et, ft, E[k], F[k], acc[TB ? 2 * k + 1 : 0]);
       }
     }
+    if constexpr (EXT) {
+#pragma unroll
+      for (int k = 0; k < Q; ++k) {
+        uint32_t h = HB[k];
+        if constexpr (TAIL) h &= in_text(k, te - 1);
+        row_max(h, kc0 + (uint32_t)(2 * k + 1) + ((uint32_t)(2 * (Q + k) + 1) << 16), M[k], MK[k], M[k],
+                MK[k]);
+      }
+      if (any_odd) take_last(last_odd);
+    }
 #pragma unroll
     for (int q = NT - 1; q > 0; --q) P[q] = __funnelshift_l(P[q - 1], P[q], 2);
     P[0] = __funnelshift_l(Pn, P[0], 2);
     Pn = Pn * four;
+  };
+
+  for (int32_t r = 0; r < Rtot;) {
+    if (!EXT || r < r_tail)
+      row_step(r, std::false_type{});
+    else
+      row_step(r, std::true_type{});
     ++r;
+    if constexpr (EXT) {
+      // Row i's books (align.rs:2580-2640), in the lane that holds the band's last cell.
+      const int32_t i = a1 + r - 1 - kw;
+      if (books && !fin && i >= 1) {
+        const int32_t rmax = (((rmax_f & ~3) + off) >> 2) - S.ext * (2 * i + W - bl);
+        const uint32_t col = (uint32_t)(i - bl + rmax_k);
+        const int32_t hi = min(i + above, n);
+        if ((S.flags & F_CLIP) && rmax > b.clip_best) {
+          b.clip_best = rmax;
+          if (S.flags & F_CELL) {
+            b.ci = (uint32_t)i;
+            b.cj = col;
+          }
+        }
+        const bool stop = (S.flags & F_CLIP) && rmax < sat_sub(b.clip_best, S.xdrop);
+        if (stop || i == m) {
+          a.out[jid] = DRes{stop ? NEG : rmax, b.clip_best, 0, NEG, stop ? 0u : col, b.ci, b.cj,
+                            (uint32_t)hi, (uint32_t)i, (uint32_t)i, band_cells(i, below, above, n)};
+          fin = true;
+        }
+      }
+    }
     if constexpr (TB) {
       if ((r & 3) == 0) {
         // Four row steps: one 16-byte store per quad of words, lane-fastest.
@@ -396,7 +525,10 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
         for (int k = 0; k < 2 * Q; ++k) acc[k] = 0;
       }
     }
-    if (r == next_end) {
+    if constexpr (EXT) {
+      if ((r & 3) == 0 && !__any_sync(FULL, books && !fin)) break;
+    }
+    if (!EXT && r == next_end) {
       // Passes whose cell (m, n) this row step computed.
       const int32_t Kend = n - m + bl, ke = (Kend >> 1) - k0;
       if (has && r == N && ke >= 0 && ke < 2 * Q) {
@@ -429,7 +561,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
         if (l + s < L) v = max(v, u);
       }
       v = __shfl_sync(FULL, v, min(seg * L, 31));
-      const int32_t delta = (int32_t)(v - kH) - (int32_t)kWTop;
+      const int32_t delta = (int32_t)(v - kH) - wtop;
       const uint32_t dd = ((uint32_t)(-delta) & 0xffffu) * kW2;
 #pragma unroll
       for (int k = 0; k < Q; ++k) {
@@ -437,6 +569,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
         HB[k] = __viaddmax_u16x2(HB[k], dd, kNegH);
         E[k] = __viaddmax_u16x2(E[k], dd, kNegE);
         F[k] = __viaddmax_u16x2(F[k], dd, kNegF);
+        if constexpr (EXT) M[k] = __viaddmax_u16x2(M[k], dd, kNegH | kW2);
       }
       off += delta;
     }
@@ -452,8 +585,8 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
   __syncwarp();
 }
 
-template <int Q, bool TB>
-__global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB)) wave16_kernel(sfk::AffLaunch a) {
+template <int Q, bool TB, bool EXT>
+__global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, EXT)) wave16_kernel(sfk::AffLaunch a) {
   const int lane = threadIdx.x & 31;
   // The first task by place; the queue hands out those after the grid's first ones.
   const uint32_t grid_tasks = (gridDim.x * blockDim.x) >> 5;
@@ -463,7 +596,7 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB)) wave16_kernel(sf
     const uint2 task = a.tasks[q];
     const int L = (int)(task.y & 0xffu), np = (int)(task.y >> 8), seg = lane / L;
     const bool has = seg < np;
-    wave_passes<Q, TB>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, np, lane, seg);
+    wave_passes<Q, TB, EXT>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, np, lane, seg);
     if (a.njobs <= grid_tasks) break;
     uint32_t next = 0;
     if (lane == 0) next = atomicAdd(a.counter, 1u);
@@ -475,12 +608,12 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB)) wave16_kernel(sf
 
 namespace sfk {
 
-template <int Q>
+template <int Q, bool EXT>
 cudaError_t launch_wave16_q(bool tb, const AffLaunch& a, int grid, cudaStream_t s) {
   if (tb)
-    wave16_kernel<Q, true><<<grid, 128, 0, s>>>(a);
+    wave16_kernel<Q, true, EXT><<<grid, 128, 0, s>>>(a);
   else
-    wave16_kernel<Q, false><<<grid, 128, 0, s>>>(a);
+    wave16_kernel<Q, false, EXT><<<grid, 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 

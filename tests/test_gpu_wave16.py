@@ -1,9 +1,10 @@
 """The anti-diagonal 16-bit kernel (sf_wave16_impl.cuh) against the oracle: scores, end cells,
-DP cells and CIGARs of Global banded passes, bit-exact, where its layout can go wrong -- every
-class filled to its last band cell, several passes of uneven length to a warp, bands that start
-at column 0 for many rows, one-base sequences, row steps around the stores (4), the window
-chunks (16) and the rebase (32), paths along the band's edges, long passes, and score sets on
-both sides of its admission rule."""
+DP cells and CIGARs of Global and Prefix banded passes, bit-exact, where its layout can go wrong
+-- every class filled to its last band cell, several passes of uneven length to a warp, bands
+that start at column 0 for many rows, one-base sequences, row steps around the stores (4), the
+window chunks (16) and the rebase (32), paths along the band's edges, long passes, score sets on
+both sides of its admission rule; for Prefix passes the clip cell, the X-drop stop at any row, the
+last row's best column and texts that end inside the band."""
 import json
 
 import numpy as np
@@ -168,3 +169,124 @@ def test_admission(ctx):
     out, kinds = _run(ctx, rows, scores)
     assert {"wave16", "affine16"} <= {k for k, _, _ in kinds}, kinds
     _check(rows, out, scores)
+
+
+def _run_prefix(ctx, rows, scores, rows_only=False):
+    """rows: (pattern, text, band, window or None, xdrop, end bonus, cigar, score index); window
+    None: an affine pass in Prefix mode, else an extension."""
+    import os
+    from spearfish_gb300 import batch as B
+    pb = B.PoolBuilder()
+    jobs = B.new_jobs(len(rows))
+    for j, (p, t, band, win, xd, bonus, cig, sci) in zip(jobs, rows):
+        j["p_off"], j["m"] = pb.add(p), len(p)
+        j["t_off"], j["n"] = pb.add(t), len(t)
+        j["band"], j["want_cigar"], j["sc_index"], j["mode"] = band, cig, sci, R.PREFIX
+        j["kind"] = B.JOB_AFFINE if win is None else B.JOB_EXTEND_WINDOW
+        if win is not None:
+            j["window"], j["xdrop"], j["end_bonus"] = win, xd, bonus
+    old = os.environ.get("SF_AFFINE16_LANES")
+    if rows_only:
+        os.environ["SF_AFFINE16_LANES"] = "32"
+    try:
+        plan = B.Plan(ctx, jobs, pb.size, scores)
+        try:
+            plan.upload(pb.build())
+            plan.execute()
+            out = plan.download()
+            kinds = {(b["kind"], b["c"], b["lanes"]) for b in json.loads(plan.describe())["buckets"]}
+        finally:
+            plan.close()
+    finally:
+        if rows_only:
+            if old is None:
+                del os.environ["SF_AFFINE16_LANES"]
+            else:
+                os.environ["SF_AFFINE16_LANES"] = old
+    return out, kinds
+
+
+def _check_prefix(rows, out, scores):
+    for q, (p, t, band, win, xd, bonus, cig, sci) in enumerate(rows):
+        r, sc = out.results[q], scores[sci]
+        where = (q, len(p), len(t), band, win, xd, sci)
+        got = (int(r["status"]), int(r["score"]), int(r["pattern_end"]), int(r["text_end"]))
+        if win is None:
+            o = O.traceback(p, t, O.TB_AFFINE, O.PREFIX, sc, band)
+            assert got == (0, o["score"], len(p), o["end_j"]), where
+        else:
+            o = O.traceback(p, t, O.TB_EXTEND, O.PREFIX, sc, band, win, bonus, xd)
+            assert got == (0, o["score"], o["end_i"], o["end_j"]), where
+            assert (*got[1:], int(r["text_read"])) == \
+                O.affine_extend_window(p, t, win, sc, band, bonus, xd), where
+        if cig:
+            assert out.cigar(q) == o["cigar"], where
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_prefix(ctx, packed):
+    rng = np.random.default_rng(2641 + packed)
+    rows = []
+
+    def add(p, t, band, extend=True):
+        t = t or [int(rng.integers(0, 4))]
+        win = len(t) + int(rng.integers(0, 40)) if extend else None
+        xd = int(rng.choice([0, 3, 8, 20, 50, R.I32_MAX]))
+        rows.append((p, t, band, win, xd, int(rng.integers(0, 9)), int(rng.integers(0, 2)),
+                     int(rng.integers(0, 2))))
+
+    # Bands that fill each class, miss it by one or pass it by one, rows that end past, at and
+    # before the text's end.
+    for cap in (48, 64, 72, 80, 96, 128, 160, 192, 256, 320, 512, 768, 1024):
+        for w in (cap - 1, cap, cap + 1):
+            band, extra = (w - 2) // 2, (w - 2) % 2
+            for cut in (0, 7, 40):
+                m = band // 2 + 30 + int(rng.integers(0, 90))
+                p, t = _shifted(rng, m, int(rng.integers(-(m // 3), m // 3 + 1)))
+                t = t[:max(1, m - cut)] + rng.integers(0, 4, extra).tolist()
+                # The window's geometry is the text's: below + above + 1 = w.
+                rows.append((p[:len(t) - extra] if cut else p, t, band, len(t), 50, 5, 1, cap % 3 % 2))
+                add(p, t, band, extend=False)
+    for m in list(range(1, 60)) + [127, 128, 129, 400]:
+        p, t = _noisy(rng, m, 0.15)
+        add(p, t + rng.integers(0, 4, int(rng.integers(0, 30))).tolist(), int(rng.integers(0, 20)))
+        add(p, t[:max(1, len(t) - int(rng.integers(0, 10)))], int(rng.integers(0, 20)), extend=False)
+    # Extensions that go wrong part of the way: the X-drop stops at any row.
+    for _ in range(PACKED - len(rows) if packed else 200):
+        m = int(np.exp(rng.uniform(np.log(8), np.log(500))))
+        good = int(rng.integers(0, m + 1))
+        p, t = _noisy(rng, m, float(rng.choice([0.0, 0.05, 0.12])))
+        t = t[:good] + rng.integers(0, 4, max(0, m + 20 - good)).tolist()
+        add(p, t, int(rng.integers(1, 40)), extend=rng.random() < 0.8)
+    scores = (R.ONT, R.HIFI)
+    out, kinds = _run_prefix(ctx, rows, scores)
+    wave = {(c, n) for k, c, n in kinds if k == "wave16x"}
+    want = {(16, 3), (24, 4), (32, 4), (32, 10), (32, 32)} if packed else \
+        {(16, 8), (16, 16), (16, 32), (24, 32), (32, 32)}
+    assert wave >= want, sorted(kinds)
+    _check_prefix(rows, out, scores)
+    # The row kernels give the same.
+    ref, rkinds = _run_prefix(ctx, rows, scores, rows_only=True)
+    assert not any(k.startswith("wave") for k, _, _ in rkinds)
+    for f in ("score", "pattern_end", "text_start", "text_end", "text_read", "cells", "n_ops",
+              "status"):
+        assert np.array_equal(out.results[f], ref.results[f]), f
+    assert np.array_equal(out.ops, ref.ops)
+
+
+def test_prefix_long(ctx):
+    """Thousands of row steps with every row's maximum in order, up to the widest class."""
+    rng = np.random.default_rng(2651)
+    rows = []
+    for m, band in ((9000, 16), (6000, 128), (4000, 300), (3000, 480)):
+        for kind in ("noisy", "half"):
+            q = rng.integers(0, 4, m).tolist()
+            t = R.mutate(q, R.rand_edits(rng, m // 10, m))
+            if kind == "half":
+                t = t[:m // 2] + rng.integers(0, 4, m // 2).tolist()
+            for xd in (50, 400, R.I32_MAX):
+                rows.append((q, t, band, len(t) + 60, xd, 5, 1, int(rng.integers(0, 2))))
+    scores = (R.ONT, R.HIFI)
+    out, kinds = _run_prefix(ctx, rows, scores)
+    assert ("wave16x", 32, 32) in kinds, kinds  # (the widest bands of all go to the row kernels)
+    _check_prefix(rows, out, scores)
