@@ -77,41 +77,30 @@ __device__ __forceinline__ uint32_t pick(uint32_t x, uint32_t y, uint32_t m) {
   return d;
 }
 
-// Walks the pass's path from its end cell, the whole warp on one pass.  Each lane caches eight band
-// offsets (two quads of four) of one group of four row steps, so the warp holds 128 row steps
-// around the path; a run of diagonal steps, which keeps its band offset, is found by one ballot
-// over the cached nibbles.
+// Walks the warp's paths from their end cells, each by its pass's lanes, side by side.  Lane d of
+// a pass caches eight band offsets (two quads of four) of the row steps 8 (H0 - d) .. + 7, eight
+// nibbles an offset, latest row first; a run of diagonal steps, which keeps its band offset, is
+// found by one ballot over the cached nibbles.  `steps`: the lane's pass's row steps.
+//
+// A stored word holds its four row steps' nibbles, each 8 low, on top of the word of the four
+// steps before, 16 bits up (the rows push and never clear): its low field needs 0x8888 added, its
+// high field that and the earlier word's low field taken off.
 template <int Q>
-__device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, int L, int lane) {
+__device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, bool has, int L, int l, int base,
+                          int32_t steps) {
   const DJob J = a.jobs[jid];
   const TJob T = a.tjobs[jid];
   const DRes R = a.out[jid];
   const int32_t m = (int32_t)J.m, n = (int32_t)J.n;
   const int32_t bl = clamp30(J.below) | 1, W = bl + clamp30(J.above) + 1;
   const int32_t a1 = (bl >> 1) + 1;  // the row step that row-step index 0 stands for
-  const int32_t gstride = (Q / 2) * L;  // uint4s per group of four row steps
+  const int32_t gstride = (Q / 2) * L, groups = (steps + 3) >> 2;  // uint4s per group of four steps
   const uint4* tb = reinterpret_cast<const uint4*>(a.tb + J.tb_word);
+  const uint32_t lanes = L == 32 ? FULL : (1u << L) - 1u;
   uint32_t* out = a.ops + T.ops_off;
   const uint32_t cap = T.ops_cap;
   uint32_t n_ops = 0, cur_op = 15, cur_len = 0;
   int status = 0;
-  auto push = [&](uint32_t op, uint32_t len) {
-    if (len == 0) return;
-    if (op == cur_op) {
-      cur_len += len;
-      return;
-    }
-    if (cur_len) {
-      if (n_ops == cap) {
-        status = -1;
-        return;
-      }
-      if (lane == 0) out[n_ops] = (cur_len << 4) | cur_op;
-      ++n_ops;
-    }
-    cur_op = op;
-    cur_len = len;
-  };
   // End cell (align.rs:2643-2650 score_col; 975-981 the window's choice).
   int32_t score = R.score, i = m, j = (int32_t)R.score_col;
   if (T.kind != 0) {
@@ -120,94 +109,130 @@ __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, int L, int lane
       score = R.clip_best;
       i = (int32_t)R.clip_i;
       j = (int32_t)R.clip_j;
-      push(4, (uint32_t)(m - i));
+      cur_op = 4;
+      cur_len = (uint32_t)(m - i);
     }
   }
   const int32_t ei = i, ej = j;
   int32_t K = j - i + bl;
-  int state = 0;                      // 0 H, 1 E, 2 F
-  int32_t G0 = -1, q0 = -1;           // lane d caches group G0 - d of offsets 4 q0 .. 4 q0 + 7
-  uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0;  // offsets 4 q0 + (0, 1), (2, 3), (4, 5), (6, 7)
-  // One quad of four offsets: the low or the high fields of its four words.
-  auto quad = [&](int32_t g, int32_t kq, uint32_t& x, uint32_t& y) {
-    x = y = 0;
-    if (g < 0 || kq < 0 || kq >= Q * L) return;
-    const int32_t ln = kq / Q, rem = kq - ln * Q, hi = rem >= Q / 2;
-    const uint4 w = tb[(int64_t)g * gstride + (rem - (hi ? Q / 2 : 0)) * L + ln];
-    const uint32_t s = hi ? 0x7632u : 0x5410u;
-    x = __byte_perm(w.x, w.y, s);
-    y = __byte_perm(w.z, w.w, s);
-  };
-  const int64_t guard = 3 * ((int64_t)m + n) + 64;
-  for (int64_t it = 0;; ++it) {
-    if (it > guard || status) {
-      if (!status) status = 1;
-      break;
-    }
-    if (state == 0 && i == 0) {
-      push(2, (uint32_t)j);
-      break;
-    }
-    if (state == 0 && j == 0) {
-      push(1, (uint32_t)i);
-      break;
-    }
-    if (i <= 0 || j <= 0 || K < 0 || K >= W) {
-      status = 1;
-      break;
-    }
-    const int32_t rho = i + (K >> 1) - a1, g = rho >> 2;
-    if (K < 4 * q0 || K >= 4 * q0 + 8 || q0 < 0 || g > G0 || g <= G0 - 32) {
-      q0 = max(K - 2, 0) >> 2;
-      G0 = g;
-      quad(g - lane, q0, c0, c1);
-      quad(g - lane, q0 + 1, c2, c3);
-    }
-    const int32_t x = K - 4 * q0;  // 0 .. 7
-    const uint32_t w01 = x & 2 ? c1 : c0, w23 = x & 2 ? c3 : c2;
-    const uint32_t w = x & 4 ? w23 : w01;
-    const uint32_t v = (x & 1) ? w >> 16 : w & 0xffffu;  // this lane's four nibbles at K
-    const int32_t d = G0 - g, r0 = rho & 3;
-    const uint32_t nib = (__shfl_sync(FULL, v, d) >> (4 * (3 - r0))) & 15u;
-    if (state == 0) {
-      const uint32_t win = nib >> 2;
-      if (win == 2u) {
-        // Row step 3 of a group is nibble 0.  Rows after the path's own count as diagonal.
-        uint32_t dg = (v >> 3) & ~(v >> 2) & 0x1111u;
-        if (lane == d) dg |= 0x1111u & ((1u << (4 * (3 - r0))) - 1u);
-        const uint32_t part = ((uint32_t)__ffs((int)(~dg & 0x11111u)) - 1u) >> 2;  // 0 .. 4
-        const uint32_t nf = __ballot_sync(FULL, dg != 0x1111u) >> d;
-        const int32_t z = nf ? __ffs((int)nf) - 1 : 32 - d;  // whole groups from lane d on
-        const int32_t tail = (int32_t)__shfl_sync(FULL, part, (d + z) & 31);
-        int32_t run = 4 * z - (3 - r0) + (nf ? tail : 0);
-        run = min(run, min(i, j));
-        push(0, (uint32_t)run);
-        i -= run;
-        j -= run;
-      } else {
-        state = win == 1u ? 2 : 1;
+  int state = 0;              // 0 H, 1 E, 2 F
+  int32_t H0 = -1, q0 = -1;   // cached: row steps up to 8 H0 + 7, offsets 4 q0 .. 4 q0 + 7
+  uint32_t c[8];
+#pragma unroll
+  for (int x = 0; x < 8; ++x) c[x] = 0;
+  // One quad of four offsets in the two groups of row steps 8 h ..: the low or the high fields of
+  // its four words, the later group's in the low half.
+  auto quad = [&](int32_t h, int32_t kq, uint32_t (&w)[4]) {
+    uint4 g[3] = {};  // groups 2 h - 1 (for the high fields), 2 h, 2 h + 1
+    uint32_t s = 0x5410u;
+    if (h >= 0 && kq >= 0 && kq < Q * L) {
+      const int32_t ln = kq / Q, rem = kq - ln * Q, hi = rem >= Q / 2;
+      const uint4* p = tb + (rem - (hi ? Q / 2 : 0)) * L + ln;
+      if (hi) s = 0x7632u;
+#pragma unroll
+      for (int u = 0; u < 3; ++u) {
+        const int32_t k = 2 * h - 1 + u;
+        if ((u > 0 || hi) && k >= 0 && k < groups) g[u] = p[(int64_t)k * gstride];
       }
     }
-    if (state == 1) {
-      push(2, 1);
-      state = (nib & 2u) ? 0 : 1;
-      --j;
-      --K;
-    } else if (state == 2) {
-      push(1, 1);
-      state = (nib & 1u) ? 2 : 0;
-      --i;
-      ++K;
+    auto both = [&](uint32_t x0, uint32_t x1, uint32_t x2) {
+      return __byte_perm(x2 - (x1 << 16) + 0x88888888u, x1 - (x0 << 16) + 0x88888888u, s);
+    };
+    w[0] = both(g[0].x, g[1].x, g[2].x);
+    w[1] = both(g[0].y, g[1].y, g[2].y);
+    w[2] = both(g[0].z, g[1].z, g[2].z);
+    w[3] = both(g[0].w, g[1].w, g[2].w);
+  };
+  const int64_t guard = 3 * ((int64_t)m + n) + 64;
+  bool done = !has;
+  for (int64_t it = 0; __any_sync(FULL, !done); ++it) {
+    const bool end = !done && state == 0 && (i == 0 || j == 0);
+    const bool bad = !done && !end && (i <= 0 || j <= 0 || K < 0 || K >= W || it > guard);
+    const bool go = !done && !end && !bad;
+    const int32_t rho = i + (K >> 1) - a1, h = rho >> 3, pos = 7 - (rho & 7);
+    if (go && (K < 4 * q0 || K >= 4 * q0 + 8 || q0 < 0 || h > H0 || h <= H0 - L)) {
+      q0 = max(K - 2, 0) >> 2;
+      H0 = h;
+      uint32_t w0[4], w1[4];
+      quad(h - l, q0, w0);
+      quad(h - l, q0 + 1, w1);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        c[x] = w0[x];
+        c[4 + x] = w1[x];
+      }
     }
+    const int32_t x = K - 4 * q0;  // 0 .. 7
+    const uint32_t x0 = x & 1 ? c[1] : c[0], x1 = x & 1 ? c[3] : c[2], x2 = x & 1 ? c[5] : c[4],
+                   x3 = x & 1 ? c[7] : c[6];
+    const uint32_t y0 = x & 2 ? x1 : x0, y1 = x & 2 ? x3 : x2;
+    const uint32_t v = x & 4 ? y1 : y0;  // this lane's eight nibbles at K
+    const int32_t d = go ? H0 - h : 0;
+    const uint32_t nib = (__shfl_sync(FULL, v, min(base + d, 31)) >> (4 * pos)) & 15u;
+    // Diagonal cells; rows after the path's own count as such.
+    uint32_t nd = ~((v >> 3) & ~(v >> 2)) & 0x11111111u;
+    if (l == d) nd &= ~((1u << (4 * pos)) - 1u);
+    const uint32_t part = nd ? (uint32_t)(__ffs((int)nd) - 1) >> 2 : 8u;
+    const uint32_t nf = ((__ballot_sync(FULL, nd != 0) >> base) & lanes) >> d;
+    const int32_t z = nf ? __ffs((int)nf) - 1 : L - d;  // whole lanes from lane d on
+    const int32_t tail = (int32_t)__shfl_sync(FULL, part, min(base + d + z, 31));
+    uint32_t op = 0, len = 0;
+    if (end) {
+      op = i == 0 ? 2 : 1;
+      len = (uint32_t)(i == 0 ? j : i);
+    }
+    if (go) {
+      if (state == 0) {
+        const uint32_t win = nib >> 2;
+        if (win == 2u) {
+          const int32_t run = min(8 * z - pos + (nf ? tail : 0), min(i, j));
+          len = (uint32_t)run;
+          i -= run;
+          j -= run;
+        } else {
+          state = win == 1u ? 2 : 1;
+        }
+      }
+      if (state == 1) {
+        op = 2;
+        len = 1;
+        state = (nib & 2u) ? 0 : 1;
+        --j;
+        --K;
+      } else if (state == 2) {
+        op = 1;
+        len = 1;
+        state = (nib & 1u) ? 2 : 0;
+        --i;
+        ++K;
+      }
+    }
+    if (len) {
+      if (op == cur_op) {
+        cur_len += len;
+      } else {
+        if (cur_len) {
+          if (n_ops == cap)
+            status = -1;
+          else if (l == 0)
+            out[n_ops] = (cur_len << 4) | cur_op;
+          ++n_ops;
+        }
+        cur_op = op;
+        cur_len = len;
+      }
+    }
+    if (bad) status = 1;
+    done = done || end || bad || status != 0;
   }
-  if (!status && cur_len) {
-    if (n_ops == cap)
-      status = -1;
-    else if (lane == 0)
-      out[n_ops] = (cur_len << 4) | cur_op;
-    ++n_ops;
-  }
-  if (lane == 0) {
+  if (has && l == 0) {
+    if (!status && cur_len) {
+      if (n_ops == cap)
+        status = -1;
+      else
+        out[n_ops] = (cur_len << 4) | cur_op;
+      ++n_ops;
+    }
     TRes tr;
     tr.score = score;
     tr.status = status;
@@ -223,7 +248,7 @@ __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, int L, int lane
 // where `has` is false: computed, not stored).
 template <int Q, bool TB, bool EXT>
 __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t jid, bool has, int L,
-                                            int np, int lane, int seg) {
+                                            int lane, int seg) {
   constexpr int NT = (2 * Q + 15) / 16;  // 16-base registers of a lane's text (pattern) window
   constexpr int NC = (Q + 7) / 8;        // registers of a step's match bits
   static_assert(Q % 2 == 0 && Q >= 4 && Q <= 16, "words per lane and parity");
@@ -380,7 +405,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       ac = ac * sixteen + y;
       ac = ec * mone + ac;
       ac = ht * four + ac;
-      ac = hs * mfour + ac;  // (winner - 2) << 2: the flush adds the 8 a nibble
+      ac = hs * mfour + ac;  // (winner - 2) << 2
       h = hs;
       eo = ec;
       fo = fc;
@@ -513,16 +538,12 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
     if constexpr (TB) {
       if ((r & 3) == 0) {
         // Four row steps: one 16-byte store per quad of words, lane-fastest.
-        const bool st = has && r < N + 4;
+        if (has && r < N + 4) {
 #pragma unroll
-        for (int q = 0; q < Q / 2; ++q) {
-          const uint4 w = make_uint4(acc[4 * q] + 0x88888888u, acc[4 * q + 1] + 0x88888888u,
-                                     acc[4 * q + 2] + 0x88888888u, acc[4 * q + 3] + 0x88888888u);
-          if (st) tbp[q * L] = w;
+          for (int q = 0; q < Q / 2; ++q)
+            tbp[q * L] = make_uint4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+          tbp += (Q / 2) * L;
         }
-        if (st) tbp += (Q / 2) * L;
-#pragma unroll
-        for (int k = 0; k < 2 * Q; ++k) acc[k] = 0;
       }
     }
     if constexpr (EXT) {
@@ -576,11 +597,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
   }
   if constexpr (TB) {
     __syncwarp();
-    for (int s = 0; s < np; ++s) {
-      const uint32_t js = __shfl_sync(FULL, jid, s * L);
-      if (__shfl_sync(FULL, (int)has, s * L)) walk_wave<Q>(a, js, L, lane);
-      __syncwarp();
-    }
+    walk_wave<Q>(a, jid, has, L, l, min(seg * L, 31), N);
   }
   __syncwarp();
 }
@@ -596,7 +613,7 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, EXT)) wave16_kern
     const uint2 task = a.tasks[q];
     const int L = (int)(task.y & 0xffu), np = (int)(task.y >> 8), seg = lane / L;
     const bool has = seg < np;
-    wave_passes<Q, TB, EXT>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, np, lane, seg);
+    wave_passes<Q, TB, EXT>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, lane, seg);
     if (a.njobs <= grid_tasks) break;
     uint32_t next = 0;
     if (lane == 0) next = atomicAdd(a.counter, 1u);
