@@ -237,6 +237,7 @@ struct sf_plan {
   // cell: -1 by the plan's passes, else as set (the autotuner's trial plans).
   int lean = -1;
   int most = 0;  // Myers pairs a warp at most, likewise (0: by the plan's passes)
+  uint64_t long_steps = 0;  // the row steps of a long pass, likewise
   // Class overrides for this plan only (the autotuner's trial plans); else the context's.
   const sfe::TuneTable* tune_override = nullptr;
   // Host-side build arrays kept between builds (sf_plan.cu).
@@ -331,7 +332,7 @@ bool ok_sc(const sf_affine_t* sc);
 bool allow16();
 int default_lanes16();
 void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax, bool use16,
-                     bool lean, PassKind& kind, int& c, bool& wide, int& lanes,
+                     uint64_t long_steps, PassKind& kind, int& c, bool& wide, int& lanes,
                      int lanes16 = 32);
 // The band cells the anti-diagonal kernel lays out for a pass.
 int64_t wave_width(const DJob& j);
@@ -339,6 +340,7 @@ int64_t wave_width(const DJob& j);
 // fastest, rather than the cheapest ones a cell.
 bool lean_plan(size_t np, int sms);
 bool plan_is_lean(const sf_plan* P);
+uint64_t plan_long_steps(const sf_plan* P);
 inline bool is_wave(int kind) { return kind == PK_WAVE16 || kind == PK_WAVE16X; }
 // Row steps of a pass on the anti-diagonal kernel.
 uint64_t wave_steps(const DJob& j, int kind);

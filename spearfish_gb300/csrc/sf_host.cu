@@ -1213,7 +1213,8 @@ int sf_batch_run(sf_context* ctx, const uint8_t* pool, uint64_t pool_bytes, cons
 namespace {
 
 // A pass's class before any override, and the Myers blocks it needs.
-int default_class(const Pass& p, bool use16, bool lean, int most, ClassKey& key, int64_t& blocks) {
+int default_class(const Pass& p, bool use16, bool lean, int most, uint64_t long_steps, ClassKey& key,
+                  int64_t& blocks) {
   if (p.kind == PK_MYERS) {
     int b = 1, lanes = 1;
     int rc = choose_myers_class(p.m, lean, most, b, lanes);
@@ -1228,7 +1229,7 @@ int default_class(const Pass& p, bool use16, bool lean, int most, ClassKey& key,
   int c = 4, lanes = 32;
   bool wide = false;
   PassKind kind = PK_AFFINE;
-  classify_affine(p, j, flags, wmax, use16, lean, kind, c, wide, lanes, default_lanes16());
+  classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, lanes, default_lanes16());
   const bool tb = p.want_cigar && p.kind != PK_LOCAL;
   key = ClassKey{kind, c, wide ? 1 : 0, tb ? 1 : 0, lanes};
   blocks = wmax;  // affine: the group's widest row
@@ -1253,12 +1254,21 @@ std::vector<ClassChoice> tune_candidates(const ClassKey& key, int64_t blocks) {
         if (!dup) out.push_back(ClassChoice{b, lanes});
       }
   } else if (is_wave(key.kind)) {
-    // The next classes that hold all the default class does (later plans' passes of it too).
-    for (int c = 0; c < sfk::kWaveN; ++c)
-      if (c != key.c && sfk::wave_cap(sfk::kWave[c]) >= sfk::wave_cap(sfk::kWave[key.c]) &&
-          (int)out.size() < 4 && (key.kind == PK_WAVE16 || sfk::kWave[c].q <= sfk::kWaveMaxX) &&
-          (c > key.c || key.c >= sfk::kWaveN0))
-        out.push_back(ClassChoice{c, key.lanes});
+    // The next classes of its range that hold all the default class does (later plans' passes of
+    // it too), and the first of the faster ones that does.
+    const int cap = sfk::wave_cap(sfk::kWave[key.c]);
+    const int ends[] = {sfk::kWaveFast, sfk::kWaveX, sfk::kWaveXFast, sfk::kWaveN};
+    const int from = key.kind == PK_WAVE16 ? 0 : 2, to = from + 2;
+    for (int u = from; u < to; ++u) {
+      const int first = u ? ends[u - 1] : 0;
+      const bool home = key.c >= first && key.c < ends[u];
+      int left = home ? 2 : (key.c < first ? 1 : 0);
+      for (int c = home ? key.c + 1 : first; c < ends[u] && left; ++c)
+        if (sfk::wave_cap(sfk::kWave[c]) >= cap) {
+          out.push_back(ClassChoice{c, key.lanes});
+          --left;
+        }
+    }
   } else if (!key.wide) {
     // The 16-bit classes for 16, 32 and 64 lanes a pass.
     auto classes16 = [](int lanes, const int*& cs, int& nc) {
@@ -1309,13 +1319,14 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   const bool use16 = allow16();
   const bool lean = plan_is_lean(P);
   const int most = most_pairs(P);
+  const uint64_t long_steps = plan_long_steps(P);
   // Group the passes by their default class.
   std::map<ClassKey, std::vector<size_t>> groups;
   std::map<ClassKey, int64_t> gblocks;
   for (size_t q = 0; q < P->passes.size(); ++q) {
     ClassKey k;
     int64_t blocks = 0;
-    int rc = default_class(P->passes[q], use16, lean, most, k, blocks);
+    int rc = default_class(P->passes[q], use16, lean, most, long_steps, k, blocks);
     if (rc) return rc;
     groups[k].push_back(q);
     gblocks[k] = std::max(gblocks[k], blocks);
@@ -1325,6 +1336,7 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   S.pool_bytes = P->pool_bytes;
   S.lean = lean;
   S.most = most;
+  S.long_steps = long_steps;
   void* uploaded = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CK(cudaEventCreate(&e0));

@@ -114,7 +114,7 @@ bool fits_wave(const Pass& p, const DJob& j, uint32_t flags, PassKind& kind) {
   const int64_t w = wave_width(j), shorter = std::min(p.m, p.n);
   if (p.m < 1 || p.n < 1 || w > (prefix ? 4 * (shorter + 1) + 64 : 2 * (shorter + 1))) return false;
   if (prefix && (int64_t)p.m > (int64_t)p.n + j.below) return false;  // ends past the text
-  if (w > sfk::wave_cap(sfk::kWave[prefix ? sfk::kWaveN - 1 : sfk::kWaveN0 - 1])) return false;
+  if (w > sfk::wave_cap(sfk::kWave[prefix ? sfk::kWaveXFast - 1 : sfk::kWaveFast - 1])) return false;
   const int64_t g = (int64_t)s.mat + 2 * s.ext;
   if (4 * g * (sfk::kWaveRebaseRows + 1) >
       std::min<int64_t>(0xffff - (int64_t)sfk::kWaveTop, sfk::kWaveNeg))
@@ -131,6 +131,40 @@ bool lean_plan(size_t np, int sms) { return np <= (size_t)sms * 20; }
 bool plan_is_lean(const sf_plan* P) {
   return P->lean >= 0 ? P->lean != 0 : lean_plan(P->passes.size(), P->ctx->sms);
 }
+// Row steps from which a pass takes its fastest class: all of them in a lean plan; else where one
+// warp would still run when the rest of the plan is done, and its longest pass on a team.  A row
+// step takes about 0.8 us on one warp among other kernels, 0.36 on a team; the plan's time is
+// estimated from its cells (2 a nanosecond with every scheduler busy, Myers 40).  Measured on
+// uneven batches: 25,000 pairs 18.4 -> 15.7 ms, 6,000 pairs 10.8 -> 8.3 (a team for every pass
+// past a third of these lengths: 20.1 and 10.1, its warps repeat lanes).
+uint64_t plan_long_steps(const sf_plan* P) {
+  if (P->long_steps) return P->long_steps;
+  if (plan_is_lean(P)) return 1;
+  constexpr int kT = 16;
+  double ns[kT] = {}, most[kT] = {};
+  parallel_chunks(P->passes.size(), 4096, kT, [&](size_t q0, size_t q1, int k) {
+    double t = 0, x = 0;
+    for (size_t q = q0; q < q1; ++q) {
+      const Pass& p = P->passes[q];
+      if (p.kind == PK_MYERS) {
+        t += (double)p.m * p.n / 40000.0;
+      } else {
+        const double band = p.band == SF_NOLIMIT ? p.n + 1.0 : 2.0 * (double)p.band + 1.0;
+        t += (double)p.m * std::min(p.n + 1.0, band) / 2000.0;
+        x = std::max(x, ((double)p.m + p.n) / 2);
+      }
+    }
+    ns[k] = t;
+    most[k] = x;
+  });
+  double total = 0, longest = 0;
+  for (int k = 0; k < kT; ++k) {
+    total += ns[k];
+    longest = std::max(longest, most[k]);
+  }
+  return std::max<uint64_t>(1, (uint64_t)(std::max(total, 360.0 * longest) / 800.0));
+}
+
 // Myers pairs a warp at most: four warps a scheduler before more pairs share one.
 int most_pairs(const sf_plan* P) {
   if (P->most) return P->most;
@@ -194,13 +228,15 @@ bool allow_w64() {
 // Kernel class of an affine or local pass: the anti-diagonal 16-bit kernel when the pass fits
 // it, else the packed 16-bit row kernel, else the 32-bit register kernel, else (rows wider than 32 * 48 cells) the wide-row kernel.
 void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax, bool use16,
-                     bool lean, PassKind& kind, int& c, bool& wide, int& lanes, int lanes16) {
+                     uint64_t long_steps, PassKind& kind, int& c, bool& wide, int& lanes,
+                     int lanes16) {
   wide = false;
   lanes = 32;
   if (use16 && lanes16 == 0 && fits_wave(p, j, flags, kind)) {
     const int64_t w = wave_width(j);
-    for (c = lean ? sfk::kWaveN0 : (kind == PK_WAVE16X ? sfk::kWaveX0 : 0); sfk::wave_cap(sfk::kWave[c]) < w; ++c) {
-    }
+    const bool fast = wave_steps(j, kind) >= long_steps;
+    c = kind == PK_WAVE16X ? (fast ? sfk::kWaveXFast : sfk::kWaveX) : (fast ? sfk::kWaveFast : 0);
+    while (sfk::wave_cap(sfk::kWave[c]) < w) ++c;
     return;
   }
   if (use16 && fits16(p, flags, wmax)) {
@@ -570,6 +606,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   const int lanes16 = default_lanes16();
   const bool lean = plan_is_lean(P);
   const int most = most_pairs(P);
+  const uint64_t long_steps = plan_long_steps(P);
   const TuneTable* tune = P->tune_override ? P->tune_override : &ctx->tune;
   const auto& word_of = S.word_of;
   auto& dj = S.dj;
@@ -683,7 +720,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       bool wide = false;
       PassKind kind = PK_AFFINE;
       int ln = 32;
-      classify_affine(p, j, flags, wmax, use16, lean, kind, c, wide, ln, lanes16);
+      classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, ln, lanes16);
       const bool tb = p.want_cigar && p.kind != PK_LOCAL;
       if (!wide) tuned(kind, c, false, tb, ln);
       TJob t{};
@@ -1057,14 +1094,16 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
       // As many pairs a warp as its lanes hold; in the fast classes fewer, while that leaves
       // schedulers empty.
       const bool my = b.kind == PK_MYERS;
-      const int64_t most =
-          my ? std::min(most_pairs(P), std::max(1, 32 / b.lanes)) : 32 / sfk::kWave[b.c].lanes;
-      const bool fast = my ? lean : b.c >= sfk::kWaveN0 && b.c < sfk::kWaveX0;
+      const int team = my ? (b.lanes > 32 ? b.lanes / 32 : 1) : sfk::wave_warps(sfk::kWave[b.c]);
+      const int64_t most = std::max(
+          1, my ? std::min(most_pairs(P), 32 / b.lanes) : 32 / sfk::kWave[b.c].lanes);
+      const bool fast = my ? lean
+                           : (b.c >= sfk::kWaveFast && b.c < sfk::kWaveX) || b.c >= sfk::kWaveXFast;
       b.per_warp = (int)(!fast ? most
                                : std::max<int64_t>(1, std::min<int64_t>(most, b.count / (4 * (int64_t)ctx->sms))));
       b.task_count = (b.count + b.per_warp - 1) / b.per_warp;
-      b.block = my && b.lanes > 32 ? b.lanes : 128;
-      b.grid = warps_grid((uint64_t)b.task_count * (my && b.lanes > 32 ? b.lanes / 32 : 1), b.block);
+      b.block = team > 1 ? 32 * team : 128;
+      b.grid = warps_grid((uint64_t)b.task_count * team, b.block);
     } else {
       // Two-warp passes: one pass per 64-thread block; otherwise a 4-warp block holds 4
       // passes (chains), or 8 with 16 lanes a pass.
@@ -1089,7 +1128,9 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
   S.tasks.clear();
   auto merges = [](const Bucket& x, const Bucket& y) {
     if (x.kind != y.kind) return false;
-    if (is_wave(x.kind)) return sfk::kWave[x.c].q == sfk::kWave[y.c].q && x.tb == y.tb;
+    if (is_wave(x.kind))
+      return sfk::kWave[x.c].q == sfk::kWave[y.c].q && x.tb == y.tb &&
+             sfk::wave_warps(sfk::kWave[x.c]) == sfk::wave_warps(sfk::kWave[y.c]);
     return x.c == y.c && (x.lanes > 32 ? x.lanes == y.lanes : y.lanes <= 32);
   };
   std::vector<uint8_t> done(nb, 0);
@@ -1115,8 +1156,8 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
         }
       }
       g.task_count = (uint32_t)S.tasks.size() - g.task_first;
-      g.grid = warps_grid((uint64_t)g.task_count * (b.kind == PK_MYERS && b.lanes > 32 ? b.lanes / 32 : 1),
-                          g.block);
+      const bool team = b.kind == PK_MYERS ? b.lanes > 32 : sfk::wave_warps(sfk::kWave[b.c]) > 1;
+      g.grid = warps_grid((uint64_t)g.task_count * (team ? g.block / 32 : 1), g.block);
     }
     g.stream = (int)(P->groups.size() % sf_context::kAux);
     P->groups.push_back(g);
@@ -1390,7 +1431,8 @@ int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* ev
         al.order = orders;
         al.tasks = tasks;
         al.njobs = task_count;
-        CK(sfk::launch_wave16(sfk::kWave[b.c].q, b.kind == PK_WAVE16X, b.tb, al, grid, bs));
+        CK(sfk::launch_wave16(sfk::kWave[b.c].q, b.kind == PK_WAVE16X, sfk::kWave[b.c].lanes > 32, b.tb,
+                              al, grid, b.block, bs));
       } else if (b.kind == PK_CHAIN16) {
         CK(sfk::launch_affine16_chain(b.c, al, b.grid, b.block, bs));
       } else if (b.kind == PK_AFFINE16 && b.lanes == 64) {
@@ -1719,13 +1761,13 @@ uint64_t plan_bytes_estimate(const std::vector<Pass>& passes, uint64_t pool_byte
     PassKind kind = PK_AFFINE;
     int ln = 32;
     uint64_t tb_wave = 0;
-    // The classes either way of `lean`: the larger traceback.
+    // The cheap and the fast class: the larger traceback.
     for (int lean = 0; lean < 2 && p.want_cigar && p.kind != PK_LOCAL; ++lean) {
-      classify_affine(p, j, flags, wmax, use16, lean != 0, kind, c, wide, ln, lanes16);
+      classify_affine(p, j, flags, wmax, use16, lean ? 0 : UINT64_MAX, kind, c, wide, ln, lanes16);
       if (!is_wave(kind)) break;
       tb_wave = std::max(tb_wave, sfk::wave_tb_words(sfk::kWave[c], wave_steps(j, kind)) * 4);
     }
-    classify_affine(p, j, flags, wmax, use16, false, kind, c, wide, ln, lanes16);
+    classify_affine(p, j, flags, wmax, use16, UINT64_MAX, kind, c, wide, ln, lanes16);
     if (p.want_cigar && p.kind != PK_LOCAL) {
       b += is_wave(kind)
                ? tb_wave

@@ -20,10 +20,11 @@ struct WaveClass {
   int q, lanes;
 };
 extern const WaveClass kWave[];
-// [0, kWaveN0): the cheapest a cell, Global; [kWaveN0, kWaveX0): the fastest a pass (Prefix
-// passes: those of up to kWaveMaxX words); [kWaveX0, kWaveN): the cheapest a cell, Prefix.
-constexpr int kWaveN0 = 24, kWaveX0 = 31, kWaveN = 43;
-constexpr int kWaveMaxX = 8;
+// Global passes: [0, kWaveFast) the cheapest a cell, [kWaveFast, kWaveX) the fastest a pass;
+// Prefix passes: [kWaveX, kWaveXFast) and [kWaveXFast, kWaveN) likewise.
+constexpr int kWaveFast = 24, kWaveX = 30, kWaveXFast = 42, kWaveN = 47;
+// More than 32 lanes: a team of warps, 30 lanes further on each.
+inline int wave_warps(const WaveClass& c) { return c.lanes > 32 ? (c.lanes - 2) / 30 : 1; }
 inline int wave_cap(const WaveClass& c) { return 4 * c.q * c.lanes; }
 // Traceback words of a pass of `steps` row steps: 2Q words a lane and group of four.
 inline uint64_t wave_tb_words(const WaveClass& c, uint64_t steps) {
@@ -36,8 +37,8 @@ __host__ __device__ constexpr int wave_blocks(int q, bool tb, bool ext) {
              : tb ? (q <= 4 ? 6 : q <= 6 ? 5 : q <= 8 ? 4 : 3) : (q <= 6 ? 8 : q <= 8 ? 6 : q <= 10 ? 5 : 4);
 }
 
-// prefix: Prefix passes, else Global ones.
-cudaError_t launch_wave16(int q, bool prefix, bool tb, const AffLaunch& a, int grid,
-                          cudaStream_t s);
+// prefix: Prefix passes, else Global ones.  block: 128, or a team's threads.
+cudaError_t launch_wave16(int q, bool prefix, bool team, bool tb, const AffLaunch& a, int grid,
+                          int block, cudaStream_t s);
 
 }  // namespace sfk

@@ -85,9 +85,11 @@ __device__ __forceinline__ uint32_t pick(uint32_t x, uint32_t y, uint32_t m) {
 // A stored word holds its four row steps' nibbles, each 8 low, on top of the word of the four
 // steps before, 16 bits up (the rows push and never clear): its low field needs 0x8888 added, its
 // high field that and the earlier word's low field taken off.
+//
+// L: the lanes of the layout; WL of them (a team: its first warp's) walk.
 template <int Q>
-__device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, bool has, int L, int l, int base,
-                          int32_t steps) {
+__device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, bool has, int L, int WL, int l,
+                          int base, int32_t steps) {
   const DJob J = a.jobs[jid];
   const TJob T = a.tjobs[jid];
   const DRes R = a.out[jid];
@@ -96,7 +98,7 @@ __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, bool has, int L
   const int32_t a1 = (bl >> 1) + 1;  // the row step that row-step index 0 stands for
   const int32_t gstride = (Q / 2) * L, groups = (steps + 3) >> 2;  // uint4s per group of four steps
   const uint4* tb = reinterpret_cast<const uint4*>(a.tb + J.tb_word);
-  const uint32_t lanes = L == 32 ? FULL : (1u << L) - 1u;
+  const uint32_t lanes = WL == 32 ? FULL : (1u << WL) - 1u;
   uint32_t* out = a.ops + T.ops_off;
   const uint32_t cap = T.ops_cap;
   uint32_t n_ops = 0, cur_op = 15, cur_len = 0;
@@ -150,7 +152,7 @@ __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, bool has, int L
     const bool bad = !done && !end && (i <= 0 || j <= 0 || K < 0 || K >= W || it > guard);
     const bool go = !done && !end && !bad;
     const int32_t rho = i + (K >> 1) - a1, h = rho >> 3, pos = 7 - (rho & 7);
-    if (go && (K < 4 * q0 || K >= 4 * q0 + 8 || q0 < 0 || h > H0 || h <= H0 - L)) {
+    if (go && (K < 4 * q0 || K >= 4 * q0 + 8 || q0 < 0 || h > H0 || h <= H0 - WL)) {
       q0 = max(K - 2, 0) >> 2;
       H0 = h;
       uint32_t w0[4], w1[4];
@@ -174,7 +176,7 @@ __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, bool has, int L
     if (l == d) nd &= ~((1u << (4 * pos)) - 1u);
     const uint32_t part = nd ? (uint32_t)(__ffs((int)nd) - 1) >> 2 : 8u;
     const uint32_t nf = ((__ballot_sync(FULL, nd != 0) >> base) & lanes) >> d;
-    const int32_t z = nf ? __ffs((int)nf) - 1 : L - d;  // whole lanes from lane d on
+    const int32_t z = nf ? __ffs((int)nf) - 1 : WL - d;  // whole lanes from lane d on
     const int32_t tail = (int32_t)__shfl_sync(FULL, part, min(base + d + z, 31));
     uint32_t op = 0, len = 0;
     if (end) {
@@ -244,15 +246,31 @@ __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, bool has, int L
   }
 }
 
+// A team's exchanges, by turns: each warp's lane 30 for the next warp's lane 0, its lane 1 for the
+// last warp's lane 31, and its largest field.
+template <int Q>
+struct WaveTeam {
+  uint4 up[2][4][Q], down[2][4][Q];
+  uint32_t top[2][4];
+  uint32_t task;
+};
+
 // One warp's passes, one per segment of L lanes: `jid` is the lane's own pass (any valid one
-// where `has` is false: computed, not stored).
-template <int Q, bool TB, bool EXT>
+// where `has` is false: computed, not stored).  TEAM: one pass over the block's warps, 30 lanes
+// further on each; a warp's outer lanes (but the first's first and the last's last) repeat its
+// neighbours' and are set right from them every 2Q row steps, which is as long as what they lack
+// at their outer side takes to cross them, a cell a step.
+template <int Q, bool TB, bool EXT, bool TEAM>
 __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t jid, bool has, int L,
-                                            int lane, int seg) {
+                                            int lane, int seg, WaveTeam<Q>* X) {
+  static_assert(!TEAM || !EXT, "teams run Global passes");
   constexpr int NT = (2 * Q + 15) / 16;  // 16-base registers of a lane's text (pattern) window
   constexpr int NC = (Q + 7) / 8;        // registers of a step's match bits
   static_assert(Q % 2 == 0 && Q >= 4 && Q <= 16, "words per lane and parity");
-  const int l = lane - seg * L;
+  const int w = TEAM ? threadIdx.x >> 5 : 0, NW = TEAM ? blockDim.x >> 5 : 1;
+  const int l = TEAM ? 30 * w + lane : lane - seg * L;
+  const bool leftmost = TEAM ? lane == 0 : l == 0, rightmost = TEAM ? lane == 31 : l == L - 1;
+  const bool own = !TEAM || ((lane > 0 || w == 0) && (lane < 31 || w == NW - 1));
   const DJob J = a.jobs[jid];
   const DParams S = a.params[jid];
   const int32_t m = (int32_t)J.m, n = (int32_t)J.n;
@@ -445,12 +463,14 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
 #pragma unroll
     for (int k = 0; k < Q; ++k) G[k] = HB[k] * one - g2;
     {
-      uint32_t sG = __shfl_up_sync(FULL, G[Q - 1], 1), sE = __shfl_up_sync(FULL, E[Q - 1], 1);
-      if (l == 0) sG = sE = kNegE;
-      const uint32_t gl = __byte_perm(sG, G[Q - 1], 0x5432), el = __byte_perm(sE, E[Q - 1], 0x5432);
+      // What the last word's cells hand to the right: its low half to the lane's own word 0.
+      const uint32_t er = __vmaxu2(G[Q - 1], E[Q - 1]);
+      uint32_t el = __shfl_up_sync(FULL, er, 1);
+      if (leftmost) el = kNegE;
+      el = __byte_perm(el, er, 0x5432);
 #pragma unroll
       for (int k = Q - 1; k >= 0; --k) {
-        const uint32_t et = __vmaxu2(k ? G[k ? k - 1 : 0] : gl, k ? E[k ? k - 1 : 0] : el);
+        const uint32_t et = k ? __vmaxu2(G[k ? k - 1 : 0], E[k ? k - 1 : 0]) : el;
         const uint32_t ft = __vmaxu2(G[k], F[k]);
         cell(k, cb, HA[k], et, ft, E[k], F[k], acc[TB ? 2 * k : 0]);
       }
@@ -477,17 +497,16 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
 #pragma unroll
     for (int k = 0; k < Q; ++k) G[k] = HA[k] * one - g2;
     {
-      uint32_t sG = __shfl_down_sync(FULL, G[0], 1), sF = __shfl_down_sync(FULL, F[0], 1);
-      if (l == L - 1) {
-        sG = kNegE;
-        sF = kNegF;
-      }
-      const uint32_t gu = __byte_perm(G[0], sG, 0x5432), fu = __byte_perm(F[0], sF, 0x5432);
+      // What word 0's cells hand down to the left, likewise.
+      const uint32_t fl = __vmaxu2(G[0], F[0]);
+      uint32_t fr = __shfl_down_sync(FULL, fl, 1);
+      if (rightmost) fr = kNegF;
+      fr = __byte_perm(fl, fr, 0x5432);
 #pragma unroll
       for (int k = 0; k < Q; ++k) {
         const uint32_t et = __vmaxu2(G[k], E[k]);
-        const uint32_t ft = __vmaxu2(k + 1 < Q ? G[k + 1 < Q ? k + 1 : 0] : gu,
-                                     k + 1 < Q ? F[k + 1 < Q ? k + 1 : 0] : fu);
+        const uint32_t ft =
+            k + 1 < Q ? __vmaxu2(G[k + 1 < Q ? k + 1 : 0], F[k + 1 < Q ? k + 1 : 0]) : fr;
         cell(k, cb, HB[k], et, ft, E[k], F[k], acc[TB ? 2 * k + 1 : 0]);
       }
     }
@@ -538,7 +557,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
     if constexpr (TB) {
       if ((r & 3) == 0) {
         // Four row steps: one 16-byte store per quad of words, lane-fastest.
-        if (has && r < N + 4) {
+        if (has && own && r < N + 4) {
 #pragma unroll
           for (int q = 0; q < Q / 2; ++q)
             tbp[q * L] = make_uint4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
@@ -552,7 +571,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
     if (!EXT && r == next_end) {
       // Passes whose cell (m, n) this row step computed.
       const int32_t Kend = n - m + bl, ke = (Kend >> 1) - k0;
-      if (has && r == N && ke >= 0 && ke < 2 * Q) {
+      if (has && own && r == N && ke >= 0 && ke < 2 * Q) {
         uint32_t u = 0;
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
@@ -571,17 +590,52 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       }
       next_end = __reduce_min_sync(FULL, has && N > r ? N : INT32_MAX);
     }
+    if constexpr (TEAM) {
+      if ((r & (2 * Q - 1)) == 0) {
+        const int turn = (r / (2 * Q)) & 1;
+        uint32_t v = 0;
+        if ((r & (kWRebase - 1)) == 0) {
+#pragma unroll
+          for (int k = 0; k < Q; ++k) v = __vimax3_u16x2(v, HA[k], HB[k]);
+          v = __reduce_max_sync(FULL, own ? max(v & 0xffffu, v >> 16) : 0u);
+          if (lane == 0) X->top[turn][w] = v;
+        }
+        if ((lane == 30 && w < NW - 1) || (lane == 1 && w > 0)) {
+          uint4* at = lane == 30 ? X->up[turn][w] : X->down[turn][w];
+#pragma unroll
+          for (int k = 0; k < Q; ++k) at[k] = make_uint4(HA[k], HB[k], E[k], F[k]);
+        }
+        __syncthreads();
+        if ((lane == 0 && w > 0) || (lane == 31 && w < NW - 1)) {
+          const uint4* at = lane == 0 ? X->up[turn][w - 1] : X->down[turn][w + 1];
+#pragma unroll
+          for (int k = 0; k < Q; ++k) {
+            const uint4 x = at[k];
+            HA[k] = x.x;
+            HB[k] = x.y;
+            E[k] = x.z;
+            F[k] = x.w;
+          }
+        }
+      }
+    }
     if ((r & (kWRebase - 1)) == 0) {
       // Each pass's largest field back to the top.
       uint32_t v = 0;
 #pragma unroll
       for (int k = 0; k < Q; ++k) v = __vimax3_u16x2(v, HA[k], HB[k]);
       v = max(v & 0xffffu, v >> 16);
-      for (int s = 1; s < L; s <<= 1) {
-        const uint32_t u = __shfl_down_sync(FULL, v, s);
-        if (l + s < L) v = max(v, u);
+      if constexpr (TEAM) {
+        const int turn = (r / (2 * Q)) & 1;
+        v = X->top[turn][0];
+        for (int u = 1; u < NW; ++u) v = max(v, X->top[turn][u]);
+      } else {
+        for (int s = 1; s < L; s <<= 1) {
+          const uint32_t u = __shfl_down_sync(FULL, v, s);
+          if (l + s < L) v = max(v, u);
+        }
+        v = __shfl_sync(FULL, v, min(seg * L, 31));
       }
-      v = __shfl_sync(FULL, v, min(seg * L, 31));
       const int32_t delta = (int32_t)(v - kH) - wtop;
       const uint32_t dd = ((uint32_t)(-delta) & 0xffffu) * kW2;
 #pragma unroll
@@ -596,8 +650,13 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
     }
   }
   if constexpr (TB) {
-    __syncwarp();
-    walk_wave<Q>(a, jid, has, L, l, min(seg * L, 31), N);
+    if constexpr (TEAM) {
+      __syncthreads();
+      if (w == 0) walk_wave<Q>(a, jid, true, L, 32, lane, 0, N);
+    } else {
+      __syncwarp();
+      walk_wave<Q>(a, jid, has, L, L, l, min(seg * L, 31), N);
+    }
   }
   __syncwarp();
 }
@@ -613,7 +672,8 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, EXT)) wave16_kern
     const uint2 task = a.tasks[q];
     const int L = (int)(task.y & 0xffu), np = (int)(task.y >> 8), seg = lane / L;
     const bool has = seg < np;
-    wave_passes<Q, TB, EXT>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, lane, seg);
+    wave_passes<Q, TB, EXT, false>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, lane, seg,
+                                   nullptr);
     if (a.njobs <= grid_tasks) break;
     uint32_t next = 0;
     if (lane == 0) next = atomicAdd(a.counter, 1u);
@@ -621,9 +681,35 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, EXT)) wave16_kern
   }
 }
 
+// One pass per block of two to four warps.
+template <int Q, bool TB>
+__global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, false)) wave16t_kernel(sfk::AffLaunch a) {
+  __shared__ WaveTeam<Q> X;
+  uint32_t q = blockIdx.x;
+  while (q < a.njobs) {
+    const uint2 task = a.tasks[q];
+    wave_passes<Q, TB, false, true>(a, a.order[task.x], true, (int)(task.y & 0xffu), threadIdx.x & 31,
+                                    0, &X);
+    if (a.njobs <= gridDim.x) break;
+    __syncthreads();
+    if (threadIdx.x == 0) X.task = gridDim.x + atomicAdd(a.counter, 1u);
+    __syncthreads();
+    q = X.task;
+  }
+}
+
 }  // namespace
 
 namespace sfk {
+
+template <int Q>
+cudaError_t launch_wave16t_q(bool tb, const AffLaunch& a, int grid, int block, cudaStream_t s) {
+  if (tb)
+    wave16t_kernel<Q, true><<<grid, block, 0, s>>>(a);
+  else
+    wave16t_kernel<Q, false><<<grid, block, 0, s>>>(a);
+  return cudaGetLastError();
+}
 
 template <int Q, bool EXT>
 cudaError_t launch_wave16_q(bool tb, const AffLaunch& a, int grid, cudaStream_t s) {
