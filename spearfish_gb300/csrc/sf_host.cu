@@ -1264,7 +1264,7 @@ std::vector<ClassChoice> tune_candidates(const ClassKey& key, int64_t blocks) {
       const bool home = key.c >= first && key.c < ends[u];
       int left = home ? 2 : (key.c < first ? 1 : 0);
       for (int c = home ? key.c + 1 : first; c < ends[u] && left; ++c)
-        if (sfk::wave_cap(sfk::kWave[c]) >= cap) {
+        if (sfk::wave_cap(sfk::kWave[c]) >= cap && (cap > 1024) == (sfk::wave_cap(sfk::kWave[c]) > 1024)) {
           out.push_back(ClassChoice{c, key.lanes});
           --left;
         }

@@ -102,8 +102,10 @@ uint64_t wave_steps(const DJob& j, int kind) {
 // for) and open >= 1.  Its fields hold four times the value: the largest rises by (mat + 2 ext) a
 // row step between rebases, and a band cell lies at most (mat + 2 ext) * width / 2 + open below it
 // (a gap from the best path, extension free in the kernel's potential); a Prefix pass's row
-// maxima rise by ext a cell across the band on either side of that.  A band much wider than the
+// maxima rise by ext a cell across the band above that, and where a row starts left of the text
+// (`below` cells at most) from the cells no path reaches.  A band much wider than the
 // text (or the pattern) is left to the row kernels, whose rows stop at the text's end.
+constexpr int64_t kWaveNarrow = 1024;  // wave_wide classes hold more cells, no others do
 bool fits_wave(const Pass& p, const DJob& j, uint32_t flags, PassKind& kind) {
   if (p.kind != PK_AFFINE || (flags & (F_FULL | F_CUT))) return false;
   const bool prefix = p.mode == SF_PREFIX;
@@ -114,14 +116,17 @@ bool fits_wave(const Pass& p, const DJob& j, uint32_t flags, PassKind& kind) {
   const int64_t w = wave_width(j), shorter = std::min(p.m, p.n);
   if (p.m < 1 || p.n < 1 || w > (prefix ? 4 * (shorter + 1) + 64 : 2 * (shorter + 1))) return false;
   if (prefix && (int64_t)p.m > (int64_t)p.n + j.below) return false;  // ends past the text
-  if (w > sfk::wave_cap(sfk::kWave[prefix ? sfk::kWaveXFast - 1 : sfk::kWaveFast - 1])) return false;
-  const int64_t g = (int64_t)s.mat + 2 * s.ext;
-  if (4 * g * (sfk::kWaveRebaseRows + 1) >
-      std::min<int64_t>(0xffff - (int64_t)sfk::kWaveTop, sfk::kWaveNeg))
-    return false;
   kind = prefix ? PK_WAVE16X : PK_WAVE16;
-  return 4 * (g * (w / 2 + 2) + 2 * (int64_t)s.open + 16) + (prefix ? 8 * (int64_t)s.ext * (w + 1) : 0) <=
-         (int64_t)sfk::kWaveTop - (int64_t)sfk::kWaveNeg;
+  const sfk::WaveClass& last = sfk::kWave[prefix ? sfk::kWaveN - 1 : sfk::kWaveX - 1];
+  if (w > sfk::wave_cap(last)) return false;
+  const int64_t g = (int64_t)s.mat + 2 * s.ext, open = s.open, ext = prefix ? s.ext : 0;
+  const bool wide = prefix && w > kWaveNarrow;
+  const int64_t top = sfk::wave_top(wide), neg = sfk::wave_neg(wide);
+  if (4 * g * (sfk::kWaveRebaseRows + 1) > std::min<int64_t>(0xffff - top, neg)) return false;
+  auto below_top = [&](int64_t cells) { return 4 * (g * (cells / 2 + 2) + 2 * open + 16); };
+  int64_t room = below_top(w);
+  if (prefix) room = std::max(room, below_top(j.below + 1) + 4 * ext * (j.below + 2));
+  return room + 4 * ext * (w + 1) <= top - neg;
 }
 
 // Few passes: each takes the fastest class.  Measured on 2 kb passes with band 128 and CIGARs:
@@ -149,7 +154,9 @@ uint64_t plan_long_steps(const sf_plan* P) {
       if (p.kind == PK_MYERS) {
         t += (double)p.m * p.n / 40000.0;
       } else {
-        const double band = p.band == SF_NOLIMIT ? p.n + 1.0 : 2.0 * (double)p.band + 1.0;
+        const double band = p.band == SF_NOLIMIT ? p.n + 1.0
+                                                 : 2.0 * (double)p.band + 1.0 +
+                                                       std::fabs((double)p.n - (double)p.m);
         t += (double)p.m * std::min(p.n + 1.0, band) / 2000.0;
         x = std::max(x, ((double)p.m + p.n) / 2);
       }

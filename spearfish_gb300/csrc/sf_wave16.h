@@ -8,10 +8,13 @@ namespace sfk {
 
 struct AffLaunch;
 
-// Fields: the largest of a pass sits at kWaveTop after a rebase (each kWaveRebaseRows row
-// steps), cells no path reaches at kWaveNeg; no more than kWaveNeg is taken off at a rebase, nor
+// Fields: the largest of a pass sits at wave_top after a rebase (each kWaveRebaseRows row
+// steps), cells no path reaches at wave_neg; no more than wave_neg is taken off at a rebase, nor
 // does the largest rise past the field in between.
-constexpr uint32_t kWaveTop = 0xf000u, kWaveNeg = 0x1000u;
+// The widest Prefix classes leave less at either end.
+__host__ __device__ constexpr bool wave_wide(int q, int lanes) { return q * lanes > 256; }
+__host__ __device__ constexpr uint32_t wave_top(bool wide) { return wide ? 0xfc00u : 0xf000u; }
+__host__ __device__ constexpr uint32_t wave_neg(bool wide) { return wide ? 0x400u : 0x1000u; }
 constexpr int kWaveRebaseRows = 32;
 
 // A class: Q words (2Q band cells) a lane and parity, L lanes a pass, 32 / L passes a warp;
@@ -22,7 +25,7 @@ struct WaveClass {
 extern const WaveClass kWave[];
 // Global passes: [0, kWaveFast) the cheapest a cell, [kWaveFast, kWaveX) the fastest a pass;
 // Prefix passes: [kWaveX, kWaveXFast) and [kWaveXFast, kWaveN) likewise.
-constexpr int kWaveFast = 24, kWaveX = 30, kWaveXFast = 42, kWaveN = 47;
+constexpr int kWaveFast = 28, kWaveX = 37, kWaveXFast = 52, kWaveN = 62;
 // More than 32 lanes: a team of warps, 30 lanes further on each.
 inline int wave_warps(const WaveClass& c) { return c.lanes > 32 ? (c.lanes - 2) / 30 : 1; }
 inline int wave_cap(const WaveClass& c) { return 4 * c.q * c.lanes; }
@@ -31,6 +34,9 @@ inline uint64_t wave_tb_words(const WaveClass& c, uint64_t steps) {
   return (steps + 3) / 4 * 2 * (uint64_t)c.q * (uint64_t)c.lanes;
 }
 
+// A team's warps at most, and the blocks of that many per SM its registers are held to.
+__host__ __device__ constexpr int wave_most_warps(int q) { return q <= 4 ? 7 : 4; }
+__host__ __device__ constexpr int wave_team_blocks(int q, bool tb) { return q <= 4 && !tb ? 4 : 3; }
 // 4-warp blocks per SM the registers are held to.
 __host__ __device__ constexpr int wave_blocks(int q, bool tb, bool ext) {
   return ext ? (tb ? (q <= 4 ? 5 : q <= 6 ? 4 : 3) : (q <= 4 ? 6 : q <= 6 ? 5 : 4))

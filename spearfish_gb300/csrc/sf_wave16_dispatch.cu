@@ -15,26 +15,30 @@ cudaError_t launch_wave16x_6(bool, const AffLaunch&, int, cudaStream_t);
 cudaError_t launch_wave16x_8(bool, const AffLaunch&, int, cudaStream_t);
 
 cudaError_t launch_wave16t_4(bool, const AffLaunch&, int, int, cudaStream_t);
+cudaError_t launch_wave16xt_4(bool, const AffLaunch&, int, int, cudaStream_t);
+cudaError_t launch_wave16xt_8(bool, const AffLaunch&, int, int, cudaStream_t);
 
 // Classes by the cells they hold, within each range.  The cheapest a band cell: a row step costs
 // a warp about 32 Q + 60 issue slots whatever it holds, so many cells a lane and many passes a
 // warp; Prefix passes keep two more registers a word and stop at 8 words.  The fastest a pass:
-// four words a lane, over two to four warps for bands past 512 cells (two words a lane over up to
+// four words a lane, over two to seven warps for bands past 512 cells (two words a lane over up to
 // seven warps took as long: a row step's chain through both shuffles is 270 cycles, 400 with
 // traceback).
 const WaveClass kWave[kWaveN] = {
     {4, 3},  {4, 4},  {6, 3},  {4, 5},  {6, 4},   {10, 3},  {8, 4},   {12, 3},
     {10, 4}, {12, 4}, {10, 5}, {12, 5}, {8, 8},   {12, 6},  {10, 8},  {12, 8},
     {10, 10}, {12, 10}, {8, 16}, {10, 16}, {12, 16}, {8, 32}, {10, 32}, {12, 32},
-    {4, 8}, {4, 16}, {4, 32}, {4, 62}, {4, 92}, {4, 122},
+    {4, 122}, {4, 152}, {4, 182}, {4, 212},
+    {4, 8}, {4, 16}, {4, 32}, {4, 62}, {4, 92}, {4, 122}, {4, 152}, {4, 182}, {4, 212},
     {4, 3}, {4, 4}, {6, 3}, {4, 5}, {6, 4}, {8, 4}, {8, 5}, {8, 6}, {8, 8}, {8, 10}, {8, 16}, {8, 32},
-    {4, 8}, {4, 16}, {4, 32}, {6, 32}, {8, 32}};
+    {8, 62}, {8, 92}, {8, 122},
+    {4, 8}, {4, 16}, {4, 32}, {4, 62}, {8, 32}, {4, 92}, {4, 122}, {4, 152}, {4, 182}, {4, 212}};
 
 cudaError_t launch_wave16(int q, bool prefix, bool team, bool tb, const AffLaunch& a, int grid,
                           int block, cudaStream_t s) {
   if (team) {
-    if (prefix || q != 4) return cudaErrorInvalidValue;
-    return launch_wave16t_4(tb, a, grid, block, s);
+    if (q == 4) return (prefix ? launch_wave16xt_4 : launch_wave16t_4)(tb, a, grid, block, s);
+    return prefix && q == 8 ? launch_wave16xt_8(tb, a, grid, block, s) : cudaErrorInvalidValue;
   }
   switch (q) {
     case 4: return prefix ? launch_wave16x_4(tb, a, grid, s) : launch_wave16_4(tb, a, grid, s);

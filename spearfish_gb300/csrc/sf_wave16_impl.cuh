@@ -48,7 +48,6 @@
 
 namespace {
 
-constexpr uint32_t kWTop = sfk::kWaveTop, kWNeg = sfk::kWaveNeg;
 constexpr uint32_t kW2 = 0x00010001u;
 constexpr int kWRebase = sfk::kWaveRebaseRows;
 
@@ -247,11 +246,14 @@ __device__ void walk_wave(const sfk::AffLaunch& a, uint32_t jid, bool has, int L
 }
 
 // A team's exchanges, by turns: each warp's lane 30 for the next warp's lane 0, its lane 1 for the
-// last warp's lane 31, and its largest field.
-template <int Q>
+// last warp's lane 31, its largest field, and whether the pass has ended.
+template <int Q, bool EXT>
 struct WaveTeam {
-  uint4 up[2][4][Q], down[2][4][Q];
-  uint32_t top[2][4];
+  static constexpr int kWarps = sfk::wave_most_warps(Q);
+  uint4 up[2][kWarps][Q], down[2][kWarps][Q];
+  uint2 row[EXT ? 2 : 1][EXT ? kWarps : 1][Q];
+  uint32_t top[2][kWarps];
+  uint32_t ended[2];
   uint32_t task;
 };
 
@@ -262,8 +264,9 @@ struct WaveTeam {
 // at their outer side takes to cross them, a cell a step.
 template <int Q, bool TB, bool EXT, bool TEAM>
 __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t jid, bool has, int L,
-                                            int lane, int seg, WaveTeam<Q>* X) {
-  static_assert(!TEAM || !EXT, "teams run Global passes");
+                                            int lane, int seg, WaveTeam<Q, EXT>* X) {
+  const bool wide = TEAM && EXT && sfk::wave_wide(Q, L);
+  const uint32_t kWTop = sfk::wave_top(wide), kWNeg = sfk::wave_neg(wide);
   constexpr int NT = (2 * Q + 15) / 16;  // 16-base registers of a lane's text (pattern) window
   constexpr int NC = (Q + 7) / 8;        // registers of a step's match bits
   static_assert(Q % 2 == 0 && Q >= 4 && Q <= 16, "words per lane and parity");
@@ -289,7 +292,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
   const uint32_t g2 = 4u * (uint32_t)S.open * kW2;
   const uint32_t v1 = (uint32_t)(S.mat + S.mis), v4 = 4u * v1;
   constexpr uint32_t kH = TB ? 2u : 0u, kF = TB ? 1u : 0u;  // a clean field's low bits
-  constexpr uint32_t kNegH = (kWNeg + kH) * kW2, kNegE = kWNeg * kW2, kNegF = (kWNeg + kF) * kW2;
+  const uint32_t kNegH = (kWNeg + kH) * kW2, kNegE = kWNeg * kW2, kNegF = (kWNeg + kF) * kW2;
 
   // EXT: M's potential rises by 4 ext a step, so the top leaves room for a row's width of them.
   const int32_t wtop = EXT ? (int32_t)kWTop - 4 * S.ext * (W + 1) : (int32_t)kWTop;
@@ -387,7 +390,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
   // The band's last cell: one lane's word and half, in the even or the odd step.
   const bool last_odd = (W - 1) & 1;
   const int32_t last_e = kw - k0;  // 0 .. 2Q - 1 in the lane that holds it
-  const bool books = EXT && has && last_e >= 0 && last_e < 2 * Q;
+  const bool books = EXT && has && own && last_e >= 0 && last_e < 2 * Q;
   const bool any_even = EXT && __any_sync(FULL, books && !last_odd);
   const bool any_odd = EXT && __any_sync(FULL, books && last_odd);
   const uint32_t pad0 = l == 0 && bl != below ? 0xffff0000u : ~0u;  // offset 0 is a pad
@@ -478,7 +481,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
     if constexpr (EXT) {
       uint32_t sM = __shfl_up_sync(FULL, M[Q - 1], 1);
       const uint32_t sK = __shfl_up_sync(FULL, MK[Q - 1], 1);
-      if (l == 0) sM = kNegH | kW2;
+      if (leftmost) sM = kNegH | kW2;
       const uint32_t ml = __byte_perm(sM, M[Q - 1], 0x5432), pl = __byte_perm(sK, MK[Q - 1], 0x5432);
 #pragma unroll
       for (int k = Q - 1; k >= 0; --k) {
@@ -566,7 +569,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       }
     }
     if constexpr (EXT) {
-      if ((r & 3) == 0 && !__any_sync(FULL, books && !fin)) break;
+      if (!TEAM && (r & 3) == 0 && !__any_sync(FULL, books && !fin)) break;
     }
     if (!EXT && r == next_end) {
       // Passes whose cell (m, n) this row step computed.
@@ -604,8 +607,14 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
           uint4* at = lane == 30 ? X->up[turn][w] : X->down[turn][w];
 #pragma unroll
           for (int k = 0; k < Q; ++k) at[k] = make_uint4(HA[k], HB[k], E[k], F[k]);
+          if constexpr (EXT)
+            if (lane == 30)
+#pragma unroll
+              for (int k = 0; k < Q; ++k) X->row[turn][w][k] = make_uint2(M[k], MK[k]);
         }
+        if (EXT && books) X->ended[turn] = fin;
         __syncthreads();
+        if (EXT && X->ended[turn]) break;
         if ((lane == 0 && w > 0) || (lane == 31 && w < NW - 1)) {
           const uint4* at = lane == 0 ? X->up[turn][w - 1] : X->down[turn][w + 1];
 #pragma unroll
@@ -616,6 +625,14 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
             E[k] = x.z;
             F[k] = x.w;
           }
+          if constexpr (EXT)
+            if (lane == 0)
+#pragma unroll
+              for (int k = 0; k < Q; ++k) {
+                const uint2 x = X->row[turn][w - 1][k];
+                M[k] = x.x;
+                MK[k] = x.y;
+              }
         }
       }
     }
@@ -681,14 +698,15 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, EXT)) wave16_kern
   }
 }
 
-// One pass per block of two to four warps.
-template <int Q, bool TB>
-__global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, false)) wave16t_kernel(sfk::AffLaunch a) {
-  __shared__ WaveTeam<Q> X;
+// One pass per block of two to seven warps.
+template <int Q, bool TB, bool EXT>
+__global__ void __launch_bounds__(32 * sfk::wave_most_warps(Q), sfk::wave_team_blocks(Q, TB))
+    wave16t_kernel(sfk::AffLaunch a) {
+  __shared__ WaveTeam<Q, EXT> X;
   uint32_t q = blockIdx.x;
   while (q < a.njobs) {
     const uint2 task = a.tasks[q];
-    wave_passes<Q, TB, false, true>(a, a.order[task.x], true, (int)(task.y & 0xffu), threadIdx.x & 31,
+    wave_passes<Q, TB, EXT, true>(a, a.order[task.x], true, (int)(task.y & 0xffu), threadIdx.x & 31,
                                     0, &X);
     if (a.njobs <= gridDim.x) break;
     __syncthreads();
@@ -702,12 +720,12 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, false)) wave16t_k
 
 namespace sfk {
 
-template <int Q>
+template <int Q, bool EXT>
 cudaError_t launch_wave16t_q(bool tb, const AffLaunch& a, int grid, int block, cudaStream_t s) {
   if (tb)
-    wave16t_kernel<Q, true><<<grid, block, 0, s>>>(a);
+    wave16t_kernel<Q, true, EXT><<<grid, block, 0, s>>>(a);
   else
-    wave16t_kernel<Q, false><<<grid, block, 0, s>>>(a);
+    wave16t_kernel<Q, false, EXT><<<grid, block, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -3,6 +3,6 @@
 
 namespace sfk {
 cudaError_t launch_wave16t_4(bool tb, const AffLaunch& a, int grid, int block, cudaStream_t s) {
-  return launch_wave16t_q<4>(tb, a, grid, block, s);
+  return launch_wave16t_q<4, false>(tb, a, grid, block, s);
 }
 }  // namespace sfk

@@ -1,0 +1,8 @@
+// Anti-diagonal 16-bit kernels with 4 words a lane and parity, a team of warps a Prefix pass.
+#include "sf_wave16_impl.cuh"
+
+namespace sfk {
+cudaError_t launch_wave16xt_4(bool tb, const AffLaunch& a, int grid, int block, cudaStream_t s) {
+  return launch_wave16t_q<4, true>(tb, a, grid, block, s);
+}
+}  // namespace sfk

@@ -273,7 +273,7 @@ def test_prefix(ctx, packed):
     out, kinds = _run_prefix(ctx, rows, scores)
     wave = {(c, n) for k, c, n in kinds if k == "wave16x"}
     want = {(16, 3), (24, 4), (32, 4), (32, 10), (32, 32)} if packed else \
-        {(16, 8), (16, 16), (16, 32), (24, 32), (32, 32)}
+        {(16, 8), (16, 16), (16, 32), (16, 62), (32, 32)}
     assert wave >= want, sorted(kinds)
     _check_prefix(rows[:checked], out, scores)
     # The row kernels give the same.
@@ -299,5 +299,48 @@ def test_prefix_long(ctx):
                 rows.append((q, t, band, len(t) + 60, xd, 5, 1, int(rng.integers(0, 2))))
     scores = (R.ONT, R.HIFI)
     out, kinds = _run_prefix(ctx, rows, scores)
-    assert ("wave16x", 32, 32) in kinds, kinds  # (the widest bands of all go to the row kernels)
+    assert ("wave16x", 16, 32) in kinds and ("wave16x", 16, 92) in kinds, kinds
     _check_prefix(rows, out, scores)
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_wide_bands(ctx, packed):
+    """Bands past one warp's cells: Global and Prefix classes of teams filled to their last cell,
+    missed or passed by one; paths along either edge (the largest spread of a row), X-drop stops
+    in every part, score sets on both sides of what the widest classes take."""
+    rng = np.random.default_rng(2661 + packed)
+    scores = (R.ONT, R.HIFI, (1, 6, 4, 3), (3, 2, 900, 1), (5, 4, 4, 2), (0, 2, 1, 1))
+    rows = []
+    for cap in (992, 1024, 1472, 1952, 1984, 2432, 2912, 2944, 3392):
+        for w in (cap - 1, cap, cap + 1):
+            for edge in (0, 1):
+                band = int(rng.integers(1, 90)) if edge else (w - 2) // 2
+                extra = w - 2 * band - 2 + (w % 2)  # below + above + 1 = w, `below` odd or even
+                m = max(band // 2 + 40, w // 4 + 20) + int(rng.integers(0, 60))
+                q = rng.integers(0, 4, m).tolist()
+                fill = rng.integers(0, 4, max(0, extra + band)).tolist()
+                good = R.mutate(q, R.rand_edits(rng, int(m * rng.choice([0.0, 0.1])), m))
+                t = (fill + good if edge and rng.random() < 0.5 else good + fill)[:m + extra]
+                t += rng.integers(0, 4, m + extra - len(t)).tolist()
+                xd = int(rng.choice([8, 50, 2000, R.I32_MAX]))
+                rows.append((q, t, band, len(t), xd, 5, 1, len(rows) % len(scores)))
+                rows.append((q, t, band, None, R.I32_MAX, 0, int(edge), (len(rows) // 2) % 3))
+    checked = len(rows)
+    if packed:
+        rows += [(p, t, b, None, R.I32_MAX, 0, 0, sci) for p, t, b, _, sci in _ballast() * 2]
+    out, kinds = _run_prefix(ctx, rows, scores)
+    wave = {(c, n) for k, c, n in kinds if k == "wave16x"}
+    want = {(32, 62), (32, 92), (32, 122)} if packed else \
+        {(16, 62), (16, 92), (16, 122), (16, 152), (16, 182), (16, 212)}
+    assert wave >= want, sorted(kinds)
+    _check_prefix(rows[:checked], out, scores)
+
+    grows = []
+    for w in (1536, 1537, 1952, 1953, 2432, 2912, 3392, 3393):
+        band, extra = (w - 2) // 2, (w - 2) % 2
+        for d in (-band, 0, band):
+            p, t = _shifted(rng, band + 30 + int(rng.integers(0, 90)), d)
+            grows.append((p, t + rng.integers(0, 4, extra).tolist(), band, 1, len(grows) % 2))
+    gout, gkinds = _run(ctx, grows + (_ballast() if packed else []), scores)
+    assert {(16, 152), (16, 182), (16, 212)} <= {(c, n) for k, c, n in gkinds if k == "wave16"}
+    _check(grows, gout, scores)
