@@ -114,6 +114,7 @@ bool fits_wave(const Pass& p, const DJob& j, uint32_t flags, PassKind& kind) {
   if (s.mat < 0 || s.mat > 1000 || s.ext < 0 || s.ext > 1000 || s.mis != 2 * s.ext) return false;
   if (s.open < 1 || s.open > 900) return false;
   const int64_t w = wave_width(j), shorter = std::min(p.m, p.n);
+  if (4 * ((int64_t)s.mat + 2 * s.ext) * ((int64_t)p.m + p.n) >= 1 << 30) return false;
   if (p.m < 1 || p.n < 1 || w > (prefix ? 4 * (shorter + 1) + 64 : 2 * (shorter + 1))) return false;
   if (prefix && (int64_t)p.m > (int64_t)p.n + j.below) return false;  // ends past the text
   kind = prefix ? PK_WAVE16X : PK_WAVE16;
@@ -136,40 +137,65 @@ bool lean_plan(size_t np, int sms) { return np <= (size_t)sms * 20; }
 bool plan_is_lean(const sf_plan* P) {
   return P->lean >= 0 ? P->lean != 0 : lean_plan(P->passes.size(), P->ctx->sms);
 }
-// Row steps from which a pass takes its fastest class: all of them in a lean plan; else where one
-// warp would still run when the rest of the plan is done, and its longest pass on a team.  A row
-// step takes about 0.8 us on one warp among other kernels, 0.36 on a team; the plan's time is
-// estimated from its cells (2 a nanosecond with every scheduler busy, Myers 40).  Measured on
-// uneven batches: 25,000 pairs 18.4 -> 15.7 ms, 6,000 pairs 10.8 -> 8.3 (a team for every pass
-// past a third of these lengths: 20.1 and 10.1, its warps repeat lanes).
+// Row steps from which a pass takes its fastest class.  The plan's longest passes do, as long as
+// their band cells together leave schedulers idle in the cheaper classes (kFastCells: 2 kb passes
+// of band 128, 1,200 of them 0.64 ms on 4 words x 32 lanes against 1.37 on 12 x 6; 4,000 equal
+// passes are a quarter faster in the cheap classes).  In a plan of many passes only those do that
+// would still run on one warp when the rest is done: a row step takes about 0.8 us on one warp
+// among other kernels, 0.36 on a team, and the plan's time is estimated from its cells (2 a
+// nanosecond with every scheduler busy, 3.5 without traceback, Myers 40).  Measured on uneven
+// batches: 25,000 pairs 18.4 -> 15.7 ms, 6,000 pairs 10.8 -> 8.3 (a team for every pass past a
+// third of these lengths: 20.1 and 10.1, its warps repeat lanes).
 uint64_t plan_long_steps(const sf_plan* P) {
   if (P->long_steps) return P->long_steps;
-  if (plan_is_lean(P)) return 1;
-  constexpr int kT = 16;
-  double ns[kT] = {}, most[kT] = {};
-  parallel_chunks(P->passes.size(), 4096, kT, [&](size_t q0, size_t q1, int k) {
+  constexpr int kT = 16, kBins = 128;
+  constexpr double kFastCells = 550000;
+  auto shape = [](const Pass& p, double& w, double& steps) {
+    const double m = p.m, n = p.n, far = std::fabs(n - m);
+    w = p.band == SF_NOLIMIT ? m + n + 1 : 2.0 * (double)p.band + far + 2.0;
+    w = std::min(w, 2.0 * (n + 1.0));
+    steps = p.mode == SF_PREFIX ? m + w / 2 : (m + n) / 2;
+  };
+  const size_t np = P->passes.size();
+  std::vector<double> ns(kT), most(kT), cells((size_t)kT * kBins);
+  parallel_chunks(np, 4096, kT, [&](size_t q0, size_t q1, int k) {
     double t = 0, x = 0;
     for (size_t q = q0; q < q1; ++q) {
       const Pass& p = P->passes[q];
       if (p.kind == PK_MYERS) {
         t += (double)p.m * p.n / 40000.0;
       } else {
-        const double band = p.band == SF_NOLIMIT ? p.n + 1.0
-                                                 : 2.0 * (double)p.band + 1.0 +
-                                                       std::fabs((double)p.n - (double)p.m);
-        t += (double)p.m * std::min(p.n + 1.0, band) / 2000.0;
-        x = std::max(x, ((double)p.m + p.n) / 2);
+        double w, steps;
+        shape(p, w, steps);
+        t += w * steps / (p.want_cigar ? 2000.0 : 3500.0);
+        x = std::max(x, steps);
       }
     }
     ns[k] = t;
     most[k] = x;
   });
-  double total = 0, longest = 0;
+  double total = 0, longest = 1;
   for (int k = 0; k < kT; ++k) {
     total += ns[k];
     longest = std::max(longest, most[k]);
   }
-  return std::max<uint64_t>(1, (uint64_t)(std::max(total, 360.0 * longest) / 800.0));
+  parallel_chunks(np, 4096, kT, [&](size_t q0, size_t q1, int k) {
+    for (size_t q = q0; q < q1; ++q) {
+      if (P->passes[q].kind == PK_MYERS) continue;
+      double w, steps;
+      shape(P->passes[q], w, steps);
+      cells[(size_t)k * kBins + (size_t)std::min(kBins - 1.0, steps / longest * kBins)] += w;
+    }
+  });
+  double sum = 0;
+  int bin = kBins;
+  for (; bin > 0; --bin) {
+    for (int k = 0; k < kT; ++k) sum += cells[(size_t)k * kBins + (size_t)bin - 1];
+    if (sum > kFastCells) break;
+  }
+  double least = bin ? longest * bin / kBins + 1 : 1;
+  if (!plan_is_lean(P)) least = std::max(least, std::max(total, 360.0 * longest) / 800.0);
+  return (uint64_t)std::max(1.0, least);
 }
 
 // Myers pairs a warp at most: four warps a scheduler before more pairs share one.
@@ -232,6 +258,23 @@ bool allow_w64() {
   return !(env && env[0] == '0');
 }
 
+// Whether a Prefix pass takes less time on the anti-diagonal kernel's class c than on the row
+// kernel, which does no more than the pattern's rows, each no wider than the text, while the
+// anti-diagonals run on until the last row has crossed the band: a short pattern in a wide band
+// is the row kernel's.  Nanoseconds a row step and a row, with the device full (a pass's share;
+// measured over 8,000 passes of widths 60-1,500, patterns 0.3-4 times that) and alone (600).
+bool wave_is_less(const Pass& p, const DJob& j, int64_t wmax, int c, bool alone) {
+  const sfk::WaveClass& k = sfk::kWave[c];
+  const double steps = (double)wave_steps(j, PK_WAVE16X), words = (double)((wmax + 31) / 32);
+  const int per_warp = std::max(1, 32 / k.lanes), warps = sfk::wave_warps(k);
+  const bool tb = p.want_cigar;
+  const double wave = alone ? (tb ? 0.36 : 0.25) + 0.015 * k.q * warps / 4
+                            : (tb ? 0.17 + 0.042 * k.q : 0.095 + 0.03 * k.q) * warps / per_warp;
+  const double row = alone ? (tb ? 0.6 + 0.0105 * words : 0.44 + 0.01 * words)
+                           : (tb ? 0.2 + 0.0243 * words : 0.14 + 0.0165 * words);
+  return steps * wave <= (double)p.m * row;
+}
+
 // Kernel class of an affine or local pass: the anti-diagonal 16-bit kernel when the pass fits
 // it, else the packed 16-bit row kernel, else the 32-bit register kernel, else (rows wider than 32 * 48 cells) the wide-row kernel.
 void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax, bool use16,
@@ -244,7 +287,7 @@ void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax,
     const bool fast = wave_steps(j, kind) >= long_steps;
     c = kind == PK_WAVE16X ? (fast ? sfk::kWaveXFast : sfk::kWaveX) : (fast ? sfk::kWaveFast : 0);
     while (sfk::wave_cap(sfk::kWave[c]) < w) ++c;
-    return;
+    if (kind == PK_WAVE16 || !fits16(p, flags, wmax) || wave_is_less(p, j, wmax, c, fast)) return;
   }
   if (use16 && fits16(p, flags, wmax)) {
     if (lanes16 == 16)

@@ -36,11 +36,15 @@ inline uint64_t wave_tb_words(const WaveClass& c, uint64_t steps) {
 
 // A team's warps at most, and the blocks of that many per SM its registers are held to.
 __host__ __device__ constexpr int wave_most_warps(int q) { return q <= 4 ? 7 : 4; }
-__host__ __device__ constexpr int wave_team_blocks(int q, bool tb) { return q <= 4 && !tb ? 4 : 3; }
-// 4-warp blocks per SM the registers are held to.
+__host__ __device__ constexpr int wave_team_blocks(int q, bool tb, bool ext) {
+  return q > 4 ? 3 : ext ? 2 : tb ? 3 : 4;
+}
+// 4-warp blocks per SM the registers are held to: as many as cost no spill or reload of constants
+// (600 2 kb windows, four words: 1.00 ms at five blocks, 0.82 at four; 20,000 Global pairs, ten
+// and twelve words: 5.19 ms at three, 5.09 at four).
 __host__ __device__ constexpr int wave_blocks(int q, bool tb, bool ext) {
-  return ext ? (tb ? (q <= 4 ? 5 : q <= 6 ? 4 : 3) : (q <= 4 ? 6 : q <= 6 ? 5 : 4))
-             : tb ? (q <= 4 ? 6 : q <= 6 ? 5 : q <= 8 ? 4 : 3) : (q <= 6 ? 8 : q <= 8 ? 6 : q <= 10 ? 5 : 4);
+  return ext ? (tb ? (q <= 6 ? 4 : 3) : 4)
+             : tb ? (q <= 4 ? 6 : q <= 6 ? 5 : 4) : (q <= 6 ? 8 : q <= 8 ? 6 : q <= 10 ? 5 : 4);
 }
 
 // prefix: Prefix passes, else Global ones.  block: 128, or a team's threads.

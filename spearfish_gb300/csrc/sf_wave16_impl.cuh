@@ -30,10 +30,12 @@
 //
 // Prefix passes (EXT) need each row's largest value and its leftmost column, in row order: for
 // the clip score, its cell and the X-drop stop, and for the last row's score.  Both travel along
-// the row from left to right, a cell a step, as E does: M(K) = max(M(K - 1), H(K)) with the
-// leftmost offset it was reached at, and leave the band at its last cell, where one lane keeps
-// the pass's books, one row a row step, in row order.  The rows that run ahead of a stop are
-// computed and left out.  Columns past the text count for nothing (the last rows of a pass).
+// the row from left to right, an even and the odd cell after it a row step, M = max(M, H even,
+// H odd) with the leftmost offset it was reached at, and leave the band at its last cell, where
+// one lane keeps the pass's books in row order, four rows at a time.  The rows that run ahead of
+// a stop are computed and left out.  Columns past the text count for nothing (the last rows).
+// 8,000 2 kb windows (band 128, CIGARs) on GB300: row kernel 8.75 ms, a cell a step with its books
+// a row at a time 5.95, now 4.83; without CIGARs 7.2 -> 2.94.
 //
 // Bound: the ALU pipe (one instruction every other cycle a scheduler): 8.5 of a word's 14.5
 // instructions with traceback, 4.5 of 6.5 without.  With 12 words a lane and 6 lanes a pass a
@@ -63,7 +65,14 @@ __device__ __forceinline__ uint32_t low_fields(int32_t c, int r) {
   return (uint32_t)((uint64_t(1) << (2 * k)) - 1u) & 0x55555555u;
 }
 
-// (x & m) | o in one instruction, with the constants in registers.
+// x * I + y on the multiply-add pipe, whatever I is: the maxima need the other one.
+template <int I>
+__device__ __forceinline__ uint32_t mad(uint32_t x, uint32_t y) {
+  uint32_t d;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "n"(I), "r"(y));
+  return d;
+}
+// (x & m) | o in one instruction.
 __device__ __forceinline__ uint32_t and_or(uint32_t x, uint32_t m, uint32_t o) {
   uint32_t d;
   asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(x), "r"(m), "r"(o));
@@ -257,6 +266,22 @@ struct WaveTeam {
   uint32_t task;
 };
 
+// A Prefix pass's books, in fields' units (four to one), without the potential, kept off the registers.  A
+// row's maximum is in the potential of offset 2 kw + 1 (an odd last cell: + 2): pot4 at row 0, row4
+// a row.  best (at row i, offset k): the largest so far; a row more than xd below it ends the pass.
+struct WaveBooks {
+  int32_t best, i, k, clip, xd, pot4, row4, row0, m, tail, at;
+};
+// Prefix passes: the words of the lane that holds a band's last cell over four row steps, by the
+// pass's place in its warp, for that lane to pick one by its offset (a select over registers
+// costs the ALU pipe 4 Q a row step), and the books.
+template <int Q, bool EXT>
+struct WaveLast {
+  static constexpr int kQuads = EXT ? (Q + 3) / 4 : 1, kSlots = EXT ? 11 : 1;
+  uint4 w[kSlots][4][3][kQuads];  // the last slot takes what the other lanes write
+  WaveBooks books[kSlots];
+};
+
 // One warp's passes, one per segment of L lanes: `jid` is the lane's own pass (any valid one
 // where `has` is false: computed, not stored).  TEAM: one pass over the block's warps, 30 lanes
 // further on each; a warp's outer lanes (but the first's first and the last's last) repeat its
@@ -264,7 +289,8 @@ struct WaveTeam {
 // at their outer side takes to cross them, a cell a step.
 template <int Q, bool TB, bool EXT, bool TEAM>
 __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t jid, bool has, int L,
-                                            int lane, int seg, WaveTeam<Q, EXT>* X) {
+                                            int lane, int seg, WaveLast<Q, EXT>& Z,
+                                            WaveTeam<Q, EXT>* X) {
   const bool wide = TEAM && EXT && sfk::wave_wide(Q, L);
   const uint32_t kWTop = sfk::wave_top(wide), kWNeg = sfk::wave_neg(wide);
   constexpr int NT = (2 * Q + 15) / 16;  // 16-base registers of a lane's text (pattern) window
@@ -285,14 +311,13 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
   const int32_t kw = (W - 1) >> 1;  // the pair of offsets the band's last cell is in
   const int32_t N = EXT ? m + kw - a1 + 1 : (m + n + 1) >> 1;
 
-  const uint32_t one = (uint32_t)opaque_one(), mone = 0u - one;
-  const uint32_t sixteen = one << 4, four = one << 2, mfour = 0u - four;
   // The tag masks, opaque so that each use is one three-input instruction.
+  const uint32_t one = (uint32_t)opaque_one();
   const uint32_t mlow = 0xfffcfffcu * one, kone = kW2 * one, ktwo = 2u * kone, msel = ~kone;
-  const uint32_t g2 = 4u * (uint32_t)S.open * kW2;
+  const uint32_t mg2 = 0u - 4u * (uint32_t)S.open * kW2;
   const uint32_t v1 = (uint32_t)(S.mat + S.mis), v4 = 4u * v1;
   constexpr uint32_t kH = TB ? 2u : 0u, kF = TB ? 1u : 0u;  // a clean field's low bits
-  const uint32_t kNegH = (kWNeg + kH) * kW2, kNegE = kWNeg * kW2, kNegF = (kWNeg + kF) * kW2;
+  const uint32_t kNegH = (kWNeg + kH) * kW2, kNegE = kWNeg * kW2, kNegF = (kWNeg + kF) * kW2, kNegM = (kWNeg + 2u) * kW2;
 
   // EXT: M's potential rises by 4 ext a step, so the top leaves room for a row's width of them.
   const int32_t wtop = EXT ? (int32_t)kWTop - 4 * S.ext * (W + 1) : (int32_t)kWTop;
@@ -309,7 +334,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
     F[k] = kNegF;
     if constexpr (TB) acc[2 * k] = acc[2 * k + 1] = 0;
     if constexpr (EXT) {
-      M[k] = kNegH | kW2;
+      M[k] = kNegM;
       MK[k] = 0;
     }
   }
@@ -375,17 +400,19 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       cb[NC - 1] = __byte_perm(eq[0], hi, 0x7632);
     }
   };
-  // EXT: the row maximum and its offset after word k's cells, from those left of them.  h: the
-  // cells' values, or 0 where they count for nothing; kc: their offsets.  The maximum is kept one
-  // step ahead (4 ext more) and with bit 0 set, which no H has: a tie keeps the left one, and bit
-  // 0 says which won.
-  const uint32_t m4 = 4u * (uint32_t)S.ext * kW2 + kW2, kc0 = 4u * (uint32_t)Q * (uint32_t)l * kW2;
-  const uint32_t ones = 0xffffu * one;
-  auto row_max = [&](uint32_t h, uint32_t kc, uint32_t ml, uint32_t pl, uint32_t& mo, uint32_t& po) {
-    const uint32_t x = __vmaxu2(ml, h);
-    const uint32_t kept = x & kW2;
-    po = pick(pl, kc, kept * ones);
-    mo = kept * mone + (x * one + m4);
+  // EXT: a row's largest value, left to right a pair of offsets (an even and an odd cell, both of
+  // one row step) at a time.  It is kept a pair ahead (8 ext more) with bit 1 set, which no cell
+  // has there, so that a tie keeps the left one and bit 1 says which won; an even cell has bit 0
+  // set, which then stands for the parity of the maximum's offset.  MK: the pair's even offset.
+  const uint32_t e4 = 4u * (uint32_t)S.ext * kW2;
+  const uint32_t ha = e4 + (TB ? ~0u * kW2 : kW2), hb = 0u - 2u * kW2;  // cells' low bits: kH
+  const uint32_t m8 = 2u * e4 + 2u * kW2, kc0 = 4u * (uint32_t)Q * (uint32_t)l * kW2;
+  auto row_max = [&](uint32_t xa, uint32_t xb, uint32_t kc, uint32_t ml, uint32_t pl, uint32_t& mo,
+                     uint32_t& po) {
+    const uint32_t x = __vimax3_u16x2(ml, xa, xb);
+    const uint32_t kept = x & (2u * kW2);
+    po = pick(pl, kc, mad<0x7fff>(kept, 0u));
+    mo = mad<-1>(kept, mad<1>(x, m8));
   };
   // The band's last cell: one lane's word and half, in the even or the odd step.
   const bool last_odd = (W - 1) & 1;
@@ -394,23 +421,32 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
   const bool any_even = EXT && __any_sync(FULL, books && !last_odd);
   const bool any_odd = EXT && __any_sync(FULL, books && last_odd);
   const uint32_t pad0 = l == 0 && bl != below ? 0xffff0000u : ~0u;  // offset 0 is a pad
-  int32_t rmax_f = 0, rmax_k = 0;  // the finished row's largest field and its offset
-  auto take_last = [&](bool mine) {
-    uint32_t u = 0, p = 0;
+  constexpr int kSpare = WaveLast<Q, EXT>::kSlots - 1, kArray = 8 * WaveLast<Q, EXT>::kQuads;
+  auto* const last = Z.w[books ? seg : kSpare];
+  auto* const even_last = Z.w[books && !last_odd ? seg : kSpare];
+  auto* const odd_last = Z.w[books && last_odd ? seg : kSpare];
+  auto put_last = [&](uint4* to, const uint32_t (&x)[EXT ? Q : 1]) {
+    if constexpr (EXT) {
 #pragma unroll
-    for (int k = 0; k < (EXT ? Q : 1); ++k) {
-      if (last_e == k || last_e == Q + k) {
-        u = M[k];
-        p = MK[k];
-      }
-    }
-    if (mine) {
-      rmax_f = (int32_t)(last_e >= Q ? u >> 16 : u & 0xffffu);
-      rmax_k = (int32_t)(last_e >= Q ? p >> 16 : p & 0xffffu);
+      for (int q = 0; q < Q / 4; ++q)
+        to[q] = make_uint4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+      if constexpr (Q % 4 != 0) *reinterpret_cast<uint2*>(to + Q / 4) = make_uint2(x[Q - 2], x[Q - 1]);
     }
   };
-  Book b;
-  bool fin = false;
+  volatile WaveBooks& bk = Z.books[books ? seg : kSpare];
+  bool open = books;
+  if constexpr (EXT) {
+    bk.at = !books ? 0 : 2 * (last_e >= Q ? last_e - Q : last_e) + (last_e >= Q ? 1 : 0);
+    bk.best = 4 * Book{}.clip_best;
+    bk.i = bk.k = 0;
+    bk.clip = S.flags & F_CLIP;
+    bk.xd = 4 * min(max(S.xdrop, -(1 << 27)), 1 << 28);
+    bk.pot4 = 4 * S.ext * (W - bl + (last_odd ? 1 : 0));
+    bk.row4 = 8 * S.ext;
+    bk.row0 = a1 - 4 - kw;         // the first row of the four steps before row step 0
+    bk.m = m;
+    bk.tail = n + bl - 2 * kw;     // rows after this: the band's last even cell lies past the text
+  }
   // Row steps from which some cell lies past the text.
   const int32_t r_tail = __reduce_min_sync(FULL, has ? n + bl - kw - a1 : INT32_MAX);
   // Word k's cells: e and f are the gap values entering them; h their diagonal, then their H.
@@ -423,10 +459,10 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       const uint32_t ht = __vimax3_u16x2(dg, fc, ec);
       const uint32_t hs = and_or(ht, mlow, ktwo);
       const uint32_t y = pick(et, ft, msel);  // E opened << 1 | F extended
-      ac = ac * sixteen + y;
-      ac = ec * mone + ac;
-      ac = ht * four + ac;
-      ac = hs * mfour + ac;  // (winner - 2) << 2
+      ac = mad<16>(ac, y);
+      ac = mad<-1>(ec, ac);
+      ac = mad<4>(ht, ac);
+      ac = mad<-4>(hs, ac);  // (winner - 2) << 2
       h = hs;
       eo = ec;
       fo = fc;
@@ -460,11 +496,17 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
     auto in_text = [&](int k, int32_t t) -> uint32_t {
       return (k <= t ? 0xffffu : 0u) | (Q + k <= t ? 0xffff0000u : 0u);
     };
+    [[maybe_unused]] uint32_t sM = 0, sK = 0;
+    if constexpr (EXT) {
+      sM = __shfl_up_sync(FULL, M[Q - 1], 1);
+      sK = __shfl_up_sync(FULL, MK[Q - 1], 1);
+      if (leftmost) sM = kNegM;
+    }
     uint32_t G[Q], cb[NC];
     // Even step: offsets 2k from their odd neighbours.
     matches(Me, cb);
 #pragma unroll
-    for (int k = 0; k < Q; ++k) G[k] = HB[k] * one - g2;
+    for (int k = 0; k < Q; ++k) G[k] = mad<1>(HB[k], mg2);
     {
       // What the last word's cells hand to the right: its low half to the lane's own word 0.
       const uint32_t er = __vmaxu2(G[Q - 1], E[Q - 1]);
@@ -478,27 +520,13 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
         cell(k, cb, HA[k], et, ft, E[k], F[k], acc[TB ? 2 * k : 0]);
       }
     }
-    if constexpr (EXT) {
-      uint32_t sM = __shfl_up_sync(FULL, M[Q - 1], 1);
-      const uint32_t sK = __shfl_up_sync(FULL, MK[Q - 1], 1);
-      if (leftmost) sM = kNegH | kW2;
-      const uint32_t ml = __byte_perm(sM, M[Q - 1], 0x5432), pl = __byte_perm(sK, MK[Q - 1], 0x5432);
-#pragma unroll
-      for (int k = Q - 1; k >= 0; --k) {
-        uint32_t h = k == 0 ? HA[0] & pad0 : HA[k];
-        if constexpr (TAIL) h &= in_text(k, te);
-        row_max(h, kc0 + (uint32_t)(2 * k) + ((uint32_t)(2 * (Q + k)) << 16), k ? M[k ? k - 1 : 0] : ml,
-                k ? MK[k ? k - 1 : 0] : pl, M[k], MK[k]);
-      }
-      if (any_even) take_last(!last_odd);
-    }
 #pragma unroll
     for (int q = 0; q < NT; ++q) T[q] = __funnelshift_r(T[q], T[q + 1], 2);
     T[NT] >>= 2;
     // Odd step: offsets 2k + 1 from their even neighbours.
     matches(Mo, cb);
 #pragma unroll
-    for (int k = 0; k < Q; ++k) G[k] = HA[k] * one - g2;
+    for (int k = 0; k < Q; ++k) G[k] = mad<1>(HA[k], mg2);
     {
       // What word 0's cells hand down to the left, likewise.
       const uint32_t fl = __vmaxu2(G[0], F[0]);
@@ -514,19 +542,40 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       }
     }
     if constexpr (EXT) {
+      uint32_t ml[Q], pl[Q];
+      ml[0] = __byte_perm(sM, M[Q - 1], 0x5432);
+      pl[0] = __byte_perm(sK, MK[Q - 1], 0x5432);
 #pragma unroll
-      for (int k = 0; k < Q; ++k) {
-        uint32_t h = HB[k];
-        if constexpr (TAIL) h &= in_text(k, te - 1);
-        row_max(h, kc0 + (uint32_t)(2 * k + 1) + ((uint32_t)(2 * (Q + k) + 1) << 16), M[k], MK[k], M[k],
-                MK[k]);
+      for (int k = 1; k < Q; ++k) {
+        ml[k] = M[k - 1];
+        pl[k] = MK[k - 1];
       }
-      if (any_odd) take_last(last_odd);
+      if (any_even) {
+        // An even last cell: what stands left of its pair, and the even cells.
+        put_last(even_last[r & 3][0], ml);
+        put_last(even_last[r & 3][1], pl);
+        put_last(even_last[r & 3][2], HA);
+      }
+#pragma unroll
+      for (int k = Q - 1; k >= 0; --k) {
+        uint32_t xa = mad<1>(HA[k], ha), xb = TB ? mad<1>(HB[k], hb) : HB[k];
+        if (k == 0) xa &= pad0;
+        if constexpr (TAIL) {
+          xa &= in_text(k, te);
+          xb &= in_text(k, te - 1);
+        }
+        row_max(xa, xb, mad<1>(kc0, (uint32_t)(2 * k) + ((uint32_t)(2 * (Q + k)) << 16)), ml[k], pl[k],
+                M[k], MK[k]);
+      }
+      if (any_odd) {
+        put_last(odd_last[r & 3][0], M);
+        put_last(odd_last[r & 3][1], MK);
+      }
     }
 #pragma unroll
     for (int q = NT - 1; q > 0; --q) P[q] = __funnelshift_l(P[q - 1], P[q], 2);
     P[0] = __funnelshift_l(Pn, P[0], 2);
-    Pn = Pn * four;
+    Pn = mad<4>(Pn, 0u);
   };
 
   for (int32_t r = 0; r < Rtot;) {
@@ -535,25 +584,72 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
     else
       row_step(r, std::true_type{});
     ++r;
-    if constexpr (EXT) {
-      // Row i's books (align.rs:2580-2640), in the lane that holds the band's last cell.
-      const int32_t i = a1 + r - 1 - kw;
-      if (books && !fin && i >= 1) {
-        const int32_t rmax = (((rmax_f & ~3) + off) >> 2) - S.ext * (2 * i + W - bl);
-        const uint32_t col = (uint32_t)(i - bl + rmax_k);
-        const int32_t hi = min(i + above, n);
-        if ((S.flags & F_CLIP) && rmax > b.clip_best) {
-          b.clip_best = rmax;
-          if (S.flags & F_CELL) {
-            b.ci = (uint32_t)i;
-            b.cj = col;
+    if (EXT && (r & 3) == 0) {
+      // The books of the four rows these steps finished (align.rs:2580-2640), in the lane that
+      // holds the band's last cell; all lanes go along.
+      const int32_t i0 = r + bk.row0, row4 = bk.row4, v0 = off - bk.pot4 - row4 * i0;
+      const int32_t best = bk.best, xd = bk.xd;
+      const bool clip = bk.clip;
+      const uint16_t* const fs = reinterpret_cast<const uint16_t*>(last[0][0]) + bk.at;
+      constexpr int kRow = 3 * kArray, kArray2 = 2 * kArray;
+      constexpr uint32_t ha1 = TB ? ~0u : 1u;
+      const uint32_t x4 = row4 / 2 + ha1;
+      auto row_of = [&](int t, uint32_t& k) {
+        uint32_t f = fs[t * kRow];
+        k = fs[t * kRow + kArray] | (~f & 1u);
+        if (any_even) {
+          // An even last cell is yet to be counted, where it lies in the text.
+          const uint32_t x = fs[t * kRow + kArray2] + x4;
+          if (!last_odd && x > f && i0 + t <= bk.tail) {
+            f = x;
+            k = (uint32_t)(2 * kw);
           }
         }
-        const bool stop = (S.flags & F_CLIP) && rmax < sat_sub(b.clip_best, S.xdrop);
-        if (stop || i == m) {
-          a.out[jid] = DRes{stop ? NEG : rmax, b.clip_best, 0, NEG, stop ? 0u : col, b.ci, b.cj,
-                            (uint32_t)hi, (uint32_t)i, (uint32_t)i, band_cells(i, below, above, n)};
-          fin = true;
+        return (int32_t)f;
+      };
+      // Together: the largest row, the first of equals (3 - t in the low bits), where no row can
+      // end the pass.
+      int32_t top = INT32_MIN, least = INT32_MAX;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        uint32_t f = fs[t * kRow];
+        if (any_even) f = max(f, last_odd ? 0u : fs[t * kRow + kArray2] + x4);
+        const int32_t v = (int32_t)and_or(f, ~3u, 3u - t) + (v0 - t * row4);
+        top = max(top, v);
+        least = min(least, v);
+      }
+      const bool slow = open && (i0 < 1 || i0 + 3 >= bk.m || i0 + 3 > bk.tail ||
+                                 (clip && least - 3 + xd < max(best, top)));
+      if (!__any_sync(FULL, slow)) {
+        if (clip && (top & ~3) > best) {
+          const int t = 3 - (top & 3);
+          uint32_t pk;
+          row_of(t, pk);
+          bk.best = top & ~3;
+          bk.i = i0 + t;
+          bk.k = (int32_t)pk;
+        }
+      } else {
+#pragma unroll 1
+        for (int t = 0; t < 4; ++t) {
+          const int32_t i = i0 + t;
+          uint32_t pk;
+          const int32_t v = (row_of(t, pk) & ~3) + (v0 - t * row4);
+          if (!open || i < 1) continue;
+          if (clip && v > bk.best) {
+            bk.best = v;
+            bk.i = i;
+            bk.k = (int32_t)pk;
+          }
+          const bool stop = clip && v + xd < bk.best;
+          if (stop || i == m) {
+            const bool cell = clip && (S.flags & F_CELL) && bk.i;
+            a.out[jid] = DRes{stop ? NEG : v >> 2, clip ? bk.best >> 2 : Book{}.clip_best, 0, NEG,
+                              stop ? 0u : (uint32_t)(i - bl) + pk, cell ? (uint32_t)bk.i : 0u,
+                              cell ? (uint32_t)(bk.i - bl + bk.k) : 0u, (uint32_t)min(i + above, n),
+                              (uint32_t)i, (uint32_t)i, band_cells(i, below, above, n)};
+            open = false;
+          }
         }
       }
     }
@@ -569,7 +665,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       }
     }
     if constexpr (EXT) {
-      if (!TEAM && (r & 3) == 0 && !__any_sync(FULL, books && !fin)) break;
+      if (!TEAM && (r & 3) == 0 && !__any_sync(FULL, open)) break;
     }
     if (!EXT && r == next_end) {
       // Passes whose cell (m, n) this row step computed.
@@ -612,7 +708,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
 #pragma unroll
               for (int k = 0; k < Q; ++k) X->row[turn][w][k] = make_uint2(M[k], MK[k]);
         }
-        if (EXT && books) X->ended[turn] = fin;
+        if (EXT && books) X->ended[turn] = !open;
         __syncthreads();
         if (EXT && X->ended[turn]) break;
         if ((lane == 0 && w > 0) || (lane == 31 && w < NW - 1)) {
@@ -661,7 +757,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
         HB[k] = __viaddmax_u16x2(HB[k], dd, kNegH);
         E[k] = __viaddmax_u16x2(E[k], dd, kNegE);
         F[k] = __viaddmax_u16x2(F[k], dd, kNegF);
-        if constexpr (EXT) M[k] = __viaddmax_u16x2(M[k], dd, kNegH | kW2);
+        if constexpr (EXT) M[k] = __viaddmax_u16x2(M[k], dd, kNegM);
       }
       off += delta;
     }
@@ -681,6 +777,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
 template <int Q, bool TB, bool EXT>
 __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, EXT)) wave16_kernel(sfk::AffLaunch a) {
   const int lane = threadIdx.x & 31;
+  __shared__ WaveLast<Q, EXT> Z[4];
   // The first task by place; the queue hands out those after the grid's first ones.
   const uint32_t grid_tasks = (gridDim.x * blockDim.x) >> 5;
   // (Every q is a shuffle's: the compiler then keeps what follows from it in uniform registers.)
@@ -690,7 +787,7 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, EXT)) wave16_kern
     const int L = (int)(task.y & 0xffu), np = (int)(task.y >> 8), seg = lane / L;
     const bool has = seg < np;
     wave_passes<Q, TB, EXT, false>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, lane, seg,
-                                   nullptr);
+                                   Z[threadIdx.x >> 5], nullptr);
     if (a.njobs <= grid_tasks) break;
     uint32_t next = 0;
     if (lane == 0) next = atomicAdd(a.counter, 1u);
@@ -700,14 +797,15 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, EXT)) wave16_kern
 
 // One pass per block of two to seven warps.
 template <int Q, bool TB, bool EXT>
-__global__ void __launch_bounds__(32 * sfk::wave_most_warps(Q), sfk::wave_team_blocks(Q, TB))
+__global__ void __launch_bounds__(32 * sfk::wave_most_warps(Q), sfk::wave_team_blocks(Q, TB, EXT))
     wave16t_kernel(sfk::AffLaunch a) {
   __shared__ WaveTeam<Q, EXT> X;
+  __shared__ WaveLast<Q, EXT> Z;
   uint32_t q = blockIdx.x;
   while (q < a.njobs) {
     const uint2 task = a.tasks[q];
     wave_passes<Q, TB, EXT, true>(a, a.order[task.x], true, (int)(task.y & 0xffu), threadIdx.x & 31,
-                                    0, &X);
+                                    0, Z, &X);
     if (a.njobs <= gridDim.x) break;
     __syncthreads();
     if (threadIdx.x == 0) X.task = gridDim.x + atomicAdd(a.counter, 1u);

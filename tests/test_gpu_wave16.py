@@ -255,6 +255,12 @@ def test_prefix(ctx, packed):
                 # The window's geometry is the text's: below + above + 1 = w.
                 rows.append((p[:len(t) - extra] if cut else p, t, band, len(t), 50, 5, 1, cap % 3 % 2))
                 add(p, t, band, extend=False)
+        if cap >= 512:
+            # (Short patterns in wide bands run on the row kernel.)
+            for w in (cap - 1, cap):
+                p, t = _shifted(rng, 2 * cap, cap // 3)
+                rows.append((p, t + rng.integers(0, 4, w % 2).tolist(), (w - 2) // 2, None,
+                             R.I32_MAX, 0, 1, w % 2))
     for m in list(range(1, 60)) + [127, 128, 129, 400]:
         p, t = _noisy(rng, m, 0.15)
         add(p, t + rng.integers(0, 4, int(rng.integers(0, 30))).tolist(), int(rng.integers(0, 20)))
@@ -325,6 +331,10 @@ def test_wide_bands(ctx, packed):
                 xd = int(rng.choice([8, 50, 2000, R.I32_MAX]))
                 rows.append((q, t, band, len(t), xd, 5, 1, len(rows) % len(scores)))
                 rows.append((q, t, band, None, R.I32_MAX, 0, int(edge), (len(rows) // 2) % 3))
+        q, t = _noisy(rng, 2 * cap, 0.1)
+        for xd in (50, R.I32_MAX):
+            rows.append((q, t + rng.integers(0, 4, cap - 200 - len(t) + 2 * cap).tolist(), 98,
+                         3 * cap - 200, xd, 5, 1, len(rows) % 2))
     checked = len(rows)
     if packed:
         rows += [(p, t, b, None, R.I32_MAX, 0, 0, sci) for p, t, b, _, sci in _ballast() * 2]
