@@ -4,6 +4,7 @@
 // and results at the C ABI (include/sf_align.h).
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
@@ -141,11 +142,11 @@ bool plan_is_lean(const sf_plan* P) {
 // their band cells together leave schedulers idle in the cheaper classes (kFastCells: 2 kb passes
 // of band 128, 1,200 of them 0.64 ms on 4 words x 32 lanes against 1.37 on 12 x 6; 4,000 equal
 // passes are a quarter faster in the cheap classes).  In a plan of many passes only those do that
-// would still run on one warp when the rest is done: a row step takes about 0.8 us on one warp
-// among other kernels, 0.36 on a team, and the plan's time is estimated from its cells (2 a
+// would still run on one warp when the rest is done: a row step takes about 1 us on one warp
+// among other kernels, 0.5 on a team, and the plan's time is estimated from its cells (2 a
 // nanosecond with every scheduler busy, 3.5 without traceback, Myers 40).  Measured on uneven
-// batches: 25,000 pairs 18.4 -> 15.7 ms, 6,000 pairs 10.8 -> 8.3 (a team for every pass past a
-// third of these lengths: 20.1 and 10.1, its warps repeat lanes).
+// batches, no team / 0.8 / 1 / 1.2 / 1.6 us: 25,000 pairs 18.5 / 16.9 / 14.4 / 14.5 / 17.6 ms,
+// 6,000 pairs 10.9 / 6.9 / 6.9 / 7.0 / 7.2 (teams repeat lanes, and take the schedulers' turns).
 uint64_t plan_long_steps(const sf_plan* P) {
   if (P->long_steps) return P->long_steps;
   constexpr int kT = 16, kBins = 128;
@@ -194,7 +195,7 @@ uint64_t plan_long_steps(const sf_plan* P) {
     if (sum > kFastCells) break;
   }
   double least = bin ? longest * bin / kBins + 1 : 1;
-  if (!plan_is_lean(P)) least = std::max(least, std::max(total, 360.0 * longest) / 800.0);
+  if (!plan_is_lean(P)) least = std::max(least, std::max(total, 360.0 * longest) / 1000.0);
   return (uint64_t)std::max(1.0, least);
 }
 
@@ -315,6 +316,20 @@ void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax,
   }
   kind = p.kind == PK_LOCAL ? PK_LOCAL : PK_AFFINE;
   choose_affine_class(wmax, c, wide);
+}
+
+// A pass's own time in cycles, roughly, on an SM it has to itself (measured: anti-diagonal row
+// steps 445 at four words with traceback, 980 at twelve; a row kernel's row 0.6 us + 0.0105 a
+// cell a lane, 0.44 + 0.01 without traceback; Myers columns 65 a block).
+uint64_t pass_cycles(const Pass& p, const DJob& j, PassKind kind, int c, uint64_t chunks) {
+  const bool tb = p.want_cigar;
+  if (is_wave(kind)) {
+    const uint64_t q = (uint64_t)sfk::kWave[c].q, step = tb ? 180 + 66 * q : 100 + 36 * q;
+    return wave_steps(j, kind) * step * (kind == PK_WAVE16X ? 7 : 5) / 5;
+  }
+  const uint64_t rows = std::max<uint32_t>(p.m, 1);
+  if (kind == PK_AFFINE16) return rows * (tb ? 1150 + 20 * (uint64_t)c : 850 + 19 * (uint64_t)c);
+  return rows * 100 * ((uint64_t)c * std::max<uint64_t>(chunks, 1) + 8);
 }
 
 // The autotuner's override for a pass's default class, if it chose one.
@@ -754,8 +769,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
         m.k = p.k;
         if (p.mode != SF_INFIX && (uint64_t)p.k < (uint64_t)p.m + p.n) kcut[worker] = true;
         per[q] = {Key2{PK_MYERS, b, 0, 0, lanes},
-                  // A step takes about (70 + 25 B) / 45 of a row's unit.
-                  Item{sl, (uint64_t)p.n, ((uint64_t)p.n + (uint64_t)lanes) * ((uint64_t)b + 3u) / 2u}};
+                  Item{sl, (uint64_t)p.n, ((uint64_t)p.n + (uint64_t)lanes) * 65u * (uint64_t)b}};
         has_item[q] = 1;
         pass_work[q] = pass_lat[q] = 0;
         continue;
@@ -802,11 +816,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       pr.ext = p.sc.ext;
       const uint64_t work = (uint64_t)std::max<uint32_t>(p.m, 1) * (uint64_t)std::max<int64_t>(wmax, 1);
       pass_work[q] = work;
-      // Anti-diagonal row steps: about (60 + 32 Q) / 45 of this unit (a row's 45 cycles).
-      const uint64_t row_cost = is_wave(kind)
-                                    ? 2u + (uint64_t)(2 * sfk::kWave[c].q / 3)
-                                    : (uint64_t)c * (wide ? (uint64_t)wide_chunks(c, wmax) : 1u) + 8u;
-      pass_lat[q] = (uint64_t)std::max<uint32_t>(p.m, 1) * row_cost;
+      pass_lat[q] = pass_cycles(p, j, kind, c, wide ? (uint64_t)wide_chunks(c, wmax) : 0);
       has_item[q] = !P->chained[q];
       if (has_item[q]) per[q] = {Key2{kind, c, wide, tb, ln}, Item{sl, work, pass_lat[q]}};
       dj[sl] = j;
@@ -1184,6 +1194,7 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
     return x.c == y.c && (x.lanes > 32 ? x.lanes == y.lanes : y.lanes <= 32);
   };
   std::vector<uint8_t> done(nb, 0);
+  double behind[sf_context::kAux] = {};
   for (size_t u = 0; u < nb; ++u) {
     if (done[u]) continue;
     Bucket& b = P->buckets[u];
@@ -1209,7 +1220,9 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
       const bool team = b.kind == PK_MYERS ? b.lanes > 32 : sfk::wave_warps(sfk::kWave[b.c]) > 1;
       g.grid = warps_grid((uint64_t)g.task_count * (team ? g.block / 32 : 1), g.block);
     }
-    g.stream = (int)(P->groups.size() % sf_context::kAux);
+    // Past one a stream, behind the shortest.
+    g.stream = (int)(std::min_element(behind, behind + sf_context::kAux) - behind);
+    behind[g.stream] += (double)b.lat + 1;
     P->groups.push_back(g);
   }
 }
