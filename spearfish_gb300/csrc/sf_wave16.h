@@ -41,10 +41,11 @@ __host__ __device__ constexpr int wave_team_blocks(int q, bool tb, bool ext) {
 }
 // 4-warp blocks per SM the registers are held to: as many as cost no spill or reload of constants
 // (600 2 kb windows, four words: 1.00 ms at five blocks, 0.82 at four; 20,000 Global pairs, ten
-// and twelve words: 5.19 ms at three, 5.09 at four).
+// and twelve words: 5.19 ms at three, 5.09 at four; without traceback 600 pairs, four words:
+// 0.312 ms at eight, 0.238 at five, and 10,000 of eight words 1.08 at six, 1.05 at five).
 __host__ __device__ constexpr int wave_blocks(int q, bool tb, bool ext) {
   return ext ? (tb ? (q <= 6 ? 4 : 3) : 4)
-             : tb ? (q <= 4 ? 6 : q <= 6 ? 5 : 4) : (q <= 6 ? 8 : q <= 8 ? 6 : q <= 10 ? 5 : 4);
+             : tb ? (q <= 4 ? 6 : q <= 6 ? 5 : 4) : (q <= 8 ? 5 : 4);
 }
 
 // prefix: Prefix passes, else Global ones.  block: 128, or a team's threads.
