@@ -116,7 +116,8 @@ enum PassKind : uint8_t {
   PK_AFFINE16 = 3,
   PK_CHAIN16 = 4,
   PK_WAVE16 = 5,
-  PK_WAVE16X = 6
+  PK_WAVE16X = 6,
+  PK_WAVE16C = 7
 };
 
 // One DP pass as the reference's `affine_dp` / `distance` / `local_band_core` receive it.
@@ -338,10 +339,11 @@ void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax,
 int64_t wave_width(const DJob& j);
 // Whether a plan of np passes takes the Myers and anti-diagonal classes that finish a pass
 // fastest, rather than the cheapest ones a cell.
+int pass_lanes16(const Pass& p, size_t np, int lanes16);
 bool lean_plan(size_t np, int sms);
 bool plan_is_lean(const sf_plan* P);
 uint64_t plan_long_steps(const sf_plan* P);
-inline bool is_wave(int kind) { return kind == PK_WAVE16 || kind == PK_WAVE16X; }
+inline bool is_wave(int kind) { return kind == PK_WAVE16 || kind == PK_WAVE16X || kind == PK_WAVE16C; }
 // Row steps of a pass on the anti-diagonal kernel.
 uint64_t wave_steps(const DJob& j, int kind);
 // A class as its reports show it: cells a lane and lanes a pass.

@@ -1213,7 +1213,7 @@ int sf_batch_run(sf_context* ctx, const uint8_t* pool, uint64_t pool_bytes, cons
 namespace {
 
 // A pass's class before any override, and the Myers blocks it needs.
-int default_class(const Pass& p, bool use16, bool lean, int most, uint64_t long_steps, ClassKey& key,
+int default_class(const Pass& p, size_t np, bool use16, bool lean, int most, uint64_t long_steps, ClassKey& key,
                   int64_t& blocks) {
   if (p.kind == PK_MYERS) {
     int b = 1, lanes = 1;
@@ -1229,7 +1229,8 @@ int default_class(const Pass& p, bool use16, bool lean, int most, uint64_t long_
   int c = 4, lanes = 32;
   bool wide = false;
   PassKind kind = PK_AFFINE;
-  classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, lanes, default_lanes16());
+  classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, lanes,
+                  pass_lanes16(p, np, default_lanes16()));
   const bool tb = p.want_cigar && p.kind != PK_LOCAL;
   key = ClassKey{kind, c, wide ? 1 : 0, tb ? 1 : 0, lanes};
   blocks = wmax;  // affine: the group's widest row
@@ -1263,11 +1264,13 @@ std::vector<ClassChoice> tune_candidates(const ClassKey& key, int64_t blocks) {
       const int first = u ? ends[u - 1] : 0;
       const bool home = key.c >= first && key.c < ends[u];
       int left = home ? 2 : (key.c < first ? 1 : 0);
-      for (int c = home ? key.c + 1 : first; c < ends[u] && left; ++c)
+      for (int c = home ? key.c + 1 : first; c < ends[u] && left; ++c) {
+        if (key.kind == PK_WAVE16C && sfk::kWave[c].lanes > 32) continue;
         if (sfk::wave_cap(sfk::kWave[c]) >= cap && (cap > 1024) == (sfk::wave_cap(sfk::kWave[c]) > 1024)) {
           out.push_back(ClassChoice{c, key.lanes});
           --left;
         }
+      }
     }
   } else if (!key.wide) {
     // The 16-bit classes for 16, 32 and 64 lanes a pass.
@@ -1326,7 +1329,7 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   for (size_t q = 0; q < P->passes.size(); ++q) {
     ClassKey k;
     int64_t blocks = 0;
-    int rc = default_class(P->passes[q], use16, lean, most, long_steps, k, blocks);
+    int rc = default_class(P->passes[q], P->passes.size(), use16, lean, most, long_steps, k, blocks);
     if (rc) return rc;
     groups[k].push_back(q);
     gblocks[k] = std::max(gblocks[k], blocks);
@@ -1395,6 +1398,7 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
                                                                : (key.kind == PK_AFFINE16 ? "affine16"
                                                                   : key.kind == PK_WAVE16  ? "wave16"
                                                                   : key.kind == PK_WAVE16X ? "wave16x"
+                                                                  : key.kind == PK_WAVE16C ? "wave16c"
                                                                                            : "affine")),
                   shown_c(key.kind, key.c), key.wide ? "true" : "false", key.tb ? "true" : "false",
                   shown_lanes(key.kind, key.c, key.lanes), g.second.size(), shown_c(key.kind, best.c),

@@ -98,7 +98,8 @@ uint64_t wave_steps(const DJob& j, int kind) {
 }
 
 // Whether a pass runs on the anti-diagonal kernel (sf_wave16_impl.cuh), and as which kind: a
-// Global pass of a finite band without clip or cut, or a Prefix pass of one without cut.  Its
+// Global pass of a finite band without clip or cut, or a Prefix pass of one (with a cut column:
+// no traceback, one warp's classes).  Its
 // band edges rest on mis = 2 ext (a mismatch costs what the two gap bases around it would extend
 // for) and open >= 1.  Its fields hold four times the value: the largest rises by (mat + 2 ext) a
 // row step between rebases, and a band cell lies at most (mat + 2 ext) * width / 2 + open below it
@@ -108,7 +109,7 @@ uint64_t wave_steps(const DJob& j, int kind) {
 // text (or the pattern) is left to the row kernels, whose rows stop at the text's end.
 constexpr int64_t kWaveNarrow = 1024;  // wave_wide classes hold more cells, no others do
 bool fits_wave(const Pass& p, const DJob& j, uint32_t flags, PassKind& kind) {
-  if (p.kind != PK_AFFINE || (flags & (F_FULL | F_CUT))) return false;
+  if (p.kind != PK_AFFINE || (flags & F_FULL)) return false;
   const bool prefix = p.mode == SF_PREFIX;
   if (!prefix && (p.mode != SF_GLOBAL || (flags & F_ROWMAX))) return false;
   const sf_affine_t& s = p.sc;
@@ -118,7 +119,9 @@ bool fits_wave(const Pass& p, const DJob& j, uint32_t flags, PassKind& kind) {
   if (4 * ((int64_t)s.mat + 2 * s.ext) * ((int64_t)p.m + p.n) >= 1 << 30) return false;
   if (p.m < 1 || p.n < 1 || w > (prefix ? 4 * (shorter + 1) + 64 : 2 * (shorter + 1))) return false;
   if (prefix && (int64_t)p.m > (int64_t)p.n + j.below) return false;  // ends past the text
-  kind = prefix ? PK_WAVE16X : PK_WAVE16;
+  const bool cut = flags & F_CUT;
+  if (cut && (!prefix || p.want_cigar || w > kWaveNarrow)) return false;
+  kind = cut ? PK_WAVE16C : prefix ? PK_WAVE16X : PK_WAVE16;
   const sfk::WaveClass& last = sfk::kWave[prefix ? sfk::kWaveN - 1 : sfk::kWaveX - 1];
   if (w > sfk::wave_cap(last)) return false;
   const int64_t g = (int64_t)s.mat + 2 * s.ext, open = s.open, ext = prefix ? s.ext : 0;
@@ -138,7 +141,7 @@ bool lean_plan(size_t np, int sms) { return np <= (size_t)sms * 20; }
 bool plan_is_lean(const sf_plan* P) {
   return P->lean >= 0 ? P->lean != 0 : lean_plan(P->passes.size(), P->ctx->sms);
 }
-// Row steps from which a pass takes its fastest class.  The plan's longest passes do, as long as
+// Row steps from which an affine pass takes its fastest class.  The plan's longest passes do, as long as
 // their band cells together leave schedulers idle in the cheaper classes (kFastCells: 2 kb passes
 // of band 128, 1,200 of them 0.64 ms on 4 words x 32 lanes against 1.37 on 12 x 6; 4,000 equal
 // passes are a quarter faster in the cheap classes).  In a plan of many passes only those do that
@@ -229,6 +232,14 @@ int default_lanes16() {
   return 32;
 }
 
+// The same for one pass of a plan of np: few passes with a cut column stay on the row kernels (500
+// sorted calls, 2,400 passes: 0.76 ms there, 1.02 on the anti-diagonal one; 900 calls 1.47 and
+// 1.70; 5,800 calls 2.18 and 1.96; 12,000 3.85 and 3.5).
+int pass_lanes16(const Pass& p, size_t np, int lanes16) {
+  constexpr size_t kCutPasses = 16384;
+  return lanes16 == 0 && p.cut != SF_NOLIMIT && np < kCutPasses ? 32 : lanes16;
+}
+
 // Row sharing between sorted texts on the GPU: SF_SORTED_CHAINS=1 in the environment runs
 // the passes of a sorted call that can share rows as chains; by default every pass runs
 // separately (the results are the same either way, and separate passes finish sooner on the
@@ -268,12 +279,13 @@ bool wave_is_less(const Pass& p, const DJob& j, int64_t wmax, int c, bool alone)
   const sfk::WaveClass& k = sfk::kWave[c];
   const double steps = (double)wave_steps(j, PK_WAVE16X), words = (double)((wmax + 31) / 32);
   const int per_warp = std::max(1, 32 / k.lanes), warps = sfk::wave_warps(k);
-  const bool tb = p.want_cigar;
+  const bool tb = p.want_cigar, cut = p.cut != SF_NOLIMIT;
+  if (cut && alone) return false;
   const double wave = alone ? (tb ? 0.36 : 0.25) + 0.015 * k.q * warps / 4
                             : (tb ? 0.17 + 0.042 * k.q : 0.095 + 0.03 * k.q) * warps / per_warp;
   const double row = alone ? (tb ? 0.6 + 0.0105 * words : 0.44 + 0.01 * words)
                            : (tb ? 0.2 + 0.0243 * words : 0.14 + 0.0165 * words);
-  return steps * wave <= (double)p.m * row;
+  return steps * wave * (cut ? 1.25 : 1.0) <= (double)p.m * row;
 }
 
 // Kernel class of an affine or local pass: the anti-diagonal 16-bit kernel when the pass fits
@@ -286,8 +298,8 @@ void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax,
   if (use16 && lanes16 == 0 && fits_wave(p, j, flags, kind)) {
     const int64_t w = wave_width(j);
     const bool fast = wave_steps(j, kind) >= long_steps;
-    c = kind == PK_WAVE16X ? (fast ? sfk::kWaveXFast : sfk::kWaveX) : (fast ? sfk::kWaveFast : 0);
-    while (sfk::wave_cap(sfk::kWave[c]) < w) ++c;
+    c = kind != PK_WAVE16 ? (fast ? sfk::kWaveXFast : sfk::kWaveX) : (fast ? sfk::kWaveFast : 0);
+    while (sfk::wave_cap(sfk::kWave[c]) < w || (kind == PK_WAVE16C && sfk::kWave[c].lanes > 32)) ++c;
     if (kind == PK_WAVE16 || !fits16(p, flags, wmax) || wave_is_less(p, j, wmax, c, fast)) return;
   }
   if (use16 && fits16(p, flags, wmax)) {
@@ -325,7 +337,7 @@ uint64_t pass_cycles(const Pass& p, const DJob& j, PassKind kind, int c, uint64_
   const bool tb = p.want_cigar;
   if (is_wave(kind)) {
     const uint64_t q = (uint64_t)sfk::kWave[c].q, step = tb ? 180 + 66 * q : 100 + 36 * q;
-    return wave_steps(j, kind) * step * (kind == PK_WAVE16X ? 7 : 5) / 5;
+    return wave_steps(j, kind) * step * (kind == PK_WAVE16 ? 5 : 7) / 5;
   }
   const uint64_t rows = std::max<uint32_t>(p.m, 1);
   if (kind == PK_AFFINE16) return rows * (tb ? 1150 + 20 * (uint64_t)c : 850 + 19 * (uint64_t)c);
@@ -784,7 +796,8 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       bool wide = false;
       PassKind kind = PK_AFFINE;
       int ln = 32;
-      classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, ln, lanes16);
+      classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, ln,
+                      pass_lanes16(p, np, lanes16));
       const bool tb = p.want_cigar && p.kind != PK_LOCAL;
       if (!wide) tuned(kind, c, false, tb, ln);
       TJob t{};
@@ -1333,6 +1346,7 @@ void describe_plan(sf_plan* P, const BuildScratch& S) {
                   : b.kind == PK_CHAIN16 ? "chain16"
                   : b.kind == PK_WAVE16  ? "wave16"
                   : b.kind == PK_WAVE16X ? "wave16x"
+                  : b.kind == PK_WAVE16C ? "wave16c"
                                          : "affine",
                   shown_c(b.kind, b.c),
                   b.wide ? "true" : "false", b.tb ? "true" : "false",
@@ -1494,8 +1508,8 @@ int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* ev
         al.order = orders;
         al.tasks = tasks;
         al.njobs = task_count;
-        CK(sfk::launch_wave16(sfk::kWave[b.c].q, b.kind == PK_WAVE16X, sfk::kWave[b.c].lanes > 32, b.tb,
-                              al, grid, b.block, bs));
+        CK(sfk::launch_wave16(sfk::kWave[b.c].q, b.kind != PK_WAVE16, b.kind == PK_WAVE16C,
+                              sfk::kWave[b.c].lanes > 32, b.tb, al, grid, b.block, bs));
       } else if (b.kind == PK_CHAIN16) {
         CK(sfk::launch_affine16_chain(b.c, al, b.grid, b.block, bs));
       } else if (b.kind == PK_AFFINE16 && b.lanes == 64) {

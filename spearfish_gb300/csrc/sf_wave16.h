@@ -48,8 +48,9 @@ __host__ __device__ constexpr int wave_blocks(int q, bool tb, bool ext) {
              : tb ? (q <= 4 ? 6 : q <= 6 ? 5 : 4) : (q <= 8 ? 5 : 4);
 }
 
-// prefix: Prefix passes, else Global ones.  block: 128, or a team's threads.
-cudaError_t launch_wave16(int q, bool prefix, bool team, bool tb, const AffLaunch& a, int grid,
+// prefix: Prefix passes, else Global ones; cut: with a cut column (no teams, no traceback).
+// block: 128, or a team's threads.
+cudaError_t launch_wave16(int q, bool prefix, bool cut, bool team, bool tb, const AffLaunch& a, int grid,
                           int block, cudaStream_t s);
 
 }  // namespace sfk

@@ -14,6 +14,10 @@ cudaError_t launch_wave16x_4(bool, const AffLaunch&, int, cudaStream_t);
 cudaError_t launch_wave16x_6(bool, const AffLaunch&, int, cudaStream_t);
 cudaError_t launch_wave16x_8(bool, const AffLaunch&, int, cudaStream_t);
 
+cudaError_t launch_wave16c_4(const AffLaunch&, int, cudaStream_t);
+cudaError_t launch_wave16c_6(const AffLaunch&, int, cudaStream_t);
+cudaError_t launch_wave16c_8(const AffLaunch&, int, cudaStream_t);
+
 cudaError_t launch_wave16t_4(bool, const AffLaunch&, int, int, cudaStream_t);
 cudaError_t launch_wave16xt_4(bool, const AffLaunch&, int, int, cudaStream_t);
 cudaError_t launch_wave16xt_8(bool, const AffLaunch&, int, int, cudaStream_t);
@@ -34,8 +38,15 @@ const WaveClass kWave[kWaveN] = {
     {8, 62}, {8, 92}, {8, 122},
     {4, 8}, {4, 16}, {4, 32}, {4, 62}, {8, 32}, {4, 92}, {4, 122}, {4, 152}, {4, 182}, {4, 212}};
 
-cudaError_t launch_wave16(int q, bool prefix, bool team, bool tb, const AffLaunch& a, int grid,
+cudaError_t launch_wave16(int q, bool prefix, bool cut, bool team, bool tb, const AffLaunch& a, int grid,
                           int block, cudaStream_t s) {
+  if (cut) {
+    if (team || tb) return cudaErrorInvalidValue;
+    return q == 4   ? launch_wave16c_4(a, grid, s)
+           : q == 6 ? launch_wave16c_6(a, grid, s)
+           : q == 8 ? launch_wave16c_8(a, grid, s)
+                    : cudaErrorInvalidValue;
+  }
   if (team) {
     if (q == 4) return (prefix ? launch_wave16xt_4 : launch_wave16t_4)(tb, a, grid, block, s);
     return prefix && q == 8 ? launch_wave16xt_8(tb, a, grid, block, s) : cudaErrorInvalidValue;

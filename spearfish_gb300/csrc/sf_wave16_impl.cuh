@@ -1,6 +1,6 @@
 // Global and Prefix banded affine (Gotoh) passes swept by anti-diagonals, two cells per 32-bit
 // register and several passes per warp (align.rs:2446-2666 `run_core` in Mode::Global without
-// clip or cut, and in Mode::Prefix with or without clip, without cut).  Results and traceback
+// clip or cut, and in Mode::Prefix with or without clip and cut).  Results and traceback
 // decisions equal the row kernels' (sf_affine16_impl.cuh).
 //
 // Cells.  Band offset K = j - i + bl of cell (i, j) sits at a fixed place: lane K / 4Q of the
@@ -34,6 +34,7 @@
 // H odd) with the leftmost offset it was reached at, and leave the band at its last cell, where
 // one lane keeps the pass's books in row order, four rows at a time.  The rows that run ahead of
 // a stop are computed and left out.  Columns past the text count for nothing (the last rows).
+// With a cut column (CUT) a second maximum, over the cells up to it, travels beside M.
 // 8,000 2 kb windows (band 128, CIGARs) on GB300: row kernel 8.75 ms, a cell a step with its books
 // a row at a time 5.95, now 4.83; without CIGARs 7.2 -> 2.94.
 //
@@ -271,6 +272,7 @@ struct WaveTeam {
 // a row.  best (at row i, offset k): the largest so far; a row more than xd below it ends the pass.
 struct WaveBooks {
   int32_t best, i, k, clip, xd, pot4, row4, row0, m, tail, at;
+  int32_t cut, cut_row, cut_tail;  // CUT: the largest up to the cut, and the last rows it matters for
 };
 // Prefix passes: the words of the lane that holds a band's last cell over four row steps, by the
 // pass's place in its warp, for that lane to pick one by its offset (a select over registers
@@ -278,7 +280,7 @@ struct WaveBooks {
 template <int Q, bool EXT>
 struct WaveLast {
   static constexpr int kQuads = EXT ? (Q + 3) / 4 : 1, kSlots = EXT ? 11 : 1;
-  uint4 w[kSlots][4][3][kQuads];  // the last slot takes what the other lanes write
+  uint4 w[kSlots][4][4][kQuads];  // the last slot takes what the other lanes write
   WaveBooks books[kSlots];
 };
 
@@ -287,7 +289,7 @@ struct WaveLast {
 // further on each; a warp's outer lanes (but the first's first and the last's last) repeat its
 // neighbours' and are set right from them every 2Q row steps, which is as long as what they lack
 // at their outer side takes to cross them, a cell a step.
-template <int Q, bool TB, bool EXT, bool TEAM>
+template <int Q, bool TB, bool EXT, bool TEAM, bool CUT>
 __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t jid, bool has, int L,
                                             int lane, int seg, WaveLast<Q, EXT>& Z,
                                             WaveTeam<Q, EXT>* X) {
@@ -321,8 +323,11 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
 
   // EXT: M's potential rises by 4 ext a step, so the top leaves room for a row's width of them.
   const int32_t wtop = EXT ? (int32_t)kWTop - 4 * S.ext * (W + 1) : (int32_t)kWTop;
+  [[maybe_unused]] const int32_t cut =
+      CUT ? (int32_t)(J.cut < (uint64_t)n + 1 ? J.cut : (uint64_t)n + 1) : 0;
   uint32_t HA[Q], HB[Q], E[Q], F[Q], acc[TB ? 2 * Q : 1];
   uint32_t M[EXT ? Q : 1], MK[EXT ? Q : 1];  // a row's largest value so far and its offset K
+  uint32_t C[CUT ? Q : 1];                   // the same up to the cut column
 #pragma unroll
   for (int k = 0; k < Q; ++k) {
     // The seed at (0, 0): offset bl, odd.
@@ -337,6 +342,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       M[k] = kNegM;
       MK[k] = 0;
     }
+    if constexpr (CUT) C[k] = kNegM;
   }
   int32_t off = -wtop;
 
@@ -446,6 +452,11 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
     bk.row0 = a1 - 4 - kw;         // the first row of the four steps before row step 0
     bk.m = m;
     bk.tail = n + bl - 2 * kw;     // rows after this: the band's last even cell lies past the text
+    if constexpr (CUT) {
+      bk.cut = 4 * Book{}.cut_best;
+      bk.cut_row = cut + below;  // rows after this start past the cut
+      bk.cut_tail = cut + bl - 2 * kw;
+    }
   }
   // Row steps from which some cell lies past the text.
   const int32_t r_tail = __reduce_min_sync(FULL, has ? n + bl - kw - a1 : INT32_MAX);
@@ -496,7 +507,11 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
     auto in_text = [&](int k, int32_t t) -> uint32_t {
       return (k <= t ? 0xffffu : 0u) | (Q + k <= t ? 0xffff0000u : 0u);
     };
-    [[maybe_unused]] uint32_t sM = 0, sK = 0;
+    [[maybe_unused]] uint32_t sM = 0, sK = 0, sC = 0;
+    if constexpr (CUT) {
+      sC = __shfl_up_sync(FULL, C[Q - 1], 1);
+      if (leftmost) sC = kNegM;
+    }
     if constexpr (EXT) {
       sM = __shfl_up_sync(FULL, M[Q - 1], 1);
       sK = __shfl_up_sync(FULL, MK[Q - 1], 1);
@@ -556,6 +571,22 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
         put_last(even_last[r & 3][1], pl);
         put_last(even_last[r & 3][2], HA);
       }
+      if constexpr (CUT) {
+        // Cells up to the cut (and the text's end): their largest, without its offset.
+        const int32_t tc = min(n, cut) + bl - (a1 + r) - k0;
+        uint32_t cl[Q];
+        cl[0] = __byte_perm(sC, C[Q - 1], 0x5432);
+#pragma unroll
+        for (int k = 1; k < Q; ++k) cl[k] = C[k - 1];
+        if (any_even) put_last(even_last[r & 3][3], cl);
+#pragma unroll
+        for (int k = Q - 1; k >= 0; --k) {
+          uint32_t xa = mad<1>(HA[k], ha);
+          if (k == 0) xa &= pad0;
+          C[k] = mad<1>(__vimax3_u16x2(cl[k], xa & in_text(k, tc), HB[k] & in_text(k, tc - 1)), 2u * e4);
+        }
+        if (any_odd) put_last(odd_last[r & 3][3], C);
+      }
 #pragma unroll
       for (int k = Q - 1; k >= 0; --k) {
         uint32_t xa = mad<1>(HA[k], ha), xb = TB ? mad<1>(HB[k], hb) : HB[k];
@@ -591,7 +622,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
       const int32_t best = bk.best, xd = bk.xd;
       const bool clip = bk.clip;
       const uint16_t* const fs = reinterpret_cast<const uint16_t*>(last[0][0]) + bk.at;
-      constexpr int kRow = 3 * kArray, kArray2 = 2 * kArray;
+      constexpr int kRow = 4 * kArray, kArray2 = 2 * kArray;
       constexpr uint32_t ha1 = TB ? ~0u : 1u;
       const uint32_t x4 = row4 / 2 + ha1;
       auto row_of = [&](int t, uint32_t& k) {
@@ -606,6 +637,13 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
           }
         }
         return (int32_t)f;
+      };
+      // A row's largest up to the cut.
+      auto cut_of = [&](int t) {
+        uint32_t f = fs[t * kRow + 3 * kArray];
+        if (any_even && !last_odd && i0 + t <= min(bk.tail, bk.cut_tail))
+          f = max(f, fs[t * kRow + kArray2] + x4);
+        return (int32_t)(f & ~3u) + (v0 - t * row4);
       };
       // Together: the largest row, the first of equals (3 - t in the low bits), where no row can
       // end the pass.
@@ -629,6 +667,13 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
           bk.i = i0 + t;
           bk.k = (int32_t)pk;
         }
+        if constexpr (CUT) {
+          int32_t c = bk.cut;
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            if (open && i0 + t <= bk.cut_row) c = max(c, cut_of(t));
+          bk.cut = c;
+        }
       } else {
 #pragma unroll 1
         for (int t = 0; t < 4; ++t) {
@@ -636,6 +681,9 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
           uint32_t pk;
           const int32_t v = (row_of(t, pk) & ~3) + (v0 - t * row4);
           if (!open || i < 1) continue;
+          const bool to_cut = CUT && i <= bk.cut_row;
+          const int32_t vc = to_cut ? cut_of(t) : 0;
+          if (to_cut && vc > bk.cut) bk.cut = vc;
           if (clip && v > bk.best) {
             bk.best = v;
             bk.i = i;
@@ -644,7 +692,8 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
           const bool stop = clip && v + xd < bk.best;
           if (stop || i == m) {
             const bool cell = clip && (S.flags & F_CELL) && bk.i;
-            a.out[jid] = DRes{stop ? NEG : v >> 2, clip ? bk.best >> 2 : Book{}.clip_best, 0, NEG,
+            a.out[jid] = DRes{stop ? NEG : v >> 2, clip ? bk.best >> 2 : Book{}.clip_best,
+                              CUT ? bk.cut >> 2 : 0, to_cut && !stop ? vc >> 2 : NEG,
                               stop ? 0u : (uint32_t)(i - bl) + pk, cell ? (uint32_t)bk.i : 0u,
                               cell ? (uint32_t)(bk.i - bl + bk.k) : 0u, (uint32_t)min(i + above, n),
                               (uint32_t)i, (uint32_t)i, band_cells(i, below, above, n)};
@@ -758,6 +807,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
         E[k] = __viaddmax_u16x2(E[k], dd, kNegE);
         F[k] = __viaddmax_u16x2(F[k], dd, kNegF);
         if constexpr (EXT) M[k] = __viaddmax_u16x2(M[k], dd, kNegM);
+        if constexpr (CUT) C[k] = __viaddmax_u16x2(C[k], dd, kNegM);
       }
       off += delta;
     }
@@ -774,7 +824,7 @@ __device__ __forceinline__ void wave_passes(const sfk::AffLaunch& a, uint32_t ji
   __syncwarp();
 }
 
-template <int Q, bool TB, bool EXT>
+template <int Q, bool TB, bool EXT, bool CUT>
 __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, EXT)) wave16_kernel(sfk::AffLaunch a) {
   const int lane = threadIdx.x & 31;
   __shared__ WaveLast<Q, EXT> Z[4];
@@ -786,7 +836,7 @@ __global__ void __launch_bounds__(128, sfk::wave_blocks(Q, TB, EXT)) wave16_kern
     const uint2 task = a.tasks[q];
     const int L = (int)(task.y & 0xffu), np = (int)(task.y >> 8), seg = lane / L;
     const bool has = seg < np;
-    wave_passes<Q, TB, EXT, false>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, lane, seg,
+    wave_passes<Q, TB, EXT, false, CUT>(a, a.order[task.x + (has ? (uint32_t)seg : 0u)], has, L, lane, seg,
                                    Z[threadIdx.x >> 5], nullptr);
     if (a.njobs <= grid_tasks) break;
     uint32_t next = 0;
@@ -804,7 +854,7 @@ __global__ void __launch_bounds__(32 * sfk::wave_most_warps(Q), sfk::wave_team_b
   uint32_t q = blockIdx.x;
   while (q < a.njobs) {
     const uint2 task = a.tasks[q];
-    wave_passes<Q, TB, EXT, true>(a, a.order[task.x], true, (int)(task.y & 0xffu), threadIdx.x & 31,
+    wave_passes<Q, TB, EXT, true, false>(a, a.order[task.x], true, (int)(task.y & 0xffu), threadIdx.x & 31,
                                     0, Z, &X);
     if (a.njobs <= gridDim.x) break;
     __syncthreads();
@@ -827,12 +877,18 @@ cudaError_t launch_wave16t_q(bool tb, const AffLaunch& a, int grid, int block, c
   return cudaGetLastError();
 }
 
+template <int Q>
+cudaError_t launch_wave16c_q(const AffLaunch& a, int grid, cudaStream_t s) {
+  wave16_kernel<Q, false, true, true><<<grid, 128, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
 template <int Q, bool EXT>
 cudaError_t launch_wave16_q(bool tb, const AffLaunch& a, int grid, cudaStream_t s) {
   if (tb)
-    wave16_kernel<Q, true, EXT><<<grid, 128, 0, s>>>(a);
+    wave16_kernel<Q, true, EXT, false><<<grid, 128, 0, s>>>(a);
   else
-    wave16_kernel<Q, false, EXT><<<grid, 128, 0, s>>>(a);
+    wave16_kernel<Q, false, EXT, false><<<grid, 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -354,3 +354,35 @@ def test_wide_bands(ctx, packed):
     gout, gkinds = _run(ctx, grows + (_ballast() if packed else []), scores)
     assert {(16, 152), (16, 182), (16, 212)} <= {(c, n) for k, c, n in gkinds if k == "wave16"}
     _check(grows, gout, scores)
+
+
+@pytest.mark.parametrize("calls", [120, 3600])
+def test_prefix_cut(ctx, calls):
+    """Sorted-texts extensions with a cut column: left of the band, in it at any parity, at and
+    past the text's end; X-drop stops in every part, even and odd last cells, bands of each class
+    (a few calls run one pass a warp, many several)."""
+    from spearfish_gb300 import tiebreak as T
+    rng = np.random.default_rng(2671)
+    scores = (R.ONT, R.HIFI)
+    got_calls, want = [], []
+    for q in range(calls):
+        m = int(np.exp(rng.uniform(np.log(1), np.log(120 if q % 40 else 1500))))
+        band = int(rng.choice([0, 1, 5, 16, 24, 32, 47])) if q % 40 else int(rng.integers(60, 400))
+        base = rng.integers(0, 4, m + int(rng.integers(0, 40))).tolist()
+        p = R.mutate(base[:m], R.rand_edits(rng, m // 12, m)) or [1]
+        texts = sorted({tuple(R.mutate(base, R.rand_edits(rng, int(rng.integers(0, 6)), len(base))))
+                        or (0,) for _ in range(int(rng.integers(1, 5)))})
+        texts = [list(t) for t in texts]
+        n = min(len(t) for t in texts)
+        cut = int(rng.choice([0, 1, max(0, n - 3), n, n + 50, int(rng.integers(0, n + 1))]))
+        xd = int(rng.choice([0, 6, 20, 50, R.I32_MAX]))
+        bonus, track, within = int(rng.integers(0, 8)), bool(q & 1), bool(q & 2)
+        diag, w, sci = bool(rng.random() < 0.2), max(len(t) for t in texts) + int(rng.integers(0, 30)), q % 2
+        got_calls.append(dict(kind=T.SORTED_EXTEND_CUT, read=p, texts=texts, band=band,
+                              end_bonus=bonus, xdrop=xd, diagonal=diag, window=w, cut=cut,
+                              track_cut=track, bonus_within_cut=within, sc_index=sci))
+        want.append(O.affine_extend_sorted_cut_bonus(p, texts, scores[sci], band, bonus, xd, diag,
+                                                     w, cut, track, within))
+    got = T.sorted_batch(ctx, got_calls, scores=scores)
+    for q in range(calls):
+        assert got[q] == want[q], (q, got_calls[q])
