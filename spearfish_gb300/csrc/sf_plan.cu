@@ -152,6 +152,12 @@ bool plan_is_lean(const sf_plan* P) {
 // 6,000 pairs 10.9 / 6.9 / 6.9 / 7.0 / 7.2 (teams repeat lanes, and take the schedulers' turns).
 uint64_t plan_long_steps(const sf_plan* P) {
   if (P->long_steps) return P->long_steps;
+  if (!P->passes.empty() && P->passes.front().kind == PK_MYERS && P->passes.back().kind == PK_MYERS) {
+    // Myers pairs only: nothing to weigh.
+    bool any = false;
+    for (size_t q = 0; q < P->passes.size() && !any; ++q) any = P->passes[q].kind != PK_MYERS;
+    if (!any) return 1;
+  }
   constexpr int kT = 16, kBins = 128;
   constexpr double kFastCells = 550000;
   auto shape = [](const Pass& p, double& w, double& steps) {
@@ -1235,7 +1241,7 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
     }
     // Past one a stream, behind the shortest.
     g.stream = (int)(std::min_element(behind, behind + sf_context::kAux) - behind);
-    behind[g.stream] += (double)b.lat + 1;
+    if (!P->groups.empty()) behind[g.stream] += (double)b.lat + 1;  // (the first runs beside them)
     P->groups.push_back(g);
   }
 }
@@ -1426,7 +1432,7 @@ int mark_stage(std::vector<cudaEvent_t>* evs, cudaStream_t s) {
 
 // The first part of an execute: the pack on `s`, then the launches, fanned out over the
 // auxiliary streams so that their tails overlap (each on its stream, rotated by `soff`; also
-// a single one with `fan_one`).  `used` collects the auxiliary
+// the first one with `fan_one`).  `used` collects the auxiliary
 // streams launched on.
 // With `evs`, everything runs in order on `s` with an event after each stage.
 int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* evs, int soff,
@@ -1461,7 +1467,10 @@ int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* ev
     const uint32_t task_count = evs ? b.task_count : P->groups[q].task_count;
     const int grid = evs ? b.grid : P->groups[q].grid;
     cudaStream_t bs = s;
-    if (fan) {
+    // The longest launch follows the pack on `s` itself and so starts first, its blocks spread
+    // over the SMs: let in later, as others leave, they crowd the first SMs to empty (55 teams of
+    // 3 ms beside 7,600 short passes: 11.2 ms, 4.4 started first).
+    if (fan && (q > 0 || fan_one)) {
       const int si = (P->groups[q].stream + soff) % sf_context::kAux;
       bs = ctx->aux[si];
       if (!mine[si]) CK(cudaStreamWaitEvent(bs, ctx->fork, 0));
