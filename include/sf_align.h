@@ -36,7 +36,7 @@
  *  - SF_SORTED_CHAINS=1: the sorted entry points run the passes that can
  *    share rows as chains (below, at sf_affine_sorted).
  *  - SF_BATCH_SEGMENTS=0: sf_batch_run builds every batch as one plan (no
- *    segments, below).
+ *    segments, below); =1: every large even batch runs in segments.
  */
 #ifndef SF_ALIGN_H
 #define SF_ALIGN_H

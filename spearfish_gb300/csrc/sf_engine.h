@@ -353,7 +353,7 @@ int choose_myers_class(uint32_t m, bool lean, int most, int& b, int& lanes);
 int most_pairs(const sf_plan* P);
 DJob make_djob(const Pass& p, uint32_t& flags);
 // Whether large sf_batch_run batches may run in segments (SF_BATCH_SEGMENTS).
-bool batch_segments_on();
+int batch_segments();
 // The plan's pinned staging: stage_done marks the end of the copies issued out of it so
 // far; stage_wait waits for that before it is written again.
 int stage_wait(sf_plan* P);

@@ -1039,38 +1039,51 @@ uint64_t pool_reach(const sf_job_t* jobs, uint64_t count, uint64_t pool_bytes) {
   return *std::max_element(mx, mx + kT);
 }
 
-// Whether a batch's jobs are even enough to run in segments: no job's estimated work above
-// 8x the mean.  A long pass in a late segment starts only when the earlier segments' blocks
+// Whether a batch's jobs are enough work, and even enough, to run in segments.  Enough: the host's
+// share of a segment has to hide behind the device's of the last one; measured in one plan and in
+// segments, affine batches cross at 5 ms of device time (18,000 pairs of 500 b with CIGARs 1.95 and
+// 2.58 ms, 20,000 of 2 kb 6.2 and 6.2, 60,000 15.1 and 13.6), Myers ones at 0.7 (18,000 of 1 kb
+// 1.47 and 1.63, 9,900 of 2 kb 1.70 and 1.50, 40,000 5.0 and 4.2).  Even: no job's estimated work
+// above 8x the mean.  A long pass in a late segment starts only when the earlier segments' blocks
 // have left the device, so it would end after the rest; one plan starts it first.  Work is
 // band cells for affine jobs and matrix cells / 24 for Myers (its cells cost about 1/24 of
 // an affine cell).
-bool batch_even(const sf_job_t* jobs, uint64_t count) {
+bool batch_in_segments(const sf_job_t* jobs, uint64_t count, bool whatever_work) {
   constexpr int kT = 16;
-  double sum[kT] = {}, mx[kT] = {};
+  constexpr double kAffineNs = 5e6, kMyersNs = 7e5;
+  double sum[kT] = {}, mx[kT] = {}, dev[kT] = {};
+  bool affine[kT] = {};
   parallel_chunks(count, 4096, kT, [&](size_t q0, size_t q1, int k) {
-    double s = 0, x = 0;
+    double s = 0, x = 0, ns = 0;
     for (size_t q = q0; q < q1; ++q) {
       const sf_job_t& j = jobs[q];
       const double m = j.m, n = j.n;
       double w;
       if (j.kind == SF_JOB_MYERS) {
         w = m * n / 24.0;
+        ns += m * n / 40000.0;
       } else {
         const double band = j.band == SF_NOLIMIT ? n + 1 : 2.0 * (double)j.band + 1;
         w = m * std::min(n + 1, band);
+        ns += w / (j.want_cigar ? 2000.0 : 3500.0);
+        affine[k] = true;
       }
       s += w;
       x = std::max(x, w);
     }
     sum[k] = s;
     mx[k] = x;
+    dev[k] = ns;
   });
-  double s = 0, x = 0;
+  double s = 0, x = 0, ns = 0;
+  bool any = false;
   for (int k = 0; k < kT; ++k) {
     s += sum[k];
     x = std::max(x, mx[k]);
+    ns += dev[k];
+    any = any || affine[k];
   }
-  return count > 0 && x <= 8.0 * (s / (double)count);
+  return count > 0 && (whatever_work || ns >= (any ? kAffineNs : kMyersNs)) && x <= 8.0 * (s / (double)count);
 }
 
 // A large batch in segments of consecutive jobs, each its own plan: the host converts and
@@ -1193,7 +1206,7 @@ int sf_batch_run(sf_context* ctx, const uint8_t* pool, uint64_t pool_bytes, cons
     ctx->cache->ctx = ctx;
   }
   const int nseg = (int)std::min<uint64_t>(count / kSegJobs, sf_context::kSegs);
-  if (nseg >= 2 && batch_segments_on() && batch_even(jobs, count))
+  if (nseg >= 2 && batch_segments() && batch_in_segments(jobs, count, batch_segments() > 1))
     return batch_run_segments(ctx, nseg, pool, pool_bytes, jobs, count, scores, n_scores, results,
                               ops, ops_cap, ops_used);
   sf_plan* P = ctx->cache.get();

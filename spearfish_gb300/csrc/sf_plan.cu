@@ -250,10 +250,11 @@ int pass_lanes16(const Pass& p, size_t np, int lanes16) {
 // the passes of a sorted call that can share rows as chains; by default every pass runs
 // separately (the results are the same either way, and separate passes finish sooner on the
 // batches measured: a chain runs its passes one after another); read once per plan.
-// Large sf_batch_run batches run in segments (SF_BATCH_SEGMENTS=0 turns it off).
-bool batch_segments_on() {
+// Large sf_batch_run batches of enough work run in segments: 1; SF_BATCH_SEGMENTS=0 turns it off
+// (0), =1 runs every large even batch so (2).
+int batch_segments() {
   const char* e = std::getenv("SF_BATCH_SEGMENTS");
-  return !(e && e[0] == '0');
+  return !e ? 1 : e[0] == '0' ? 0 : 2;
 }
 
 // Capped Global and Prefix Myers pairs stop at the first column wholly past their cap
