@@ -40,9 +40,9 @@
 //
 // Bound: the ALU pipe (one instruction every other cycle a scheduler): 8.5 of a word's 14.5
 // instructions with traceback, 4.5 of 6.5 without.  With 12 words a lane and 6 lanes a pass a
-// row step issues 443 instructions for five 2 kb passes of band 128 (258 on the ALU pipe), the
-// row kernel 254 for one; score only 221 against 150.  20,000 such pairs on GB300: 10.25 ->
-// 5.2 ms with CIGARs, 5.7 -> 2.4 ms without.
+// row step issues 459 instructions for five 2 kb passes of band 128 (266 on the ALU pipe, 73% of
+// its rate), the row kernel 254 for one; score only 221 (87%) against 150.  20,000 such pairs on
+// GB300: 10.25 -> 4.8 ms with CIGARs, 5.7 -> 2.4 ms without.
 #pragma once
 #include <type_traits>
 
