@@ -134,9 +134,8 @@ bool fits_wave(const Pass& p, const DJob& j, uint32_t flags, PassKind& kind) {
   return room + 4 * ext * (w + 1) <= top - neg;
 }
 
-// Few passes: each takes the fastest class.  Measured on 2 kb passes with band 128 and CIGARs:
-// 600 passes 0.47 ms on 4 words x 32 lanes, 0.84 on 10 x 8; 1,200 passes 0.64 against 1.37 on
-// 12 x 6; 8,200 passes 3.49 against 2.54 (four a warp): the lines cross near 20 an SM.
+// Few passes: Myers pairs take one block a lane, and an affine pass needs only to be among the
+// longest to take a fast class (plan_long_steps).
 bool lean_plan(size_t np, int sms) { return np <= (size_t)sms * 20; }
 bool plan_is_lean(const sf_plan* P) {
   return P->lean >= 0 ? P->lean != 0 : lean_plan(P->passes.size(), P->ctx->sms);
