@@ -339,6 +339,7 @@ void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax,
 int64_t wave_width(const DJob& j);
 // Whether a plan of np passes takes the Myers and anti-diagonal classes that finish a pass
 // fastest, rather than the cheapest ones a cell.
+int myers_team(const sf_plan* P);
 int pass_lanes16(const Pass& p, size_t np, int lanes16);
 bool lean_plan(size_t np, int sms);
 bool plan_is_lean(const sf_plan* P);
@@ -349,7 +350,7 @@ uint64_t wave_steps(const DJob& j, int kind);
 // A class as its reports show it: cells a lane and lanes a pass.
 int shown_c(int kind, int c);
 int shown_lanes(int kind, int c, int lanes);
-int choose_myers_class(uint32_t m, bool lean, int most, int& b, int& lanes);
+int choose_myers_class(uint32_t m, int team, int most, int& b, int& lanes);
 int most_pairs(const sf_plan* P);
 DJob make_djob(const Pass& p, uint32_t& flags);
 // Whether large sf_batch_run batches may run in segments (SF_BATCH_SEGMENTS).

@@ -1226,11 +1226,11 @@ int sf_batch_run(sf_context* ctx, const uint8_t* pool, uint64_t pool_bytes, cons
 namespace {
 
 // A pass's class before any override, and the Myers blocks it needs.
-int default_class(const Pass& p, size_t np, bool use16, bool lean, int most, uint64_t long_steps, ClassKey& key,
+int default_class(const Pass& p, size_t np, bool use16, int team, int most, uint64_t long_steps, ClassKey& key,
                   int64_t& blocks) {
   if (p.kind == PK_MYERS) {
     int b = 1, lanes = 1;
-    int rc = choose_myers_class(p.m, lean, most, b, lanes);
+    int rc = choose_myers_class(p.m, team, most, b, lanes);
     if (rc) return rc;
     key = ClassKey{PK_MYERS, b, 0, 0, lanes};
     blocks = ((int64_t)p.m + 63) / 64;
@@ -1334,7 +1334,7 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   const auto t0 = std::chrono::steady_clock::now();
   const bool use16 = allow16();
   const bool lean = plan_is_lean(P);
-  const int most = most_pairs(P);
+  const int most = most_pairs(P), team = myers_team(P);
   const uint64_t long_steps = plan_long_steps(P);
   // Group the passes by their default class.
   std::map<ClassKey, std::vector<size_t>> groups;
@@ -1342,7 +1342,7 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   for (size_t q = 0; q < P->passes.size(); ++q) {
     ClassKey k;
     int64_t blocks = 0;
-    int rc = default_class(P->passes[q], P->passes.size(), use16, lean, most, long_steps, k, blocks);
+    int rc = default_class(P->passes[q], P->passes.size(), use16, team, most, long_steps, k, blocks);
     if (rc) return rc;
     groups[k].push_back(q);
     gblocks[k] = std::max(gblocks[k], blocks);

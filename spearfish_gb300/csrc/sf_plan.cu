@@ -213,6 +213,13 @@ int most_pairs(const sf_plan* P) {
   return (int)std::max<size_t>(1, std::min<size_t>(32, P->passes.size() / ((size_t)P->ctx->sms * 16)));
 }
 
+// Warps a pair of a small plan may take: as long as that leaves schedulers idle (1,762 Global pairs
+// of 4.8 kb in one call: 2.19 ms on four warps of one block a lane, 1.36 on one of three; 450 of 5 kb 0.61, 0.49).
+int myers_team(const sf_plan* P) {
+  if (!plan_is_lean(P)) return 0;
+  return (int)std::min<size_t>(4, (size_t)P->ctx->sms * 10 / std::max<size_t>(1, P->passes.size()));
+}
+
 int shown_c(int kind, int c) { return is_wave(kind) ? 4 * sfk::kWave[c].q : c; }
 int shown_lanes(int kind, int c, int lanes) {
   return is_wave(kind) ? sfk::kWave[c].lanes : lanes;
@@ -366,20 +373,21 @@ bool myers_class_ok(uint32_t m) { return m <= SF_MYERS_MAX_PATTERN; }
 // was measured at 74, 140, 190 and 250 cycles of a scheduler, whatever its lanes hold: many
 // pairs take the B whose share of a step is least, of at most `most` pairs a warp (10,000 1 kb
 // pairs: 0.33 ms at 2 x 8 and 1 x 16 lanes, 0.36 at 4 x 4, which leaves two warps a scheduler);
-// few pairs one block a lane, over several warps from 33 blocks on (100 of 5 kb: 0.29 ms at
-// 1 x 128, 0.58 at 4 x 32).  Past 128 blocks a pair takes four warps either way (a 20 kb pattern
+// few pairs one block a lane, over several warps (`team` at most) from 33 blocks on (100 of 5 kb:
+// 0.29 ms at 1 x 128, 0.58 at 4 x 32).  Past 128 blocks a pair takes four warps either way (a 20 kb pattern
 // on one warp ran 8.1 ms alone, and among other kernels it set an uneven batch's time; on four
 // 2.3 ms).
-int choose_myers_class(uint32_t m, bool lean, int most, int& b, int& lanes) {
+int choose_myers_class(uint32_t m, int team, int most, int& b, int& lanes) {
   if (m > SF_MYERS_MAX_PATTERN) return fail(SF_ERR_TOO_LONG, "Myers pattern longer than SF_MYERS_MAX_PATTERN");
   const int blocks = std::max(1, (int)((m + 63) / 64));
-  if (blocks > 128 || (lean && blocks > 32)) {
-    lanes = lean && blocks <= 64 ? 64 : 128;
+  const bool pair_of_warps = blocks <= 64 && team >= 2;
+  if (blocks > 128 || (blocks > 32 && (pair_of_warps || team >= 4))) {
+    lanes = pair_of_warps ? 64 : 128;
     b = (blocks + lanes - 1) / lanes;
     return SF_OK;
   }
   int best = INT32_MAX;
-  for (int c = 1; c <= (lean ? 1 : sfk::kMyersMaxB); ++c) {
+  for (int c = 1; c <= sfk::kMyersMaxB; ++c) {
     const int p = (blocks + c - 1) / c;
     if (p > 32) continue;
     constexpr int kStep[sfk::kMyersMaxB] = {74, 140, 190, 250};
@@ -688,7 +696,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   const size_t np = P->passes.size();
   const int lanes16 = default_lanes16();
   const bool lean = plan_is_lean(P);
-  const int most = most_pairs(P);
+  const int most = most_pairs(P), team = myers_team(P);
   const uint64_t long_steps = plan_long_steps(P);
   const TuneTable* tune = P->tune_override ? P->tune_override : &ctx->tune;
   const auto& word_of = S.word_of;
@@ -718,7 +726,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   for (int k = 0; k < kT; ++k) {
     if (bad[k] != UINT64_MAX) {
       int b = 1, l = 1;
-      return choose_myers_class(P->passes[bad[k]].m, lean, 1, b, l);  // sets the error
+      return choose_myers_class(P->passes[bad[k]].m, 0, 1, b, l);  // sets the error
     }
     nmy[k + 1] += nmy[k];
   }
@@ -775,7 +783,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       const uint32_t sl = P->slot[q];
       if (p.kind == PK_MYERS) {
         int b = 1, lanes = 1;
-        (void)choose_myers_class(p.m, lean, most, b, lanes);
+        (void)choose_myers_class(p.m, team, most, b, lanes);
         tuned(PK_MYERS, b, false, false, lanes);
         MJob& m = mj[sl];
         m = MJob{};
