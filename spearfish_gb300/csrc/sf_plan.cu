@@ -103,7 +103,9 @@ uint64_t wave_steps(const DJob& j, int kind) {
 // band edges rest on mis = 2 ext (a mismatch costs what the two gap bases around it would extend
 // for) and open >= 1.  Its fields hold four times the value: the largest rises by (mat + 2 ext) a
 // row step between rebases, and a band cell lies at most (mat + 2 ext) * width / 2 + open below it
-// (a gap from the best path, extension free in the kernel's potential); a Prefix pass's row
+// (a gap from the best path, extension free in the kernel's potential); a cell no path reaches
+// gives up a gap's opening like any other and must not go below zero (it would borrow from the
+// field beside it), so open ends at wave_neg / 4, 256 in the widest classes; a Prefix pass's row
 // maxima rise by ext a cell across the band above that, and where a row starts left of the text
 // (`below` cells at most) from the cells no path reaches.  A band much wider than the
 // text (or the pattern) is left to the row kernels, whose rows stop at the text's end.
@@ -128,6 +130,7 @@ bool fits_wave(const Pass& p, const DJob& j, uint32_t flags, PassKind& kind) {
   const bool wide = prefix && w > kWaveNarrow;
   const int64_t top = sfk::wave_top(wide), neg = sfk::wave_neg(wide);
   if (4 * g * (sfk::kWaveRebaseRows + 1) > std::min<int64_t>(0xffff - top, neg)) return false;
+  if (4 * open > neg) return false;
   auto below_top = [&](int64_t cells) { return 4 * (g * (cells / 2 + 2) + 2 * open + 16); };
   int64_t room = below_top(w);
   if (prefix) room = std::max(room, below_top(j.below + 1) + 4 * ext * (j.below + 2));

@@ -9,8 +9,8 @@ namespace sfk {
 struct AffLaunch;
 
 // Fields: the largest of a pass sits at wave_top after a rebase (each kWaveRebaseRows row
-// steps), cells no path reaches at wave_neg; no more than wave_neg is taken off at a rebase, nor
-// does the largest rise past the field in between.
+// steps), cells no path reaches at wave_neg; no more than wave_neg is taken off at a rebase or for
+// a gap's opening, nor does the largest rise past the field in between.
 // The widest Prefix classes leave less at either end.
 __host__ __device__ constexpr bool wave_wide(int q, int lanes) { return q * lanes > 256; }
 __host__ __device__ constexpr uint32_t wave_top(bool wide) { return wide ? 0xfc00u : 0xf000u; }

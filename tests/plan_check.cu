@@ -1,0 +1,45 @@
+// Runs the plan build's host phases (spearfish_gb300/csrc/sf_plan.cu) without a GPU: reads a plan
+// from the file named on the command line -- four 64-bit words (SMs, pool bytes, scores, jobs),
+// the scores, the jobs -- and prints its description, each job's bucket and the sizes it takes.
+#include "../spearfish_gb300/csrc/sf_plan.cu"
+
+#include <cstdio>
+
+using namespace sfe;
+
+int main(int, char** argv) {
+  FILE* f = std::fopen(argv[1], "rb");
+  uint64_t head[4];
+  if (!f || std::fread(head, 8, 4, f) != 4) return 2;
+  std::vector<sf_affine_t> scores(head[2]);
+  std::vector<sf_job_t> jobs(head[3]);
+  if (std::fread(scores.data(), sizeof(sf_affine_t), scores.size(), f) != scores.size() ||
+      std::fread(jobs.data(), sizeof(sf_job_t), jobs.size(), f) != jobs.size())
+    return 2;
+  std::fclose(f);
+  sf_context ctx;
+  ctx.sms = (int)head[0];
+  sf_plan P;
+  P.ctx = &ctx;
+  P.pool_bytes = head[1];
+  P.scratch.reset(new BuildScratch);
+  BuildScratch& S = *P.scratch;
+  if (jobs_to_passes(jobs.data(), jobs.size(), scores.data(), (uint32_t)scores.size(), head[1], P.passes) ||
+      build_sequences(&P, S)) {
+    std::printf("%s\n", last_error().c_str());
+    return 1;
+  }
+  choose_chains(&P, S, allow16());
+  if (describe_passes(&P, S, allow16())) return 1;
+  lay_out_outputs(&P, S);
+  build_chains(&P, S);
+  build_buckets(&P, S);
+  describe_plan(&P, S);
+  std::vector<uint32_t> at(jobs.size());
+  if (plan_job_buckets(&P, at.data(), at.size())) return 1;
+  std::printf("{\"plan\": %s, \"job_buckets\": [", P.desc.c_str());
+  for (size_t q = 0; q < at.size(); ++q) std::printf("%s%d", q ? ", " : "", (int)at[q]);
+  std::printf("], \"tb_words\": %llu, \"pool_words\": %llu, \"sequences\": %zu}\n",
+              (unsigned long long)P.tb_words, (unsigned long long)P.pool_words, P.seq_len.size());
+  return 0;
+}

@@ -386,3 +386,31 @@ def test_prefix_cut(ctx, calls):
     got = T.sorted_batch(ctx, got_calls, scores=scores)
     for q in range(calls):
         assert got[q] == want[q], (q, got_calls[q])
+
+
+@pytest.mark.parametrize("op", [255, 256, 257, 300, 900])
+def test_wide_prefix_open(ctx, op):
+    """Large gap-open costs on both sides of what the classes past 1,024 cells take (a cell no
+    path reaches gives up the opening too), at their first and last widths and below them."""
+    rng = np.random.default_rng(2681 + op)
+    scores = ((3, 2, op, 1), (3, 0, op, 0), (0, 2, op, 1))
+    for cells in (1024, 1025, 1222, 1984, 3392, 1026):
+        rows = []
+        half = (cells - 2) // 2
+        wide = (half | 1) + half + (cells - 2) % 2 + 1 > 1024
+        for sci in range(len(scores)):
+            for kind in ("noisy", "shifted", "half"):
+                band, extra = (cells - 2) // 2, (cells - 2) % 2
+                m = cells // 2 + 300 + int(rng.integers(0, 60))
+                p, t = _noisy(rng, m, 0.05) if kind == "noisy" else \
+                    _shifted(rng, m, int(rng.integers(-m // 3, m // 3 + 1)))
+                if kind == "half":
+                    t = t[:m // 2] + rng.integers(0, 4, m).tolist()
+                t = (t + rng.integers(0, 4, m).tolist())[:m + extra]
+                rows.append((p, t, band, None, R.I32_MAX, 0, 1, sci))
+                rows += [(p, t, band, len(t), xd, 5, 1, sci) for xd in (50, R.I32_MAX)]
+        out, kinds = _run_prefix(ctx, rows, scores)
+        team = any(k == "wave16x" and lanes > 32 for k, _, lanes in kinds)
+        assert any(k == "wave16x" for k, _, _ in kinds) == (op <= 256 or not wide), (cells, kinds)
+        assert team == (op <= 256 and wide), (cells, kinds)
+        _check_prefix(rows, out, scores)

@@ -1,0 +1,72 @@
+"""The plan build's host phases on the CPU (tests/plan_check.cu): which kernel class each job gets
+and the sizes the plan takes."""
+import json
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import refcases as R
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    from spearfish_gb300 import build
+    lib = build.build()
+    exe = str(tmp_path_factory.mktemp("plan") / "plan_check")
+    cmd = [build.nvcc(), *build.ARCH, "-std=c++17", "-O1", "--expt-relaxed-constexpr", "-I", build.INCLUDE,
+           os.path.join(ROOT, "tests", "plan_check.cu"), lib, "-o", exe,
+           "-Xlinker", "-rpath," + os.path.dirname(lib)]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+    def run(jobs, scores=(R.ONT,), pool_bytes=None, sms=152):
+        if pool_bytes is None:
+            pool_bytes = int(max((jobs["p_off"] + jobs["m"]).max(), (jobs["t_off"] + jobs["n"]).max()))
+        path = exe + ".in"
+        with open(path, "wb") as f:
+            np.array([sms, pool_bytes, len(scores), len(jobs)], np.uint64).tofile(f)
+            np.array([tuple(s) for s in scores], np.int32).tofile(f)
+            jobs.tofile(f)
+        out = subprocess.run([exe, path], capture_output=True, text=True, timeout=120)
+        assert out.returncode == 0, out.stdout + out.stderr
+        plan = json.loads(out.stdout)
+        plan["kinds"] = [plan["plan"]["buckets"][b]["kind"] for b in plan["job_buckets"]]
+        return plan
+    return run
+
+
+def _jobs(rows):
+    """rows: dicts of job fields; patterns and texts one after another in the pool."""
+    from spearfish_gb300 import batch as B
+    jobs, at = B.new_jobs(len(rows)), 0
+    for j, r in zip(jobs, rows):
+        j["p_off"], j["t_off"] = at, at + r["m"]
+        at += r["m"] + r["n"]
+        for k, v in r.items():
+            j[k] = v
+    return jobs
+
+
+@pytest.mark.parametrize("ext", [0, 1])
+def test_wide_prefix_open(check, ext):
+    """A cell no path reaches gives up a gap's opening: four times it at most what such cells hold,
+    256 in the classes past 1,024 cells, and past 900 in no class."""
+    from spearfish_gb300 import batch as B
+    rows, want, scores = [], [], []
+    for op in (255, 256, 257, 300, 900, 901):
+        scores.append((3, 2 * ext, op, ext))
+        for cells in (1023, 1025, 1222, 1984, 3391):
+            for kind in (B.JOB_AFFINE, B.JOB_EXTEND_WINDOW):
+                rows.append(dict(m=2000, n=2000, band=(cells - 1) // 2, kind=kind, mode=R.PREFIX,
+                                 window=2000, xdrop=50, sc_index=len(scores) - 1, want_cigar=1))
+                # below + above + 1 cells, below made odd.
+                below = (cells - 1) // 2
+                w = (below | 1) + below + 1
+                want.append(op <= (256 if w > 1024 else 900))
+    plan = check(_jobs(rows), scores)
+    for r, k, ok in zip(rows, plan["kinds"], want):
+        assert (k == "wave16x") == ok, (r, scores[r["sc_index"]], k)
