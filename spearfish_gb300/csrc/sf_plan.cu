@@ -1843,35 +1843,36 @@ uint64_t plan_bytes_estimate(const std::vector<Pass>& passes, uint64_t pool_byte
   // Mirrors plan_build's sizes: byte pool, packed pool, descriptors, results, traceback
   // arena, CIGAR slots (twice: slots and compacted), wide-row scratch; DevBuf keeps 25%
   // headroom on each.
-  uint64_t b = pool_bytes + 256 * 4 + 4096;
+  constexpr uint64_t kSeqs = 2 * 20, kOrder = 4 + sizeof(uint2);  // order and task
+  constexpr uint64_t kAffine = sizeof(DJob) + sizeof(DParams) + sizeof(DRes) + sizeof(TJob) + sizeof(TRes) + 8 + 4;
+  constexpr uint64_t kMyers = sizeof(MJob) + 4;
+  uint64_t b = pool_bytes + 512 * 4 + 8192;
   uint64_t scratch = 0;
   const bool use16 = allow16();
   const int lanes16 = default_lanes16();
   for (const Pass& p : passes) {
-    b += (uint64_t)(p.m + p.n + 34) / 4 + 40 + 200;
+    b += (uint64_t)(p.m + p.n + 34) / 4 + kSeqs + kOrder + (p.kind == PK_MYERS ? kMyers : kAffine);
     if (p.kind == PK_MYERS) continue;
     uint32_t flags = 0;
     DJob j = make_djob(p, flags);
     const int64_t wmax = band_wmax(j, flags);
-    int c = 4;
-    bool wide = false;
-    PassKind kind = PK_AFFINE;
-    int ln = 32;
-    uint64_t tb_wave = 0;
-    // The cheap and the fast class: the larger traceback.
-    for (int lean = 0; lean < 2 && p.want_cigar && p.kind != PK_LOCAL; ++lean) {
-      classify_affine(p, j, flags, wmax, use16, lean ? 0 : UINT64_MAX, kind, c, wide, ln, lanes16);
-      if (!is_wave(kind)) break;
-      tb_wave = std::max(tb_wave, sfk::wave_tb_words(sfk::kWave[c], wave_steps(j, kind)) * 4);
+    const bool tb = p.want_cigar && p.kind != PK_LOCAL;
+    // A pass gets its cheap or its fast class by the plan it is in, and either may be a row or an
+    // anti-diagonal one (a short pattern in a wide band: rows among many, a team among few): the larger.
+    uint64_t tb_bytes = 0;
+    for (const uint64_t long_steps : {UINT64_MAX, uint64_t(0)}) {
+      int c = 4, ln = 32;
+      bool wide = false;
+      PassKind kind = PK_AFFINE;
+      classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, ln, lanes16);
+      const uint64_t words = is_wave(kind)
+                                 ? sfk::wave_tb_words(sfk::kWave[c], wave_steps(j, kind))
+                                 : (uint64_t)p.m * (tb_row_words(c, wide ? wide_chunks(c, wmax) : 1) * (uint64_t)ln / 32);
+      if (tb) tb_bytes = std::max(tb_bytes, words * 4);
+      if (wide) scratch = std::max<uint64_t>(scratch, (uint64_t)wide_chunks(c, wmax) * 32 * c);
     }
-    classify_affine(p, j, flags, wmax, use16, UINT64_MAX, kind, c, wide, ln, lanes16);
-    if (p.want_cigar && p.kind != PK_LOCAL) {
-      b += is_wave(kind)
-               ? tb_wave
-               : (uint64_t)p.m * tb_row_words(c, wide ? wide_chunks(c, wmax) : 1) * 4 * ln / 32;
-      b += 2 * ((uint64_t)p.m + p.n + 2) * 4;
-    }
-    if (wide) scratch = std::max<uint64_t>(scratch, (uint64_t)wide_chunks(c, wmax) * 32 * c);
+    b += tb_bytes;
+    if (tb) b += 2 * ((uint64_t)p.m + p.n + 2) * 4;
   }
   // Wide buckets (with and without traceback): up to 2 blocks/SM x 4 warps x 4 rows each.
   b += scratch * 4 * 2 * 304 * 4 * 4 * 2;

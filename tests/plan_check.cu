@@ -39,7 +39,16 @@ int main(int, char** argv) {
   if (plan_job_buckets(&P, at.data(), at.size())) return 1;
   std::printf("{\"plan\": %s, \"job_buckets\": [", P.desc.c_str());
   for (size_t q = 0; q < at.size(); ++q) std::printf("%s%d", q ? ", " : "", (int)at[q]);
-  std::printf("], \"tb_words\": %llu, \"pool_words\": %llu, \"sequences\": %zu}\n",
-              (unsigned long long)P.tb_words, (unsigned long long)P.pool_words, P.seq_len.size());
+  // What upload_plan asks for, buffer by buffer.
+  const uint64_t needs = P.pool_bytes + 4 * P.pool_words + 20 * P.seq_len.size() +
+                         S.dj.size() * (sizeof(DJob) + sizeof(DParams) + sizeof(DRes) + sizeof(TJob) + sizeof(TRes)) +
+                         S.mj.size() * (sizeof(MJob) + 4) + 4 * P.tb_words + 8 * P.ops_words + 12 * S.wlist.size() +
+                         4 * S.order.size() + sizeof(uint2) * S.tasks.size() + 4 * P.buckets.size() +
+                         4 * S.scratch_total + 14 * 64;
+  std::printf("], \"tb_words\": %llu, \"pool_words\": %llu, \"sequences\": %zu, \"needs\": %llu, "
+              "\"estimate\": %llu}\n",
+              (unsigned long long)P.tb_words, (unsigned long long)P.pool_words, P.seq_len.size(),
+              (unsigned long long)(needs + needs / 4 + 14 * 256),
+              (unsigned long long)plan_bytes_estimate(P.passes, P.pool_bytes));
   return 0;
 }

@@ -70,3 +70,17 @@ def test_wide_prefix_open(check, ext):
     plan = check(_jobs(rows), scores)
     for r, k, ok in zip(rows, plan["kinds"], want):
         assert (k == "wave16x") == ok, (r, scores[r["sc_index"]], k)
+
+
+@pytest.mark.parametrize("count", [1, 40, 4000])
+@pytest.mark.parametrize("m,n,band", [(1000, 1060, 600), (1000, 650, 600), (400, 460, 300), (90, 100, 30),
+                                      (60, 300, 120), (2000, 2100, 64)])
+def test_estimate_is_an_upper_bound(check, m, n, band, count):
+    """plan_bytes_estimate, which the server admits requests by, against what the plan takes: short
+    patterns in wide bands, whose passes run on rows or on a team by how many there are."""
+    from spearfish_gb300 import batch as B
+    for kind in (B.JOB_AFFINE, B.JOB_EXTEND_WINDOW):
+        for cigar in (0, 1):
+            row = dict(m=m, n=n, band=band, kind=kind, mode=R.PREFIX, window=n, xdrop=100, want_cigar=cigar)
+            plan = check(_jobs([row] * count))
+            assert plan["estimate"] >= plan["needs"], (plan["kinds"][0], plan["estimate"], plan["needs"])
