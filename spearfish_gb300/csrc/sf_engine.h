@@ -238,6 +238,7 @@ struct sf_plan {
   // cell: -1 by the plan's passes, else as set (the autotuner's trial plans).
   int lean = -1;
   int most = 0;  // Myers pairs a warp at most, likewise (0: by the plan's passes)
+  int team = -1;            // warps a Myers pair may take, likewise
   uint64_t long_steps = 0;  // the row steps of a long pass, likewise
   // Class overrides for this plan only (the autotuner's trial plans); else the context's.
   const sfe::TuneTable* tune_override = nullptr;
@@ -337,13 +338,16 @@ void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax,
                      int lanes16 = 32);
 // The band cells the anti-diagonal kernel lays out for a pass.
 int64_t wave_width(const DJob& j);
-// Whether a plan of np passes takes the Myers and anti-diagonal classes that finish a pass
-// fastest, rather than the cheapest ones a cell.
 int myers_team(const sf_plan* P);
 int pass_lanes16(const Pass& p, size_t np, int lanes16);
+// Whether a plan of np passes takes the Myers and anti-diagonal classes that finish a pass
+// fastest, rather than the cheapest ones a cell.
 bool lean_plan(size_t np, int sms);
 bool plan_is_lean(const sf_plan* P);
 uint64_t plan_long_steps(const sf_plan* P);
+// Sets on S all that a pass's default class depends on beside the pass: S, of some of P's passes,
+// then gives them the classes P does.
+void choose_as(const sf_plan* P, sf_plan* S);
 inline bool is_wave(int kind) { return kind == PK_WAVE16 || kind == PK_WAVE16X || kind == PK_WAVE16C; }
 // Row steps of a pass on the anti-diagonal kernel.
 uint64_t wave_steps(const DJob& j, int kind);

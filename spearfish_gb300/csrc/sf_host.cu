@@ -1333,7 +1333,6 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   if (reps == 0) reps = 1;
   const auto t0 = std::chrono::steady_clock::now();
   const bool use16 = allow16();
-  const bool lean = plan_is_lean(P);
   const int most = most_pairs(P), team = myers_team(P);
   const uint64_t long_steps = plan_long_steps(P);
   // Group the passes by their default class.
@@ -1350,9 +1349,7 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   sf_plan S;  // trial plan, its buffers reused across trials
   S.ctx = ctx;
   S.pool_bytes = P->pool_bytes;
-  S.lean = lean;
-  S.most = most;
-  S.long_steps = long_steps;
+  choose_as(P, &S);
   void* uploaded = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CK(cudaEventCreate(&e0));

@@ -219,8 +219,16 @@ int most_pairs(const sf_plan* P) {
 // Warps a pair of a small plan may take: as long as that leaves schedulers idle (1,762 Global pairs
 // of 4.8 kb in one call: 2.19 ms on four warps of one block a lane, 1.36 on one of three; 450 of 5 kb 0.61, 0.49).
 int myers_team(const sf_plan* P) {
+  if (P->team >= 0) return P->team;
   if (!plan_is_lean(P)) return 0;
   return (int)std::min<size_t>(4, (size_t)P->ctx->sms * 10 / std::max<size_t>(1, P->passes.size()));
+}
+
+void choose_as(const sf_plan* P, sf_plan* S) {
+  S->lean = plan_is_lean(P);
+  S->most = most_pairs(P);
+  S->team = myers_team(P);
+  S->long_steps = plan_long_steps(P);
 }
 
 int shown_c(int kind, int c) { return is_wave(kind) ? 4 * sfk::kWave[c].q : c; }

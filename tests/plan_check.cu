@@ -39,13 +39,34 @@ int main(int, char** argv) {
   if (plan_job_buckets(&P, at.data(), at.size())) return 1;
   std::printf("{\"plan\": %s, \"job_buckets\": [", P.desc.c_str());
   for (size_t q = 0; q < at.size(); ++q) std::printf("%s%d", q ? ", " : "", (int)at[q]);
+  // The passes of each class in a plan of their own, as the autotuner times them: how many get
+  // another class there.
+  std::map<std::tuple<int, int, int, int, int>, std::vector<size_t>> alike;
+  for (size_t q = 0; q < jobs.size(); ++q) {
+    const BucketKey& k = S.per[q].first;
+    alike[{k.kind, k.c, k.wide, k.tb, k.lanes}].push_back(q);
+  }
+  size_t strays = 0;
+  for (const auto& g : alike) {
+    sf_plan T;
+    T.ctx = &ctx;
+    T.pool_bytes = P.pool_bytes;
+    T.scratch.reset(new BuildScratch);
+    choose_as(&P, &T);
+    for (size_t q : g.second) T.passes.push_back(P.passes[q]);
+    if (build_sequences(&T, *T.scratch)) return 1;
+    choose_chains(&T, *T.scratch, allow16());
+    if (describe_passes(&T, *T.scratch, allow16())) return 1;
+    for (const auto& it : T.scratch->per) strays += !(it.first == S.per[g.second[0]].first);
+  }
+  std::printf("], \"strays\": %zu", strays);
   // What upload_plan asks for, buffer by buffer.
   const uint64_t needs = P.pool_bytes + 4 * P.pool_words + 20 * P.seq_len.size() +
                          S.dj.size() * (sizeof(DJob) + sizeof(DParams) + sizeof(DRes) + sizeof(TJob) + sizeof(TRes)) +
                          S.mj.size() * (sizeof(MJob) + 4) + 4 * P.tb_words + 8 * P.ops_words + 12 * S.wlist.size() +
                          4 * S.order.size() + sizeof(uint2) * S.tasks.size() + 4 * P.buckets.size() +
                          4 * S.scratch_total + 14 * 64;
-  std::printf("], \"tb_words\": %llu, \"pool_words\": %llu, \"sequences\": %zu, \"needs\": %llu, "
+  std::printf(", \"tb_words\": %llu, \"pool_words\": %llu, \"sequences\": %zu, \"needs\": %llu, "
               "\"estimate\": %llu}\n",
               (unsigned long long)P.tb_words, (unsigned long long)P.pool_words, P.seq_len.size(),
               (unsigned long long)(needs + needs / 4 + 14 * 256),

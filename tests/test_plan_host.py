@@ -84,3 +84,15 @@ def test_estimate_is_an_upper_bound(check, m, n, band, count):
             row = dict(m=m, n=n, band=band, kind=kind, mode=R.PREFIX, window=n, xdrop=100, want_cigar=cigar)
             plan = check(_jobs([row] * count))
             assert plan["estimate"] >= plan["needs"], (plan["kinds"][0], plan["estimate"], plan["needs"])
+
+
+@pytest.mark.parametrize("others,pairs", [(700, 300), (100, 40), (20, 1500), (3000, 900)])
+def test_trial_plans_keep_the_classes(check, others, pairs):
+    """The autotuner times the passes of one class in a plan of their own, which is smaller: they
+    must get the same default class there, or the candidates it names would not be what runs."""
+    from spearfish_gb300 import batch as B
+    rows = [dict(m=500 + 7 * (q % 50), n=560, band=40, kind=B.JOB_AFFINE, mode=R.GLOBAL, want_cigar=1)
+            for q in range(others)]
+    rows += [dict(m=m, n=m, kind=B.JOB_MYERS, mode=R.INFIX) for m in (700, 40 * 64, 100 * 64, 200 * 64)
+             for _ in range(pairs // 4)]
+    assert check(_jobs(rows))["strays"] == 0
