@@ -528,12 +528,15 @@ int stage_done(sf_plan* P) {
 // pattern for u even, its text for u odd).  A pattern (text) is packed once for a run of
 // consecutive passes that name it -- a read's distance and alignment, a read against its
 // candidates; one named again later is packed again, which costs less than finding it: 160,000
-// flanks in no order took 11 ms to sort and 0.05 ms to pack.  Sequences of at least kLongSeq
-// bases, where a copy would weigh, are looked up.
+// flanks in no order took 11 ms to sort and 0.05 ms to pack.  Where copies would weigh, they are
+// looked up: sequences of at least kLongSeq bases, and of kShared once the passes name more than
+// twice the bases there are (a few transcripts named by many reads in turn: 200,000 reads on 100
+// transcripts of 10-60 kb held 2.17 GB unshared, 0.08 looked up, in 42.5 and 41.3 ms a call; with
+// 1-3 kb ones, a million reads, 0.98 GB in 32 ms, but 0.33 in 43 looked up).
 int build_sequences(sf_plan* P, BuildScratch& S) {
   const sf_context* ctx = P->ctx;
   const size_t np = P->passes.size();
-  constexpr uint32_t kLongSeq = 1u << 16;
+  constexpr uint32_t kLongSeq = 1u << 16, kShared = 1u << 12;
   constexpr int kChunks = 16;
   auto bad_pass = [&](const Pass& p) {
     return (p.p_off & kOffMask) + p.m > P->pool_bytes ||
@@ -549,8 +552,9 @@ int build_sequences(sf_plan* P, BuildScratch& S) {
   };
   // Per chunk of passes (the same chunks below): its new sequences and their words.
   size_t cnt[kChunks] = {};
-  uint64_t wsum[kChunks] = {}, first_bad[kChunks];
-  bool has_long[kChunks] = {};
+  uint64_t wsum[kChunks] = {}, bases[kChunks] = {}, first_bad[kChunks];
+  uint32_t longest[kChunks] = {};
+  bool stored[kChunks] = {};
   std::fill(first_bad, first_bad + kChunks, UINT64_MAX);
   parallel_chunks(np, 2048, kChunks, [&](size_t q0, size_t q1, int k) {
     for (size_t q = q0; q < q1; ++q) {
@@ -563,12 +567,15 @@ int build_sequences(sf_plan* P, BuildScratch& S) {
       if (q == q0 || new_p(q)) {
         cnt[k]++;
         wsum[k] += seq_words(p.m);
+        bases[k] += p.m;
       }
       if (q == q0 || new_t(q)) {
         cnt[k]++;
         wsum[k] += seq_words(p.n);
+        bases[k] += p.n;
       }
-      has_long[k] = has_long[k] || p.m >= kLongSeq || p.n >= kLongSeq;
+      longest[k] = std::max({longest[k], p.m, p.n});
+      stored[k] = stored[k] || (p.t_off & kStoreFlag);
     }
   });
   const uint64_t bad = *std::min_element(first_bad, first_bad + kChunks);
@@ -582,28 +589,100 @@ int build_sequences(sf_plan* P, BuildScratch& S) {
   auto& word_of = S.word_of;
   word_of.resize(2 * np);
   uint64_t words = 0;
-  if (std::any_of(has_long, has_long + kChunks, [](bool v) { return v; })) {
-    // In pass order, long sequences by (offset, length).
-    std::map<std::pair<uint64_t, uint32_t>, uint64_t> seen;
+  uint64_t named = 0, there = P->pool_bytes;
+  for (int k = 0; k < kChunks; ++k) named += bases[k];
+  if (std::any_of(stored, stored + kChunks, [](bool v) { return v; })) there += ctx->store->bases;
+  const uint32_t least = named / 2 > there ? kShared : kLongSeq;
+  if (*std::max_element(longest, longest + kChunks) >= least) {
+    // In pass order; a long sequence once a chunk of passes, and where a chunk names it again,
+    // once among the chunks.
+    struct Seq {
+      uint64_t off;
+      uint32_t len;
+      bool again;
+    };
+    // Sequences by (offset, length): places in a list of at most `most`.
+    struct Seen {
+      std::vector<uint32_t> at;
+      size_t mask;
+      explicit Seen(size_t most) {
+        size_t n = 16;
+        while (n < 2 * most) n *= 2;
+        at.assign(n, UINT32_MAX);
+        mask = n - 1;
+      }
+      // The place in `list` of (off, len); UINT32_MAX if it is not there (it goes to the list's end).
+      uint32_t find(const std::vector<Seq>& list, uint64_t off, uint32_t len) {
+        const uint64_t h = (off ^ (uint64_t)len << 40) * 0x9e3779b97f4a7c15ull;
+        for (size_t u = (size_t)(h >> 32) & mask;; u = (u + 1) & mask) {
+          if (at[u] == UINT32_MAX) {
+            at[u] = (uint32_t)list.size();
+            return UINT32_MAX;
+          }
+          if (list[at[u]].off == off && list[at[u]].len == len) return at[u];
+        }
+      }
+    };
+    std::vector<Seq> mine[kChunks];
+    std::vector<uint64_t> at[kChunks];
+    parallel_chunks(np, 2048, kChunks, [&](size_t q0, size_t q1, int k) {
+      Seen seen(cnt[k]);
+      uint64_t wp = 0, wt = 0;
+      auto place = [&](uint64_t off, uint32_t len) {
+        if (len >= least) {
+          const uint32_t u = seen.find(mine[k], off, len);
+          if (u != UINT32_MAX) {
+            mine[k][u].again = true;
+            return (uint64_t)u;
+          }
+        }
+        mine[k].push_back(Seq{off, len, false});
+        return (uint64_t)mine[k].size() - 1;
+      };
+      for (size_t q = q0; q < q1; ++q) {
+        const Pass& p = P->passes[q];
+        if (q == q0 || new_p(q)) wp = place(p.p_off, p.m);
+        if (q == q0 || new_t(q)) wt = place(p.t_off, p.n);
+        word_of[2 * q] = wp;
+        word_of[2 * q + 1] = wt;
+      }
+    });
+    size_t total = 0, shared = 0;
+    for (const auto& list : mine) {
+      total += list.size();
+      for (const Seq& q : list) shared += q.again || q.len >= kLongSeq;
+    }
+    Seen seen(shared);
+    std::vector<Seq> first;            // the shared sequences
+    std::vector<uint64_t> first_word;  // and their words
     P->seq_boff.clear();
     P->seq_len.clear();
     P->seq_woff.clear();
-    auto place = [&](uint64_t off, uint32_t len) {
-      if (len >= kLongSeq) {
-        const auto it = seen.emplace(std::make_pair(off, len), words);
-        if (!it.second) return it.first->second;
+    P->seq_boff.reserve(total);
+    P->seq_len.reserve(total);
+    P->seq_woff.reserve(total);
+    for (int k = 0; k < kChunks; ++k) {
+      at[k].reserve(mine[k].size());
+      for (const Seq& q : mine[k]) {
+        if (q.again || q.len >= kLongSeq) {
+          const uint32_t u = seen.find(first, q.off, q.len);
+          if (u != UINT32_MAX) {
+            at[k].push_back(first_word[u]);
+            continue;
+          }
+          first.push_back(q);
+          first_word.push_back(words);
+        }
+        at[k].push_back(words);
+        P->seq_boff.push_back(q.off);
+        P->seq_len.push_back(q.len);
+        P->seq_woff.push_back(words);
+        words += seq_words(q.len);
       }
-      P->seq_boff.push_back(off);
-      P->seq_len.push_back(len);
-      P->seq_woff.push_back(words);
-      words += seq_words(len);
-      return P->seq_woff.back();
-    };
-    for (size_t q = 0; q < np; ++q) {
-      const Pass& p = P->passes[q];
-      word_of[2 * q] = new_p(q) ? place(p.p_off, p.m) : word_of[2 * q - 2];
-      word_of[2 * q + 1] = new_t(q) ? place(p.t_off, p.n) : word_of[2 * q - 1];
     }
+    parallel_chunks(np, 2048, kChunks, [&](size_t q0, size_t q1, int k) {
+      for (size_t u = 2 * q0; u < 2 * q1; ++u) word_of[u] = at[k][word_of[u]];
+    });
   } else {
     // Each chunk's new sequences at their places, from the counts above.
     size_t at0[kChunks] = {}, total = 0;

@@ -29,6 +29,15 @@ int main(int, char** argv) {
     std::printf("%s\n", last_error().c_str());
     return 1;
   }
+  // Each pass's sequences lie where its words begin.
+  std::map<uint64_t, std::pair<uint64_t, uint32_t>> placed;
+  for (size_t u = 0; u < P.seq_len.size(); ++u) placed[P.seq_woff[u]] = {P.seq_boff[u], P.seq_len[u]};
+  for (size_t q = 0; q < jobs.size(); ++q) {
+    const Pass& p = P.passes[q];
+    if (placed[S.word_of[2 * q]] != std::make_pair(p.p_off, p.m) ||
+        placed[S.word_of[2 * q + 1]] != std::make_pair(p.t_off, p.n))
+      return 3;
+  }
   choose_chains(&P, S, allow16());
   if (describe_passes(&P, S, allow16())) return 1;
   lay_out_outputs(&P, S);

@@ -96,3 +96,27 @@ def test_trial_plans_keep_the_classes(check, others, pairs):
     rows += [dict(m=m, n=m, kind=B.JOB_MYERS, mode=R.INFIX) for m in (700, 40 * 64, 100 * 64, 200 * 64)
              for _ in range(pairs // 4)]
     assert check(_jobs(rows))["strays"] == 0
+
+
+@pytest.mark.parametrize("count", [1, 12, 2047, 50000])
+@pytest.mark.parametrize("text", [300, 4096, 40000, 70000])
+def test_shared_sequences(check, text, count):
+    """Many reads that name a few transcripts in turn: each transcript is packed once where its
+    copies would weigh, and every pass finds its own sequences."""
+    from spearfish_gb300 import batch as B
+    rng = np.random.default_rng(31)
+    texts = 7
+    jobs = B.new_jobs(count)
+    jobs["kind"], jobs["mode"] = B.JOB_MYERS, R.INFIX
+    jobs["m"] = rng.integers(0, 200, count)
+    which = np.arange(count) % texts
+    jobs["n"] = text + which % 2
+    jobs["t_off"] = which * (text + 1)
+    jobs["p_off"] = texts * (text + 1) + np.concatenate([[0], np.cumsum(jobs["m"])[:-1]])
+    plan = check(jobs)
+    packed = 16 * plan["pool_words"]
+    there = texts * (text + 1) + int(jobs["m"].sum())
+    if text >= 4096:
+        assert packed <= 2 * there + 16 * (plan["sequences"] + 512)
+    if text >= 4096 and count > 20 * texts:
+        assert plan["sequences"] <= count + texts
