@@ -118,7 +118,8 @@ bool fits_wave(const Pass& p, const DJob& j, uint32_t flags, PassKind& kind) {
   if (s.mat < 0 || s.mat > 1000 || s.ext < 0 || s.ext > 1000 || s.mis != 2 * s.ext) return false;
   if (s.open < 1 || s.open > 900) return false;
   const int64_t w = wave_width(j), shorter = std::min(p.m, p.n);
-  if (4 * ((int64_t)s.mat + 2 * s.ext) * ((int64_t)p.m + p.n) >= 1 << 30) return false;
+  // Scores and row steps in 32 bits (scores of zero too).
+  if (4 * std::max<int64_t>(1, (int64_t)s.mat + 2 * s.ext) * ((int64_t)p.m + p.n) >= 1 << 30) return false;
   if (p.m < 1 || p.n < 1 || w > (prefix ? 4 * (shorter + 1) + 64 : 2 * (shorter + 1))) return false;
   if (prefix && (int64_t)p.m > (int64_t)p.n + j.below) return false;  // ends past the text
   const bool cut = flags & F_CUT;

@@ -120,3 +120,14 @@ def test_shared_sequences(check, text, count):
         assert packed <= 2 * there + 16 * (plan["sequences"] + 512)
     if text >= 4096 and count > 20 * texts:
         assert plan["sequences"] <= count + texts
+
+
+@pytest.mark.parametrize("scores", [(0, 0, 1, 0), (2, 4, 4, 2)])
+def test_longest_sequences(check, scores):
+    """Sequences whose row steps (or scores) would pass 32 bits stay off the anti-diagonal kernel,
+    also where every step scores zero."""
+    from spearfish_gb300 import batch as B
+    for mode in (R.GLOBAL, R.PREFIX):
+        rows = [dict(m=m, n=m, band=20, kind=B.JOB_AFFINE, mode=mode) for m in (1 << 20, (1 << 30) + 5)]
+        kinds = check(_jobs(rows), [scores])["kinds"]
+        assert kinds[0].startswith("wave16") and not kinds[1].startswith("wave16"), kinds
