@@ -206,7 +206,7 @@ struct sf_plan {
   std::vector<uint32_t> slot;
   uint32_t n_aff = 0, n_my = 0, n_walk = 0;
   uint32_t n_tasks = 0;  // tasks of all launches (d_tasks: the tasks, then the job order)
-  bool myers_kcut = false;  // a Myers pass is Global or Prefix with k < m + n
+  bool myers_kcut = false;  // a Myers pass is Global or Prefix and myers_capped
   std::vector<Bucket> buckets;
   std::vector<Group> groups;
   uint64_t tb_words = 0, ops_words = 0, scratch_cells = 0;

@@ -884,7 +884,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
         m.n = p.n;
         m.mode = p.mode;
         m.k = p.k;
-        if (p.mode != SF_INFIX && (uint64_t)p.k < (uint64_t)p.m + p.n) kcut[worker] = true;
+        if (p.mode != SF_INFIX && myers_capped(p.k, p.m, p.n)) kcut[worker] = true;
         per[q] = {Key2{PK_MYERS, b, 0, 0, lanes},
                   Item{sl, (uint64_t)p.n, ((uint64_t)p.n + (uint64_t)lanes) * 65u * (uint64_t)b}};
         has_item[q] = 1;

@@ -68,7 +68,7 @@ int main(int, char** argv) {
     if (describe_passes(&T, *T.scratch, allow16())) return 1;
     for (const auto& it : T.scratch->per) strays += !(it.first == S.per[g.second[0]].first);
   }
-  std::printf("], \"strays\": %zu", strays);
+  std::printf("], \"strays\": %zu, \"myers_kcut\": %s", strays, P.myers_kcut ? "true" : "false");
   // What upload_plan asks for, buffer by buffer.
   const uint64_t needs = P.pool_bytes + 4 * P.pool_words + 20 * P.seq_len.size() +
                          S.dj.size() * (sizeof(DJob) + sizeof(DParams) + sizeof(DRes) + sizeof(TJob) + sizeof(TRes)) +

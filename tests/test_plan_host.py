@@ -131,3 +131,14 @@ def test_longest_sequences(check, scores):
         rows = [dict(m=m, n=m, band=20, kind=B.JOB_AFFINE, mode=mode) for m in (1 << 20, (1 << 30) + 5)]
         kinds = check(_jobs(rows), [scores])["kinds"]
         assert kinds[0].startswith("wave16") and not kinds[1].startswith("wave16"), kinds
+
+
+@pytest.mark.parametrize("mode", [R.INFIX, R.PREFIX, R.GLOBAL])
+def test_caps_that_stop_pairs(check, mode):
+    """A capped Global or Prefix pair may stop early where the kernel's column scores, 32 bits,
+    hold its cap; caps of 2^30 and more (texts of more than 2^30 columns) never do."""
+    from spearfish_gb300 import batch as B
+    for n, k in ((900, 0), (900, 1799), (900, 1800), (1500000000, (1 << 30) - 1), (1500000000, 1 << 30),
+                 (1500000000, 1200000000), (900, 0xFFFFFFFF)):
+        plan = check(_jobs([dict(m=900, n=n, kind=B.JOB_MYERS, mode=mode, k=k)]))
+        assert plan["myers_kcut"] == (mode != R.INFIX and k < 900 + n and k < 1 << 30), (n, k)
