@@ -558,6 +558,10 @@ int build_sequences(sf_plan* P, BuildScratch& S) {
   bool stored[kChunks] = {};
   std::fill(first_bad, first_bad + kChunks, UINT64_MAX);
   parallel_chunks(np, 2048, kChunks, [&](size_t q0, size_t q1, int k) {
+    size_t c = 0;
+    uint64_t w = 0, b = 0;
+    uint32_t most = 0;
+    bool store = false;
     for (size_t q = q0; q < q1; ++q) {
       const Pass& p = P->passes[q];
       if (bad_pass(p)) {
@@ -566,18 +570,23 @@ int build_sequences(sf_plan* P, BuildScratch& S) {
       }
       // A chunk's first pass starts anew: its chunk knows nothing of the one before.
       if (q == q0 || new_p(q)) {
-        cnt[k]++;
-        wsum[k] += seq_words(p.m);
-        bases[k] += p.m;
+        c++;
+        w += seq_words(p.m);
+        b += p.m;
       }
       if (q == q0 || new_t(q)) {
-        cnt[k]++;
-        wsum[k] += seq_words(p.n);
-        bases[k] += p.n;
+        c++;
+        w += seq_words(p.n);
+        b += p.n;
       }
-      longest[k] = std::max({longest[k], p.m, p.n});
-      stored[k] = stored[k] || (p.t_off & kStoreFlag);
+      most = std::max({most, p.m, p.n});
+      store = store || (p.t_off & kStoreFlag);
     }
+    cnt[k] = c;
+    wsum[k] = w;
+    bases[k] = b;
+    longest[k] = most;
+    stored[k] = store;
   });
   const uint64_t bad = *std::min_element(first_bad, first_bad + kChunks);
   if (bad != UINT64_MAX) {
