@@ -180,6 +180,7 @@ struct Group {
   uint32_t bucket = 0;                      // its first bucket (kind, c, tb)
   uint32_t task_first = 0, task_count = 0;  // none: the bucket's own order range
   int grid = 0, block = 128, stream = 0;
+  bool lead = false;  // starts before the others, on the plan's own stream
 };
 
 }  // namespace sfe
@@ -209,6 +210,7 @@ struct sf_plan {
   bool myers_kcut = false;  // a Myers pass is Global or Prefix and myers_capped
   std::vector<Bucket> buckets;
   std::vector<Group> groups;
+  int streams = 1;  // auxiliary streams its launches share
   uint64_t tb_words = 0, ops_words = 0, scratch_cells = 0;
   int wide_warps = 0;
   std::string desc;
@@ -271,10 +273,12 @@ struct sf_context {
   int dev = 0;
   int sms = 0;
   cudaStream_t s = nullptr;
-  // Auxiliary streams that launches share round robin: as many as the device has hardware
-  // queues by default.  More would share queues, and a launch would wait for another stream's
-  // (with twelve, config 3's four streams past the eighth held back a third of its buckets).
-  static constexpr int kAux = 8;
+  // Auxiliary streams that launches share.  A plan of few passes has all of them: its launches
+  // leave the device idle one after another (644 pairs of 984 bases, bands 5-600, 14 launches: 1.20
+  // ms over 8, 0.86 over 16).  A plan of many has kBusy, one (the leading launch's, as a rule) more
+  // than the device has hardware queues by default: more crowd each other's blocks (5,447
+  // extensions, 30 launches: 7.8 ms over 9, 9.3 over 13).
+  static constexpr int kAux = 16, kBusy = 9;
   cudaStream_t aux[kAux] = {};
   cudaEvent_t fork = nullptr, join[kAux] = {};
   std::unique_ptr<sf_plan> cache;  // reused by sf_batch_run

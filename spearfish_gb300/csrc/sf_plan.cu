@@ -1320,6 +1320,7 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
              sfk::wave_warps(sfk::kWave[x.c]) == sfk::wave_warps(sfk::kWave[y.c]);
     return x.c == y.c && (x.lanes > 32 ? x.lanes == y.lanes : y.lanes <= 32);
   };
+  P->streams = lean ? sf_context::kAux : sf_context::kBusy;
   std::vector<uint8_t> done(nb, 0);
   double behind[sf_context::kAux] = {};
   for (size_t u = 0; u < nb; ++u) {
@@ -1348,8 +1349,14 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
       g.grid = warps_grid((uint64_t)g.task_count * (team ? g.block / 32 : 1), g.block);
     }
     // Past one a stream, behind the shortest.
-    g.stream = (int)(std::min_element(behind, behind + sf_context::kAux) - behind);
-    if (!P->groups.empty()) behind[g.stream] += (double)b.lat + 1;  // (the first runs beside them)
+    g.stream = (int)(std::min_element(behind, behind + P->streams) - behind);
+    behind[g.stream] += (double)b.lat + 1;
+    // The longest starts first, so that its blocks spread over the SMs: let in later, as others
+    // leave, they crowd the first SMs to empty (55 teams of 3 ms beside 7,600 short passes: 11.2 ms,
+    // 4.4 started first).  With a warp a scheduler it is on every SM in any order, and alone it would
+    // leave the others the tail (7,225 pairs in six launches, the first of 3,656 warps: 1.50 ms, 1.27
+    // beside them).
+    g.lead = P->groups.empty() && (int64_t)g.grid * (g.block / 32) <= 4 * (int64_t)ctx->sms;
     P->groups.push_back(g);
   }
 }
@@ -1575,11 +1582,9 @@ int plan_launch_buckets(sf_plan* P, cudaStream_t s, std::vector<cudaEvent_t>* ev
     const uint32_t task_count = evs ? b.task_count : P->groups[q].task_count;
     const int grid = evs ? b.grid : P->groups[q].grid;
     cudaStream_t bs = s;
-    // The longest launch follows the pack on `s` itself and so starts first, its blocks spread
-    // over the SMs: let in later, as others leave, they crowd the first SMs to empty (55 teams of
-    // 3 ms beside 7,600 short passes: 11.2 ms, 4.4 started first).
-    if (fan && (q > 0 || fan_one)) {
-      const int si = (P->groups[q].stream + soff) % sf_context::kAux;
+    // (The leading launch follows the pack on `s` itself.)
+    if (fan && (!P->groups[q].lead || fan_one)) {
+      const int si = (P->groups[q].stream + soff) % P->streams;
       bs = ctx->aux[si];
       if (!mine[si]) CK(cudaStreamWaitEvent(bs, ctx->fork, 0));
       mine[si] = used[si] = true;

@@ -48,6 +48,10 @@ int main(int, char** argv) {
   if (plan_job_buckets(&P, at.data(), at.size())) return 1;
   std::printf("{\"plan\": %s, \"job_buckets\": [", P.desc.c_str());
   for (size_t q = 0; q < at.size(); ++q) std::printf("%s%d", q ? ", " : "", (int)at[q]);
+  std::printf("], \"launches\": [");
+  for (size_t q = 0; q < P.groups.size(); ++q)
+    std::printf("%s{\"stream\": %d, \"lead\": %s, \"warps\": %d}", q ? ", " : "", P.groups[q].stream,
+                P.groups[q].lead ? "true" : "false", P.groups[q].grid * P.groups[q].block / 32);
   // The passes of each class in a plan of their own, as the autotuner times them: how many get
   // another class there.
   std::map<std::tuple<int, int, int, int, int>, std::vector<size_t>> alike;

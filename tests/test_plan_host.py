@@ -142,3 +142,21 @@ def test_caps_that_stop_pairs(check, mode):
                  (1500000000, 1200000000), (900, 0xFFFFFFFF)):
         plan = check(_jobs([dict(m=900, n=n, kind=B.JOB_MYERS, mode=mode, k=k)]))
         assert plan["myers_kcut"] == (mode != R.INFIX and k < 900 + n and k < 1 << 30), (n, k)
+
+
+@pytest.mark.parametrize("passes", [644, 2900, 20000])
+def test_streams_of_launches(check, passes):
+    """Few passes: a launch of each class on a stream of its own.  The first launch starts before the
+    others only while it leaves schedulers empty."""
+    from spearfish_gb300 import batch as B
+    odd = ((1, 3, 5, 2),)  # on the row kernels, a launch a class
+    rows = [dict(m=900, n=900, band=20 + 640 * (q % 14) // 14, kind=B.JOB_AFFINE, mode=R.GLOBAL, want_cigar=1)
+            for q in range(passes)]
+    launches = check(_jobs(rows), odd)["launches"]
+    streams = [x["stream"] for x in launches]
+    assert 9 < len(launches) <= 16
+    if passes <= 20 * 152:
+        assert len(set(streams)) == len(launches)
+    else:
+        assert max(streams) < 9
+    assert [x["lead"] for x in launches] == [launches[0]["warps"] <= 4 * 152] + [False] * (len(launches) - 1)
