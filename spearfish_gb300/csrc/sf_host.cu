@@ -228,7 +228,7 @@ const char* sf_last_error(void) { return last_error().c_str(); }
 
 const char* sf_version(void) {
   return "spearfish_gb300 sf_align 0.1 (sm_103a; affine C={4,6,8,9,10,11,12,14,16,20,24,28,32,40,48}+wide; "
-         "myers B={1,2,3,4})";
+         "wave16 Q={4,6,8,10,12}; myers B={1,2,3,4})";
 }
 
 int sf_set_device(int device) {
@@ -1225,8 +1225,9 @@ int sf_batch_run(sf_context* ctx, const uint8_t* pool, uint64_t pool_bytes, cons
 
 namespace {
 
-// A pass's class before any override, and the Myers blocks it needs.
-int default_class(const Pass& p, size_t np, bool use16, int team, int most, uint64_t long_steps, ClassKey& key,
+// A pass's class before any override, and the Myers blocks it needs.  (A plan's jobs have no cut
+// column.)
+int default_class(const Pass& p, bool use16, int team, int most, uint64_t long_steps, ClassKey& key,
                   int64_t& blocks) {
   if (p.kind == PK_MYERS) {
     int b = 1, lanes = 1;
@@ -1242,8 +1243,7 @@ int default_class(const Pass& p, size_t np, bool use16, int team, int most, uint
   int c = 4, lanes = 32;
   bool wide = false;
   PassKind kind = PK_AFFINE;
-  classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, lanes,
-                  pass_lanes16(p, np, default_lanes16()));
+  classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, lanes, default_lanes16());
   const bool tb = p.want_cigar && p.kind != PK_LOCAL;
   key = ClassKey{kind, c, wide ? 1 : 0, tb ? 1 : 0, lanes};
   blocks = wmax;  // affine: the group's widest row
@@ -1278,7 +1278,6 @@ std::vector<ClassChoice> tune_candidates(const ClassKey& key, int64_t blocks) {
       const bool home = key.c >= first && key.c < ends[u];
       int left = home ? 2 : (key.c < first ? 1 : 0);
       for (int c = home ? key.c + 1 : first; c < ends[u] && left; ++c) {
-        if (key.kind == PK_WAVE16C && sfk::kWave[c].lanes > 32) continue;
         if (sfk::wave_cap(sfk::kWave[c]) >= cap && (cap > 1024) == (sfk::wave_cap(sfk::kWave[c]) > 1024)) {
           out.push_back(ClassChoice{c, key.lanes});
           --left;
@@ -1341,7 +1340,7 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   for (size_t q = 0; q < P->passes.size(); ++q) {
     ClassKey k;
     int64_t blocks = 0;
-    int rc = default_class(P->passes[q], P->passes.size(), use16, team, most, long_steps, k, blocks);
+    int rc = default_class(P->passes[q], use16, team, most, long_steps, k, blocks);
     if (rc) return rc;
     groups[k].push_back(q);
     gblocks[k] = std::max(gblocks[k], blocks);
@@ -1408,7 +1407,6 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
                                                                : (key.kind == PK_AFFINE16 ? "affine16"
                                                                   : key.kind == PK_WAVE16  ? "wave16"
                                                                   : key.kind == PK_WAVE16X ? "wave16x"
-                                                                  : key.kind == PK_WAVE16C ? "wave16c"
                                                                                            : "affine")),
                   shown_c(key.kind, key.c), key.wide ? "true" : "false", key.tb ? "true" : "false",
                   shown_lanes(key.kind, key.c, key.lanes), g.second.size(), shown_c(key.kind, best.c),

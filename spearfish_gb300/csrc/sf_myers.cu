@@ -86,7 +86,6 @@ __device__ __forceinline__ void myers_block(uint2& pv, uint2& mv, uint2 eq, uint
 }
 
 // Shared memory: the warps' match masks, then (teams) the chunk's words and votes by parity.
-template <int B>
 struct Team {
   uint32_t acc[2][4][2];
   uint32_t past[2][4];
@@ -96,7 +95,7 @@ struct Team {
 template <int B, bool TEAM>
 __global__ void __launch_bounds__(128, B <= 2 ? 8 : (B == 3 ? 6 : 5)) myers_kernel(sfk::MyersLaunch a) {
   extern __shared__ uint64_t smem[];
-  __shared__ Team<B> X;
+  __shared__ Team X;
   const int lane = threadIdx.x & 31, w = TEAM ? threadIdx.x >> 5 : 0;
   const int W = TEAM ? blockDim.x >> 5 : 1;
   // A lane's masks: code c of block bb at byte bb * kBlockBytes + c * kCodeBytes + 8 * lane.

@@ -264,10 +264,6 @@ int pass_lanes16(const Pass& p, size_t np, int lanes16) {
   return lanes16 == 0 && p.cut != SF_NOLIMIT && np < kCutPasses ? 32 : lanes16;
 }
 
-// Row sharing between sorted texts on the GPU: SF_SORTED_CHAINS=1 in the environment runs
-// the passes of a sorted call that can share rows as chains; by default every pass runs
-// separately (the results are the same either way, and separate passes finish sooner on the
-// batches measured: a chain runs its passes one after another); read once per plan.
 // Large sf_batch_run batches of enough work run in segments: 1; SF_BATCH_SEGMENTS=0 turns it off
 // (0), =1 runs every large even batch so (2).
 int batch_segments() {
@@ -282,6 +278,10 @@ bool allow_myers_stop() {
   return !(env && env[0] == '0');
 }
 
+// Row sharing between sorted texts on the GPU: SF_SORTED_CHAINS=1 in the environment runs
+// the passes of a sorted call that can share rows as chains; by default every pass runs
+// separately (the results are the same either way, and separate passes finish sooner on the
+// batches measured: a chain runs its passes one after another); read once per plan.
 bool allow_chains() {
   const char* env = std::getenv("SF_SORTED_CHAINS");
   return env && env[0] == '1';
@@ -795,7 +795,6 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   const sf_context* ctx = P->ctx;
   const size_t np = P->passes.size();
   const int lanes16 = default_lanes16();
-  const bool lean = plan_is_lean(P);
   const int most = most_pairs(P), team = myers_team(P);
   const uint64_t long_steps = plan_long_steps(P);
   const TuneTable* tune = P->tune_override ? P->tune_override : &ctx->tune;
