@@ -211,6 +211,7 @@ struct sf_plan {
   std::vector<Bucket> buckets;
   std::vector<Group> groups;
   int streams = 1;  // auxiliary streams its launches share
+  bool shared = false;  // other plans run beside it as a rule (a server's slots)
   uint64_t tb_words = 0, ops_words = 0, scratch_cells = 0;
   int wide_warps = 0;
   std::string desc;
@@ -275,7 +276,8 @@ struct sf_context {
   cudaStream_t s = nullptr;
   // Auxiliary streams that launches share.  A plan of few passes has all of them: its launches
   // leave the device idle one after another (644 pairs of 984 bases, bands 5-600, 14 launches: 1.20
-  // ms over 8, 0.86 over 16).  A plan of many has kBusy, one (the leading launch's, as a rule) more
+  // ms over 8, 0.86 over 16).  A plan of many, or beside others (40 served batches of up to 1,500
+  // reads: 33.0 ms over 9, 35.0 over 16), has kBusy, one (the leading launch's, as a rule) more
   // than the device has hardware queues by default: more crowd each other's blocks (5,447
   // extensions, 30 launches: 7.8 ms over 9, 9.3 over 13).
   static constexpr int kAux = 16, kBusy = 9;

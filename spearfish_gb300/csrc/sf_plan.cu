@@ -1319,7 +1319,7 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
              sfk::wave_warps(sfk::kWave[x.c]) == sfk::wave_warps(sfk::kWave[y.c]);
     return x.c == y.c && (x.lanes > 32 ? x.lanes == y.lanes : y.lanes <= 32);
   };
-  P->streams = lean ? sf_context::kAux : sf_context::kBusy;
+  P->streams = lean && !P->shared ? sf_context::kAux : sf_context::kBusy;
   std::vector<uint8_t> done(nb, 0);
   double behind[sf_context::kAux] = {};
   for (size_t u = 0; u < nb; ++u) {

@@ -242,6 +242,7 @@ int sf_server_create(const sf_server_opts* opts, sf_server** out) {
     sl.plan.reset(new sf_plan);
     sl.plan->ctx = sl.ctx;
     sl.plan->owns_ctx = true;
+    sl.plan->shared = true;
     CK(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
     S->slots.push_back(std::move(sl));
   }

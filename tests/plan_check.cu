@@ -7,7 +7,7 @@
 
 using namespace sfe;
 
-int main(int, char** argv) {
+int main(int argc, char** argv) {
   FILE* f = std::fopen(argv[1], "rb");
   uint64_t head[4];
   if (!f || std::fread(head, 8, 4, f) != 4) return 2;
@@ -21,6 +21,7 @@ int main(int, char** argv) {
   ctx.sms = (int)head[0];
   sf_plan P;
   P.ctx = &ctx;
+  P.shared = argc > 2;  // as a server's slot
   P.pool_bytes = head[1];
   P.scratch.reset(new BuildScratch);
   BuildScratch& S = *P.scratch;

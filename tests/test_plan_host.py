@@ -23,7 +23,7 @@ def check(tmp_path_factory):
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
 
-    def run(jobs, scores=(R.ONT,), pool_bytes=None, sms=152):
+    def run(jobs, scores=(R.ONT,), pool_bytes=None, sms=152, shared=False):
         if pool_bytes is None:
             pool_bytes = int(max((jobs["p_off"] + jobs["m"]).max(), (jobs["t_off"] + jobs["n"]).max()))
         path = exe + ".in"
@@ -31,7 +31,7 @@ def check(tmp_path_factory):
             np.array([sms, pool_bytes, len(scores), len(jobs)], np.uint64).tofile(f)
             np.array([tuple(s) for s in scores], np.int32).tofile(f)
             jobs.tofile(f)
-        out = subprocess.run([exe, path], capture_output=True, text=True, timeout=120)
+        out = subprocess.run([exe, path] + ["shared"] * shared, capture_output=True, text=True, timeout=120)
         assert out.returncode == 0, out.stdout + out.stderr
         plan = json.loads(out.stdout)
         plan["kinds"] = [plan["plan"]["buckets"][b]["kind"] for b in plan["job_buckets"]]
@@ -144,18 +144,18 @@ def test_caps_that_stop_pairs(check, mode):
         assert plan["myers_kcut"] == (mode != R.INFIX and k < 900 + n and k < 1 << 30), (n, k)
 
 
-@pytest.mark.parametrize("passes", [644, 2900, 20000])
-def test_streams_of_launches(check, passes):
-    """Few passes: a launch of each class on a stream of its own.  The first launch starts before the
-    others only while it leaves schedulers empty."""
+@pytest.mark.parametrize("passes,shared", [(644, False), (644, True), (2900, False), (20000, False)])
+def test_streams_of_launches(check, passes, shared):
+    """Few passes, not in a server: a launch of each class on a stream of its own.  The first launch
+    starts before the others only while it leaves schedulers empty."""
     from spearfish_gb300 import batch as B
     odd = ((1, 3, 5, 2),)  # on the row kernels, a launch a class
     rows = [dict(m=900, n=900, band=20 + 640 * (q % 14) // 14, kind=B.JOB_AFFINE, mode=R.GLOBAL, want_cigar=1)
             for q in range(passes)]
-    launches = check(_jobs(rows), odd)["launches"]
+    launches = check(_jobs(rows), odd, shared=shared)["launches"]
     streams = [x["stream"] for x in launches]
     assert 9 < len(launches) <= 16
-    if passes <= 20 * 152:
+    if passes <= 20 * 152 and not shared:
         assert len(set(streams)) == len(launches)
     else:
         assert max(streams) < 9
