@@ -240,7 +240,8 @@ struct sf_plan {
   // Whether passes take the class that finishes one fastest (few passes) or the cheapest a
   // cell: -1 by the plan's passes, else as set (the autotuner's trial plans).
   int lean = -1;
-  int most = 0;  // Myers pairs a warp at most, likewise (0: by the plan's passes)
+  int most = 0;   // Myers pairs a warp at most as classes are chosen, likewise (0: by the plan's passes)
+  int share = 0;  // and as many share a warp of a class that holds them, likewise
   int team = -1;            // warps a Myers pair may take, likewise
   uint64_t long_steps = 0;  // the row steps of a long pass, likewise
   // Class overrides for this plan only (the autotuner's trial plans); else the context's.
@@ -362,6 +363,7 @@ int shown_c(int kind, int c);
 int shown_lanes(int kind, int c, int lanes);
 int choose_myers_class(uint32_t m, int team, int most, int& b, int& lanes);
 int most_pairs(const sf_plan* P);
+int share_pairs(const sf_plan* P);
 DJob make_djob(const Pass& p, uint32_t& flags);
 // Whether large sf_batch_run batches may run in segments (SF_BATCH_SEGMENTS).
 int batch_segments();

@@ -211,10 +211,22 @@ uint64_t plan_long_steps(const sf_plan* P) {
   return (uint64_t)std::max(1.0, least);
 }
 
-// Myers pairs a warp at most: four warps a scheduler before more pairs share one.
+// Myers pairs a warp at most as classes are chosen: four warps a scheduler before blocks are put in
+// fewer lanes for more pairs a warp.
 int most_pairs(const sf_plan* P) {
   if (P->most) return P->most;
   return (int)std::max<size_t>(1, std::min<size_t>(32, P->passes.size() / ((size_t)P->ctx->sms * 16)));
+}
+
+// Myers pairs that share a warp of a class that holds them: as many as leave each warp a scheduler
+// of its own.  A warp's step fills the ALU pipe for 74 cycles and takes about 97 alone, so a second
+// warp on a scheduler costs more than a second pair in the warp does (4,500 pairs of 150 bases: 82 us
+// with four warps a scheduler before pairs share one, 35 so; 3,000 of 363: 92 and 46; 735 of 1 kb: 93
+// and 76).
+int share_pairs(const sf_plan* P) {
+  if (P->share) return P->share;
+  const size_t schedulers = (size_t)P->ctx->sms * 4;
+  return (int)std::max<size_t>(1, std::min<size_t>(32, (P->passes.size() + schedulers - 1) / schedulers));
 }
 
 // Warps a pair of a small plan may take: as long as that leaves schedulers idle (1,762 Global pairs
@@ -228,6 +240,7 @@ int myers_team(const sf_plan* P) {
 void choose_as(const sf_plan* P, sf_plan* S) {
   S->lean = plan_is_lean(P);
   S->most = most_pairs(P);
+  S->share = share_pairs(P);
   S->team = myers_team(P);
   S->long_steps = plan_long_steps(P);
 }
@@ -1277,16 +1290,15 @@ void build_buckets(sf_plan* P, BuildScratch& S) {
   };
   for (auto& b : P->buckets) {
     if (b.kind == PK_MYERS || is_wave(b.kind)) {
-      // As many pairs a warp as its lanes hold; in the fast classes fewer, while that leaves
+      // As many passes a warp as its lanes hold; in the fast classes fewer, while that leaves
       // schedulers empty.
       const bool my = b.kind == PK_MYERS;
       const int team = my ? (b.lanes > 32 ? b.lanes / 32 : 1) : sfk::wave_warps(sfk::kWave[b.c]);
-      const int64_t most = std::max(
-          1, my ? std::min(most_pairs(P), 32 / b.lanes) : 32 / sfk::kWave[b.c].lanes);
-      const bool fast = my ? lean
-                           : (b.c >= sfk::kWaveFast && b.c < sfk::kWaveX) || b.c >= sfk::kWaveXFast;
-      b.per_warp = (int)(!fast ? most
-                               : std::max<int64_t>(1, std::min<int64_t>(most, b.count / (4 * (int64_t)ctx->sms))));
+      const int64_t hold = std::max(1, 32 / (my ? b.lanes : sfk::kWave[b.c].lanes));
+      const bool fast = (b.c >= sfk::kWaveFast && b.c < sfk::kWaveX) || b.c >= sfk::kWaveXFast;
+      b.per_warp = (int)(my      ? std::min<int64_t>(hold, share_pairs(P))
+                         : !fast ? hold
+                                 : std::max<int64_t>(1, std::min<int64_t>(hold, b.count / (4 * (int64_t)ctx->sms))));
       b.task_count = (b.count + b.per_warp - 1) / b.per_warp;
       b.block = team > 1 ? 32 * team : 128;
       b.grid = warps_grid((uint64_t)b.task_count * team, b.block);

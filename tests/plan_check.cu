@@ -51,8 +51,9 @@ int main(int argc, char** argv) {
   for (size_t q = 0; q < at.size(); ++q) std::printf("%s%d", q ? ", " : "", (int)at[q]);
   std::printf("], \"launches\": [");
   for (size_t q = 0; q < P.groups.size(); ++q)
-    std::printf("%s{\"stream\": %d, \"lead\": %s, \"warps\": %d}", q ? ", " : "", P.groups[q].stream,
-                P.groups[q].lead ? "true" : "false", P.groups[q].grid * P.groups[q].block / 32);
+    std::printf("%s{\"stream\": %d, \"lead\": %s, \"warps\": %d, \"tasks\": %u}", q ? ", " : "",
+                P.groups[q].stream, P.groups[q].lead ? "true" : "false",
+                P.groups[q].grid * P.groups[q].block / 32, P.groups[q].task_count);
   // The passes of each class in a plan of their own, as the autotuner times them: how many get
   // another class there.
   std::map<std::tuple<int, int, int, int, int>, std::vector<size_t>> alike;

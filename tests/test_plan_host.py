@@ -160,3 +160,15 @@ def test_streams_of_launches(check, passes, shared):
     else:
         assert max(streams) < 9
     assert [x["lead"] for x in launches] == [launches[0]["warps"] <= 4 * 152] + [False] * (len(launches) - 1)
+
+
+@pytest.mark.parametrize("m", [60, 150, 363, 700, 1000])
+@pytest.mark.parametrize("pairs", [1, 608, 609, 1500, 3000, 4500, 20000])
+def test_pairs_that_share_a_warp(check, pairs, m):
+    """Myers pairs share a warp as soon as each warp has a scheduler of its own, as far as its lanes
+    hold them."""
+    from spearfish_gb300 import batch as B
+    plan = check(_jobs([dict(m=m, n=m + 100, kind=B.JOB_MYERS, mode=R.INFIX)] * pairs))
+    (bucket,), (launch,) = plan["plan"]["buckets"], plan["launches"]
+    share = min(32 // bucket["lanes"], -(-pairs // 608))
+    assert launch["tasks"] == -(-pairs // share), (bucket, launch)
