@@ -207,7 +207,7 @@ struct sf_plan {
   std::vector<uint32_t> slot;
   uint32_t n_aff = 0, n_my = 0, n_walk = 0;
   uint32_t n_tasks = 0;  // tasks of all launches (d_tasks: the tasks, then the job order)
-  bool myers_kcut = false;  // a Myers pass is Global or Prefix and myers_capped
+  bool myers_kcut = false;  // Myers pairs may stop early: one is Global or Prefix with k < m + n
   std::vector<Bucket> buckets;
   std::vector<Group> groups;
   int streams = 1;  // auxiliary streams its launches share

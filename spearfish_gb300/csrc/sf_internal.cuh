@@ -62,12 +62,6 @@ struct MJob {
   uint32_t mode, k;
 };
 
-// Whether a Global or Prefix pair may stop early under its cap: it can exceed it (no distance is
-// above m + n), and the kernel's 32-bit column scores hold the cap and what it adds to it.
-__host__ __device__ inline bool myers_capped(uint32_t k, uint32_t m, uint32_t n) {
-  return k < 0x40000000u && (uint64_t)k < (uint64_t)m + (uint64_t)n;
-}
-
 // Traceback walk: which end cell, and where the CIGAR goes.
 struct TJob {
   uint64_t ops_off;   // first op slot
@@ -249,7 +243,8 @@ struct MyersLaunch {
   const uint32_t* pool;
   uint32_t* out;
   int team;   // one pair per block of 2 or 4 warps
-  int kcut;   // some pair is Global or Prefix and myers_capped: stop pairs early (see kernel)
+  int kcut;   // some pair is Global or Prefix with k < m + n, none with such a k of 2^30 or more:
+              // stop pairs early (see kernel)
 };
 // Pairs of up to 64 * blocks_per_lane * lanes pattern bases; blocks_per_lane 1 .. kMyersMaxB.
 cudaError_t launch_myers(int blocks_per_lane, const MyersLaunch& a, int grid, int block,

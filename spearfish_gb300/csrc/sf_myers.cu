@@ -168,8 +168,8 @@ __global__ void __launch_bounds__(128, B <= 2 ? 8 : (B == 3 ? 6 : 5)) myers_kern
     int score = m, best = glob ? INT32_MAX : m;
     // This lane's bottom score in its current column (D[i][0] = i), for the cap.
     int bottom = max((l + 1) * B * 64 - free_rows, 0);
-    const bool capped = a.kcut && has && !infix && sf::myers_capped(J.k, J.m, J.n);
-    const int far = (int)min(J.k, 0x40000000u) + (TEAM ? 34 : 2);
+    const bool capped = a.kcut && has && !infix && (uint64_t)J.k < (uint64_t)m + (uint64_t)n;
+    const int far = (int)min((uint64_t)J.k, (uint64_t)0x3fffffff) + (TEAM ? 34 : 2);
     const bool any_cap = __any_sync(FULL, capped);
     bool dead = false;
     uint32_t out_p = 0, out_m = 0;  // the deltas leaving this lane

@@ -869,7 +869,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   has_item.resize(np);
   constexpr int kMaxThreads = 16;
   uint64_t scratch_max[kMaxThreads] = {};
-  bool kcut[kMaxThreads] = {};
+  bool kcut[kMaxThreads] = {}, kfar[kMaxThreads] = {};
   // Descriptors of passes [q0, q1), each written at its slot.
   auto describe = [&](size_t q0, size_t q1, int worker) {
     // The tune table's answers, memoised per class (a batch has few classes).
@@ -905,7 +905,10 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
         m.n = p.n;
         m.mode = p.mode;
         m.k = p.k;
-        if (p.mode != SF_INFIX && myers_capped(p.k, p.m, p.n)) kcut[worker] = true;
+        if (p.mode != SF_INFIX && (uint64_t)p.k < (uint64_t)p.m + p.n) {
+          kcut[worker] = true;
+          kfar[worker] = kfar[worker] || p.k >= 1u << 30;
+        }
         per[q] = {Key2{PK_MYERS, b, 0, 0, lanes},
                   Item{sl, (uint64_t)p.n, ((uint64_t)p.n + (uint64_t)lanes) * 65u * (uint64_t)b}};
         has_item[q] = 1;
@@ -964,7 +967,10 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
     }
   };
   parallel_chunks(np, 2048, kMaxThreads, describe);
-  P->myers_kcut = allow_myers_stop() && std::any_of(kcut, kcut + kMaxThreads, [](bool v) { return v; });
+  // (The kernel's 32-bit column scores hold caps below 2^30: a plan with a larger one has no pair
+  // stop early.)
+  auto any = [](const bool* v) { return std::any_of(v, v + kMaxThreads, [](bool x) { return x; }); };
+  P->myers_kcut = allow_myers_stop() && any(kcut) && !any(kfar);
   uint64_t scratch_cells = 0;
   for (int w = 0; w < kMaxThreads; ++w) scratch_cells = std::max(scratch_cells, scratch_max[w]);
   P->scratch_cells = scratch_cells;
