@@ -244,6 +244,7 @@ struct sf_plan {
   int share = 0;  // and as many share a warp of a class that holds them, likewise
   int team = -1;            // warps a Myers pair may take, likewise
   uint64_t long_steps = 0;  // the row steps of a long pass, likewise
+  bool short_rows = false;  // and whether there are only few and short ones
   // Class overrides for this plan only (the autotuner's trial plans); else the context's.
   const sfe::TuneTable* tune_override = nullptr;
   // Host-side build arrays kept between builds (sf_plan.cu).
@@ -342,7 +343,7 @@ bool allow16();
 int default_lanes16();
 void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax, bool use16,
                      uint64_t long_steps, PassKind& kind, int& c, bool& wide, int& lanes,
-                     int lanes16 = 32);
+                     int lanes16 = 32, bool short_rows = false);
 // The band cells the anti-diagonal kernel lays out for a pass.
 int64_t wave_width(const DJob& j);
 int myers_team(const sf_plan* P);
@@ -351,7 +352,8 @@ int pass_lanes16(const Pass& p, size_t np, int lanes16);
 // fastest, rather than the cheapest ones a cell.
 bool lean_plan(size_t np, int sms);
 bool plan_is_lean(const sf_plan* P);
-uint64_t plan_long_steps(const sf_plan* P);
+// The row steps from which a pass of P is long; short_rows: P is of few passes, all of short patterns.
+uint64_t plan_long_steps(const sf_plan* P, bool& short_rows);
 // Sets on S all that a pass's default class depends on beside the pass: S, of some of P's passes,
 // then gives them the classes P does.
 void choose_as(const sf_plan* P, sf_plan* S);

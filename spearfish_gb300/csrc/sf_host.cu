@@ -1227,8 +1227,8 @@ namespace {
 
 // A pass's class before any override, and the Myers blocks it needs.  (A plan's jobs have no cut
 // column.)
-int default_class(const Pass& p, bool use16, int team, int most, uint64_t long_steps, ClassKey& key,
-                  int64_t& blocks) {
+int default_class(const Pass& p, bool use16, int team, int most, uint64_t long_steps, bool short_rows,
+                  ClassKey& key, int64_t& blocks) {
   if (p.kind == PK_MYERS) {
     int b = 1, lanes = 1;
     int rc = choose_myers_class(p.m, team, most, b, lanes);
@@ -1243,7 +1243,8 @@ int default_class(const Pass& p, bool use16, int team, int most, uint64_t long_s
   int c = 4, lanes = 32;
   bool wide = false;
   PassKind kind = PK_AFFINE;
-  classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, lanes, default_lanes16());
+  classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, lanes, default_lanes16(),
+                  short_rows);
   const bool tb = p.want_cigar && p.kind != PK_LOCAL;
   key = ClassKey{kind, c, wide ? 1 : 0, tb ? 1 : 0, lanes};
   blocks = wmax;  // affine: the group's widest row
@@ -1333,14 +1334,15 @@ int sf_plan_tune(sf_plan* P, const uint8_t* pool, uint32_t reps, char* report, u
   const auto t0 = std::chrono::steady_clock::now();
   const bool use16 = allow16();
   const int most = most_pairs(P), team = myers_team(P);
-  const uint64_t long_steps = plan_long_steps(P);
+  bool short_rows = false;
+  const uint64_t long_steps = plan_long_steps(P, short_rows);
   // Group the passes by their default class.
   std::map<ClassKey, std::vector<size_t>> groups;
   std::map<ClassKey, int64_t> gblocks;
   for (size_t q = 0; q < P->passes.size(); ++q) {
     ClassKey k;
     int64_t blocks = 0;
-    int rc = default_class(P->passes[q], use16, team, most, long_steps, k, blocks);
+    int rc = default_class(P->passes[q], use16, team, most, long_steps, short_rows, k, blocks);
     if (rc) return rc;
     groups[k].push_back(q);
     gblocks[k] = std::max(gblocks[k], blocks);

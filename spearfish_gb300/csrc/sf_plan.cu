@@ -153,7 +153,13 @@ bool plan_is_lean(const sf_plan* P) {
 // nanosecond with every scheduler busy, 3.5 without traceback, Myers 40).  Measured on uneven
 // batches, no team / 0.8 / 1 / 1.2 / 1.6 us: 25,000 pairs 18.5 / 16.9 / 14.4 / 14.5 / 17.6 ms,
 // 6,000 pairs 10.9 / 6.9 / 6.9 / 7.0 / 7.2 (teams repeat lanes, and take the schedulers' turns).
-uint64_t plan_long_steps(const sf_plan* P) {
+//
+// Few passes, all of patterns shorter than kShortRows, leave the Prefix ones without traceback to
+// the row kernel: pass by pass the two kernels are near each other there, and a second launch costs
+// such a plan more than it saves (span ends of 512 hits, flanks up to 40 / 67 bases: 298 / 305 us
+// split, 252 / 265 on rows alone; up to 130: 300 and 292; up to 250: 333 and 351).
+uint64_t plan_long_steps(const sf_plan* P, bool& short_rows) {
+  short_rows = P->short_rows;
   if (P->long_steps) return P->long_steps;
   if (!P->passes.empty() && P->passes.front().kind == PK_MYERS && P->passes.back().kind == PK_MYERS) {
     // Myers pairs only: nothing to weigh.
@@ -170,9 +176,12 @@ uint64_t plan_long_steps(const sf_plan* P) {
     steps = p.mode == SF_PREFIX ? m + w / 2 : (m + n) / 2;
   };
   const size_t np = P->passes.size();
+  constexpr uint32_t kShortRows = 100;
   std::vector<double> ns(kT), most(kT), cells((size_t)kT * kBins);
+  uint32_t rows[kT] = {};
   parallel_chunks(np, 4096, kT, [&](size_t q0, size_t q1, int k) {
     double t = 0, x = 0;
+    uint32_t r = 0;
     for (size_t q = q0; q < q1; ++q) {
       const Pass& p = P->passes[q];
       if (p.kind == PK_MYERS) {
@@ -182,16 +191,19 @@ uint64_t plan_long_steps(const sf_plan* P) {
         shape(p, w, steps);
         t += w * steps / (p.want_cigar ? 2000.0 : 3500.0);
         x = std::max(x, steps);
+        r = std::max(r, p.m);
       }
     }
     ns[k] = t;
     most[k] = x;
+    rows[k] = r;
   });
   double total = 0, longest = 1;
   for (int k = 0; k < kT; ++k) {
     total += ns[k];
     longest = std::max(longest, most[k]);
   }
+  short_rows = plan_is_lean(P) && *std::max_element(rows, rows + kT) < kShortRows;
   parallel_chunks(np, 4096, kT, [&](size_t q0, size_t q1, int k) {
     for (size_t q = q0; q < q1; ++q) {
       if (P->passes[q].kind == PK_MYERS) continue;
@@ -242,7 +254,7 @@ void choose_as(const sf_plan* P, sf_plan* S) {
   S->most = most_pairs(P);
   S->share = share_pairs(P);
   S->team = myers_team(P);
-  S->long_steps = plan_long_steps(P);
+  S->long_steps = plan_long_steps(P, S->short_rows);
 }
 
 int shown_c(int kind, int c) { return is_wave(kind) ? 4 * sfk::kWave[c].q : c; }
@@ -330,7 +342,7 @@ bool wave_is_less(const Pass& p, const DJob& j, int64_t wmax, int c, bool alone)
 // it, else the packed 16-bit row kernel, else the 32-bit register kernel, else (rows wider than 32 * 48 cells) the wide-row kernel.
 void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax, bool use16,
                      uint64_t long_steps, PassKind& kind, int& c, bool& wide, int& lanes,
-                     int lanes16) {
+                     int lanes16, bool short_rows) {
   wide = false;
   lanes = 32;
   if (use16 && lanes16 == 0 && fits_wave(p, j, flags, kind)) {
@@ -338,7 +350,8 @@ void classify_affine(const Pass& p, const DJob& j, uint32_t flags, int64_t wmax,
     const bool fast = wave_steps(j, kind) >= long_steps;
     c = kind != PK_WAVE16 ? (fast ? sfk::kWaveXFast : sfk::kWaveX) : (fast ? sfk::kWaveFast : 0);
     while (sfk::wave_cap(sfk::kWave[c]) < w || (kind == PK_WAVE16C && sfk::kWave[c].lanes > 32)) ++c;
-    if (kind == PK_WAVE16 || !fits16(p, flags, wmax) || wave_is_less(p, j, wmax, c, fast)) return;
+    const bool rows = short_rows && !p.want_cigar;
+    if (kind == PK_WAVE16 || !fits16(p, flags, wmax) || (!rows && wave_is_less(p, j, wmax, c, fast))) return;
   }
   if (use16 && fits16(p, flags, wmax)) {
     if (lanes16 == 16)
@@ -809,7 +822,8 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
   const size_t np = P->passes.size();
   const int lanes16 = default_lanes16();
   const int most = most_pairs(P), team = myers_team(P);
-  const uint64_t long_steps = plan_long_steps(P);
+  bool short_rows = false;
+  const uint64_t long_steps = plan_long_steps(P, short_rows);
   const TuneTable* tune = P->tune_override ? P->tune_override : &ctx->tune;
   const auto& word_of = S.word_of;
   auto& dj = S.dj;
@@ -926,7 +940,7 @@ int describe_passes(sf_plan* P, BuildScratch& S, bool use16) {
       PassKind kind = PK_AFFINE;
       int ln = 32;
       classify_affine(p, j, flags, wmax, use16, long_steps, kind, c, wide, ln,
-                      pass_lanes16(p, np, lanes16));
+                      pass_lanes16(p, np, lanes16), short_rows);
       const bool tb = p.want_cigar && p.kind != PK_LOCAL;
       if (!wide) tuned(kind, c, false, tb, ln);
       TJob t{};

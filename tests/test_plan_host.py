@@ -172,3 +172,20 @@ def test_pairs_that_share_a_warp(check, pairs, m):
     (bucket,), (launch,) = plan["plan"]["buckets"], plan["launches"]
     share = min(32 // bucket["lanes"], -(-pairs // 608))
     assert launch["tasks"] == -(-pairs // share), (bucket, launch)
+
+
+@pytest.mark.parametrize("longest", [40, 99, 100, 250])
+@pytest.mark.parametrize("count", [1, 1200, 5000])
+def test_few_short_prefix_passes(check, count, longest):
+    """Few Prefix passes without traceback, all of short patterns, run on one kernel (the rows);
+    with a long one among them, or many, each where it takes less time."""
+    from spearfish_gb300 import batch as B
+    rows = [dict(m=longest if q == 0 else 5 + q % 36, n=90, band=16, kind=B.JOB_EXTEND_WINDOW, mode=R.PREFIX,
+                 window=90, xdrop=50, want_cigar=0) for q in range(count)]
+    rows[0]["n"] = rows[0]["window"] = longest + 20
+    plan = check(_jobs(rows))
+    if count <= 3040 and longest < 100:
+        assert set(plan["kinds"]) == {"affine16"}, set(plan["kinds"])
+    else:
+        assert "wave16x" in plan["kinds"]
+    assert plan["strays"] == 0
