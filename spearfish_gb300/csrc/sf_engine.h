@@ -278,11 +278,12 @@ struct sf_context {
   cudaStream_t s = nullptr;
   // Auxiliary streams that launches share.  A plan of few passes has all of them: its launches
   // leave the device idle one after another (644 pairs of 984 bases, bands 5-600, 14 launches: 1.20
-  // ms over 8, 0.86 over 16).  A plan of many, or beside others (40 served batches of up to 1,500
-  // reads: 33.0 ms over 9, 35.0 over 16), has kBusy, one (the leading launch's, as a rule) more
-  // than the device has hardware queues by default: more crowd each other's blocks (5,447
-  // extensions, 30 launches: 7.8 ms over 9, 9.3 over 13).
-  static constexpr int kAux = 16, kBusy = 9;
+  // ms over 8, 0.86 over 12 or 16; 2,000 Infix ones on the 32-bit rows 1.30 over 12, 1.37 over 16).
+  // A plan of many, or beside others (40 served batches of up to 1,500 reads: 33.0 ms over 9, 35.0
+  // over 16), has kBusy, one (the leading launch's, as a rule) more than the device has hardware
+  // queues by default: more crowd each other's blocks (5,447 extensions, 30 launches: 7.8 ms over
+  // 9, 9.3 over 13).
+  static constexpr int kAux = 12, kBusy = 9;
   cudaStream_t aux[kAux] = {};
   cudaEvent_t fork = nullptr, join[kAux] = {};
   std::unique_ptr<sf_plan> cache;  // reused by sf_batch_run

@@ -146,7 +146,7 @@ def test_caps_that_stop_pairs(check, mode):
 
 @pytest.mark.parametrize("passes,shared", [(644, False), (644, True), (2900, False), (20000, False)])
 def test_streams_of_launches(check, passes, shared):
-    """Few passes, not in a server: a launch of each class on a stream of its own.  The first launch
+    """Few passes, not in a server: up to twelve launches on streams of their own.  The first launch
     starts before the others only while it leaves schedulers empty."""
     from spearfish_gb300 import batch as B
     odd = ((1, 3, 5, 2),)  # on the row kernels, a launch a class
@@ -156,7 +156,7 @@ def test_streams_of_launches(check, passes, shared):
     streams = [x["stream"] for x in launches]
     assert 9 < len(launches) <= 16
     if passes <= 20 * 152 and not shared:
-        assert len(set(streams)) == len(launches)
+        assert len(set(streams)) == min(12, len(launches))
     else:
         assert max(streams) < 9
     assert [x["lead"] for x in launches] == [launches[0]["warps"] <= 4 * 152] + [False] * (len(launches) - 1)
