@@ -1984,7 +1984,7 @@ uint64_t plan_bytes_estimate(const std::vector<Pass>& passes, uint64_t pool_byte
   const bool use16 = allow16();
   const int lanes16 = default_lanes16();
   for (const Pass& p : passes) {
-    b += (uint64_t)(p.m + p.n + 34) / 4 + kSeqs + kOrder + (p.kind == PK_MYERS ? kMyers : kAffine);
+    b += ((uint64_t)p.m + p.n + 34) / 4 + kSeqs + kOrder + (p.kind == PK_MYERS ? kMyers : kAffine);
     if (p.kind == PK_MYERS) continue;
     uint32_t flags = 0;
     DJob j = make_djob(p, flags);
